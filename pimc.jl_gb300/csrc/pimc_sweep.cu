@@ -738,57 +738,132 @@ cudaError_t launch_measure(const ChainDesc *desc, ChainVar *var, double *dpool, 
 // Composite 8-point Gauss-Legendre in FP64: geometric panels from 1e-10 to 0.5
 // (the log behaviour at k -> 0), then uniform panels of a quarter of the
 // shortest oscillation period up to K with exp(-tau K^2) = 1e-18.  CUDA's j0 /
-// y0 are library calls.  One thread per entry of the upper triangle.
+// y0 are library calls.
+//
+// With t(k) = 1/s(k), s = (2/pi)(gamma + log(k/2)) - 4/g0, the weights
+// t^2/(1+t^2) = wa = 1/(1+s^2) and t/(1+t^2) = wb = s/(1+s^2) stay finite where
+// t has its pole, and the integrand factors over the two radii:
+//   -wa J1 J2 - wb (J1 Y2 + J2 Y1) + wa Y1 Y2 = Y1 U2 + J1 V2,
+//   U = wa Y - wb J, V = -(wa J + wb Y).
+// So the n K distinct Bessel arguments are evaluated once (k_contact_nodes)
+// and the table is the product [Y J]^T [U V] over the nodes
+// (k_contact_product).  Evaluating the four functions per (entry, node)
+// instead took 529 ms for n = 600, K = 4656 nodes (180300 entries, 3.4 G
+// function values); the factored form has 5.6 M of them and 1.7 G FP64 FMAs,
+// which the FP64 pipe (2 lanes per SM clock) bounds at 2.9 ms; the whole
+// call, copy to the host included, takes 4.7 ms.
 // ---------------------------------------------------------------------------
 struct ContactQuad {
   double tau, g0, K, k0, du;
   int ngraded, nuniform;
 };
 
-// the integrand of the three Bessel integrals (Gautier et al., supplementary
-// S28; src/propagator.jl:50-64) combined, T = (-I1 - I2 + I3) / (2 pi).  With
-// t(k) = 1/s(k), s = (2/pi)(gamma + log(k/2)) - 4/g0, the weights
-// t^2/(1+t^2) = 1/(1+s^2) and t/(1+t^2) = s/(1+s^2) are taken in s, which
-// stays finite where t has its pole.
-__device__ __forceinline__ double contact_integrand(double k, double r1, double r2, const ContactQuad &q) {
-  const double sk = (2.0 / 3.141592653589793) * (0.5772156649015329 + log(0.5 * k)) - 4.0 / q.g0;
-  const double den = 1.0 / (1.0 + sk * sk), wa = den, wb = sk * den;
-  const double J1 = j0(k * r1), J2 = j0(k * r2), Y1 = y0(k * r1), Y2 = y0(k * r2);
-  return k * exp(-q.tau * k * k) * (-wa * J1 * J2 - wb * (J1 * Y2 + J2 * Y1) + wa * Y1 * Y2);
-}
-
-__device__ double contact_entry(double r1, double r2, const ContactQuad &q) {
+// node q of the rule: the wave number and its weight
+__device__ __forceinline__ void contact_node(const ContactQuad &c, int q, double &k, double &w) {
   const double xs[4] = {0.18343464249564978, 0.525532409916329, 0.7966664774136267, 0.9602898564975362};
   const double ws[4] = {0.36268378337836166, 0.3137066458778869, 0.22238103445337443, 0.10122853629037706};
-  double sum = 0.0;
-  auto panel = [&](double a, double b) {
-    const double c = 0.5 * (a + b), hw = 0.5 * (b - a);
-    double ps = 0.0;
-    for (int i = 0; i < 4; ++i)
-      ps += ws[i] * (contact_integrand(c - hw * xs[i], r1, r2, q) + contact_integrand(c + hw * xs[i], r1, r2, q));
-    sum += hw * ps;
-  };
-  double a = 1e-10;
-  for (int p = 0; p < q.ngraded; ++p) {
-    const double b = p + 1 == q.ngraded ? q.k0 : 2.0 * a;
-    panel(a, b);
-    a = b;
+  const int p = q >> 3, i = (q >> 1) & 3;
+  double a, b;
+  if (p < c.ngraded) {
+    a = ldexp(1e-10, p);
+    b = p + 1 == c.ngraded ? c.k0 : 2.0 * a;
+  } else {
+    a = c.k0 + (p - c.ngraded) * c.du;
+    b = c.k0 + (p - c.ngraded + 1) * c.du;
   }
-  for (int p = 0; p < q.nuniform; ++p) panel(q.k0 + p * q.du, q.k0 + (p + 1) * q.du);
-  return sum / (2.0 * 3.141592653589793);
+  const double mid = 0.5 * (a + b), hw = 0.5 * (b - a);
+  k = (q & 1) ? mid + hw * xs[i] : mid - hw * xs[i];
+  w = hw * ws[i];
 }
 
-__global__ void k_contact_table(double *tab, int n, double r0, double h, ContactQuad q) {
-  const long long ntri = (long long)n * (n + 1) / 2;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < ntri;
-       e += (long long)gridDim.x * blockDim.x) {
-    // row i1 of the upper triangle holds n - i1 entries
-    int i1 = (int)((2.0 * n + 1.0 - sqrt((2.0 * n + 1.0) * (2.0 * n + 1.0) - 8.0 * (double)e)) / 2.0);
-    if (i1 < 0) i1 = 0;
-    while (i1 > 0 && (long long)i1 * (2 * n - i1 + 1) / 2 > e) --i1;
-    while ((long long)(i1 + 1) * (2 * n - i1) / 2 <= e) ++i1;
-    const int i2 = i1 + (int)(e - (long long)i1 * (2 * n - i1 + 1) / 2);
-    const double v = contact_entry(r0 + i1 * h, r0 + i2 * h, q);
+// rows of the product for nodes [q0, q0 + kc): f[r][kc][ld], r = Y, J, U, V
+__global__ void __launch_bounds__(128) k_contact_nodes(double *f, int n, int ld, int q0, int kc, double r0,
+                                                        double h, ContactQuad c) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= ld) return;
+  const size_t plane = (size_t)kc * ld;
+  for (int q = blockIdx.y; q < kc; q += gridDim.y) {
+    double k, w;
+    contact_node(c, q0 + q, k, w);
+    const double s = (2.0 / 3.141592653589793) * (0.5772156649015329 + log(0.5 * k)) - 4.0 / c.g0;
+    const double wa = w * k * exp(-c.tau * k * k) / (1.0 + s * s) / (2.0 * 3.141592653589793), wb = s * wa;
+    double J = 0.0, Y = 0.0;
+    if (i < n) {
+      const double x = k * (r0 + i * h);
+      J = j0(x);
+      Y = y0(x);
+    }
+    const size_t at = (size_t)q * ld + i;
+    f[at] = Y;
+    f[plane + at] = J;
+    f[2 * plane + at] = wa * Y - wb * J;
+    f[3 * plane + at] = -(wa * J + wb * Y);
+  }
+}
+
+// 32 x 32 tiles of the upper triangle, 64 threads of 4 x 4 entries, blockIdx.y
+// a range of the nodes; part[split][ntile][32][32].  The FP64 pipe bounds it
+// (16 FMAs per 4 shared-memory loads of a thread and row), so the tiles are
+// small enough that little work falls on entries below the diagonal or past
+// n (7 % at n = 600), and the nodes are split to fill the SMs.
+constexpr int CT_T = 32, CT_K = 16;
+__global__ void __launch_bounds__(64) k_contact_product(const double *f, double *part, int ld, int kc,
+                                                         int per) {
+  __shared__ double sa[2][CT_K][CT_T], sb[2][CT_K][CT_T];
+  int ti = 0, rest = blockIdx.x;
+  const int nt = ld / CT_T;
+  while (rest >= nt - ti) rest -= nt - ti++;  // row ti of tiles holds nt - ti of them
+  const int tj = ti + rest;
+  const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
+  const size_t plane = (size_t)kc * ld;
+  const int k_lo = blockIdx.y * per, k_hi = min(kc, k_lo + per);
+  double acc[4][4] = {};
+  for (int k0 = k_lo; k0 < k_hi; k0 += CT_K) {
+    for (int e = tid; e < 2 * CT_K * CT_T; e += 64) {
+      const int r = e / (CT_K * CT_T), kk = (e / CT_T) % CT_K, col = e % CT_T;
+      const bool in = k0 + kk < k_hi;
+      const size_t at = (size_t)r * plane + (size_t)(k0 + kk) * ld + col;
+      sa[r][kk][col] = in ? f[at + (size_t)ti * CT_T] : 0.0;
+      sb[r][kk][col] = in ? f[at + 2 * plane + (size_t)tj * CT_T] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int kk = 0; kk < CT_K; ++kk)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        double a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          a[u] = sa[r][kk][ty + 8 * u];
+          b[u] = sb[r][kk][tx + 8 * u];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) acc[u][v] = fma(a[u], b[v], acc[u][v]);
+      }
+    __syncthreads();
+  }
+  double *o = part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (CT_T * CT_T);
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) o[(ty + 8 * u) * CT_T + tx + 8 * v] = acc[u][v];
+}
+
+// the splits' tiles summed in order into both triangles; add: onto the table
+// (later ranges of nodes)
+__global__ void __launch_bounds__(256) k_contact_gather(const double *part, double *tab, int n, int ld,
+                                                         int ntile, int nsplit, int add) {
+  const int nt = ld / CT_T;
+  int ti = 0, rest = blockIdx.x;
+  while (rest >= nt - ti) rest -= nt - ti++;
+  const int tj = ti + rest;
+  for (int e = threadIdx.x; e < CT_T * CT_T; e += blockDim.x) {
+    const int i1 = ti * CT_T + e / CT_T, i2 = tj * CT_T + e % CT_T;
+    if (i1 > i2 || i2 >= n) continue;
+    double v = add ? tab[(size_t)i1 * n + i2] : 0.0;
+    for (int s = 0; s < nsplit; ++s) v += part[((size_t)s * ntile + blockIdx.x) * (CT_T * CT_T) + e];
     tab[(size_t)i1 * n + i2] = v;
     tab[(size_t)i2 * n + i1] = v;
   }
@@ -805,14 +880,40 @@ cudaError_t launch_contact_table(double *dtab, int n, double range, double g0, d
   // the Bessel products oscillate with period >= 2 pi / (2 range): quarter
   // periods per panel
   const double period = 2.0 * 3.141592653589793 / (2.0 * range);
-  q.nuniform = (int)ceil((q.K - q.k0) / (0.25 * period));
-  if (q.nuniform < 1) q.nuniform = 1;
+  const double nu = ceil((q.K - q.k0) / (0.25 * period));
+  if (!(nu < (1 << 27))) return cudaErrorInvalidValue;  // more nodes than an int counts
+  q.nuniform = nu < 1.0 ? 1 : (int)nu;
   q.du = (q.K - q.k0) / q.nuniform;
   const double r0 = 1e-20, h = (range - r0) / (n - 1);
-  const long long ntri = (long long)n * (n + 1) / 2;
-  const int blocks = (int)std::min<long long>((ntri + 127) / 128, 65535);
-  k_contact_table<<<blocks, 128, 0, s>>>(dtab, n, r0, h, q);
-  return cudaGetLastError();
+  const int nodes = 8 * (q.ngraded + q.nuniform);
+  const int ld = (n + CT_T - 1) / CT_T * CT_T, nt = ld / CT_T, ntile = nt * (nt + 1) / 2;
+  // about 3000 tile products in flight (ten CTAs of 64 threads per SM and a
+  // second wave), never fewer than 64 nodes each
+  const int nsplit = std::max(1, std::min({3000 / ntile, (nodes + 63) / 64, 64}));
+  const size_t npart = (size_t)nsplit * ntile * CT_T * CT_T;
+  // ranges of nodes whose four rows fit a scratch of 128 MB, less when the
+  // device has no such room left
+  double *ws = nullptr;
+  int kc = 0;
+  cudaError_t e = cudaErrorMemoryAllocation;
+  for (size_t room = (size_t)128 << 20; room >= ((size_t)1 << 18) && e == cudaErrorMemoryAllocation; room >>= 1) {
+    kc = (int)std::min<size_t>(nodes, std::max<size_t>(CT_K, room / (32 * (size_t)ld)));
+    e = cudaMalloc(&ws, 8 * (4 * (size_t)kc * ld + npart));
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+  }
+  if (e != cudaSuccess) return e;
+  double *part = ws + 4 * (size_t)kc * ld;
+  for (int q0 = 0; q0 < nodes && e == cudaSuccess; q0 += kc) {
+    const int m = std::min(kc, nodes - q0);
+    const int per = ((m + nsplit - 1) / nsplit + CT_K - 1) / CT_K * CT_K;
+    k_contact_nodes<<<dim3((ld + 127) / 128, std::min(m, 4096)), 128, 0, s>>>(ws, n, ld, q0, m, r0, h, q);
+    k_contact_product<<<dim3(ntile, nsplit), 64, 0, s>>>(ws, part, ld, m, per);
+    k_contact_gather<<<ntile, 256, 0, s>>>(part, dtab, n, ld, ntile, nsplit, q0 > 0);
+    e = cudaGetLastError();
+  }
+  const cudaError_t es = cudaStreamSynchronize(s);
+  cudaFree(ws);
+  return e != cudaSuccess ? e : es;
 }
 
 // ---------------------------------------------------------------------------
