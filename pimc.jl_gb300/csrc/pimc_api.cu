@@ -115,7 +115,8 @@ struct Handle {
   // the batched adjoint's pool and block maps, made on its first call (the
   // chains' shapes are fixed for the handle's lifetime)
   double *d_badj = nullptr;
-  AdjBatchArgs badj{};
+  AdjArgs badj{};
+  double *badj_dSdr = nullptr;  // dS/dr of every chain in the host layout
   bool badj_ready = false;
   // the batch's 32 x 32 (particle, slice) tiles: first tile of each chain
   int *d_tile_off = nullptr;
@@ -165,6 +166,7 @@ ChainDesc make_desc(const pimc_params &p, int chain) {
   d.lambda = p.lambda;
   d.mu = p.mu;
   d.hcoef = 0.5 * p.harmonic_omega * p.harmonic_omega;
+  d.omega = p.harmonic_omega;
   d.V0 = p.lattice_V0;
   d.lat_k = p.lattice_V0 != 0.0 ? 1.0 / p.lattice_a : 0.0;
   d.g = p.pair_g;
@@ -1845,47 +1847,39 @@ int pimc_reset_measurements(void *handle) {
   return sync_check(h);
 }
 
-int pimc_adjoint(void *handle, int chain, double *dSdr, double *dSdtheta, double *extra) {
-  Handle *h = H(handle);
-  if (check_chain(h, chain)) return PIMC_EARG;
-  const ChainDesc &d = h->desc[chain];
-  if (d.flags & PF_CONTACT)
-    return fail(PIMC_EARG, "the adjoint covers the Gaussian pair; chain " + std::to_string(chain) +
-                               " uses the contact table, which has no parameter derivative");
+// doubles of a single-chain adjoint's scratch: dS/dr in both layouts, the
+// CTAs' partial rows, the totals, the inverse permutation
+static size_t adjoint_doubles(const ChainDesc &d, int ib) {
   const size_t nbd = (size_t)d.N * d.M;
-  const int nblocks = (int)((nbd + 255) / 256);
-  const size_t need = 4 * nbd + (size_t)d.N + 8 * (size_t)nblocks + 16 + (size_t)d.dim * nbd;
-  if (need > h->n_adj) {
-    if (h->d_adj) cudaFree(h->d_adj);
-    h->d_adj = nullptr;
-    h->n_adj = 0;
-    CK(cudaMalloc(&h->d_adj, need * sizeof(double)));
-    h->n_adj = need;
-  }
-  AdjArgs a;
+  return 2 * (size_t)d.dim * nbd + 9 * (size_t)adjoint_ctas(d.N, d.M, ib) + 16 + ((size_t)d.N + 1) / 2;
+}
+
+// the adjoint of one chain with its scratch at `base`
+static int adjoint_run(Handle *h, int chain, int ib, double *base, double *dSdr, double *dSdtheta,
+                       double *extra) {
+  const ChainDesc &d = h->desc[chain];
+  const size_t nx = (size_t)d.dim * d.N * d.M;
+  AdjArgs a{};
   a.desc = h->d_desc;
   a.dpool = h->d_dpool;
   a.ipool = h->d_ipool;
   a.chain = chain;
-  a.omega = h->params[chain].harmonic_omega;
-  a.gA = h->d_adj;
-  a.gB = a.gA + 2 * nbd;
-  a.part = a.gB + 2 * nbd;
-  a.nblocks = nblocks;
-  a.totals = a.part + 8 * (size_t)nblocks;
-  a.sum_rg = a.totals + 8;
-  a.dSdr = a.sum_rg + 8;
-  a.inv = (int *)(a.dSdr + (size_t)d.dim * nbd);
-  // inv needs N ints: the buffer has N doubles of room after dSdr
-  CK(cudaMemsetAsync(a.sum_rg, 0, sizeof(double), h->stream));
-  CK(launch_adjoint(a, (int)nbd, h->stream));
+  a.nchains = 1;
+  a.ib = ib;
+  a.nctas = (int)adjoint_ctas(d.N, d.M, ib);
+  double *out = base + nx;
+  a.grad = dSdr ? base : nullptr;
+  a.totals = out + nx;
+  a.part = a.totals + 16;
+  a.inv = (int *)(a.part + 9 * (size_t)a.nctas);
+  const int ntiles = ((d.N + 31) / 32) * ((d.M + 31) / 32);
+  CK(launch_adjoint(a, d.N, nullptr, ntiles, dSdr ? out : nullptr, h->stream));
   double tot[9];
-  CK(cudaMemcpyAsync(tot, a.totals, 8 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(tot + 8, a.sum_rg, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  if (dSdr) CK(cudaMemcpyAsync(dSdr, a.dSdr, sizeof(double) * d.dim * nbd, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(tot, a.totals, 9 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  if (dSdr) CK(cudaMemcpyAsync(dSdr, out, sizeof(double) * nx, cudaMemcpyDeviceToHost, h->stream));
   int rc = sync_check(h);
   if (rc) return rc;
-  // totals: S_ext, dV0, domega, S_pair, dg, pair virial, r.g_ext
+  // totals: S_ext, dV0, domega, S_pair, dg, pair virial, r.g_ext, 0, r.dS/dr
   if (dSdtheta) {
     dSdtheta[0] = tot[1];
     dSdtheta[1] = tot[2];
@@ -1899,6 +1893,25 @@ int pimc_adjoint(void *handle, int chain, double *dSdr, double *dSdtheta, double
     extra[3] = tot[8];
   }
   return PIMC_OK;
+}
+
+int pimc_adjoint(void *handle, int chain, double *dSdr, double *dSdtheta, double *extra) {
+  Handle *h = H(handle);
+  if (check_chain(h, chain)) return PIMC_EARG;
+  const ChainDesc &d = h->desc[chain];
+  if (d.flags & PF_CONTACT)
+    return fail(PIMC_EARG, "the adjoint covers the Gaussian pair; chain " + std::to_string(chain) +
+                               " uses the contact table, which has no parameter derivative");
+  const int ib = adjoint_ib(d.M, (long long)d.M * ((d.N + 31) / 32), d.N, h->num_sms, h->max_dyn_smem);
+  const size_t need = adjoint_doubles(d, ib);
+  if (need > h->n_adj) {
+    if (h->d_adj) cudaFree(h->d_adj);
+    h->d_adj = nullptr;
+    h->n_adj = 0;
+    CK(cudaMalloc(&h->d_adj, need * sizeof(double)));
+    h->n_adj = need;
+  }
+  return adjoint_run(h, chain, ib, h->d_adj, dSdr, dSdtheta, extra);
 }
 
 // the adjoint with its scratch in static device memory instead of a buffer
@@ -1912,9 +1925,8 @@ int pimc_adjoint_noalloc(void *handle, int chain, double *dSdr, double *dSdtheta
     return fail(PIMC_EARG, "the adjoint covers the Gaussian pair; chain " + std::to_string(chain) +
                                " uses the contact table, which has no parameter derivative");
   const size_t nbd = (size_t)d.N * d.M;
-  const int nblocks = (int)((nbd + 255) / 256);
-  const size_t need = 4 * nbd + (size_t)d.N + 8 * (size_t)nblocks + 16 + (size_t)d.dim * nbd;
-  if (nbd > (size_t)kNoAllocBeads || d.N > kNoAllocParticles || need > kNoAllocDoubles)
+  const int ib = adjoint_ib(d.M, (long long)d.M * ((d.N + 31) / 32), d.N, h->num_sms, h->max_dyn_smem);
+  if (nbd > (size_t)kNoAllocBeads || d.N > kNoAllocParticles || adjoint_doubles(d, ib) > kNoAllocDoubles)
     return fail(PIMC_EARG, "pimc_adjoint_noalloc serves chains of at most " +
                                std::to_string(kNoAllocBeads) + " beads (N*M) and " +
                                std::to_string(kNoAllocParticles) + " particles; chain " +
@@ -1928,121 +1940,66 @@ int pimc_adjoint_noalloc(void *handle, int chain, double *dSdr, double *dSdtheta
                                std::to_string(cur) + ")");
   double *base = nullptr;
   CK(adjoint_static_scratch(&base));
-  AdjArgs a;
-  a.desc = h->d_desc;
-  a.dpool = h->d_dpool;
-  a.ipool = h->d_ipool;
-  a.chain = chain;
-  a.omega = h->params[chain].harmonic_omega;
-  a.gA = base;
-  a.gB = a.gA + 2 * nbd;
-  a.part = a.gB + 2 * nbd;
-  a.nblocks = nblocks;
-  a.totals = a.part + 8 * (size_t)nblocks;
-  a.sum_rg = a.totals + 8;
-  a.dSdr = a.sum_rg + 8;
-  a.inv = (int *)(a.dSdr + (size_t)d.dim * nbd);
-  // the only accumulator the kernels do not overwrite
-  CK(cudaMemsetAsync(a.sum_rg, 0, sizeof(double), h->stream));
-  CK(launch_adjoint(a, (int)nbd, h->stream));
-  double tot[9];
-  CK(cudaMemcpyAsync(tot, a.totals, 8 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(tot + 8, a.sum_rg, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  if (dSdr) CK(cudaMemcpyAsync(dSdr, a.dSdr, sizeof(double) * d.dim * nbd, cudaMemcpyDeviceToHost, h->stream));
-  int rc = sync_check(h);
-  if (rc) return rc;
-  if (dSdtheta) {
-    dSdtheta[0] = tot[1];
-    dSdtheta[1] = tot[2];
-    dSdtheta[2] = tot[4];
-  }
-  if (extra) {
-    const double Mt = d.M * d.tau;
-    extra[0] = tot[0];
-    extra[1] = tot[3];
-    extra[2] = (tot[0] + 0.5 * tot[6]) / Mt + (tot[3] + 0.5 * tot[5]) / Mt;
-    extra[3] = tot[8];
-  }
-  return PIMC_OK;
+  return adjoint_run(h, chain, ib, base, dSdr, dSdtheta, extra);
 }
 
-// the batched adjoint's pool: per bead gA, gB (2 doubles each), per block a
-// row of 9 partials, per chain 9 totals, dS/dr in the host layout of every
-// chain, per chain omega, then the int maps (block -> chain, first block,
-// inverse-permutation offsets, the inverse permutations) and the bead
-// offsets.  One cudaMalloc for the handle's lifetime.
+// the batched adjoint's pool: dS/dr of every chain in both layouts, per CTA a
+// row of 9 partials, per chain 9 totals, then the int maps (first CTA of each
+// chain, inverse-permutation offsets, the inverse permutations).  One
+// cudaMalloc for the handle's lifetime.
 static int batch_adjoint_setup(Handle *h) {
   if (h->badj_ready) return PIMC_OK;
   const int nc = h->nchains;
-  std::vector<int> blk_chain, blk_first(nc), inv_off(nc);
-  std::vector<long long> bead_off(nc);
-  std::vector<double> omega(nc);
-  long long tb = 0;
+  long long rows32 = 0, slices = 0;
+  for (const ChainDesc &d : h->desc) {
+    slices += d.M;
+    rows32 += (long long)d.M * ((d.N + 31) / 32);
+  }
+  const int ib = adjoint_ib(slices, rows32, h->maxN, h->num_sms, h->max_dyn_smem);
+  std::vector<int> map(2 * (size_t)nc + 1);  // cta_first[nc + 1], inv_off[nc]
+  long long nctas = 0;
   int ninv = 0;
   for (int c = 0; c < nc; ++c) {
-    const ChainDesc &d = h->desc[c];
-    const long long nm = (long long)d.N * d.M;
-    blk_first[c] = (int)blk_chain.size();
-    for (long long b = 0; b < (nm + 255) / 256; ++b) blk_chain.push_back(c);
-    bead_off[c] = tb;
-    tb += nm;
-    inv_off[c] = ninv;
-    ninv += d.N;
-    omega[c] = h->params[c].harmonic_omega;
+    map[c] = (int)nctas;
+    nctas += adjoint_ctas(h->desc[c].N, h->desc[c].M, ib);
+    if (nctas > 0x7fffffffLL) return fail(PIMC_EARG, "batch too large for the adjoint");
+    map[nc + 1 + c] = ninv;
+    ninv += h->desc[c].N;
   }
-  const size_t nblocks = blk_chain.size();
-  if (nblocks > (size_t)0x7fffffff) return fail(PIMC_EARG, "batch too large for the adjoint");
-  // one CTA per chain slice when every chain's accumulators (32 N bytes, and
-  // 12 KB for the kernel's static reduction buffer, queues and descriptor)
-  // fit the device's shared memory
-  std::vector<int> slice_first(nc);
-  long long ns = 0;
-  for (int c = 0; c < nc; ++c) {
-    slice_first[c] = (int)ns;
-    ns += h->desc[c].M;
-  }
-  const bool slices = 32LL * h->maxN + 12288 <= (long long)h->max_dyn_smem && ns < 0x7fffffffLL;
-  const size_t nd = 4 * (size_t)tb + 9 * nblocks + 9 * (size_t)nc + h->n_stage + (size_t)nc +
-                    8 * (size_t)ns;
-  const size_t ni = nblocks + 3 * (size_t)nc + (size_t)ninv;
-  const size_t bytes = 8 * nd + 4 * ((ni + 1) & ~(size_t)1) + 8 * (size_t)nc;
+  map[nc] = (int)nctas;
+  int rc = ensure_tiles(h);
+  if (rc) return rc;
+  const size_t nd = 2 * h->n_stage + 9 * (size_t)nctas + 9 * (size_t)nc;
+  const size_t bytes = 8 * nd + 4 * (map.size() + (size_t)ninv);
   double *pool = nullptr;
-  if (cudaMalloc(&pool, bytes) != cudaSuccess)
+  if (cudaMalloc(&pool, bytes) != cudaSuccess) {
+    cudaGetLastError();
     return fail(PIMC_ENOMEM, "batched adjoint pool of " + std::to_string(bytes) + " bytes");
-  AdjBatchArgs &a = h->badj;
+  }
+  h->d_badj = pool;
+  AdjArgs a{};
   a.desc = h->d_desc;
   a.dpool = h->d_dpool;
   a.ipool = h->d_ipool;
-  a.gA = pool;
-  a.gB = a.gA + 2 * (size_t)tb;
-  a.part = a.gB + 2 * (size_t)tb;
-  a.totals = a.part + 9 * nblocks;
-  a.dSdr = a.totals + 9 * (size_t)nc;
-  double *om = a.dSdr + h->n_stage;
-  a.part_s = om + nc;
-  int *ip = (int *)(a.part_s + 8 * (size_t)ns);
-  int *bc = ip, *bf = bc + nblocks, *io = bf + nc, *sf = io + nc, *inv = sf + nc;
-  long long *bo = (long long *)(ip + ((ni + 1) & ~(size_t)1));
-  a.omega = om;
-  a.blk_chain = bc;
-  a.blk_first = bf;
-  a.inv_off = io;
-  a.inv = inv;
-  a.bead_off = bo;
-  a.nblocks = (int)nblocks;
   a.nchains = nc;
-  a.use_slices = slices ? 1 : 0;
-  a.nslices = (int)ns;
-  a.slice_first = sf;
-  h->d_badj = pool;
-  CK(cudaMemcpyAsync(om, omega.data(), 8 * (size_t)nc, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(bc, blk_chain.data(), 4 * nblocks, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(bf, blk_first.data(), 4 * (size_t)nc, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(io, inv_off.data(), 4 * (size_t)nc, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(sf, slice_first.data(), 4 * (size_t)nc, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(bo, bead_off.data(), 8 * (size_t)nc, cudaMemcpyHostToDevice, h->stream));
-  int rc = sync_check(h);
-  if (rc) return rc;
+  a.ib = ib;
+  a.nctas = (int)nctas;
+  a.grad = pool;
+  h->badj_dSdr = pool + h->n_stage;
+  a.part = h->badj_dSdr + h->n_stage;
+  a.totals = a.part + 9 * (size_t)nctas;
+  int *ip = (int *)(a.totals + 9 * (size_t)nc);
+  a.cta_first = ip;
+  a.inv_off = ip + nc + 1;
+  a.inv = ip + map.size();
+  h->badj = a;
+  const cudaError_t e = cudaMemcpyAsync(ip, map.data(), 4 * map.size(), cudaMemcpyHostToDevice, h->stream);
+  rc = e == cudaSuccess ? sync_check(h) : fail(PIMC_ECUDA, cudaGetErrorString(e));
+  if (rc) {
+    cudaFree(pool);
+    h->d_badj = nullptr;
+    return rc;
+  }
   h->badj_ready = true;
   return PIMC_OK;
 }
@@ -2056,21 +2013,21 @@ int pimc_batch_adjoint(void *handle, double *dSdtheta, double *extra, double *dS
                                  " uses the contact table, which has no parameter derivative");
   int rc = batch_adjoint_setup(h);
   if (rc) return rc;
-  AdjBatchArgs a = h->badj;
-  if (!dSdr_all) a.dSdr = nullptr;
+  AdjArgs a = h->badj;
+  if (!dSdr_all) a.grad = nullptr;
   CK(cudaEventRecord(h->ev0, h->stream));
-  CK(launch_adjoint_batch(a, h->maxN, h->stream));
+  CK(launch_adjoint(a, h->maxN, h->d_tile_off, h->ntiles, dSdr_all ? h->badj_dSdr : nullptr, h->stream));
   CK(cudaEventRecord(h->ev1, h->stream));
   std::vector<double> tot(9 * (size_t)h->nchains);
   CK(cudaMemcpyAsync(tot.data(), a.totals, 8 * tot.size(), cudaMemcpyDeviceToHost, h->stream));
   if (dSdr_all)
-    CK(cudaMemcpyAsync(dSdr_all, a.dSdr, 8 * h->n_stage, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(dSdr_all, h->badj_dSdr, 8 * h->n_stage, cudaMemcpyDeviceToHost, h->stream));
   rc = sync_check(h);
   if (rc) return rc;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, h->ev0, h->ev1);
   h->last_ms = ms;
-  h->last_launches = 4;
+  h->last_launches = dSdr_all ? 4 : 3;
   for (int c = 0; c < h->nchains; ++c) {
     const double *t = tot.data() + 9 * (size_t)c;
     const ChainDesc &d = h->desc[c];
@@ -2252,6 +2209,7 @@ int pimc_set_potential(void *handle, int chain, double V0, double omega, double 
   d.V0 = V0;
   d.lat_k = V0 != 0.0 ? 1.0 / p.lattice_a : 0.0;
   d.hcoef = 0.5 * omega * omega;
+  d.omega = omega;
   d.g = g;
   d.mhtau_g = -0.5 * d.tau * d.g;
   d.flags &= ~(PF_LATT | PF_HARM);

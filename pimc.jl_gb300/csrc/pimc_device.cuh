@@ -646,9 +646,15 @@ constexpr int EXPTAB_N = 2560;
 static __device__ double g_exptab[EXPTAB_N + 1];
 
 __device__ __forceinline__ double exp_neg(double x) {
-  if (!(x >= -40.0)) return exp(x);
-  const int k = __double2int_rn(x * -64.0);
-  const double f = fma((double)k, 0.015625, x);
+  // -x > 40 on the bits (x <= 0): a compare or a conversion costs the FP64
+  // pipe as much as a product, so the rounding to k goes through the low word
+  // of -64 x + 1.5 2^52
+  if ((unsigned long long)__double_as_longlong(x) > (unsigned long long)__double_as_longlong(-40.0) ||
+      __double_as_longlong(x) > 0)
+    return exp(x);
+  const double t = fma(x, -64.0, 6755399441055744.0);
+  const int k = __double2loint(t);
+  const double f = fma(t - 6755399441055744.0, 0.015625, x);
   double p = fma(f, 1.0 / 120.0, 1.0 / 24.0);
   p = fma(p, f, 1.0 / 6.0);
   p = fma(p, f, 0.5);
@@ -688,12 +694,18 @@ __device__ __forceinline__ double2 bridge_w(const CV &c, int m, int t) {
   return make_double2(sqrt(2.0 * c.d->lambda * a * c.d->tau) / (m - t), (double)(m - t));
 }
 
+// |x| > y, y >= 0, on the bits: a double compare takes the FP64 pipe's 16
+// cycles per warp, an integer one does not (a NaN x counts as greater)
+__device__ __forceinline__ bool abs_gt(double x, double y) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > __double_as_longlong(y);
+}
+
 // minimum-image difference a - b: the same magnitude as dist1 (|a-b| when it
 // is at most L, else 2L - |a-b|, both exactly rounded), with one subtraction
 // and a rarely taken wrap
 __device__ __forceinline__ double mi1(double a, double b, double L, double L2) {
   double dx = a - b;
-  if (fabs(dx) > L) dx -= copysign(L2, dx);
+  if (abs_gt(dx, L)) dx -= copysign(L2, dx);
   return dx;
 }
 

@@ -54,45 +54,30 @@ struct EvalArgs {
   double *out;
 };
 
+// the adjoint of one chain (cta_first null) or of every chain of a batch: a
+// warp per ib particles of a slice, four warps per CTA, chain after chain
 struct AdjArgs {
   const ChainDesc *desc;
   double *dpool;
   int *ipool;
-  int chain;
-  double omega;
-  double *gA, *gB;    // [N*M][2] scratch
-  int *inv;           // [N] scratch
-  double *part;       // [nblocks][8] scratch
-  int nblocks;
-  double *dSdr;       // [dim][N][M] or null
-  double *totals;     // [8]
-  double *sum_rg;     // [1], zeroed before the launch
+  int chain;            // the chain of a single-chain call
+  int nchains;
+  int ib;               // particles per warp, or ADJ_SLICES (adjoint_ib)
+  int nctas;
+  const int *cta_first; // [nchains + 1] first CTA of each chain, or null
+  const int *inv_off;   // [nchains] offset of each chain's inverse permutation
+  int *inv;             // inverse permutations
+  double *part;         // [nctas][9]
+  double *totals;       // [chains][9]: S_ext, dV0, domega, S_pair, dg, pair
+                        // virial, r.g_ext, 0, r.dS/dr
+  double *grad;         // dS/dr in the device layout [j][n][d], chains at
+                        // desc.host_off (a batch) or 0, or null
 };
-
-// the adjoint of every chain of a batch (pimc_batch_adjoint): beads in
-// blocks of 256, chain after chain
-struct AdjBatchArgs {
-  const ChainDesc *desc;
-  double *dpool;
-  int *ipool;
-  const double *omega;        // [nchains] trap frequency (d/domega)
-  const int *blk_chain;       // [nblocks] chain of each block
-  const int *blk_first;       // [nchains] first block of each chain
-  const long long *bead_off;  // [nchains] first bead of each chain in gA / gB
-  const int *inv_off;         // [nchains] offset of each chain's inverse permutation
-  double *gA, *gB;            // [total beads][2]
-  int *inv;                   // [sum of N]
-  double *part;               // [nblocks][9]
-  double *dSdr;               // host layout of every chain (desc.host_off), or null
-  double *totals;             // [nchains][9]: S_ext, dV0, domega, S_pair, dg, pair
-                              // virial, r.g_ext, 0, r.dS/dr
-  int nblocks, nchains;
-  // the slice kernel (one CTA per chain slice, 32 maxN bytes of shared
-  // memory): used when use_slices != 0
-  int use_slices, nslices;
-  const int *slice_first;     // [nchains] first slice CTA of each chain
-  double *part_s;             // [nslices][8]
-};
+constexpr int ADJ_SLICES = 0;  // ib: a CTA per slice instead
+inline long long adjoint_ctas(int N, int M, int ib) {
+  if (ib == ADJ_SLICES) return M;
+  return ((long long)M * ((N + ib - 1) / ib) + 3) / 4;
+}
 
 // mode 0: one CTA per chain (k_sweep); mode 1: one warp per chain (k_sweep_warp)
 cudaError_t launch_sweep(const SweepArgs &a, int mode, int grid, int block, size_t smem,
@@ -138,10 +123,12 @@ cudaError_t launch_transpose_tiles(bool import, const ChainDesc *desc, double *d
                                    int ntiles, int grid, cudaStream_t s);
 cudaError_t launch_measure(const ChainDesc *desc, ChainVar *var, double *dpool, int *ipool,
                            unsigned long long *upool, int chain0, int nchains, cudaStream_t s);
-cudaError_t launch_adjoint(const AdjArgs &a, int nbeads, cudaStream_t s);
-// four launches over every chain (inverse permutations, beads, gradients,
-// per-chain totals)
-cudaError_t launch_adjoint_batch(const AdjBatchArgs &a, int maxN, cudaStream_t s);
+int adjoint_ib(long long slices, long long rows32, int maxN, int num_sms, int max_dyn_smem);
+// inverse permutations, the gather, the totals, and with dSdr (host layout,
+// chains as in grad) the transpose of grad over the ntiles tiles of tile_off
+// (null: one chain)
+cudaError_t launch_adjoint(const AdjArgs &a, int maxN, const int *tile_off, int ntiles, double *dSdr,
+                           cudaStream_t s);
 cudaError_t upload_exp_table();
 // PIMC_CHECK builds: the device check word (code << 32 | chain of the first
 // failed bounds check, 0 if none), cleared by the read; always 0 otherwise

@@ -74,22 +74,27 @@ __device__ __forceinline__ int tile_chain(const int *tile_off, int c_lo, int c_h
   return lo;
 }
 
+// dev: a device-layout buffer of its own, chain c at host_off (per-bead forces)
+// instead of the positions in the pool; tile_off null: the tiles of chain c_lo
+// alone, both buffers holding nothing else.
 template <bool IMPORT>
 __global__ void __launch_bounds__(256) k_transpose_tiles(const ChainDesc *desc, double *dpool,
                                                           double *host, const int *tile_off,
-                                                          int c_lo, int c_hi) {
+                                                          int c_lo, int c_hi, double *dev) {
   __shared__ double tile[2][32][33];
-  const int t_end = tile_off[c_hi];
+  const int t_begin = tile_off ? tile_off[c_lo] : 0;
+  const int t_end = tile_off ? tile_off[c_hi] : ((desc[c_lo].N + 31) >> 5) * ((desc[c_lo].M + 31) >> 5);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int t = tile_off[c_lo] + blockIdx.x; t < t_end; t += gridDim.x) {
-    const int c = tile_chain(tile_off, c_lo, c_hi, t);
+  for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
+    const int c = tile_off ? tile_chain(tile_off, c_lo, c_hi, t) : c_lo;
     const ChainDesc &d = desc[c];
     const int N = d.N, M = d.M, dim = d.dim;
-    const int tj = (M + 31) >> 5, lt = t - tile_off[c];
+    const int tj = (M + 31) >> 5, lt = tile_off ? t - tile_off[c] : t;
     const int n0 = (lt / tj) * 32, j0 = (lt % tj) * 32;
     const int nn = min(32, N - n0), nj = min(32, M - j0);
-    double *x = dpool + d.x_off;
-    double *hx = host + d.host_off;
+    const long long off = tile_off ? d.host_off : 0;
+    double *x = dev ? dev + off : dpool + d.x_off;
+    double *hx = host + off;
     if (IMPORT) {
       // host rows (k, n): 32 consecutive slices per warp-wide read
       for (int r = w; r < dim * nn; r += 8) {
@@ -272,357 +277,388 @@ __global__ void __launch_bounds__(256) k_measure(const ChainDesc *desc, ChainVar
 }
 
 // ---------------------------------------------------------------------------
-// adjoint of the potential action S_pot = -sum lnV - sum lnU:
-// per-bead dS/dr and dS/d(V0, omega, g).  Bead-parallel over one chain;
-// consecutive threads are consecutive particles of one slice, so the slice
-// row they scan is shared.
-// part[block][8]: S_ext, dV0, domega, S_pair, dg, pair virial, r.g_ext, 0
+// adjoint of the potential action S_pot = -sum lnV - sum lnU: per-bead dS/dr
+// and dS/d(V0, omega, g), one chain or every chain of a batch.
+//
+// A pair (i, b) of slice j enters two links: the one it starts (when it is
+// within reach at j) and the one it ends (when its beads one slice earlier,
+// along the paths, were within reach there).  Both uses carry the same
+// exponential at slice j, so k_adjoint_gather evaluates it once per pair and
+// slice, times the number of uses, and gathers it into the bead: no second
+// pass over the links' ends and no atomics.
+//
+// A warp takes `ib` particles of one slice.  For each, the lanes test 32
+// partners at a time on the mirror words of slices j and j-1 (integer), push
+// the ones in reach at either onto a ring in shared memory, and evaluate 32
+// of them at once in FP64 -- the FP64 pipe (16 cycles of an SM per warp
+// instruction, whatever the active lanes) is the bound, so its instructions
+// run on full warps, compares run on the bits, and the earlier slice's reach
+// is settled on the mirror unless it lies within the mirror's error of the
+// cut-off.  Before, one thread per bead scanned its partners (5.6 of 32 lanes
+// active in the FP64 branch) and a batch's CTA per slice added forces through
+// FP64 shared atomics (compare-and-swap loops).  Whole calls: one chain of N =
+// 1024, M = 64 (lattice, trap, pair) 5.97 -> 0.42 ms; 60 chains of 8 to 512
+// particles with every bead's force 29.3 -> 5.9 ms, of which k_adjoint_slices
+// takes 5.2 at 85 % of the FP64 pipe.
+//
+// Partial sums per CTA: part[cta][9] = S_ext, dV0, domega, S_pair, dg, pair
+// virial, r.g_ext, 0, r.dS/dr.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double mi_signed(double a, double b, double L) {
-  double s = a - b;
-  if (s > L) s -= 2.0 * L;
-  else if (s < -L) s += 2.0 * L;
-  return s;
-}
-
-// adjoint terms of bead k (slice-major k = j N + i) of one chain: v[8] the
-// block partials above, ga the bead's gradient from the external potential
-// and from the pair terms of the link it starts, gb the gradient of the next
-// bead of its path (in_, jn) from the pair terms of that link
-__device__ __forceinline__ void adjoint_bead(const ChainDesc &d, const CV &c, int k, double omega,
-                                             double (&v)[8], double (&ga)[2], double (&gb)[2]) {
-  const int N = c.N, M = c.M, dim = c.dim;
-  const int j = k / N, i = k % N;
-  const int in = j == M - 1 ? c.next[i] : i, jn = j + 1 == M ? 0 : j + 1;
-  const double tau = d.tau;
-  const double ax = c.X(0, i, j), ay = c.Xd(1, i, j);
-  const double anx = c.X(0, in, jn), any = c.Xd(1, in, jn);
-  double ge[2];
-  grad_vext(d, ax, ay, ge[0], ge[1]);
-  ge[0] *= tau;
-  ge[1] *= tau;
-  v[0] = tau * vext(d, ax, ay);
-  if (d.flags & PF_LATT) {
-    const double sx = sinpi(ax * d.lat_k), sy = dim > 1 ? sinpi(ay * d.lat_k) : 0.0;
-    v[1] = tau * (sx * sx + sy * sy);
-  }
-  if (d.flags & PF_HARM) v[2] = tau * omega * (ax * ax + ay * ay);
-  v[6] = ax * ge[0] + ay * ge[1];
-  double go[2] = {0.0, 0.0}, gn[2] = {0.0, 0.0};
-  if (d.flags & PF_PAIR) {
-    const double rc2 = d.rc * d.rc, cg = d.inv2s2, h = 0.5 * tau;
-    Prefilter f;
-    f.init_q(c.Q(i, j), d.q_lim_rc);
-    const unsigned *row = c.xq + (size_t)j * c.ldn;
-    for (int b = 0; b < N; ++b) {
-      if (b == i || !f.pass(row[b])) continue;
-      const double bxv = c.X(0, b, j), byv = c.Xd(1, b, j);
-      const double d1x = mi_signed(ax, bxv, d.L), d1y = dim > 1 ? mi_signed(ay, byv, d.L) : 0.0;
-      const double r2a = mi2(d, ax, ay, bxv, byv);
-      if (r2a > rc2) continue;
-      const int bn = j == M - 1 ? c.next[b] : b;
-      const double bnx = c.X(0, bn, jn), bny = c.Xd(1, bn, jn);
-      const double d2x = mi_signed(anx, bnx, d.L), d2y = dim > 1 ? mi_signed(any, bny, d.L) : 0.0;
-      const double r2b = mi2(d, anx, any, bnx, bny);
-      const double e1 = exp_neg(-r2a * cg), e2 = exp_neg(-r2b * cg);
-      const double v1 = d.g * e1, v2 = d.g * e2;
-      go[0] += h * (-2.0 * cg * v1) * d1x;
-      go[1] += h * (-2.0 * cg * v1) * d1y;
-      gn[0] += h * (-2.0 * cg * v2) * d2x;
-      gn[1] += h * (-2.0 * cg * v2) * d2y;
-      // each unordered pair is visited from both sides
-      v[3] += 0.5 * h * (v1 + v2);
-      v[4] += 0.5 * h * (e1 + e2);
-      v[5] += 0.5 * h * (-2.0 * cg) * (r2a * v1 + r2b * v2);
-    }
-  }
-  ga[0] = ge[0] + go[0];
-  ga[1] = ge[1] + go[1];
-  gb[0] = gn[0];
-  gb[1] = gn[1];
-}
-
-__global__ void __launch_bounds__(256) k_adjoint_beads(AdjArgs a) {
-  __shared__ double red[256];
-  __shared__ ChainDesc d;
-  if (threadIdx.x == 0) d = a.desc[a.chain];
-  __syncthreads();
-  CV c = make_cv(&d, a.dpool, a.ipool, nullptr);
-  const int N = c.N, M = c.M;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (k < N * M) {
-    double ga[2], gb[2];
-    adjoint_bead(d, c, k, a.omega, v, ga, gb);
-    // per-bead buffers in the chain's [i][j] order (k2 = i*M + j)
-    const int j = k / N, i = k % N;
-    const size_t k2 = (size_t)i * M + j;
-    for (int q = 0; q < 2; ++q) {
-      a.gA[k2 * 2 + q] = ga[q];
-      a.gB[k2 * 2 + q] = gb[q];
-    }
-  }
-  block_sum_k<8>(v, red);
-  if (threadIdx.x == 0)
-    for (int q = 0; q < 8; ++q) a.part[(size_t)blockIdx.x * 8 + q] = v[q];
-}
-
-__global__ void k_inverse_next(AdjArgs a) {
-  const ChainDesc &d = a.desc[a.chain];
-  const int *next = a.ipool + d.next_off;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.N; i += gridDim.x * blockDim.x)
-    a.inv[next[i]] = i;
-}
-
-__global__ void __launch_bounds__(256) k_adjoint_finish(AdjArgs a) {
-  __shared__ double red[256];
-  __shared__ ChainDesc d;
-  if (threadIdx.x == 0) d = a.desc[a.chain];
-  __syncthreads();
-  CV c = make_cv(&d, a.dpool, a.ipool, nullptr);
-  const int N = c.N, M = c.M, dim = c.dim;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;  // k = i*M + j
-  double rg[1] = {0.0};
-  if (k < N * M) {
-    const int i = k / M, j = k % M;
-    const int kp = j > 0 ? k - 1 : a.inv[i] * M + (M - 1);
-    for (int q = 0; q < dim; ++q) {
-      const double g = a.gA[(size_t)k * 2 + q] + a.gB[(size_t)kp * 2 + q];
-      if (a.dSdr) a.dSdr[(size_t)q * N * M + k] = g;
-      rg[0] += c.X(q, i, j) * g;
-    }
-  }
-  block_sum_k<1>(rg, red);
-  if (threadIdx.x == 0) atomicAdd(a.sum_rg, rg[0]);
-  if (blockIdx.x == 0) {
-    double t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int b = threadIdx.x; b < a.nblocks; b += blockDim.x)
-      for (int q = 0; q < 8; ++q) t[q] += a.part[(size_t)b * 8 + q];
-    block_sum_k<8>(t, red);
-    if (threadIdx.x == 0)
-      for (int q = 0; q < 8; ++q) a.totals[q] = t[q];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// batched adjoint: every chain of a batch in one launch per stage.  Blocks of
-// 256 beads are laid out chain after chain (blk_first[c] is chain c's first
-// block, blk_chain[b] the chain of block b), so one grid covers chains of any
-// size; each block works on one chain only and writes its partial sums to
-// its own row of part, which k_adjoint_totals_b reduces per chain.
-// ---------------------------------------------------------------------------
-__global__ void k_adjoint_inv_b(AdjBatchArgs a) {
-  const int ch = blockIdx.y;
+__global__ void k_adjoint_inv(AdjArgs a) {
+  const int ch = a.cta_first ? (int)blockIdx.y : a.chain;
   const ChainDesc &d = a.desc[ch];
   const int *next = a.ipool + d.next_off;
-  int *inv = a.inv + a.inv_off[ch];
+  int *inv = a.inv + (a.cta_first ? a.inv_off[ch] : 0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.N; i += gridDim.x * blockDim.x)
     inv[next[i]] = i;
 }
 
-__global__ void __launch_bounds__(256) k_adjoint_beads_b(AdjBatchArgs a) {
-  __shared__ double red[256];
-  __shared__ ChainDesc d;
-  __shared__ int ch, lb;
-  if (threadIdx.x == 0) {
-    ch = a.blk_chain[blockIdx.x];
-    lb = blockIdx.x - a.blk_first[ch];
-    d = a.desc[ch];
+// the sums over the warp of eight values a lane: lane l ends with the sum of
+// value l & 7 (nine FP64 additions instead of forty)
+__device__ __forceinline__ double warp_sum8(const double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+  double a[4], b[2];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const bool up = lane & 4;
+    a[q] = (up ? v[q + 4] : v[q]) + __shfl_xor_sync(0xffffffffu, up ? v[q] : v[q + 4], 4);
   }
-  __syncthreads();
-  CV c = make_cv(&d, a.dpool, a.ipool, nullptr);
-  const int N = c.N, M = c.M;
-  const int k = lb * blockDim.x + threadIdx.x;
-  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (k < N * M) {
-    double ga[2], gb[2];
-    adjoint_bead(d, c, k, a.omega[ch], v, ga, gb);
-    const int j = k / N, i = k % N;
-    const size_t k2 = (size_t)a.bead_off[ch] + (size_t)i * M + j;
-    for (int q = 0; q < 2; ++q) {
-      a.gA[k2 * 2 + q] = ga[q];
-      a.gB[k2 * 2 + q] = gb[q];
-    }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const bool up = lane & 2;
+    b[q] = (up ? a[q + 2] : a[q]) + __shfl_xor_sync(0xffffffffu, up ? a[q] : a[q + 2], 2);
   }
-  block_sum_k<8>(v, red);
-  if (threadIdx.x == 0)
-    for (int q = 0; q < 8; ++q) a.part[(size_t)blockIdx.x * 9 + q] = v[q];
+  const bool up = lane & 1;
+  double c = (up ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 1);
+  c += __shfl_xor_sync(0xffffffffu, c, 8);
+  c += __shfl_xor_sync(0xffffffffu, c, 16);
+  return c;
 }
 
-// the pair terms and the external potential of one slice of one chain per
-// CTA (blocks slice_first[c] .. slice_first[c] + M - 1 are chain c's slices):
-// warps take particles i, lanes scan the higher-numbered partners b of the
-// slice through the mirror prefilter and queue the survivors, and every
-// queued pair is evaluated once in FP64, 32 at a time on full warps; its
-// force goes to both particles through accumulators in shared memory
-// (4 doubles per particle: the bead's gradient from the link it starts, and
-// the gradient of its next bead from the same link).  Needs 32 N bytes of
-// dynamic shared memory.  The accumulators add the pair forces in the order
-// the atomics land, so results repeat to rounding, not bit for bit.  Partial
-// sums to part_s[cta][8] as k_adjoint_beads.
-__global__ void __launch_bounds__(256) k_adjoint_slice_b(AdjBatchArgs a) {
-  extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ double red[256];
-  __shared__ ChainDesc d;
-  __shared__ int ch, j;
-  __shared__ unsigned long long qbuf[8 * PQ_CAP];
+constexpr int ADJ_RING = 128;  // ring entries per warp (at most 31 + 64 in use)
+// whether the pair's mirror words at a slice (ci, wc) or at the one before
+// (pi, wp) may lie within reach, and its ring entry: the partner, and for the
+// earlier slice 0 beyond, 1 within, 2 within the mirror's error of the cut-off
+__device__ __forceinline__ bool adjoint_reach(unsigned ci, unsigned pi, unsigned wc, unsigned wp,
+                                              unsigned lim_lo, unsigned lim_hi, int b, unsigned &e) {
+  const unsigned d2c = qdist2(ci, wc), d2p = qdist2(pi, wp);
+  const unsigned st = d2p < lim_lo ? 1u : (d2p <= lim_hi ? 2u : 0u);
+  e = (unsigned)b | (st << 16);
+  return d2c <= lim_hi || st;
+}
+
+// the uses of a pair at slice j -- the link it starts (r2 within reach) and the
+// link it ends (the earlier beads' reach, settled by the entry or exactly)
+__device__ __forceinline__ int adjoint_uses(const CV &c, const ChainDesc &d, unsigned e, double r2, int i, int b,
+                                            int jp, const int *inv) {
+  int uses = __double_as_longlong(r2) <= __double_as_longlong(d.rc2) ? 1 : 0;
+  const unsigned st = e >> 16;
+  if (st == 1u) {
+    ++uses;
+  } else if (st == 2u) {
+    const int ip = inv ? inv[i] : i, bp = inv ? inv[b] : b;
+    if (mi2(d, c.X(0, ip, jp), c.Xd(1, ip, jp), c.X(0, bp, jp), c.Xd(1, bp, jp)) <= d.rc2) ++uses;
+  }
+  return uses;
+}
+
+// a bead's external terms of the adjoint: its gradient, and its shares of the
+// partial sums
+__device__ __forceinline__ void adjoint_ext(const ChainDesc &d, double ax, double ay, double &gx, double &gy,
+                                            double (&v)[8]) {
+  const double tau = d.tau;
+  double ge[2];
+  grad_vext(d, ax, ay, ge[0], ge[1]);
+  gx = ge[0] * tau;
+  gy = ge[1] * tau;
+  v[0] += tau * vext(d, ax, ay);
+  if (d.flags & PF_LATT) {
+    const double sx = sinpi(ax * d.lat_k), sy = d.dim > 1 ? sinpi(ay * d.lat_k) : 0.0;
+    v[1] += tau * (sx * sx + sy * sy);
+  }
+  if (d.flags & PF_HARM) v[2] += tau * d.omega * (ax * ax + ay * ay);
+  v[6] += ax * gx + ay * gy;
+}
+
+// the block's chain and its CTA within it; every thread calls it
+__device__ __forceinline__ void adjoint_cta(const AdjArgs &a, const int *first, ChainDesc *d, int *ch_, int *lb_) {
   if (threadIdx.x == 0) {
-    int lo = 0, hi = a.nchains;  // slice_first[lo] <= blockIdx.x < slice_first[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (a.slice_first[mid] <= (int)blockIdx.x) lo = mid; else hi = mid;
+    int ch = a.chain, lb = blockIdx.x;
+    if (first) {
+      int lo = 0, hi = a.nchains;  // first[lo] <= blockIdx.x < first[hi]
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= (int)blockIdx.x) lo = mid; else hi = mid;
+      }
+      ch = lo;
+      lb -= first[lo];
     }
-    ch = lo;
-    j = blockIdx.x - a.slice_first[lo];
-    d = a.desc[lo];
+    *ch_ = ch;
+    *lb_ = lb;
+    *d = a.desc[ch];
   }
   __syncthreads();
-  CV c = make_cv(&d, a.dpool, a.ipool, nullptr);
-  const int N = c.N, M = c.M, dim = c.dim, jn = j + 1 == M ? 0 : j + 1;
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = nt >> 5;
-  double *acc = reinterpret_cast<double *>(dsm);  // [4][N]: ga.x, ga.y, gb.x, gb.y
-  for (int e = tid; e < 4 * N; e += nt) acc[e] = 0.0;
+}
+
+// the CTA's row of partial sums: four warps' v[0..7] and r.dS/dr
+__device__ __forceinline__ void adjoint_part(const AdjArgs &a, const double (&v)[8], double rg, double (*red)[9]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double s8 = warp_sum8(v);
+  rg = warp_sum(rg);
+  if (lane < 8) red[warp][lane] = s8;
+  if (lane == 8) red[warp][8] = rg;
   __syncthreads();
-  const double tau = d.tau;
-  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (d.flags & PF_PAIR) {
-    const double cg = d.inv2s2, h = 0.5 * tau, rc2 = d.rc * d.rc;
-    unsigned long long *q = qbuf + (size_t)warp * PQ_CAP;
-    const unsigned lt = (1u << lane) - 1u;
-    const unsigned *row = c.xq + (size_t)j * c.ldn;
-    int qn = 0;
-    auto flush = [&]() {
-      const int k = qn < 32 ? qn : 32;
-      if (lane < k) {
-        const unsigned long long e = q[lane];
-        const int i = (int)(e >> 32), b = (int)(e & 0xffffffffu);
-        const double ax = c.X(0, i, j), ay = c.Xd(1, i, j);
-        const double bx = c.X(0, b, j), by = c.Xd(1, b, j);
-        const double r2a = mi2(d, ax, ay, bx, by);
-        if (r2a <= rc2) {
-          const int in = j == M - 1 ? c.next[i] : i, bn = j == M - 1 ? c.next[b] : b;
-          const double anx = c.X(0, in, jn), any = c.Xd(1, in, jn);
-          const double bnx = c.X(0, bn, jn), bny = c.Xd(1, bn, jn);
-          const double d1x = mi_signed(ax, bx, d.L), d1y = dim > 1 ? mi_signed(ay, by, d.L) : 0.0;
-          const double d2x = mi_signed(anx, bnx, d.L), d2y = dim > 1 ? mi_signed(any, bny, d.L) : 0.0;
-          const double r2b = mi2(d, anx, any, bnx, bny);
-          const double e1 = exp_neg(-r2a * cg), e2 = exp_neg(-r2b * cg);
-          const double v1 = d.g * e1, v2 = d.g * e2;
-          const double f1 = h * (-2.0 * cg * v1), f2 = h * (-2.0 * cg * v2);
-          atomicAdd(&acc[i], f1 * d1x);
-          atomicAdd(&acc[b], -f1 * d1x);
-          atomicAdd(&acc[2 * N + i], f2 * d2x);
-          atomicAdd(&acc[2 * N + b], -f2 * d2x);
-          if (dim > 1) {
-            atomicAdd(&acc[N + i], f1 * d1y);
-            atomicAdd(&acc[N + b], -f1 * d1y);
-            atomicAdd(&acc[3 * N + i], f2 * d2y);
-            atomicAdd(&acc[3 * N + b], -f2 * d2y);
+  if (threadIdx.x < 9)
+    a.part[(size_t)blockIdx.x * 9 + threadIdx.x] =
+        (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
+}
+
+// the sums over the warp of two values: lanes 0-15 end with x's, 16-31 with
+// y's (five FP64 additions)
+__device__ __forceinline__ double warp_sum2(double x, double y) {
+  const bool up = (threadIdx.x & 16) != 0;
+  double f = (up ? y : x) + __shfl_xor_sync(0xffffffffu, up ? x : y, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+  return f;
+}
+
+__global__ void __launch_bounds__(128) k_adjoint_gather(AdjArgs a) {
+  __shared__ ChainDesc d;
+  __shared__ int s_ch, s_lb;
+  __shared__ unsigned ring_s[4][ADJ_RING];
+  __shared__ double red[4][9];
+  adjoint_cta(a, a.cta_first, &d, &s_ch, &s_lb);
+  CV c = make_cv(&d, a.dpool, a.ipool, nullptr);
+  const int N = c.N, M = c.M, dim = c.dim;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nib = (N + a.ib - 1) / a.ib, unit = s_lb * 4 + warp;
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, rg = 0.0;
+  if (unit < M * nib) {
+    const int j = unit / nib, i0 = (unit % nib) * a.ib, ni = min(a.ib, N - i0);
+    const int jp = j ? j - 1 : M - 1;
+    const int *inv = j ? nullptr : a.inv + (a.cta_first ? a.inv_off[s_ch] : 0);
+    const unsigned *row = c.xq + (size_t)j * c.ldn, *rowp = c.xq + (size_t)jp * c.ldn;
+    const bool own = lane < ni;
+    const int me = i0 + lane;
+    double ax = 0.0, ay = 0.0, gx = 0.0, gy = 0.0;
+    unsigned qc = 0u, qp = 0u;
+    if (own) {
+      ax = c.X(0, me, j);
+      ay = c.Xd(1, me, j);
+      qc = row[me];
+      qp = rowp[inv ? inv[me] : me];
+      adjoint_ext(d, ax, ay, gx, gy, v);
+    }
+    if ((d.flags & PF_PAIR) && N > 1) {
+      const double cg = d.inv2s2, h = 0.5 * d.tau;
+      const double kf = -2.0 * cg * h * d.g;  // the force's factor
+      const unsigned lim_lo = d.q_lim_lo, lim_hi = d.q_lim_hi, lt = (1u << lane) - 1u;
+      unsigned *ring = ring_s[warp];
+      double se = 0.0, sr = 0.0;  // sums over ordered pairs of e and r^2 e
+      for (int ii = 0; ii < ni; ++ii) {
+        const int i = i0 + ii;
+        const double px = __shfl_sync(0xffffffffu, ax, ii), py = __shfl_sync(0xffffffffu, ay, ii);
+        const unsigned ci = __shfl_sync(0xffffffffu, qc, ii), pi = __shfl_sync(0xffffffffu, qp, ii);
+        double fx = 0.0, fy = 0.0;
+        int head = 0, tail = 0;
+        auto eval = [&](int k) {
+          if (lane < k) {
+            const unsigned e = ring[(head + lane) & (ADJ_RING - 1)];
+            const int b = (int)(e & 0xffffu);
+            const double dx = mi1(px, c.X(0, b, j), d.L, d.L2);
+            const double dy = dim > 1 ? mi1(py, c.X(1, b, j), d.L, d.L2) : 0.0;
+            double r2 = dx * dx;
+            if (dim > 1) r2 = fma(dy, dy, r2);
+            const int uses = adjoint_uses(c, d, e, r2, i, b, jp, inv);
+            if (uses) {
+              double w = exp_neg(-r2 * cg);
+              if (uses == 2) w += w;
+              se += w;
+              sr = fma(r2, w, sr);
+              fx = fma(w, dx, fx);
+              fy = fma(w, dy, fy);
+            }
           }
-          v[3] += h * (v1 + v2);
-          v[4] += h * (e1 + e2);
-          v[5] += h * (-2.0 * cg) * (r2a * v1 + r2b * v2);
+          head += k;
+          __syncwarp();
+        };
+        // two blocks of 32 partners an iteration: four loads in flight; the
+        // ring then holds at most 31 + 64 entries
+        for (int b0 = 0; b0 < N; b0 += 64) {
+          unsigned wc[2], wp[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int b = b0 + 32 * u + lane;
+            wc[u] = b < N ? row[b] : 0u;
+            wp[u] = b < N ? rowp[inv ? inv[b] : b] : 0u;
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int b = b0 + 32 * u + lane;
+            unsigned e = 0u;
+            const bool p = b < N && b != i && adjoint_reach(ci, pi, wc[u], wp[u], lim_lo, lim_hi, b, e);
+            const unsigned mk = __ballot_sync(0xffffffffu, p);
+            if (p) ring[(tail + __popc(mk & lt)) & (ADJ_RING - 1)] = e;
+            tail += __popc(mk);
+          }
+          __syncwarp();
+          while (tail - head >= 32) eval(32);
+        }
+        if (tail > head) eval(tail - head);
+        if (tail > 0) {
+          const double f = warp_sum2(fx, fy);
+          const double tx = __shfl_sync(0xffffffffu, f, 0), ty = __shfl_sync(0xffffffffu, f, 16);
+          if (lane == ii) {
+            gx = fma(kf, tx, gx);
+            gy = fma(kf, ty, gy);
+          }
         }
       }
-      __syncwarp();
-      unsigned long long rest[2];
-      const int nr = qn - k;
-      for (int r = 0; r < 2; ++r) rest[r] = (lane + 32 * r < nr) ? q[32 + lane + 32 * r] : 0ull;
-      __syncwarp();
-      for (int r = 0; r < 2; ++r)
-        if (lane + 32 * r < nr) q[lane + 32 * r] = rest[r];
-      __syncwarp();
-      qn = nr;
-    };
-    for (int i = warp; i < N; i += nwarps) {
-      Prefilter f;
-      f.init_q(row[i], d.q_lim_rc);
-      for (int b0 = i + 1; b0 < N; b0 += 32) {
-        const int b = b0 + lane;
-        const bool p = b < N && f.pass(row[b]);
-        const unsigned mk = __ballot_sync(0xffffffffu, p);
-        if (p) q[qn + __popc(mk & lt)] = ((unsigned long long)(unsigned)i << 32) | (unsigned)b;
-        qn += __popc(mk);
+      // ordered pairs: half of each sum
+      v[4] = 0.5 * h * se;
+      v[3] = d.g * v[4];
+      v[5] = 0.5 * h * (-2.0 * cg) * d.g * sr;
+    }
+    if (own) {
+      if (a.grad) {
+        double *o = a.grad + (a.cta_first ? d.host_off : 0) + ((size_t)j * N + me) * dim;
+        o[0] = gx;
+        if (dim > 1) o[1] = gy;
+      }
+      rg = dim > 1 ? fma(ay, gy, ax * gx) : ax * gx;
+    }
+  }
+  adjoint_part(a, v, rg, red);
+}
+
+// the same adjoint with every unordered pair evaluated once, for batches with
+// a CTA per (chain, slice) to spare: warp w takes the particles w, w + 4, ...
+// and their partners of higher index; the force goes to the particle by a
+// warp sum and to the partners through the warp's own accumulators in shared
+// memory (within a round of 32 the partners differ, so plain loads and stores
+// do; 64 N bytes for the four warps, summed at the end).  Half of the
+// gather's evaluations, at two more FP64 operations each.
+__global__ void __launch_bounds__(128) k_adjoint_slices(AdjArgs a) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  __shared__ ChainDesc d;
+  __shared__ int s_ch, s_lb;
+  __shared__ unsigned ring_s[4][ADJ_RING];
+  __shared__ double red[4][9];
+  adjoint_cta(a, a.cta_first, &d, &s_ch, &s_lb);
+  CV c = make_cv(&d, a.dpool, a.ipool, nullptr);
+  const int N = c.N, M = c.M, dim = c.dim, j = s_lb, jp = j ? j - 1 : M - 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int *inv = j ? nullptr : a.inv + (a.cta_first ? a.inv_off[s_ch] : 0);
+  const unsigned *row = c.xq + (size_t)j * c.ldn, *rowp = c.xq + (size_t)jp * c.ldn;
+  double2 *acc = reinterpret_cast<double2 *>(dsm) + (size_t)warp * N;
+  const bool pair = (d.flags & PF_PAIR) && N > 1;
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, rg = 0.0;
+  const double cg = d.inv2s2, h = 0.5 * d.tau;
+  const double kf = -2.0 * cg * h * d.g;  // the force's factor
+  if (pair) {
+    for (int b = lane; b < N; b += 32) acc[b] = make_double2(0.0, 0.0);
+    __syncwarp();
+    const unsigned lim_lo = d.q_lim_lo, lim_hi = d.q_lim_hi, lt = (1u << lane) - 1u;
+    unsigned *ring = ring_s[warp];
+    double se = 0.0, sr = 0.0;
+    for (int i = warp; i < N; i += 4) {
+      const double px = c.X(0, i, j), py = c.Xd(1, i, j);
+      const unsigned ci = row[i], pi = rowp[inv ? inv[i] : i];
+      double fx = 0.0, fy = 0.0;
+      int head = 0, tail = 0;
+      auto eval = [&](int k) {
+        if (lane < k) {
+          const unsigned e = ring[(head + lane) & (ADJ_RING - 1)];
+          const int b = (int)(e & 0xffffu);
+          const double dx = mi1(px, c.X(0, b, j), d.L, d.L2);
+          const double dy = dim > 1 ? mi1(py, c.X(1, b, j), d.L, d.L2) : 0.0;
+          double r2 = dx * dx;
+          if (dim > 1) r2 = fma(dy, dy, r2);
+          const int uses = adjoint_uses(c, d, e, r2, i, b, jp, inv);
+          if (uses) {
+            double w = exp_neg(-r2 * cg);
+            if (uses == 2) w += w;
+            se += w;
+            sr = fma(r2, w, sr);
+            fx = fma(w, dx, fx);
+            fy = fma(w, dy, fy);
+            double2 t = acc[b];
+            t.x = fma(-w, dx, t.x);
+            t.y = fma(-w, dy, t.y);
+            acc[b] = t;
+          }
+        }
+        head += k;
         __syncwarp();
-        if (qn >= 32) flush();
+      };
+      for (int b0 = (i + 1) & ~31; b0 < N; b0 += 64) {
+        unsigned wc[2], wp[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int b = b0 + 32 * u + lane;
+          wc[u] = b < N ? row[b] : 0u;
+          wp[u] = b < N ? rowp[inv ? inv[b] : b] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int b = b0 + 32 * u + lane;
+          unsigned e = 0u;
+          const bool p = b < N && b > i && adjoint_reach(ci, pi, wc[u], wp[u], lim_lo, lim_hi, b, e);
+          const unsigned mk = __ballot_sync(0xffffffffu, p);
+          if (p) ring[(tail + __popc(mk & lt)) & (ADJ_RING - 1)] = e;
+          tail += __popc(mk);
+        }
+        __syncwarp();
+        while (tail - head >= 32) eval(32);
+      }
+      if (tail > head) eval(tail - head);
+      if (tail > 0) {
+        const double f = warp_sum2(fx, fy);
+        const double ty = __shfl_sync(0xffffffffu, f, 16);
+        if (lane == 0) {
+          double2 t = acc[i];
+          t.x += f;
+          t.y += ty;
+          acc[i] = t;
+        }
+        __syncwarp();
       }
     }
-    while (qn > 0) flush();
+    v[4] = h * se;
+    v[3] = d.g * v[4];
+    v[5] = h * (-2.0 * cg) * d.g * sr;
   }
   __syncthreads();
-  // the external potential per bead, and the per-bead buffers in the
-  // chain's [i][j] order (k2 = i M + j)
-  for (int i = tid; i < N; i += nt) {
+  const double2 *all = reinterpret_cast<const double2 *>(dsm);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
     const double ax = c.X(0, i, j), ay = c.Xd(1, i, j);
-    double ge[2];
-    grad_vext(d, ax, ay, ge[0], ge[1]);
-    ge[0] *= tau;
-    ge[1] *= tau;
-    v[0] += tau * vext(d, ax, ay);
-    if (d.flags & PF_LATT) {
-      const double sx = sinpi(ax * d.lat_k), sy = dim > 1 ? sinpi(ay * d.lat_k) : 0.0;
-      v[1] += tau * (sx * sx + sy * sy);
+    double gx, gy;
+    adjoint_ext(d, ax, ay, gx, gy, v);
+    if (pair) {
+      const double2 t0 = all[i], t1 = all[N + i], t2 = all[2 * N + i], t3 = all[3 * N + i];
+      gx = fma(kf, (t0.x + t1.x) + (t2.x + t3.x), gx);
+      if (dim > 1) gy = fma(kf, (t0.y + t1.y) + (t2.y + t3.y), gy);
     }
-    if (d.flags & PF_HARM) v[2] += tau * a.omega[ch] * (ax * ax + ay * ay);
-    v[6] += ax * ge[0] + ay * ge[1];
-    const size_t k2 = (size_t)a.bead_off[ch] + (size_t)i * M + j;
-    a.gA[k2 * 2] = ge[0] + acc[i];
-    a.gA[k2 * 2 + 1] = ge[1] + acc[N + i];
-    a.gB[k2 * 2] = acc[2 * N + i];
-    a.gB[k2 * 2 + 1] = acc[3 * N + i];
+    if (a.grad) {
+      double *o = a.grad + (a.cta_first ? d.host_off : 0) + ((size_t)j * N + i) * dim;
+      o[0] = gx;
+      if (dim > 1) o[1] = gy;
+    }
+    rg += dim > 1 ? fma(ay, gy, ax * gx) : ax * gx;
   }
-  block_sum_k<8>(v, red);
-  if (tid == 0)
-    for (int q = 0; q < 8; ++q) a.part_s[(size_t)blockIdx.x * 8 + q] = v[q];
+  adjoint_part(a, v, rg, red);
 }
 
-// per bead the full gradient gA[k] + gB[prev(k)]: dS/dr (host layout
-// x[d][n][j] of the chain at desc.host_off, when requested) and r . dS/dr
-__global__ void __launch_bounds__(256) k_adjoint_finish_b(AdjBatchArgs a) {
+// totals[c][9]: the partial rows of chain c's CTAs summed
+__global__ void __launch_bounds__(256) k_adjoint_totals(AdjArgs a) {
   __shared__ double red[256];
-  __shared__ int ch, lb;
-  if (threadIdx.x == 0) {
-    ch = a.blk_chain[blockIdx.x];
-    lb = blockIdx.x - a.blk_first[ch];
-  }
-  __syncthreads();
-  const ChainDesc &d = a.desc[ch];
-  const int N = d.N, M = d.M, dim = d.dim;
-  const double *x = a.dpool + d.x_off;
-  const int k = lb * blockDim.x + threadIdx.x;  // k = i*M + j
-  double rg[1] = {0.0};
-  if (k < N * M) {
-    const int i = k / M, j = k % M;
-    const size_t base = (size_t)a.bead_off[ch];
-    const int kp = j > 0 ? k - 1 : a.inv[a.inv_off[ch] + i] * M + (M - 1);
-    for (int q = 0; q < dim; ++q) {
-      const double g = a.gA[(base + k) * 2 + q] + a.gB[(base + kp) * 2 + q];
-      if (a.dSdr) a.dSdr[(size_t)d.host_off + (size_t)q * N * M + k] = g;
-      rg[0] += x[((size_t)j * N + i) * dim + q] * g;
-    }
-  }
-  block_sum_k<1>(rg, red);
-  if (threadIdx.x == 0) a.part[(size_t)blockIdx.x * 9 + 8] = rg[0];
-}
-
-// totals[c][9]: the partial rows of chain c's blocks summed (its slice CTAs'
-// rows when the slice kernel ran)
-__global__ void __launch_bounds__(256) k_adjoint_totals_b(AdjBatchArgs a) {
-  __shared__ double red[256];
-  const int ch = blockIdx.x;
-  const int b0 = a.blk_first[ch];
-  const int b1 = ch + 1 < a.nchains ? a.blk_first[ch + 1] : a.nblocks;
+  const int ch = a.cta_first ? (int)blockIdx.x : 0;
+  const int b0 = a.cta_first ? a.cta_first[ch] : 0, b1 = a.cta_first ? a.cta_first[ch + 1] : a.nctas;
   double t[8] = {0, 0, 0, 0, 0, 0, 0, 0}, r[1] = {0.0};
   for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
-    if (!a.use_slices)
-      for (int q = 0; q < 8; ++q) t[q] += a.part[(size_t)b * 9 + q];
+    for (int q = 0; q < 8; ++q) t[q] += a.part[(size_t)b * 9 + q];
     r[0] += a.part[(size_t)b * 9 + 8];
-  }
-  if (a.use_slices) {
-    const int s0 = a.slice_first[ch], s1 = s0 + a.desc[ch].M;
-    for (int b = s0 + threadIdx.x; b < s1; b += blockDim.x)
-      for (int q = 0; q < 8; ++q) t[q] += a.part_s[(size_t)b * 8 + q];
   }
   block_sum_k<8>(t, red);
   block_sum_k<1>(r, red);
@@ -695,8 +731,8 @@ cudaError_t launch_transpose_tiles(bool import, const ChainDesc *desc, double *d
                                    double *host, const int *tile_off, int c_lo, int c_hi,
                                    int ntiles, int grid, cudaStream_t s) {
   const int g = std::max(1, std::min(grid, ntiles));
-  if (import) k_transpose_tiles<true><<<g, 256, 0, s>>>(desc, dpool, host, tile_off, c_lo, c_hi);
-  else k_transpose_tiles<false><<<g, 256, 0, s>>>(desc, dpool, host, tile_off, c_lo, c_hi);
+  if (import) k_transpose_tiles<true><<<g, 256, 0, s>>>(desc, dpool, host, tile_off, c_lo, c_hi, nullptr);
+  else k_transpose_tiles<false><<<g, 256, 0, s>>>(desc, dpool, host, tile_off, c_lo, c_hi, nullptr);
   return cudaGetLastError();
 }
 cudaError_t launch_init_world(const ChainDesc *desc, double *dpool, int *ipool, int chain0,
@@ -966,8 +1002,8 @@ cudaError_t fp64_peak(int num_sms, cudaStream_t st, double *tflops) {
 // ---------------------------------------------------------------------------
 // adjoint scratch in static device memory (pimc_adjoint_noalloc): room for a
 // chain of up to kNoAllocBeads beads and kNoAllocParticles particles in the
-// layout of the allocating adjoint (gA, gB, partials, totals, dS/dr, inverse
-// permutation), 3.2 MB per device
+// layout of the allocating adjoint (dS/dr in both layouts, partials, totals,
+// inverse permutation), 3.2 MB per device
 // ---------------------------------------------------------------------------
 static __device__ __align__(256) double g_adj_static[kNoAllocDoubles];
 
@@ -1044,27 +1080,33 @@ cudaError_t check_word_take(cudaStream_t s, unsigned long long *w) {
   return e;
 }
 
-cudaError_t launch_adjoint_batch(const AdjBatchArgs &a, int maxN, cudaStream_t s) {
-  dim3 gi((unsigned)std::max(1, (maxN + 255) / 256), (unsigned)a.nchains);
-  k_adjoint_inv_b<<<gi, 256, 0, s>>>(a);
-  if (a.use_slices) {
-    const size_t sm = 32 * (size_t)maxN;
-    cudaError_t e = cudaFuncSetAttribute(k_adjoint_slice_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    k_adjoint_slice_b<<<a.nslices, 256, sm, s>>>(a);
-  } else {
-    k_adjoint_beads_b<<<a.nblocks, 256, 0, s>>>(a);
-  }
-  k_adjoint_finish_b<<<a.nblocks, 256, 0, s>>>(a);
-  k_adjoint_totals_b<<<a.nchains, 256, 0, s>>>(a);
-  return cudaGetLastError();
+// ADJ_SLICES (a CTA per slice, every pair once) when the slices give every SM
+// at least four CTAs and the accumulators of the largest chain fit the shared
+// memory; else the gather, with as many particles per warp as still make
+// sixteen warps per SM, from 32 down to 8, so that a small chain spreads over
+// the SMs
+int adjoint_ib(long long slices, long long rows32, int maxN, int num_sms, int max_dyn_smem) {
+  if (slices >= 4LL * num_sms && 64LL * maxN + 8192 <= max_dyn_smem) return ADJ_SLICES;
+  const long long want = 16LL * num_sms;
+  return rows32 >= want ? 32 : (2 * rows32 >= want ? 16 : 8);
 }
 
-cudaError_t launch_adjoint(const AdjArgs &a, int nbeads, cudaStream_t s) {
-  const int nb = (nbeads + 255) / 256;
-  k_inverse_next<<<4, 256, 0, s>>>(a);
-  k_adjoint_beads<<<nb, 256, 0, s>>>(a);
-  k_adjoint_finish<<<nb, 256, 0, s>>>(a);
+cudaError_t launch_adjoint(const AdjArgs &a, int maxN, const int *tile_off, int ntiles, double *dSdr,
+                           cudaStream_t s) {
+  const int nc = a.cta_first ? a.nchains : 1;
+  k_adjoint_inv<<<dim3((maxN + 255) / 256, nc), 256, 0, s>>>(a);
+  if (a.ib == ADJ_SLICES) {
+    const size_t sm = 64 * (size_t)maxN;
+    const cudaError_t e = cudaFuncSetAttribute(k_adjoint_slices, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k_adjoint_slices<<<a.nctas, 128, sm, s>>>(a);
+  } else {
+    k_adjoint_gather<<<a.nctas, 128, 0, s>>>(a);
+  }
+  k_adjoint_totals<<<nc, 256, 0, s>>>(a);
+  if (dSdr)
+    k_transpose_tiles<false><<<std::max(1, std::min(ntiles, 4096)), 256, 0, s>>>(
+        a.desc, a.dpool, dSdr, tile_off, tile_off ? 0 : a.chain, tile_off ? a.nchains : a.chain + 1, a.grad);
   return cudaGetLastError();
 }
 

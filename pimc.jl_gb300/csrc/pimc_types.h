@@ -40,6 +40,7 @@ struct ChainDesc {
   int wtab;         // bridge-coefficient table covers windows m < wtab
   double L, tau, lambda, beta;
   double hcoef, V0, lat_k;
+  double omega;         // trap frequency (hcoef = omega^2 / 2; the adjoint's d/domega)
   double g, inv2s2, rc, hard_a, mu;
   double dens_bw;
   double L2;            // 2L

@@ -36,3 +36,68 @@ def test_contact_table_in_several_ranges_of_nodes(engine_lib):
     big = contact_table(2.0, 1.0 / 2000, 13.0, 601)
     small = contact_table(2.0, 1.0 / 2000, 13.0, 4)
     np.testing.assert_allclose(big[::200, ::200], small, rtol=0, atol=1e-11 * np.abs(small).max())
+
+
+def _adjoint_reference(x, nxt, T, L, omega, V0, g, sigma, r_a, pair):
+    """dS/dr and dS/d(V0, omega, g) of the potential action in FP64 numpy"""
+    dim, N, M = x.shape
+    tau, h, c = 1.0 / (T * M), 0.5 / (T * M), 0.5 / sigma ** 2
+    grad = tau * (omega ** 2 * x + V0 * np.pi * np.sin(2 * np.pi * x))
+    th = np.array([tau * np.sum(np.sin(np.pi * x) ** 2) if V0 else 0.0, tau * omega * np.sum(x * x), 0.0])
+    if pair:
+        rc = 2 * L / np.floor(2 * L / r_a)
+        for j in range(M):
+            jn, own = (j + 1) % M, nxt if j == M - 1 else np.arange(N)
+            for a, rows in ((x[:, :, j], None), (x[:, own, jn], own)):
+                d = a[:, :, None] - a[:, None, :]
+                d -= 2 * L * np.round(d / (2 * L))
+                first = x[:, :, j][:, :, None] - x[:, :, j][:, None, :]
+                first -= 2 * L * np.round(first / (2 * L))
+                on = (np.sum(first ** 2, 0) <= rc * rc) & ~np.eye(N, dtype=bool)
+                e = on * np.exp(-c * np.sum(d * d, 0))
+                th[2] += 0.5 * h * e.sum()
+                f = (-2 * c * h * g) * np.sum(e * d, axis=2)
+                if rows is None:
+                    grad[:, :, j] += f
+                else:
+                    np.add.at(grad, (slice(None), rows, jn), f)
+    return grad, th
+
+
+@pytest.mark.parametrize("N,M,dim,pair", [(1, 4, 2, True), (2, 5, 2, True), (7, 9, 1, True), (8, 6, 2, False),
+                                          (9, 33, 2, True), (31, 8, 2, True), (32, 8, 1, True),
+                                          (33, 40, 2, True), (200, 65, 2, True), (300, 70, 1, True)])
+def test_adjoint_gather_edges(N, M, dim, pair, engine_lib):
+    """the adjoint around its blocks of particles and rings of 32 pairs, crowded
+    and sparse, alone (a warp per particles of a slice) and in a batch of at
+    least 700 slices (a CTA per slice), against FP64 numpy.  A force sums at most 2 N terms no larger than the largest force's
+    scale, each with a few rounding errors: 1e-12 of that scale"""
+    from pimc.engine import ChainParams, Engine
+    rng = np.random.default_rng(N * 100 + M)
+    kw = dict(dim=dim, N=N, M=M, L=4.0, T=0.5, lam=0.5, harmonic_omega=0.7, lattice_V0=1.5,
+              lattice_a=1.0, interactions=pair, pair_g=1.3, pair_sigma=0.5, r_a=1.2, semantics=1)
+    for spread in (0.4, 2.0):
+        x = np.clip(rng.normal(scale=spread, size=(dim, N, M)), -3.99, 3.99)
+        nxt = rng.permutation(N).astype(np.int32)
+        e = Engine([ChainParams(**kw)] + [ChainParams(**dict(kw, N=3)) for _ in range(700 // M + 1)])
+        e.set_beads(x)
+        e.set_next(nxt)
+        want, th_want = _adjoint_reference(x, nxt, 0.5, 4.0, 0.7, 1.5, 1.3, 0.5, 1.2, pair)
+        scale = np.abs(want).max()
+        g, th, _ = e.adjoint(0)
+        gb, thb, _ = e.batch_adjoint(want_beads=True)
+        for got, t in ((g, th), (gb[0], thb[0])):
+            np.testing.assert_allclose(got, want, rtol=0, atol=1e-12 * scale)
+            np.testing.assert_allclose(t, th_want, rtol=1e-12, atol=1e-13)
+        e.close()
+
+
+def test_batch_adjoint_follows_a_new_trap(engine_lib):
+    """dS/domega after set_potential uses the new frequency"""
+    from pimc.engine import ChainParams, Engine
+    e = Engine([ChainParams(dim=2, N=5, M=8, L=4.0, T=1.0, lam=0.5, harmonic_omega=1.0, seed=i) for i in range(2)])
+    e.batch_adjoint()
+    e.set_potential(0.0, 0.5, 0.0, chain=1)
+    _, th, _ = e.batch_adjoint()
+    _, one, _ = e.adjoint(1)
+    np.testing.assert_allclose(th[1], one, rtol=1e-13)
