@@ -123,22 +123,39 @@ __device__ __forceinline__ double u53(unsigned a, unsigned b) {
   return (double)x * 0x1.0p-53;
 }
 
+// x 2^-53 of an integer x <= 2^53, rounded to the nearest float.  The 64-bit
+// integer conversion would take the FP64 pipe's 16 cycles per warp; here the
+// leading 32 bits, their last bit set when anything lies below, go through the
+// 32-bit conversion, which then rounds as the whole integer would.
+__device__ __forceinline__ float u53_float(unsigned long long x) {
+  const int lz = __clzll((long long)x);
+  const unsigned long long y = x << (lz & 63);
+  const unsigned top = (unsigned)(y >> 32) | ((unsigned)y != 0u);
+  return __uint2float_rn(top) * __int_as_float((127 + 32 - 53 - lz) << 23);
+}
+
 // Box-Muller pair from two 53-bit uniforms.  The transcendental functions
 // run in FP32 (CUDA's logf / sincospif / sqrtf as library calls): the FP64
 // pipe of this part issues 2 lanes per SM clock, and a normal's relative
 // error of about 1e-7 distorts the sampled Gaussian far below any Monte Carlo
 // error.  u1 keeps its 53-bit range (as a float, exponent intact), so the
 // tails reach 8.6 sigma.  Injected-draw attempts take their normals as given.
-__device__ __forceinline__ void normal2(uint4 r, double &z0, double &z1) {
+__device__ __forceinline__ void normal2f(uint4 r, float &z0, float &z1) {
   const unsigned long long x1 = ((((unsigned long long)r.x) << 32) | r.y) >> 11;
   const unsigned long long x2 = ((((unsigned long long)r.z) << 32) | r.w) >> 11;
-  const float u1 = __ull2float_rn((1ull << 53) - x1) * 0x1.0p-53f;  // (0, 1]
-  const float u2 = __ull2float_rn(x2) * 0x1.0p-53f;                 // [0, 1]
+  const float u1 = u53_float((1ull << 53) - x1);  // (0, 1]
+  const float u2 = u53_float(x2);                 // [0, 1]
   const float rad = sqrtf(-2.f * logf(u1));
   float s, c;
   sincospif(2.f * u2, &s, &c);
-  z0 = (double)(rad * c);
-  z1 = (double)(rad * s);
+  z0 = rad * c;
+  z1 = rad * s;
+}
+__device__ __forceinline__ void normal2(uint4 r, double &z0, double &z1) {
+  float a, b;
+  normal2f(r, a, b);
+  z0 = (double)a;
+  z1 = (double)b;
 }
 
 struct Stream {
@@ -182,6 +199,10 @@ struct GenDraws {
     normal2(s.at((unsigned)k), a, b);
     z[0] = a;
     if (dim > 1) z[1] = b;
+  }
+  // the same normals as the floats they are
+  __device__ __forceinline__ void bead_normals_f(int k, float &a, float &b) const {
+    normal2f(s.at((unsigned)k), a, b);
   }
   __device__ __forceinline__ void consumed(int) {}
   __device__ __forceinline__ double normal() {
@@ -530,19 +551,30 @@ __device__ __forceinline__ double dist1(double a, double b, double L) {
   return o < dx ? o : dx;
 }
 
+// |x| > y, y >= 0, on the bits: a double compare takes the FP64 pipe's 16
+// cycles per warp, an integer one does not (a NaN x counts as greater)
+__device__ __forceinline__ bool abs_gt(double x, double y) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > __double_as_longlong(y);
+}
+
 // teleport(x, L) = (x+L) - floor(x/2L + 1/2) 2L - L (src/propagator.jl:30-32).
 // The quotient is formed by a multiplication; when it lands within 1e-9 of an
 // integer the IEEE division of the reference is used instead, so the floor is
 // always the reference's.
 // Inside the box the floor is 0 and the result is (x + L) - L, the same bits
 // as the full expression; that path skips the floor and its guard.
-__device__ __forceinline__ double teleport(double x, double L, double inv2L) {
-  if (fabs(x) < 0.999999 * L) return (x + L) - L;
+// (out of line past the box: its division would otherwise be evaluated ahead
+// of the test)
+static __device__ __noinline__ double teleport_far(double x, double L, double inv2L) {
   const double q = x * inv2L + 0.5;
   double f = floor(q);
   const double fr = q - f;
   if (fr < 1e-9 || fr > 1.0 - 1e-9) f = floor(x / (2.0 * L) + 0.5);
   return (x + L) - f * (2.0 * L) - L;
+}
+__device__ __forceinline__ double teleport(double x, double L, double inv2L) {
+  if (fabs(x) < 0.999999 * L) return (x + L) - L;
+  return teleport_far(x, L, inv2L);
 }
 
 // teleport in the sweeps (SWEEP): a coordinate inside the box is kept as it
@@ -552,8 +584,8 @@ __device__ __forceinline__ double teleport(double x, double L, double inv2L) {
 // the reference's bits.
 template <bool SWEEP>
 __device__ __forceinline__ double teleport_s(double x, double L, double inv2L) {
-  if (SWEEP && fabs(x) < L) return x;
-  return teleport(x, L, inv2L);
+  if (SWEEP && !abs_gt(x, L) && __double_as_longlong(fabs(x)) != __double_as_longlong(L)) return x;
+  return teleport_far(x, L, inv2L);
 }
 
 __device__ __forceinline__ double sgn(double v) { return v > 0.0 ? 1.0 : (v < 0.0 ? -1.0 : 0.0); }
@@ -674,10 +706,15 @@ __device__ __forceinline__ double lnU2(const ChainDesc &d, double r2a, double r2
 // bridge coefficients alpha_t = (m-t)/(m+1-t), sigma_t = sqrt(2 lambda alpha tau)
 // (src/updates/helper.jl:154,165); tabulated per chain with the same
 // expression for m < wtab
+// (the untabulated form out of line: inlined, the compiler evaluates its
+// divisions and root beside the table read, some forty FP64 instructions)
+static __device__ __noinline__ double2 bridge_coef_far(double lambda, double tau, int m, int t) {
+  const double a = (double)(m - t) / (double)(m + 1 - t);
+  return make_double2(a, sqrt(2.0 * lambda * a * tau));
+}
 __device__ __forceinline__ double2 bridge_coef(const CV &c, int m, int t) {
   if (m < c.d->wtab) return c.tab[m * c.d->wtab + t];
-  const double a = (double)(m - t) / (double)(m + 1 - t);
-  return make_double2(a, sqrt(2.0 * c.d->lambda * a * c.d->tau));
+  return bridge_coef_far(c.d->lambda, c.d->tau, m, t);
 }
 
 // the sweeps' closed form of the same bridge.  With q_t = p_t - e and
@@ -687,17 +724,14 @@ __device__ __forceinline__ double2 bridge_coef(const CV &c, int m, int t) {
 // a prefix sum in place of the recursion (two FP64 operations a coordinate
 // per bead, or a plain scan across lanes).  bridge_w(c, m, t) = (w_t, m-t)
 // for t >= 1 and (1/m, m) for t = 0; tabulated per chain for m < wtab
-__device__ __forceinline__ double2 bridge_w(const CV &c, int m, int t) {
-  if (m < c.d->wtab) return c.tabw[m * c.d->wtab + t];
+static __device__ __noinline__ double2 bridge_w_far(double lambda, double tau, int m, int t) {
   if (t == 0) return make_double2(1.0 / m, (double)m);
   const double a = (double)(m - t) / (double)(m + 1 - t);
-  return make_double2(sqrt(2.0 * c.d->lambda * a * c.d->tau) / (m - t), (double)(m - t));
+  return make_double2(sqrt(2.0 * lambda * a * tau) / (m - t), (double)(m - t));
 }
-
-// |x| > y, y >= 0, on the bits: a double compare takes the FP64 pipe's 16
-// cycles per warp, an integer one does not (a NaN x counts as greater)
-__device__ __forceinline__ bool abs_gt(double x, double y) {
-  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > __double_as_longlong(y);
+__device__ __forceinline__ double2 bridge_w(const CV &c, int m, int t) {
+  if (m < c.d->wtab) return c.tabw[m * c.d->wtab + t];
+  return bridge_w_far(c.d->lambda, c.d->tau, m, t);
 }
 
 // minimum-image difference a - b: the same magnitude as dist1 (|a-b| when it

@@ -70,22 +70,46 @@ __device__ __forceinline__ int warp_min_int(int v) {
   return v;
 }
 
+// the choices of 32 consecutive swaps of a sweep, drawn together: a lane per
+// swap, so that their FP64 products take full warps
+constexpr int SWAP_DRAWS = 32;
+struct SwapDraws {
+  int j0[SWAP_DRAWS], m[SWAP_DRAWS], n1[SWAP_DRAWS];
+  float up[SWAP_DRAWS];  // the partner choice's uniform
+  float lu[SWAP_DRAWS];  // log of the Metropolis uniform (-inf for 0)
+};
+// partial sums of one swap: per bridge the pair-free change of the action, in
+// FP64 and as a float; per warp the pair estimate and its bound
+struct SwapSums {
+  double p[2];
+  float pf[2];
+  float est[16][2];
+};
+// weights of particle chunks at an odd stride (no bank conflicts for the lanes'
+// sequential sums): room for two buffers of 32 * (chunk | 1) floats
+constexpr int SWAP_WPAD = 64;
+__host__ __device__ inline int swap_wstride(int N) { return 32 * (((N + 31) / 32) | 1); }
+
 // shared scratch of the swap
 struct SwapScratch {
-  double *w;                                   // N heat-bath weights
+  double *w;                                   // N heat-bath weights (sweeps: two buffers of
+                                               // swap_wstride floats)
   double *r1x, *r1y, *r2x, *r2y, *vb1, *vb2;   // WMAX+1 each
   double *z;                                   // 4*WMAX normals
   unsigned long long *q;                       // PQ_CAP neighbour queue per warp
   unsigned *q1, *q2;                           // WMAX+1 mirror words each
   int *iv;                                     // 4 ints: group broadcasts
+  SwapSums *sums;                              // a sweep's partial sums
+  SwapDraws *draws;                            // a sweep's next choices
   static __host__ __device__ size_t bytes(int N, int nwarps) {
-    return sizeof(double) * ((size_t)N + 6 * (WMAX + 1) + 4 * WMAX) +
+    return sizeof(double) * ((size_t)N + SWAP_WPAD + 6 * (WMAX + 1) + 4 * WMAX) +
            sizeof(unsigned long long) * PQ_CAP * (size_t)nwarps +
-           sizeof(unsigned) * 2 * (WMAX + 1) + sizeof(int) * 4;
+           sizeof(unsigned) * 2 * (WMAX + 1) + sizeof(int) * 4 + sizeof(SwapDraws) +
+           sizeof(SwapSums);
   }
   __device__ void carve(void *base, int N, int nwarps) {
     double *p = (double *)base;
-    w = p; p += N;
+    w = p; p += N + SWAP_WPAD;
     r1x = p; p += WMAX + 1; r1y = p; p += WMAX + 1;
     r2x = p; p += WMAX + 1; r2y = p; p += WMAX + 1;
     vb1 = p; p += WMAX + 1; vb2 = p; p += WMAX + 1;
@@ -94,6 +118,8 @@ struct SwapScratch {
     q1 = (unsigned *)(q + (size_t)PQ_CAP * nwarps);
     q2 = q1 + (WMAX + 1);
     iv = (int *)(q2 + (WMAX + 1));
+    sums = (SwapSums *)(iv + 4);  // 8-byte aligned: an even count of words above
+    draws = (SwapDraws *)(sums + 1);
   }
 };
 
@@ -940,6 +966,524 @@ template <bool FAST, class D>
 __device__ int swap_warp(const CV &c, int j0, int m, int n1, double u_pick, D &dr,
                          SwapScratch &S, double *prop, int *n2_out) {
   return swap_group<true, FAST>(c, j0, m, n1, u_pick, dr, S, nullptr, prop, n2_out);
+}
+
+// ---------------------------------------------------------------------------
+// the same swap in the sweeps (generator draws, no hard core, windows of at
+// most SWAP_LANES links, so that a warp holds a bridge's beads, one a lane).
+//
+// What bounds it: a chain's swaps follow one another, so an attempt's latency
+// counts, and FP64: a warp instruction takes one of the SM's four FP64 pipes
+// for 64 cycles, whatever its active lanes.  So
+//  - warp b forms bridge b, both coordinates at once in its half warps (m <=
+//    17), with its potentials and its sum of link changes; no other warp
+//    repeats FP64 work, compares run on the bits, and sums meet as floats;
+//  - decisions compare in FP32 with margins that cover every rounding; inside
+//    the margin the exact FP64 sums and exp decide, so the outcome is the FP64
+//    formula's (decide_f);
+//  - every warp searches the partner from the shared weights (no broadcast);
+//    weights and normals are double-buffered, so that a skipped or rejected
+//    attempt needs no closing barrier;
+//  - the choices of 32 swaps are drawn at once, a lane each;
+//  - rarely taken FP64 code (untabulated bridges, far teleports, unwrapped
+//    ends) is out of line: inlined, the compiler evaluates it beside the
+//    common case, and an instruction of no active lane costs as much.
+// Against swap_group, whose FP64 work every warp of the CTA repeated (cycles of
+// an attempt, then whole calls): 4096 uneven chains, CTAs of 64 threads 40 k
+// -> 22 k, 34.5 -> 28.4 ms; 768 chains of at most 48 particles 6.75 -> 4.13 ms;
+// one chain of 64 free particles under the physical rules 22 k -> 7.3 k, 4.26
+// -> 1.81 ms.
+// ---------------------------------------------------------------------------
+constexpr int SWAP_LANES = 31;
+
+// choices of swaps a0 .. a0 + 31 of a sweep, by one warp
+__device__ __forceinline__ void swap_draws(SwapDraws &D, const ChainDesc &d, unsigned long long sweep, int a0,
+                                           int n, int M, int N, int mmax, int sm) {
+  const int lane = threadIdx.x & 31;
+  if (a0 + lane < n) {
+    const Stream ss = make_stream(d, sweep, PH_SWAP, (unsigned)(a0 + lane));
+    const uint4 r0 = ss.at(DRAW_CHOICE), r1 = ss.at(DRAW_CHOICE + 1);
+    D.j0[lane] = min(M - 1, (int)(u53(r0.x, r0.y) * M));
+    D.m[lane] = min(mmax, 2 + (int)(u53(r0.z, r0.w) * (sm - 1)));
+    D.n1[lane] = min(N - 1, (int)(u53(r1.x, r1.y) * N));
+    D.up[lane] = (float)u53(r1.z, r1.w);
+    const double u = ss.uni(DRAW_ACCEPT);
+    D.lu[lane] = u > 0.0 ? logf((float)u) : -INFINITY;
+  }
+}
+
+// the Metropolis decision of a log ratio known to lie in [s - r, s + r], from
+// lu = log u: 1 accept, 0 reject, -1 undecided.  The margin covers logf and
+// the roundings of u, s and r (floats: 6e-8 each); lu = -inf is undecided.
+__device__ __forceinline__ int decide_f(float s, float r, float lu) {
+  const float mg = r * 1.00001f + 1e-5f * (1.f + fabsf(lu)) + 1e-6f * fabsf(s);
+  if (s - mg > lu && lu > -3e38f) return 1;
+  if (s + mg < lu) return 0;
+  return -1;
+}
+
+// a bridge's end e taken to the start s's side of the periodic box; returns
+// s - e (out of line: rarely taken, five FP64 instructions otherwise)
+static __device__ __noinline__ double2 unwrap_end_far(double s, double e, double L) {
+  e += sgn(s) * (2.0 * L);
+  return make_double2(s - e, e);
+}
+__device__ __forceinline__ double unwrap_end(double s, double &e, double L) {
+  const double2 r = unwrap_end_far(s, e, L);
+  e = r.y;
+  return r.x;
+}
+
+template <bool WARP, int SPEC>
+__device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, unsigned wmagic, SwapScratch &S,
+                          double *red) {
+  using G = Group<WARP>;
+  const ChainDesc &d = *c.d;
+  constexpr bool GEN = SPEC == SWAP_ANY;
+  const bool f_phys = GEN && (d.flags & PF_PHYS), f_contact = GEN && (d.flags & PF_CONTACT);
+  const bool pair = (d.flags & PF_PAIR) != 0;
+  const int N = c.N, M = c.M, dim = c.dim, lane = threadIdx.x & 31;
+  const int tid = G::rank(), nt = G::size();
+  const int warp = WARP ? 0 : (int)(threadIdx.x >> 5), nwarps = WARP ? 1 : (int)(blockDim.x >> 5);
+  const int slot = a & (SWAP_DRAWS - 1), buf = a & 1;
+  const int j0 = S.draws->j0[slot], m = S.draws->m[slot], n1 = S.draws->n1[slot];
+  const float lu = S.draws->lu[slot];
+  if (!check_ok(m >= 2 && m <= SWAP_LANES && m < M && j0 >= 0 && j0 < M, DERR_WINDOW, d) ||
+      !check_ok(n1 >= 0 && n1 < N, DERR_INDEX, d))
+    return RES_SKIP;
+  PROF_DECL;
+  PROF_COUNT(0);
+  HeatBath<true> hb;
+  hb.c = &c;
+  hb.j0 = j0;
+  hb.wrap = (j0 + m) >= M;
+  hb.se = hb.wrap ? j0 + m - M : j0 + m;
+  hb.inv_den = 0.0;
+  hb.inv_denf = d.hb_unit / (float)m;
+  const int se = hb.se;
+  const bool wrap = hb.wrap;
+  const unsigned Aq = c.Q(n1, j0);
+  const int e1p = hb.endp(n1);
+  const unsigned E1q = c.Q(e1p, se);
+  GenDraws dr = gen_draws(ss);
+  float *Sw = reinterpret_cast<float *>(S.w) + buf * wstride;
+  float *Sz = reinterpret_cast<float *>(S.z) + buf * (4 * WMAX);
+  // the bridges' normals depend on the move's stream alone
+  for (int k = tid; k < 2 * (m - 1); k += nt) {
+    float z0, z1;
+    dr.bead_normals_f(k, z0, z1);
+    Sz[2 * k] = z0;
+    Sz[2 * k + 1] = z1;
+  }
+  // heat-bath weights, four candidates per thread at a time (swap_group): lane
+  // l's chunk of particles starts at l * (chunk | 1)
+  const int chunk = (N + 31) / 32;
+  auto widx = [&](int i) { return (chunk & 1) ? i : i + (int)__umulhi((unsigned)i, wmagic); };
+  {
+    constexpr int U = 4;
+    for (int i0 = tid; i0 < N; i0 += U * nt) {
+      int ie[U];
+      unsigned qa[U], qe[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * nt;
+        ie[u] = i < N ? (wrap ? c.next[i] : i) : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * nt;
+        qa[u] = i < N ? c.Q(i, j0) : 0u;
+        qe[u] = i < N ? c.Q(ie[u], se) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * nt;
+        if (i < N) {
+          const float s2 = (float)qdist2(Aq, qe[u]) + (float)qdist2(qa[u], E1q);
+          Sw[widx(i)] = __expf(-s2 * hb.inv_denf);
+        }
+      }
+    }
+  }
+  G::sync();
+  PROF_MARK(0);
+  // the partner, by every warp: sums over the lanes' chunks in particle order,
+  // then the first particle whose cumulative weight reaches u times the sum
+  float wmax = 0.f, ssum;
+  int n2;
+  {
+    const int i0 = min(N, lane * chunk), i1 = min(N, i0 + chunk);
+    float *mine = Sw + lane * (chunk | 1);
+    const int len = i1 - i0;
+    float ls = 0.f;
+    for (int k = 0; k < len; ++k) ls += mine[k];
+    ssum = warp_sum(ls);
+    if (!(ssum > 0.f)) {
+      // every weight underflowed: exponents shifted by their largest.  One warp
+      // rewrites the weights, between barriers every warp reaches (ssum is
+      // the same for all)
+      if (!WARP) __syncthreads();
+      if (warp == 0) {
+        const HBead A{0.0, 0.0, Aq}, E{0.0, 0.0, E1q};
+        float mx = -INFINITY;
+        for (int k = 0; k < len; ++k) {
+          const float v = hb.expo(i0 + k, A, E);
+          mine[k] = v;
+          mx = v > mx ? v : mx;
+        }
+        wmax = warp_max(mx);
+        for (int k = 0; k < len; ++k) mine[k] = hb.ex_(mine[k] - wmax);
+        if (lane == 0) S.sums->pf[0] = wmax;
+      }
+      G::sync();
+      wmax = S.sums->pf[0];
+      ls = 0.f;
+      for (int k = 0; k < len; ++k) ls += mine[k];
+      ssum = warp_sum(ls);
+      G::sync();
+    }
+    const float target = S.draws->up[slot] * ssum;
+    float cw = warp_exclusive_scan(ls);
+    int cand = 0x7fffffff;
+    for (int k = 0; k < len; ++k) {
+      cw += mine[k];
+      if (cw >= target) { cand = i0 + k; break; }
+    }
+    n2 = __reduce_min_sync(0xffffffffu, (unsigned)cand);
+    if (n2 >= N || n2 < 0) n2 = N - 1;
+  }
+  PROF_MARK(1);
+  if (n2 == n1) {
+    PROF_COUNT(1);
+    return RES_SKIP;
+  }
+  const int nx1 = c.next[n1], nx2 = c.next[n2];
+  const int e2p = wrap ? nx2 : n2;
+  auto own = [&](int b, int t) { return j0 + t < M ? (b ? n2 : n1) : (b ? nx2 : nx1); };
+  auto slc = [&](int t) { return (j0 + t < M) ? j0 + t : j0 + t - M; };
+
+  // the physical rules' partner-choice ratio (swap_group): its sums now, in
+  // FP32; its logarithms in FP32 with a bound, in FP64 only for an exact
+  // decision
+  float mx3[3] = {0.f, 0.f, 0.f}, s34[4] = {0.f, 0.f, 0.f, 0.f};
+  float lrf = 0.f, lre = 0.f;
+  if (f_phys) {
+    const HBead A{0.0, 0.0, Aq}, E1{0.0, 0.0, E1q};
+    const HBead B{0.0, 0.0, c.Q(n2, j0)}, E2{0.0, 0.0, c.Q(e2p, se)};
+    auto expo_p = [&](int i, const HBead &s_, const HBead &f_) {
+      if (i != n1 && i != n2) return hb.expo(i, s_, f_);
+      return hb.expo(i, s_, f_, i == n1 ? &E2 : &E1);
+    };
+    float mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int i = tid; i < N; i += nt) {
+      const float a0 = hb.expo(i, B, E2), a1 = expo_p(i, A, E2), a2 = expo_p(i, B, E1);
+      mx[0] = a0 > mx[0] ? a0 : mx[0];
+      mx[1] = a1 > mx[1] ? a1 : mx[1];
+      mx[2] = a2 > mx[2] ? a2 : mx[2];
+    }
+    G::template max<3>(mx, red);
+    for (int i = tid; i < N; i += nt) {
+      s34[0] += hb.ex_(hb.expo(i, B, E2) - mx[0]);
+      s34[1] += hb.ex_(expo_p(i, A, E2) - mx[1]);
+      s34[2] += hb.ex_(expo_p(i, B, E1) - mx[2]);
+    }
+    // S_1 rides along in the fourth slot
+    s34[3] = tid == 0 ? ssum : 0.f;
+    G::template sum<4>(s34, red);
+    for (int k = 0; k < 3; ++k) mx3[k] = mx[k];
+    const float l1 = wmax + logf(s34[3]), l2 = mx[0] + logf(s34[0]);
+    const float l1p = mx[1] + logf(s34[1]), l2p = mx[2] + logf(s34[2]);
+    const float hp = fmaxf(-l1p, -l2p), ho = fmaxf(-l1, -l2);
+    lrf = (hp + log1pf(__expf(-fabsf(l1p - l2p)))) - (ho + log1pf(__expf(-fabsf(l1 - l2))));
+    lre = 2e-6f * (2.f + fabsf(l1) + fabsf(l2) + fabsf(l1p) + fabsf(l2p));
+  }
+  auto log_ratio = [&]() -> double {  // as swap_group's
+    if (!f_phys) return 0.0;
+    const double l1 = (double)wmax + log((double)s34[3]), l2 = (double)mx3[0] + log((double)s34[0]);
+    const double l1p = (double)mx3[1] + log((double)s34[1]), l2p = (double)mx3[2] + log((double)s34[2]);
+    return logaddexp(-l1p, -l2p) - logaddexp(-l1, -l2);
+  };
+  PROF_MARK(2);
+
+  // bridge b by warp b (one warp: both in turn): closed form (bridge_w), new
+  // beads, potentials and links, one bead a lane
+  const double L = d.L, inv2L = d.inv2L, mhtau = -0.5 * d.tau;
+  const double2 *bw = c.tabw + m * d.wtab;  // m <= M - 1 and m <= 32: always tabulated
+  if (tid == 0) S.iv[3] = 0;
+  for (int b = warp; b < 2; b += nwarps) {
+    double *rx = b ? S.r2x : S.r1x, *ry = b ? S.r2y : S.r1y, *vb = b ? S.vb2 : S.vb1;
+    unsigned *qb = b ? S.q2 : S.q1;
+    const int ns = b ? n2 : n1, ne = b ? e1p : e2p;  // exchanged ends
+    const double vold = lane < m ? c.Vl(own(b, lane), slc(lane)) : 0.0;
+    const double sx = c.X(0, ns, j0), sy = c.Xd(1, ns, j0);
+    double ex = c.X(0, ne, se), ey = c.Xd(1, ne, se);
+    double dx = sx - ex, dy = dim > 1 ? sy - ey : 0.0;
+    if (abs_gt(dx, L)) dx = unwrap_end(sx, ex, L);
+    if (dim > 1 && abs_gt(dy, L)) dy = unwrap_end(sy, ey, L);
+    const double inv_m = bw[0].x;
+    const float *z = Sz + 2 * (b * (m - 1));
+    double x, y;
+    if (m <= 17) {
+      const int t = (lane & 15) + 1, k = lane >> 4;
+      const bool act = t < m && k < dim;
+      double v = 0.0, kt = 0.0;
+      if (act) {
+        const double2 wk = bw[t];
+        v = (double)z[2 * (t - 1) + k] * wk.x;
+        kt = wk.y;
+      }
+      const double carry = (k ? dy : dx) * inv_m;
+#pragma unroll
+      for (int off = 1; off < 16; off <<= 1) {
+        const double vp = __shfl_up_sync(0xffffffffu, v, off, 16);
+        if ((lane & 15) >= off) v += vp;
+      }
+      const double p = fma(kt, carry + v, k ? ey : ex);
+      x = __shfl_sync(0xffffffffu, p, (lane - 1) & 15);
+      y = __shfl_sync(0xffffffffu, p, 16 | ((lane - 1) & 15));
+    } else {
+      const int t = lane + 1;
+      const bool act = t < m;
+      const double2 wk = act ? bw[t] : make_double2(0.0, 0.0);
+      double vx = act ? (double)z[2 * lane] * wk.x : 0.0, vy = 0.0;
+      if (dim > 1) vy = act ? (double)z[2 * lane + 1] * wk.x : 0.0;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const double px = __shfl_up_sync(0xffffffffu, vx, off);
+        if (lane >= off) vx += px;
+      }
+      x = __shfl_up_sync(0xffffffffu, fma(wk.y, dx * inv_m + vx, ex), 1);
+      y = 0.0;
+      if (dim > 1) {
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const double py = __shfl_up_sync(0xffffffffu, vy, off);
+          if (lane >= off) vy += py;
+        }
+        y = __shfl_up_sync(0xffffffffu, fma(wk.y, dy * inv_m + vy, ey), 1);
+      }
+    }
+    // lane t holds bead t, 0 and m the fixed ends
+    if (lane == 0) { x = sx; y = sy; }
+    if (lane == m) { x = ex; y = ey; }
+    double v = 0.0;
+    if (lane <= m) {
+      x = teleport_s<true>(x, L, inv2L);
+      y = dim > 1 ? teleport_s<true>(y, L, inv2L) : 0.0;
+      rx[lane] = x;
+      ry[lane] = y;
+      v = vext(d, x, y);
+      if (pair) qb[lane] = qpos(d, x, y);
+    }
+    const double vn = __shfl_down_sync(0xffffffffu, v, 1);
+    double dw = 0.0;
+    if (lane < m) {
+      const double link = mhtau * (v + vn);
+      vb[lane] = link;
+      dw = link - vold;
+    }
+    dw = warp_sum(dw);
+    if (lane == 0) {
+      S.sums->p[b] = dw;
+      S.sums->pf[b] = (float)dw;
+    }
+  }
+  G::sync();
+  PROF_MARK(3);
+  // the pair-free change of the action, w_update - w_initial without pairs
+  const float pf = S.sums->pf[0] + S.sums->pf[1] + lrf;
+  const float pfe = lre + 3e-7f * (fabsf(S.sums->pf[0]) + fabsf(S.sums->pf[1]) + fabsf(lrf));
+  auto exact_pf = [&]() { return S.sums->p[0] + S.sums->p[1] + log_ratio(); };
+  const bool fast = !(d.flags & PF_EXACT);
+  // the move's Metropolis test on an FP64 value
+  auto exact_test = [&](double dS) -> int {
+    const int k = fast ? decide_f((float)dS, 0.f, lu) : -1;
+    if (k >= 0) return k;
+    const double u = dr.uniform_accept(), delta = exp(dS);
+    return delta >= 1.0 || delta > u;
+  };
+  // Under the reference's rules every pair term (-tau/2 g (..) <= 0 for g >= 0)
+  // enters w_initial, so it can only raise w_update - w_initial: when the
+  // pair-free part already accepts, the pair sums cannot change the decision,
+  // and a lower bound of the pair sums that reaches `need` accepts as well
+  int dec = -1;
+  const bool rising = fast && pair && !f_contact && !f_phys && d.g >= 0.0;
+  if (!pair || rising) {
+    if (fast) dec = decide_f(pf, pfe, lu);
+    if (dec == -1 || (dec == 0 && pair)) {
+      if (dec == -1) dec = exact_test(exact_pf());
+      if (dec == 0 && pair) dec = -1;  // the pairs may still accept
+    }
+  }
+  PROF_MARK(5);
+  if (dec == 1 && pair) PROF_COUNT(2);
+  if (dec == -1) {
+    // the 2m links of the two moving paths in contiguous ranges per warp
+    const int per = (2 * m + nwarps - 1) / nwarps;
+    const int a0 = min(2 * m, warp * per), a1 = min(2 * m, a0 + per);
+    auto seg_of = [&](int b) {
+      return SwapSeg{&c, j0, M, b == 0 ? n1 : n2, b == 0 ? nx1 : nx2, n1, nx1, n2, nx2,
+                     b == 0 ? S.r1x : S.r2x, b == 0 ? S.r1y : S.r2y, !f_phys, b == 0 ? S.q1 : S.q2};
+    };
+    // the pair of the two moving paths, old and new (physical rules), exact
+    double w2[2] = {0.0, 0.0};  // pair parts of w_initial, w_update
+    if (f_phys)
+      for (int t = tid; t < m; t += nt) {
+        const int j = slc(t), jn = slc(t + 1);
+        const int o1 = own(0, t), o1n = own(0, t + 1), o2 = own(1, t), o2n = own(1, t + 1);
+        const double ox = c.X(0, o1, j), oy = c.Xd(1, o1, j);
+        const double r2o = mi2(d, ox, oy, c.X(0, o2, j), c.Xd(1, o2, j));
+        if (r2o <= d.rc2) {
+          if (f_contact)
+            w2[0] += contact_link(d, ox, oy, c.X(0, o2, j), c.Xd(1, o2, j), c.X(0, o1n, jn),
+                                  c.Xd(1, o1n, jn), c.X(0, o2n, jn), c.Xd(1, o2n, jn));
+          else
+            w2[0] += lnU2(d, r2o, mi2(d, c.X(0, o1n, jn), c.Xd(1, o1n, jn), c.X(0, o2n, jn), c.Xd(1, o2n, jn)));
+        }
+        const double r2n = mi2(d, S.r1x[t], S.r1y[t], S.r2x[t], S.r2y[t]);
+        if (r2n <= d.rc2) {
+          if (f_contact)
+            w2[1] += contact_link(d, S.r1x[t], S.r1y[t], S.r2x[t], S.r2y[t], S.r1x[t + 1],
+                                  S.r1y[t + 1], S.r2x[t + 1], S.r2y[t + 1]);
+          else
+            w2[1] += lnU2(d, r2n, mi2(d, S.r1x[t + 1], S.r1y[t + 1], S.r2x[t + 1], S.r2y[t + 1]));
+        }
+      }
+    if (fast && !f_contact) {
+      // bounded estimate from the mirror: decides the move unless the log
+      // acceptance ratio's interval straddles the threshold.  With rising pairs
+      // a warp whose own lower bound already accepts raises a flag in shared
+      // memory, and every warp stops at its next link
+      PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
+      const float gh = (float)(-d.mhtau_g);  // tau g / 2, within 6e-8
+      const float need = lu - pf + pfe + 1e-5f * (1.f + fabsf(lu)) + 1e-6f * (fabsf(lu) + fabsf(pf));
+      const bool monotone = rising && d.g > 0.0 && lu > -3e38f;
+      volatile int *flag = S.iv + 3;
+      // the lane's estimate and the bound on its error, with the FP32
+      // accumulation (two ulp per term) and the sums over the warp and the
+      // warps (below 16 additions of 6e-8 each) covered
+      auto lane_sum = [&](const PairEst &q, float &t, float &r) {
+        t = f_phys ? q.so - q.sn : q.so + q.sn;
+        const float ro = 2.4e-7f * (float)(q.ko + 1), rn = 2.4e-7f * (float)(q.kn + 1);
+        r = (q.bo * (1.f + ro) + ro * q.so + q.bn * (1.f + rn) + rn * q.sn + 2e-6f * (q.so + q.sn)) * 1.00001f + 1e-30f;
+      };
+      auto stop = [&](const PairEst &q) -> bool {
+        if (!monotone) return false;
+        if (*flag) return true;
+        float t, r;
+        lane_sum(q, t, r);
+        const float lb = warp_sum(t - r);
+        if (gh * lb * (lb > 0.f ? 0.99999f : 1.00001f) > need) {
+          if (lane == 0) *flag = 1;
+          return true;
+        }
+        return false;
+      };
+      for (int b = 0; b < 2; ++b) {
+        const int t0 = max(a0 - b * m, 0), t1 = min(a1 - b * m, m);
+        if (t0 < t1 && segment_estimate(c, seg_of(b), t0, t1, e, lane, stop)) break;
+      }
+      float t, r;
+      lane_sum(e, t, r);
+      t = warp_sum(t);
+      r = warp_sum(r);
+      if (f_phys) {
+        // the exact cross term rides along (its lanes' float sums)
+        const float x = warp_sum((float)(w2[1] - w2[0])), xa = warp_sum((float)(fabs(w2[0]) + fabs(w2[1])));
+        t = t * gh + x;
+        r = r * fabsf(gh) + 2e-6f * xa + 2e-7f * fabsf(t);
+      } else {
+        t *= gh;
+        r = r * fabsf(gh) + 2e-7f * fabsf(t);
+      }
+      if (lane == 0) {
+        S.sums->est[warp][0] = t;
+        S.sums->est[warp][1] = r;
+      }
+      G::sync();
+      if (monotone && *flag) {
+        dec = 1;
+      } else {
+        float ts = 0.f, rs = 0.f, as = 0.f;
+        for (int w = 0; w < nwarps; ++w) {
+          ts += S.sums->est[w][0];
+          rs += S.sums->est[w][1];
+          as += fabsf(S.sums->est[w][0]);
+        }
+        dec = decide_f(pf + ts, pfe + rs + 1e-6f * (as + fabsf(pf)), lu);
+      }
+      if (dec != -1) PROF_COUNT(3);
+    }
+    PROF_MARK(6);
+    if (dec == -1) {
+      PROF_COUNT(4);
+      for (int b = 0; b < 2; ++b) {
+        const int t0 = max(a0 - b * m, 0), t1 = min(a1 - b * m, m);
+        if (t0 >= t1) continue;
+        double wo = 0.0, wn = 0.0;
+        segment_pairs<GEN>(c, seg_of(b), t0, t1, true, true, S.q + (size_t)warp * PQ_CAP, wo, wn, lane);
+        // the reference adds the new paths' pair terms to w_initial and lets
+        // the old ones see the other moving path (reshape.jl:166-240)
+        w2[0] += wo;
+        if (f_phys) w2[1] += wn; else w2[0] += wn;
+      }
+      G::template sum<2>(w2, red);
+      // every thread holds the same sums and decides alone
+      dec = exact_test(exact_pf() + (w2[1] - w2[0]));
+    }
+  }
+  PROF_MARK(8);
+  if (!dec) {
+    PROF_COUNT(6);
+    return RES_REJECT;
+  }
+  PROF_COUNT(5);
+  // accept: exchange next, write the bridges along the new cycles, exchange
+  // the tails (reshape.jl:247-279)
+  auto nown = [&](int b, int t) { return (j0 + t < M) ? (b ? n2 : n1) : (b ? nx1 : nx2); };
+  for (int b = warp; b < 2; b += nwarps) {
+    const double *rx = b ? S.r2x : S.r1x, *ry = b ? S.r2y : S.r1y, *vb = b ? S.vb2 : S.vb1;
+    const unsigned *qb = b ? S.q2 : S.q1;
+    if (lane <= m) {
+      const int j = slc(lane), n = nown(b, lane);
+      const double x = rx[lane], y = ry[lane];
+      if (lane > 0) {
+        c.X(0, n, j) = x;
+        if (dim > 1) c.X(1, n, j) = y;
+        c.xq[(size_t)j * c.ldn + n] = pair ? qb[lane] : qpos(d, x, y);
+      }
+      if (lane < m) c.Vl(n, j) = vb[lane];
+    }
+  }
+  if (c.cl && warp == 0 && lane > 0 && lane <= m) {
+    // a slice's marks come from one thread, in a fixed order
+    c.cl->mark(nown(0, lane), slc(lane));
+    c.cl->mark(nown(1, lane), slc(lane));
+  }
+  if (j0 + m < M - 1)
+    for (int j = se + 1 + tid; j < M; j += nt) c.exchange_linked(n1, n2, j);
+  if (tid == 0) {
+    c.next[n1] = nx2;
+    c.next[n2] = nx1;
+    if (f_phys && !wrap) {
+      // the link leaving the end bead moves with the tail
+      const double v = c.Vl(n1, se);
+      c.Vl(n1, se) = c.Vl(n2, se);
+      c.Vl(n2, se) = v;
+    }
+  }
+  G::sync();
+  PROF_MARK(9);
+  return RES_ACCEPT;
+}
+
+// swaps that swap_sweep does not take (windows past SWAP_LANES links, hard
+// cores), out of line: their code stays out of its way
+template <bool WARP, int SPEC>
+static __device__ __noinline__ int swap_general(CV c, int j0, int m, int n1, double u_pick, Stream ss,
+                                                SwapScratch S, double *red) {
+  GenDraws dr = gen_draws(ss);
+  return swap_group<WARP, true, GenDraws, SPEC>(c, j0, m, n1, u_pick, dr, S, red, nullptr, nullptr);
 }
 
 // ---------------------------------------------------------------------------

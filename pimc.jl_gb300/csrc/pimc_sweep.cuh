@@ -286,34 +286,53 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
 
   // ---- permutation swaps (ReshapeSwapLinear), one at a time by the group
   if ((PH & SW_SWAP) && N > 1 && mix.swaps_per_sweep > 0) {
-    double tal[4] = {0, 0, 0, 0};
     SwapScratch S;
     S.carve(scratch, N, nwarps);
     const int mmax = max(2, min(mix.swap_max, min(M - 1, WMAX)));
     const int sm = max(2, sc.v.swap_m);
     const bool lists = (d.flags & (PF_PAIR | PF_HARD)) && build_lists();
-    const CV &cs = lists ? cq : c;
+    CV cs = c;
+    if (lists) cs.cl = cq.cl;
+    const int wstride = swap_wstride(N), chunk = (N + 31) / 32;
+    const unsigned wmagic = chunk > 1 ? 0xffffffffu / (unsigned)chunk + 1u : 0u;  // i / chunk = umulhi(i, wmagic)
+    // integer tallies (attempts, accepts, skips, beads): FP64 additions would
+    // hold the leading warp up after every attempt
+    int n_att = 0, n_acc = 0, n_skip = 0;
+    long long n_bead = 0;
     for (int a = 0; a < mix.swaps_per_sweep; ++a) {
+      if ((a & (SWAP_DRAWS - 1)) == 0) {
+        G::sync();
+        if (warp == 0) swap_draws(*S.draws, d, sweep, a, mix.swaps_per_sweep, M, N, mmax, sm);
+        G::sync();
+      }
       const Stream ss = make_stream(d, sweep, PH_SWAP, (unsigned)a);
-      const uint4 r0 = ss.at(DRAW_CHOICE), r1 = ss.at(DRAW_CHOICE + 1);
-      const int j0 = min(M - 1, (int)(u53(r0.x, r0.y) * M));
-      const int m = min(mmax, 2 + (int)(u53(r0.z, r0.w) * (sm - 1)));
-      const int n1 = min(N - 1, (int)(u53(r1.x, r1.y) * N));
-      const double upick = u53(r1.z, r1.w);
-      GenDraws dr = gen_draws(ss);
-      const int r = swap_group<WARP, true, GenDraws, SPEC>(cs, j0, m, n1, upick, dr, S, red, nullptr,
-                                                           nullptr);
-      if (tid == 0) {
-        if (r == RES_SKIP) {
-          tal[2] += 1.0;
-        } else {
-          tal[0] += 1.0;
-          tal[1] += r == RES_ACCEPT;
-          if (r != RES_HARDCORE) tal[3] += 2.0 * (m - 1);
-        }
+      const int m = S.draws->m[a & (SWAP_DRAWS - 1)];
+      int r;
+      if (m <= SWAP_LANES && !(SPEC == SWAP_ANY && (d.flags & PF_HARD))) {
+        r = swap_sweep<WARP, SPEC>(cs, a, ss, wstride, wmagic, S, red);
+      } else {
+        const uint4 r1 = ss.at(DRAW_CHOICE + 1);
+        G::sync();
+        r = swap_general<WARP, SPEC>(cs, S.draws->j0[a & (SWAP_DRAWS - 1)], m, S.draws->n1[a & (SWAP_DRAWS - 1)],
+                                     u53(r1.z, r1.w), ss, S, red);
+        G::sync();
+      }
+      if (r == RES_SKIP) {
+        ++n_skip;
+      } else {
+        ++n_att;
+        n_acc += r == RES_ACCEPT;
+        if (r != RES_HARDCORE) n_bead += 2 * (m - 1);
       }
     }
     G::sync();
+    double tal[4] = {0, 0, 0, 0};
+    if (tid == 0) {
+      tal[0] = n_att;
+      tal[1] = n_acc;
+      tal[2] = n_skip;
+      tal[3] = (double)n_bead;
+    }
     close_phase<WARP>(sc, red, MV_SWAP, tal);
   }
 
