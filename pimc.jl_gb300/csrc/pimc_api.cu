@@ -201,6 +201,21 @@ ChainDesc make_desc(const pimc_params &p, int chain) {
     d.q_u2i = (float)(u * u * d.inv2s2);
     d.q_lim_lo = rq > e ? (unsigned)std::floor((rq - e) * (rq - e)) : 0u;
     d.q_lim_hi = (unsigned)std::min(std::ceil((rq + e) * (rq + e)), (double)d.q_lim_rc);
+    {
+      // the argument of exp(-u2i d^2) is off by at most u2i (2 e d + e^2), and
+      // 2 d <= d^2 / s + s with s the reach; the exponential turns an argument
+      // error D into expm1(D) <= D exp(D), D at three reaches (beyond, the terms
+      // are below exp(-9 y(s))); the FP32 product and ex2.approx add 5e-7 (1 + y)
+      const double u2i = u * u * d.inv2s2, sr = std::sqrt((double)d.q_lim_hi) + 1.0;
+      const double fac = 1.01 * std::exp(std::min(60.0, u2i * e * (6.0 * sr + e)));
+      d.est_a = (float)(fac * u2i * e / sr + 5e-7 * u2i);
+      d.est_b = (float)(fac * u2i * e * (sr + e) + 5e-7);
+      d.est_x = (float)(-u2i * 1.4426950408889634);
+      d.f_scale = 4294967296.0 / (2.0 * p.L);
+      const double fu = 1.0 / d.f_scale;
+      d.f_unit = (float)fu;
+      d.est2 = (float)(1e-6 + 8.0 * d.rc * fu * d.inv2s2);
+    }
     d.hb_unit = (float)((double)d.q_unit2 / (4.0 * d.tau * d.lambda));
     d.q_Lf = (float)p.L;
     d.q_scalef = (float)d.q_scale;

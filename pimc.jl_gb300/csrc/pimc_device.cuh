@@ -36,10 +36,11 @@ namespace pimc {
 constexpr int WMAX = 64;     // largest staging / swap window m handled on the device
 constexpr int TWMAX = 32;    // thread-per-window variant handles m <= TWMAX
 // doubles of per-warp scratch of window_warp: new beads x, y, their external
-// potential, normals (2 per bead), the neighbour queue (96 entries), the
-// new beads' mirror words, and 4 doubles through which the warps of a
+// potential, normals (2 per bead; the centres in fixed point once the bridge is
+// drawn), the neighbour queue (96 entries), the old and new beads' mirror
+// words, and 4 doubles through which the warps of a
 // staging team exchange their partial sums
-constexpr int TEAM_SLOT_D = 5 * (WMAX + 1) + 96 + (WMAX + 2) / 2;
+constexpr int TEAM_SLOT_D = 5 * (WMAX + 1) + 96 + (WMAX + 1);
 constexpr int WARP_SCRATCH_D = TEAM_SLOT_D + 4;
 
 // move outcomes (PIMC_REJECT / ACCEPT / SKIP / HARDCORE of pimc.h)
@@ -1194,11 +1195,9 @@ struct WindowSeg {
   const CV *c;
   int n, nx, j0, M;
   const double *px, *py;
-  const unsigned *pq;   // mirror words of the new beads
+  const unsigned *pq;   // mirror words of the old and the new beads, in turn
   __device__ __forceinline__ int own(int t) const { return j0 + t < M ? n : nx; }
-  __device__ __forceinline__ unsigned curq(int side, int t) const {
-    return side ? pq[t] : c->Q(own(t), slice(t));
-  }
+  __device__ __forceinline__ unsigned curq(int side, int t) const { return pq[2 * t + side]; }
   __device__ __forceinline__ unsigned nxtq(int side, int t) const { return curq(side, t + 1); }
   __device__ __forceinline__ int slice(int t) const { return j0 + t < M ? j0 + t : j0 + t - M; }
   __device__ __forceinline__ void cur(int side, int t, double &x, double &y) const {
@@ -1258,6 +1257,10 @@ __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+
+}  // namespace pimc
+#include "pimc_scan.cuh"
+namespace pimc {
 
 // ---------------------------------------------------------------------------
 // Levy staging window, one thread (pair-free acceptance, no hard core)
@@ -1431,7 +1434,11 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
     sx_[t] = qx;
     sy_[t] = qy;
     svb[t] = vext(d, qx, qy);
-    if (phys_pair) sq[t] = qpos(d, qx, qy);
+    if (phys_pair) {
+      const int a = j0 + t;
+      sq[2 * t] = a < M ? c.Q(n, a) : c.Q(nx, a - M);
+      sq[2 * t + 1] = qpos(d, qx, qy);
+    }
   }
   __syncwarp();
   double wi = 0.0, wu = 0.0;
@@ -1444,17 +1451,31 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
   if (phys_pair) {
     WindowSeg seg{&c, n, nx, j0, M, sx_, sy_, sq};
     if (D::kSweep && !(d.flags & (PF_EXACT | PF_CONTACT))) {
-      // bounded estimate from the mirror; the exact sums only when its
-      // interval straddles the Metropolis threshold
+      // bracketed from the mirror, then from the positions in fixed point;
+      // the exact sums only when both straddle the Metropolis threshold
+      const double u = dr.uniform_accept();
+      const float lu = u > 0.0 ? logf((float)u) : -INFINITY;
+      const float dw = (float)warp_sum(wu - wi), gh = (float)(-d.mhtau_g);
+      const ScanSkip<2> skip{n, -1, true};
       PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
-      segment_estimate(c, seg, 0, m, e, lane);
-      double v[4];
-      est_reduce_lanes(e, v);
-      for (int k = 0; k < 4; ++k) v[k] = warp_sum(v[k]);
-      const double h = d.mhtau_g;
-      const double centre = warp_sum(wu) - warp_sum(wi) + h * (v[2] - v[0]);
-      const double radius = fabs(h) * (v[1] + v[3]);
-      dec = decide_interval(centre - radius, centre + radius, dr.uniform_accept());
+      scan_mirror<2>(c, j0, m, sq, skip, 0, 1, e, lane, NoStop());
+      float t, r;
+      est_lane(e, -1.f, t, r);
+      dec = decide_f(fmaf(gh, warp_sum(t), dw), fabsf(gh) * warp_sum(r) + 1e-6f * fabsf(dw), lu);
+      if (dec == -1) {
+        uint2 *cf = reinterpret_cast<uint2 *>(sz);
+        for (int k = lane; k < 2 * (m + 1); k += 32) {
+          double x, y;
+          seg.cur(k & 1, k >> 1, x, y);
+          cf[k] = make_uint2(fix32(d, x), fix32(d, y));
+        }
+        __syncwarp();
+        e = {0.f, 0.f, 0.f, 0.f, 0, 0};
+        scan_fixed<2>(c, j0, m, cf, skip, 0, 1, e, lane);
+        est_lane(e, -1.f, t, r);
+        dec = decide_f(fmaf(gh, warp_sum(t), dw), fabsf(gh) * warp_sum(r) + 1e-6f * fabsf(dw), lu);
+        __syncwarp();
+      }
     }
     if (dec == -1)
       segment_pairs(c, seg, 0, m, true, true, (unsigned long long *)(sb + 5 * (WMAX + 1)), wi, wu,
@@ -1556,7 +1577,9 @@ __device__ int window_team(const CV &c, const Team &tm, int n, int j0, int m, D 
     sx_[t] = qx;
     sy_[t] = qy;
     svb[t] = vext(d, qx, qy);
-    sq[t] = qpos(d, qx, qy);
+    const int a = j0 + t;
+    sq[2 * t] = a < M ? c.Q(n, a) : c.Q(nx, a - M);
+    sq[2 * t + 1] = qpos(d, qx, qy);
   }
   tm.sync();
   double wi = 0.0, wu = 0.0;

@@ -90,6 +90,9 @@ struct SwapSums {
 constexpr int SWAP_WPAD = 64;
 __host__ __device__ inline int swap_wstride(int N) { return 32 * (((N + 31) / 32) | 1); }
 
+// windows of a sweep's swap_sweep: at most SWAP_LANES links
+constexpr int SWAP_LANES = 31, SWAP_BEADS = SWAP_LANES + 1;
+
 // shared scratch of the swap
 struct SwapScratch {
   double *w;                                   // N heat-bath weights (sweeps: two buffers of
@@ -99,17 +102,19 @@ struct SwapScratch {
   unsigned long long *q;                       // PQ_CAP neighbour queue per warp
   unsigned *q1, *q2;                           // WMAX+1 mirror words each
   int *iv;                                     // 4 ints: group broadcasts
+  uint4 *cq;                                   // mirror words per bead: old 1, new 1, old 2, new 2
   SwapSums *sums;                              // a sweep's partial sums
   SwapDraws *draws;                            // a sweep's next choices
   static __host__ __device__ size_t bytes(int N, int nwarps) {
-    return sizeof(double) * ((size_t)N + SWAP_WPAD + 6 * (WMAX + 1) + 4 * WMAX) +
+    return sizeof(uint4) * SWAP_BEADS + sizeof(double) * ((((size_t)N + 1) & ~(size_t)1) + SWAP_WPAD + 6 * (WMAX + 1) + 4 * WMAX) +
            sizeof(unsigned long long) * PQ_CAP * (size_t)nwarps +
            sizeof(unsigned) * 2 * (WMAX + 1) + sizeof(int) * 4 + sizeof(SwapDraws) +
            sizeof(SwapSums);
   }
   __device__ void carve(void *base, int N, int nwarps) {
-    double *p = (double *)base;
-    w = p; p += N + SWAP_WPAD;
+    cq = (uint4 *)base;
+    double *p = (double *)(cq + SWAP_BEADS);
+    w = p; p += ((N + 1) & ~1) + SWAP_WPAD;
     r1x = p; p += WMAX + 1; r1y = p; p += WMAX + 1;
     r2x = p; p += WMAX + 1; r2y = p; p += WMAX + 1;
     vb1 = p; p += WMAX + 1; vb2 = p; p += WMAX + 1;
@@ -994,8 +999,6 @@ __device__ int swap_warp(const CV &c, int j0, int m, int n1, double u_pick, D &d
 // one chain of 64 free particles under the physical rules 22 k -> 7.3 k, 4.26
 // -> 1.81 ms.
 // ---------------------------------------------------------------------------
-constexpr int SWAP_LANES = 31;
-
 // choices of swaps a0 .. a0 + 31 of a sweep, by one warp
 __device__ __forceinline__ void swap_draws(SwapDraws &D, const ChainDesc &d, unsigned long long sweep, int a0,
                                            int n, int M, int N, int mmax, int sm) {
@@ -1010,16 +1013,6 @@ __device__ __forceinline__ void swap_draws(SwapDraws &D, const ChainDesc &d, uns
     const double u = ss.uni(DRAW_ACCEPT);
     D.lu[lane] = u > 0.0 ? logf((float)u) : -INFINITY;
   }
-}
-
-// the Metropolis decision of a log ratio known to lie in [s - r, s + r], from
-// lu = log u: 1 accept, 0 reject, -1 undecided.  The margin covers logf and
-// the roundings of u, s and r (floats: 6e-8 each); lu = -inf is undecided.
-__device__ __forceinline__ int decide_f(float s, float r, float lu) {
-  const float mg = r * 1.00001f + 1e-5f * (1.f + fabsf(lu)) + 1e-6f * fabsf(s);
-  if (s - mg > lu && lu > -3e38f) return 1;
-  if (s + mg < lu) return 0;
-  return -1;
 }
 
 // a bridge's end e taken to the start s's side of the periodic box; returns
@@ -1273,7 +1266,11 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
       rx[lane] = x;
       ry[lane] = y;
       v = vext(d, x, y);
-      if (pair) qb[lane] = qpos(d, x, y);
+      if (pair) {
+        const unsigned q = qpos(d, x, y);
+        qb[lane] = q;
+        reinterpret_cast<uint2 *>(S.cq + lane)[b] = make_uint2(c.Q(own(b, lane), slc(lane)), q);
+      }
     }
     const double vn = __shfl_down_sync(0xffffffffu, v, 1);
     double dw = 0.0;
@@ -1350,28 +1347,21 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
         }
       }
     if (fast && !f_contact) {
-      // bounded estimate from the mirror: decides the move unless the log
-      // acceptance ratio's interval straddles the threshold.  With rising pairs
-      // a warp whose own lower bound already accepts raises a flag in shared
-      // memory, and every warp stops at its next link
-      PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
+      // bracketed from the mirror, and where that straddles the threshold from
+      // the positions in fixed point (pimc_scan.cuh); the warps split the
+      // particles.  With rising pairs a warp whose own lower bound already
+      // accepts raises a flag in shared memory, and every warp stops at its
+      // next block
       const float gh = (float)(-d.mhtau_g);  // tau g / 2, within 6e-8
+      const float sgn_new = f_phys ? -1.f : 1.f;
       const float need = lu - pf + pfe + 1e-5f * (1.f + fabsf(lu)) + 1e-6f * (fabsf(lu) + fabsf(pf));
       const bool monotone = rising && d.g > 0.0 && lu > -3e38f;
       volatile int *flag = S.iv + 3;
-      // the lane's estimate and the bound on its error, with the FP32
-      // accumulation (two ulp per term) and the sums over the warp and the
-      // warps (below 16 additions of 6e-8 each) covered
-      auto lane_sum = [&](const PairEst &q, float &t, float &r) {
-        t = f_phys ? q.so - q.sn : q.so + q.sn;
-        const float ro = 2.4e-7f * (float)(q.ko + 1), rn = 2.4e-7f * (float)(q.kn + 1);
-        r = (q.bo * (1.f + ro) + ro * q.so + q.bn * (1.f + rn) + rn * q.sn + 2e-6f * (q.so + q.sn)) * 1.00001f + 1e-30f;
-      };
       auto stop = [&](const PairEst &q) -> bool {
         if (!monotone) return false;
         if (*flag) return true;
         float t, r;
-        lane_sum(q, t, r);
+        est_lane(q, sgn_new, t, r);
         const float lb = warp_sum(t - r);
         if (gh * lb * (lb > 0.f ? 0.99999f : 1.00001f) > need) {
           if (lane == 0) *flag = 1;
@@ -1379,38 +1369,50 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
         }
         return false;
       };
-      for (int b = 0; b < 2; ++b) {
-        const int t0 = max(a0 - b * m, 0), t1 = min(a1 - b * m, m);
-        if (t0 < t1 && segment_estimate(c, seg_of(b), t0, t1, e, lane, stop)) break;
-      }
-      float t, r;
-      lane_sum(e, t, r);
-      t = warp_sum(t);
-      r = warp_sum(r);
+      const ScanSkip<4> skip{n1, n2, f_phys};
+      // the exact cross term rides along (its lanes' float sums)
+      float xs = 0.f, xr = 0.f;
       if (f_phys) {
-        // the exact cross term rides along (its lanes' float sums)
-        const float x = warp_sum((float)(w2[1] - w2[0])), xa = warp_sum((float)(fabs(w2[0]) + fabs(w2[1])));
-        t = t * gh + x;
-        r = r * fabsf(gh) + 2e-6f * xa + 2e-7f * fabsf(t);
-      } else {
-        t *= gh;
-        r = r * fabsf(gh) + 2e-7f * fabsf(t);
+        xs = warp_sum((float)(w2[1] - w2[0]));
+        xr = 2e-6f * warp_sum((float)(fabs(w2[0]) + fabs(w2[1])));
       }
-      if (lane == 0) {
-        S.sums->est[warp][0] = t;
-        S.sums->est[warp][1] = r;
-      }
-      G::sync();
-      if (monotone && *flag) {
-        dec = 1;
-      } else {
-        float ts = 0.f, rs = 0.f, as = 0.f;
-        for (int w = 0; w < nwarps; ++w) {
-          ts += S.sums->est[w][0];
-          rs += S.sums->est[w][1];
-          as += fabsf(S.sums->est[w][0]);
+      for (int level = 0; level < 2 && dec == -1; ++level) {
+        PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
+        if (level == 0) {
+          scan_mirror<4>(c, j0, m, reinterpret_cast<const unsigned *>(S.cq), skip, warp, nwarps, e, lane, stop);
+        } else {
+          uint2 *cf = reinterpret_cast<uint2 *>(Sz);  // the normals are spent
+          for (int k = tid; k < 4 * (m + 1); k += nt) {
+            double x, y;
+            seg_of((k >> 1) & 1).cur(k & 1, k >> 2, x, y);
+            cf[k] = make_uint2(fix32(d, x), fix32(d, y));
+          }
+          G::sync();
+          scan_fixed<4>(c, j0, m, cf, skip, warp, nwarps, e, lane);
         }
-        dec = decide_f(pf + ts, pfe + rs + 1e-6f * (as + fabsf(pf)), lu);
+        float t, r;
+        est_lane(e, sgn_new, t, r);
+        t = warp_sum(t);
+        r = warp_sum(r);
+        t = t * gh + xs;
+        r = r * fabsf(gh) + xr + 2e-7f * fabsf(t);
+        if (lane == 0) {
+          S.sums->est[warp][0] = t;
+          S.sums->est[warp][1] = r;
+        }
+        G::sync();
+        if (level == 0 && monotone && *flag) {
+          dec = 1;
+        } else {
+          float ts = 0.f, rs = 0.f, as = 0.f;
+          for (int w = 0; w < nwarps; ++w) {
+            ts += S.sums->est[w][0];
+            rs += S.sums->est[w][1];
+            as += fabsf(S.sums->est[w][0]);
+          }
+          dec = decide_f(pf + ts, pfe + rs + 1e-6f * (as + fabsf(pf)), lu);
+        }
+        if (level == 0 && dec == -1) G::sync();  // the sums are read before the next level's
       }
       if (dec != -1) PROF_COUNT(3);
     }

@@ -56,6 +56,12 @@ struct ChainDesc {
   // which it is surely beyond (kQErr units of mirror error on a distance)
   float q_u2i;
   unsigned q_lim_lo, q_lim_hi;
+  // scan_mirror's exponential at squared mirror distance d2: ex2(est_x d2),
+  // relative error at most est_a d2 + est_b; scan_fixed's fixed point: 2^32 / 2L,
+  // its unit, and the constant part of its exponentials' relative error
+  float est_a, est_b, est_x;
+  float f_unit, est2;
+  double f_scale;
   // the sweeps' FP32 heat-bath exponent scale per window length m:
   // hb_unit / m = (squared mirror unit) / (4 lambda m tau)
   float hb_unit;

@@ -101,3 +101,35 @@ def test_batch_adjoint_follows_a_new_trap(engine_lib):
     _, th, _ = e.batch_adjoint()
     _, one, _ = e.adjoint(1)
     np.testing.assert_allclose(th[1], one, rtol=1e-13)
+
+
+@pytest.mark.parametrize("sem", [0, 1])
+@pytest.mark.parametrize("ell,M", [(5, 9), (17, 40), (18, 36), (31, 40), (32, 40), (33, 70), (64, 70)])
+def test_sweep_paths_decide_as_exact_sums(sem, ell, M, engine_lib):
+    """sweeps around the windows' edges (half-warp and warp bridges, the longest
+    swap of a warp, the longest window), crowded and sparse, one and two
+    dimensions: bracketed decisions give the beads, permutations and
+    acceptance counts of exact FP64 ones, bit for bit"""
+    from pimc.engine import ChainParams, Engine, Mix, OPT_EXACT_DECISIONS
+    ps = [ChainParams(dim=dim, N=N, M=M, L=L, T=1.0, lam=0.5, harmonic_omega=om, interactions=pair,
+                      pair_g=g, pair_sigma=0.4, r_a=1.0, semantics=sem, seed=900 + i)
+          for i, (N, dim, L, om, pair, g) in enumerate(
+              [(2, 2, 4.0, 1.0, True, 1.5), (31, 2, 3.0, 1.0, True, 1.0), (32, 1, 6.0, 0.5, True, 2.0),
+               (33, 2, 8.0, 0.0, True, 1.0), (70, 2, 3.0, 2.0, True, 0.7), (64, 2, 5.0, 1.0, False, 0.0),
+               (20, 2, 3.0, 1.0, True, 0.0)])]
+    out = []
+    for exact in (0, 1):
+        e = Engine(ps)
+        for i, p in enumerate(ps):
+            e.set_mix(Mix(stage_slices=ell, stage_min=2, stage_max=ell, stage_minacc=0.0, stage_maxacc=1.0,
+                          swaps_per_sweep=p.N + 40, swap_slices=ell, swap_min=2, swap_max=ell,
+                          swap_minacc=0.0, swap_maxacc=1.0, com_phases=1, com_step=0.5,
+                          com_minstep=0.1, com_maxstep=2.0), chain=i)
+        e.set_option(OPT_EXACT_DECISIONS, exact)
+        e.run_batched(6)
+        out.append([(e.get_beads(c), e.get_next(c), e.stats(c).accepts) for c in range(len(ps))])
+        e.close()
+    for (xa, na, aa), (xb, nb, ab) in zip(*out):
+        np.testing.assert_array_equal(xa, xb)
+        np.testing.assert_array_equal(na, nb)
+        assert aa == ab and np.isfinite(xa).all()
