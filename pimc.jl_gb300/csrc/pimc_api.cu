@@ -82,6 +82,7 @@ struct Handle {
   int *d_queue = nullptr;
   int *d_order = nullptr;
   int *d_iout = nullptr;
+  SlotTally *d_tally = nullptr;  // k_stage_slots' counters per chain
   double *d_buf = nullptr;
   size_t n_buf = 0;
   double *d_adj = nullptr;
@@ -517,9 +518,11 @@ int create_impl(const pimc_params *params, int nchains, void **out) {
       cudaMalloc(&h->d_queue, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&h->d_order, sizeof(int) * nchains) != cudaSuccess ||
       cudaMalloc(&h->d_iout, sizeof(int) * 16) != cudaSuccess ||
+      cudaMalloc(&h->d_tally, sizeof(SlotTally) * nchains) != cudaSuccess ||
       cudaMalloc(&h->d_stage, sizeof(double) * std::max<size_t>(h->n_stage, 1)) != cudaSuccess)
     return cleanup(fail(PIMC_ENOMEM, "device allocation failed"));
   cudaMemsetAsync(h->d_dpool, 0, sizeof(double) * h->n_dpool, h->stream);
+  cudaMemsetAsync(h->d_tally, 0, sizeof(SlotTally) * nchains, h->stream);
   cudaMemsetAsync(h->d_upool, 0, sizeof(unsigned long long) * h->n_upool, h->stream);
   // bridge coefficient tables: alpha = (m-t)/(m+1-t), sigma = sqrt(2 lambda
   // alpha tau); then the sweeps' closed form of the same bridge, (w, k) =
@@ -654,22 +657,119 @@ SweepArgs sweep_args(Handle *h, const Plan &p) {
   a.warp_scratch_d = p.warp_scratch_d;
   a.warp_bytes = p.warp_bytes;
   a.teams = 0;
+  a.slot_bytes = 0;
+  a.stage_par = 0;
+  a.stage_phase = 0;
+  a.stage_slots = 0;
+  a.tally = h->d_tally;
   return a;
 }
 
-// plain path: one launch of one CTA per chain per sweep, no queue, no graph
+// chains whose windows depend on one another (chain_serial_local) and, of
+// those, the ones that stage_slot takes (stage_by_slots)
+bool desc_serial(const ChainDesc &d) {
+  return ((d.flags & PF_PAIR) && (d.flags & PF_PHYS)) || (d.flags & PF_HARD);
+}
+bool desc_slots(const ChainDesc &d) {
+  return (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && !(d.flags & (PF_HARD | PF_CONTACT | PF_EXACT));
+}
+
+// what the slot-wise staging of chains [c0, c1) needs under their current
+// mixes: slots of the longest chain, staging phases, shared bytes of a CTA of
+// `block` threads.  par as SweepArgs::stage_par.
+struct StagePlan {
+  int slots = 0, phases = 0;
+  size_t smem = 0;
+  bool whole = false;  // some chain is staged by the whole-chain kernel
+};
+StagePlan stage_plan(const Handle *h, int par, int block, int c0, int c1) {
+  StagePlan s;
+  int ell = 0;
+  for (int c = c0; c < c1; ++c) {
+    const ChainDesc &d = h->desc[c];
+    const MixDev &m = h->mix[c];
+    if (par == 1 && !desc_serial(d)) {
+      s.whole = true;
+      continue;
+    }
+    // adapted lengths stay between stage_min and stage_max; the current one may
+    // lie below the minimum until it is adapted
+    const int lo = std::max(2, std::min({m.stage_min, h->umix[c].stage_slices, h->umix[c].stage_max, d.M - 1}));
+    s.slots = std::max(s.slots, (d.M + lo - 1) / lo);
+    s.phases = std::max(s.phases, m.staging_phases);
+    if (desc_slots(d)) ell = std::max(ell, std::min({std::max(m.stage_max, lo), d.M - 1, 64}));
+  }
+  const int nw = block / 32;
+  s.smem = (size_t)nw * window_scratch_doubles() * sizeof(double);
+  if (ell > 0) {
+    const size_t b = slot_scratch_bytes(ell, nw);
+    if (h->max_dyn_smem <= 0 || b <= (size_t)h->max_dyn_smem) s.smem = std::max(s.smem, b);
+  }
+  s.smem = (s.smem + 15) & ~(size_t)15;
+  return s;
+}
+
+// dynamic shared bytes of a fused launch of one CTA per chain: the plan's, or
+// more where the slot-wise staging of its chains fits
+size_t fused_smem(const Handle *h, const Plan &p) {
+  if (p.mode != 0 || p.split) return p.dyn_smem;
+  bool any = false;
+  for (const auto &d : h->desc) any = any || desc_slots(d);
+  if (!any) return p.dyn_smem;
+  const size_t want = (size_t)p.state_bytes + stage_plan(h, 1, p.block, 0, h->nchains).smem;
+  return want > p.dyn_smem && (h->max_dyn_smem <= 0 || want <= (size_t)h->max_dyn_smem) ? want : p.dyn_smem;
+}
+
+// plain path: each chain's sweep as its own launches, no queue, no graph.  A
+// chain of at most block / 4 pair-free windows sweeps in one launch of one CTA
+// (10 particles, 20 slices, 30 windows: 143 us a sweep, 147 in four launches);
+// others get a CTA per staging slot, then one CTA each for the swaps and the
+// rest (64 particles, 32 slices, 128 windows: 0.40 ms a sweep against 0.45).
 int run_plain(Handle *h, long long n) {
   const Plan &p = h->one;
-  CK(sweep_set_smem(p.mode, p.dyn_smem));
+  std::vector<StagePlan> sp(h->nchains);
+  std::vector<char> spec(h->nchains), fused(h->nchains);
+  bool any_fused = false;
+  size_t stage_smem = 0;
+  for (int c = 0; c < h->nchains; ++c) {
+    sp[c] = stage_plan(h, 2, p.block, c, c + 1);
+    stage_smem = std::max(stage_smem, sp[c].smem);
+    spec[c] = !(h->desc[c].flags & (PF_PHYS | PF_HARD | PF_CONTACT));
+    const MixDev &m = h->mix[c];
+    const int ell = std::max(2, std::min({h->umix[c].stage_slices, m.stage_max, h->desc[c].M - 1, 64}));
+    fused[c] = !desc_serial(h->desc[c]) && ell <= 32 &&
+               h->desc[c].N * ((h->desc[c].M + ell - 1) / ell) <= p.block / 4;
+    any_fused = any_fused || fused[c];
+  }
+  if (any_fused) CK(sweep_set_smem(0, p.dyn_smem));
+  CK(stage_slots_set_smem(stage_smem));
+  for (int sc = 0; sc < 2; ++sc) CK(sweep_phase_set_smem(1, 0, sc, 0, p.dyn_smem));
+  CK(sweep_phase_set_smem(2, 0, 0, 0, p.dyn_smem));
   SweepArgs a = sweep_args(h, p);
   a.nchains = 1;
-  a.teams = 1;  // a lone chain is latency-bound: idle warps join its slots
+  a.stage_par = 2;
   CK(cudaEventRecord(h->ev0, h->stream));
   long long launches = 0;
   for (long long s = 0; s < n; ++s)
     for (int c = 0; c < h->nchains; ++c) {
       a.chain0 = c;
-      CK(launch_sweep(a, p.mode, 1, p.block, p.dyn_smem, h->stream));
+      if (fused[c]) {
+        CK(launch_sweep(a, 0, 1, p.block, p.dyn_smem, h->stream));
+        ++launches;
+        continue;
+      }
+      a.stage_slots = sp[c].slots;
+      for (int ph = 0; ph < sp[c].phases; ++ph) {
+        a.stage_phase = ph;
+        CK(launch_stage_slots(a, sp[c].slots, p.block, sp[c].smem, h->stream));
+      }
+      if (sp[c].phases > 0) CK(launch_stage_close(a, h->stream));
+      launches += sp[c].phases + (sp[c].phases > 0);
+      if (h->mix[c].swaps_per_sweep > 0 && h->desc[c].N > 1) {
+        CK(launch_sweep_phase(a, 1, 0, spec[c], 0, 1, p.block, p.dyn_smem, h->stream));
+        ++launches;
+      }
+      CK(launch_sweep_phase(a, 2, 0, 0, 0, 1, p.block, p.dyn_smem, h->stream));
       ++launches;
     }
   CK(cudaEventRecord(h->ev1, h->stream));
@@ -700,7 +800,7 @@ int grid_for(Handle *h, const Plan &p, int phase = -1, int nch = -1) {
   const cudaError_t e = phase >= 0
                             ? sweep_phase_occupancy(phase, p.pwarp[phase], swap_spec(h), p.pregs[phase],
                                                     phase_block(p, phase), phase_smem(p, phase), &per_sm)
-                            : sweep_occupancy(p.mode, p.block, p.dyn_smem, &per_sm);
+                            : sweep_occupancy(p.mode, p.block, fused_smem(h, p), &per_sm);
   if (e != cudaSuccess || per_sm < 1) per_sm = 1;
   const bool warp = phase >= 0 ? p.pwarp[phase] != 0 : p.mode == 1;
   const int units_per_cta = warp ? phase_block(p, phase >= 0 ? phase : 0) / 32 : 1;
@@ -716,19 +816,64 @@ bool launch_teams(Handle *h, const Plan &p) {
   int per_sm = 0;
   if (p.mode != 0) return false;
   const cudaError_t e = p.split ? sweep_phase_occupancy(0, 0, 0, 0, phase_block(p, 0), phase_smem(p, 0), &per_sm)
-                                : sweep_occupancy(p.mode, p.block, p.dyn_smem, &per_sm);
+                                : sweep_occupancy(p.mode, p.block, fused_smem(h, p), &per_sm);
   if (e != cudaSuccess) return false;
   return h->nchains <= per_sm * h->num_sms;
 }
 
 // the dynamic shared-memory attribute of every kernel the plan launches
 cudaError_t plan_set_smem(const Handle *h, const Plan &p) {
-  if (!p.split) return sweep_set_smem(p.mode, p.dyn_smem);
+  if (!p.split) return sweep_set_smem(p.mode, fused_smem(h, p));
+  const StagePlan sp = stage_plan(h, 1, phase_block(p, 0), 0, h->nchains);
+  if (sp.slots > 0) {
+    const cudaError_t e = stage_slots_set_smem(sp.smem);
+    if (e != cudaSuccess) return e;
+  }
   for (int ph = 0; ph < 3; ++ph) {
     const cudaError_t e = sweep_phase_set_smem(ph, p.pwarp[ph], swap_spec(h), p.pregs[ph], phase_smem(p, ph));
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+// one phase of a split sweep of the a.nchains chains that a.order names, from
+// a reset work queue.  Staging: the chains whose windows depend on one another
+// by (chain, slot) items, the others by whole chains.
+cudaError_t issue_phase(Handle *h, const Plan &p, const SweepArgs &a, int ph, long long *launches) {
+  SweepArgs b = a;
+  b.sweeps = 1;
+  if (p.pwarp[ph]) b.warp_bytes = p.pwarp_bytes[ph];
+  bool whole = true;
+  if (ph == 0) {
+    const int block = phase_block(p, 0);
+    const StagePlan sp = stage_plan(h, 1, block, 0, h->nchains);
+    b.stage_par = 1;
+    whole = sp.whole;
+    if (sp.slots > 0 && sp.phases > 0) {
+      b.stage_slots = sp.slots;
+      int per_sm = 0;
+      if (stage_slots_occupancy(block, sp.smem, &per_sm) != cudaSuccess || per_sm < 1) per_sm = 1;
+      const long long items = (long long)sp.slots * a.nchains;
+      const int grid = (int)std::min<long long>(items, (long long)per_sm * h->num_sms);
+      cudaError_t e = cudaSuccess;
+      for (int q = 0; q < sp.phases && e == cudaSuccess; ++q) {
+        b.stage_phase = q;
+        e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
+        if (e == cudaSuccess) e = launch_stage_slots(b, grid, block, sp.smem, h->stream);
+        if (launches) *launches += 1;
+      }
+      if (e == cudaSuccess) e = launch_stage_close(b, h->stream);
+      if (launches) *launches += 1;
+      if (e != cudaSuccess) return e;
+    }
+  }
+  if (!whole) return cudaSuccess;
+  cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
+  if (e == cudaSuccess)
+    e = launch_sweep_phase(b, ph, p.pwarp[ph], swap_spec(h), p.pregs[ph], grid_for(h, p, ph, a.nchains),
+                           phase_block(p, ph), phase_smem(p, ph), h->stream);
+  if (launches) *launches += 1;
+  return e;
 }
 
 // n sweeps of every chain as launches on the stream: one launch of n sweeps,
@@ -739,23 +884,18 @@ cudaError_t plan_set_smem(const Handle *h, const Plan &p) {
 cudaError_t issue_sweeps(Handle *h, const Plan &p, SweepArgs a, int n, long long *launches) {
   if (!p.split) {
     a.sweeps = n;
+    const size_t smem = fused_smem(h, p);
+    if (p.mode == 0) a.slot_bytes = (int)(smem - p.state_bytes);
     cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
     if (e == cudaSuccess)
-      e = launch_sweep(a, p.mode, grid_for(h, p, -1, a.nchains), p.block, p.dyn_smem, h->stream);
+      e = launch_sweep(a, p.mode, grid_for(h, p, -1, a.nchains), p.block, smem, h->stream);
     if (launches) *launches += 1;
     return e;
   }
-  a.sweeps = 1;
   for (int s = 0; s < n; ++s)
     for (int ph = 0; ph < 3; ++ph) {
-      SweepArgs b = a;
-      if (p.pwarp[ph]) b.warp_bytes = p.pwarp_bytes[ph];
-      cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
-      if (e == cudaSuccess)
-        e = launch_sweep_phase(b, ph, p.pwarp[ph], swap_spec(h), p.pregs[ph], grid_for(h, p, ph, a.nchains),
-                               phase_block(p, ph), phase_smem(p, ph), h->stream);
+      const cudaError_t e = issue_phase(h, p, a, ph, launches);
       if (e != cudaSuccess) return e;
-      if (launches) *launches += 1;
     }
   return cudaSuccess;
 }
@@ -980,6 +1120,7 @@ int pimc_destroy(void *handle) {
   cudaFree(h->d_queue);
   cudaFree(h->d_order);
   cudaFree(h->d_iout);
+  cudaFree(h->d_tally);
   cudaFree(h->d_buf);
   cudaFree(h->d_adj);
   cudaFree(h->d_stage);
@@ -1275,6 +1416,13 @@ int pimc_set_move_mix(void *handle, int chain, const pimc_move_mix *mix) {
   }
   CK(cudaMemcpyAsync(h->d_var, v.data(), sizeof(ChainVar) * h->nchains, cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->d_mix, h->mix.data(), sizeof(MixDev) * h->nchains, cudaMemcpyHostToDevice, h->stream));
+  // the captured launches depend on the mixes where chains are staged by slots
+  bool slots = false;
+  for (const auto &d : h->desc) slots = slots || desc_serial(d);
+  if (slots && h->gexec) {
+    cudaGraphExecDestroy(h->gexec);
+    h->gexec = nullptr;
+  }
   return sync_check(h);
 }
 
@@ -1376,18 +1524,7 @@ int pimc_batch_phase_times(void *handle, long long n, double ms[3]) {
   for (long long s = 0; s < n && e == cudaSuccess; ++s) {
     cudaEventRecord(ev[0], h->stream);
     for (int ph = 0; ph < nph && e == cudaSuccess; ++ph) {
-      e = cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->stream);
-      if (e != cudaSuccess) break;
-      if (p.split) {
-        SweepArgs b = a;
-        b.sweeps = 1;
-        if (p.pwarp[ph]) b.warp_bytes = p.pwarp_bytes[ph];
-        e = launch_sweep_phase(b, ph, p.pwarp[ph], swap_spec(h), p.pregs[ph], grid_for(h, p, ph),
-                               phase_block(p, ph), phase_smem(p, ph), h->stream);
-      } else {
-        a.sweeps = 1;
-        e = launch_sweep(a, p.mode, grid_for(h, p), p.block, p.dyn_smem, h->stream);
-      }
+      e = p.split ? issue_phase(h, p, a, ph, nullptr) : issue_sweeps(h, p, a, 1, nullptr);
       if (e == cudaSuccess) e = cudaEventRecord(ev[ph + 1], h->stream);
     }
     if (e == cudaSuccess) e = cudaEventSynchronize(ev[nph]);

@@ -139,13 +139,12 @@ __global__ void k_eval_weights(EvalArgs a) {
   }
   if ((d.flags & PF_PAIR) && (d.flags & PF_PHYS)) {
     __shared__ double wx[WMAX + 1], wy[WMAX + 1];
-    __shared__ unsigned wq[2 * (WMAX + 1)];
+    __shared__ unsigned wq[WMAX + 1];
     __shared__ unsigned long long q[PQ_CAP];
     for (int t = lane; t <= m; t += 32) {
       wx[t] = px(t);
       wy[t] = py(t);
-      wq[2 * t] = j0 + t < M ? c.Q(n, j0 + t) : c.Q(nx, j0 + t - M);
-      wq[2 * t + 1] = qpos(d, wx[t], wy[t]);
+      wq[t] = qpos(d, wx[t], wy[t]);
     }
     __syncwarp();
     WindowSeg seg{&c, n, nx, j0, M, wx, wy, wq};

@@ -36,11 +36,11 @@ namespace pimc {
 constexpr int WMAX = 64;     // largest staging / swap window m handled on the device
 constexpr int TWMAX = 32;    // thread-per-window variant handles m <= TWMAX
 // doubles of per-warp scratch of window_warp: new beads x, y, their external
-// potential, normals (2 per bead; the centres in fixed point once the bridge is
-// drawn), the neighbour queue (96 entries), the old and new beads' mirror
-// words, and 4 doubles through which the warps of a
+// potential, normals (2 per bead; once the bridge is drawn the centres' mirror
+// words, then their fixed-point positions), the neighbour queue (96 entries),
+// the new beads' mirror words, and 4 doubles through which the warps of a
 // staging team exchange their partial sums
-constexpr int TEAM_SLOT_D = 5 * (WMAX + 1) + 96 + (WMAX + 1);
+constexpr int TEAM_SLOT_D = 5 * (WMAX + 1) + 96 + (WMAX + 2) / 2;
 constexpr int WARP_SCRATCH_D = TEAM_SLOT_D + 4;
 
 // move outcomes (PIMC_REJECT / ACCEPT / SKIP / HARDCORE of pimc.h)
@@ -242,6 +242,7 @@ struct InjDraws {
       z[d] = i < n_nrm ? nrm[i] : 0.0;
     }
   }
+  __device__ __forceinline__ void bead_normals_f(int, float &a, float &b) const { a = b = 0.f; }  // sweeps only
   __device__ __forceinline__ void consumed(int cnt) { pn += cnt; }
   __device__ __forceinline__ double normal() {
     if (pn < n_nrm) return nrm[pn++];
@@ -590,6 +591,18 @@ __device__ __forceinline__ double teleport_s(double x, double L, double inv2L) {
 }
 
 __device__ __forceinline__ double sgn(double v) { return v > 0.0 ? 1.0 : (v < 0.0 ? -1.0 : 0.0); }
+
+// a bridge's end e taken to the start s's side of the periodic box; returns
+// s - e (out of line: rarely taken, five FP64 instructions otherwise)
+static __device__ __noinline__ double2 unwrap_end_far(double s, double e, double L) {
+  e += sgn(s) * (2.0 * L);
+  return make_double2(s - e, e);
+}
+__device__ __forceinline__ double unwrap_end(double s, double &e, double L) {
+  const double2 r = unwrap_end_far(s, e, L);
+  e = r.y;
+  return r.x;
+}
 
 // engine-known external potential: hcoef |r|^2 + V0 sum sin^2(pi r_d / a)
 // the optical lattice's normalized intensity (examples/tools/potentialtools.jl:1-16):
@@ -1195,9 +1208,11 @@ struct WindowSeg {
   const CV *c;
   int n, nx, j0, M;
   const double *px, *py;
-  const unsigned *pq;   // mirror words of the old and the new beads, in turn
+  const unsigned *pq;   // mirror words of the new beads
   __device__ __forceinline__ int own(int t) const { return j0 + t < M ? n : nx; }
-  __device__ __forceinline__ unsigned curq(int side, int t) const { return pq[2 * t + side]; }
+  __device__ __forceinline__ unsigned curq(int side, int t) const {
+    return side ? pq[t] : c->Q(own(t), slice(t));
+  }
   __device__ __forceinline__ unsigned nxtq(int side, int t) const { return curq(side, t + 1); }
   __device__ __forceinline__ int slice(int t) const { return j0 + t < M ? j0 + t : j0 + t - M; }
   __device__ __forceinline__ void cur(int side, int t, double &x, double &y) const {
@@ -1346,6 +1361,70 @@ __device__ int window_thread(const CV &c, int n, int j0, int m, D &dr, bool rewr
   return acc ? 1 : 0;
 }
 
+// the interior beads t = 1 .. m-1 of a sweep's bridge from (sx, sy) to (ex, ey),
+// by one warp into X[t], Y[t]: the closed form (bridge_w), whose sum of w_t
+// z_t is a prefix scan over 32-bead chunks; both coordinates at once in the
+// half warps where m <= 17 (the scan's additions are the same, so every launch
+// shape gets the same bits)
+template <class D>
+__device__ __forceinline__ void bridge_beads(const CV &c, int m, const D &dr, double sx, double sy,
+                                             double ex, double ey, double *X, double *Y, int lane) {
+  const int dim = c.dim;
+  const double inv_m = bridge_w(c, m, 0).x;
+  if (m <= 17) {
+    const int t = (lane & 15) + 1, k = lane >> 4;
+    float z0 = 0.f, z1 = 0.f;
+    if (lane < m - 1) dr.bead_normals_f(lane, z0, z1);
+    z1 = __shfl_sync(0xffffffffu, z1, lane & 15);
+    double v = 0.0, kt = 0.0;
+    if (t < m) {
+      const double2 wk = bridge_w(c, m, t);
+      v = (double)(k ? z1 : z0) * wk.x;
+      kt = wk.y;
+    }
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) {
+      const double vp = __shfl_up_sync(0xffffffffu, v, off, 16);
+      if ((lane & 15) >= off) v += vp;
+    }
+    const double e = k ? ey : ex, s = k ? sy : sx;
+    const double p = fma(kt, (s - e) * inv_m + v, e);
+    if (t < m && k < dim) (k ? Y : X)[t] = p;
+  } else {
+    double cx = (sx - ex) * inv_m, cy = (sy - ey) * inv_m;
+    for (int c0 = 1; c0 < m; c0 += 32) {
+      const int t = c0 + lane;
+      const bool act = t < m;
+      float z0 = 0.f, z1 = 0.f;
+      double2 wk = make_double2(0.0, 0.0);
+      if (act) {
+        dr.bead_normals_f(t - 1, z0, z1);
+        wk = bridge_w(c, m, t);
+      }
+      double vx = (double)z0 * wk.x, vy = 0.0;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const double px = __shfl_up_sync(0xffffffffu, vx, off);
+        if (lane >= off) vx += px;
+      }
+      cx += vx;
+      if (act) X[t] = fma(wk.y, cx, ex);
+      cx = __shfl_sync(0xffffffffu, cx, 31);
+      if (dim > 1) {
+        vy = (double)z1 * wk.x;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const double py = __shfl_up_sync(0xffffffffu, vy, off);
+          if (lane >= off) vy += py;
+        }
+        cy += vy;
+        if (act) Y[t] = fma(wk.y, cy, ey);
+        cy = __shfl_sync(0xffffffffu, cy, 31);
+      }
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Levy staging window, one warp: pair terms (physical semantics) and the
 // hard-core retry loop.  sb: per-warp shared scratch of 5*(WMAX+1) doubles
@@ -1374,7 +1453,9 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
   if (fabs(sx - ex) > L) ex += sgn(sx) * (2.0 * L);
   if (dim > 1 && fabs(sy - ey) > L) ey += sgn(sy) * (2.0 * L);
   int fail = 0;
-  if (!hard) {
+  if (!hard && D::kSweep) {
+    bridge_beads(c, m, dr, sx, sy, ex, ey, sx_, sy_, lane);
+  } else if (!hard) {
     for (int t = 1 + lane; t < m; t += 32) {
       double z[2];
       dr.bead_normals(t - 1, dim, z);
@@ -1434,11 +1515,7 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
     sx_[t] = qx;
     sy_[t] = qy;
     svb[t] = vext(d, qx, qy);
-    if (phys_pair) {
-      const int a = j0 + t;
-      sq[2 * t] = a < M ? c.Q(n, a) : c.Q(nx, a - M);
-      sq[2 * t + 1] = qpos(d, qx, qy);
-    }
+    if (phys_pair) sq[t] = qpos(d, qx, qy);
   }
   __syncwarp();
   double wi = 0.0, wu = 0.0;
@@ -1457,8 +1534,15 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
       const float lu = u > 0.0 ? logf((float)u) : -INFINITY;
       const float dw = (float)warp_sum(wu - wi), gh = (float)(-d.mhtau_g);
       const ScanSkip<2> skip{n, -1, true};
+      unsigned *cq = reinterpret_cast<unsigned *>(sz);
+      for (int k = lane; k <= m; k += 32) {
+        cq[2 * k] = seg.curq(0, k);
+        cq[2 * k + 1] = sq[k];
+      }
+      __syncwarp();
       PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
-      scan_mirror<2>(c, j0, m, sq, skip, 0, 1, e, lane, NoStop());
+      scan_mirror<2>(c, j0, m, cq, skip, 0, 1, e, lane, NoStop());
+      __syncwarp();
       float t, r;
       est_lane(e, -1.f, t, r);
       dec = decide_f(fmaf(gh, warp_sum(t), dw), fabsf(gh) * warp_sum(r) + 1e-6f * fabsf(dw), lu);
@@ -1542,7 +1626,6 @@ __device__ int window_team(const CV &c, const Team &tm, int n, int j0, int m, D 
   const double L = d.L, inv2L = d.inv2L, mhtau = -0.5 * d.tau;
   double *b0 = sb(0);
   double *sx_ = b0, *sy_ = b0 + (WMAX + 1), *svb = b0 + 2 * (WMAX + 1);
-  double *sz = b0 + 3 * (WMAX + 1);
   unsigned *sq = (unsigned *)(b0 + 5 * (WMAX + 1) + 96);
   const int nx = c.next[n];
   const int jend = j0 + m;
@@ -1551,23 +1634,7 @@ __device__ int window_team(const CV &c, const Team &tm, int n, int j0, int m, D 
   double ex = c.X(0, oe, je), ey = c.Xd(1, oe, je);
   if (fabs(sx - ex) > L) ex += sgn(sx) * (2.0 * L);
   if (dim > 1 && fabs(sy - ey) > L) ey += sgn(sy) * (2.0 * L);
-  for (int t = 1 + tid; t < m; t += nt) {
-    double z[2];
-    dr.bead_normals(t - 1, dim, z);
-    sz[2 * t] = z[0];
-    sz[2 * t + 1] = dim > 1 ? z[1] : 0.0;
-  }
-  tm.sync();
-  if (tm.w == 0 && lane < dim) {
-    double p = lane == 0 ? sx : sy;
-    const double e = lane == 0 ? ex : ey;
-    double *dst = lane == 0 ? sx_ : sy_;
-    for (int t = 1; t < m; ++t) {
-      const double2 ab = bridge_coef(c, m, t);
-      p = ab.x * p + (1.0 - ab.x) * e + sz[2 * t + lane] * ab.y;
-      dst[t] = p;
-    }
-  }
+  if (tm.w == 0) bridge_beads(c, m, dr, sx, sy, ex, ey, sx_, sy_, lane);
   tm.sync();
   for (int t = tid; t <= m; t += nt) {
     double qx = t == 0 ? sx : (t == m ? ex : sx_[t]);
@@ -1577,9 +1644,7 @@ __device__ int window_team(const CV &c, const Team &tm, int n, int j0, int m, D 
     sx_[t] = qx;
     sy_[t] = qy;
     svb[t] = vext(d, qx, qy);
-    const int a = j0 + t;
-    sq[2 * t] = a < M ? c.Q(n, a) : c.Q(nx, a - M);
-    sq[2 * t + 1] = qpos(d, qx, qy);
+    sq[t] = qpos(d, qx, qy);
   }
   tm.sync();
   double wi = 0.0, wu = 0.0;

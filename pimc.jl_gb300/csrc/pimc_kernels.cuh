@@ -86,8 +86,8 @@ struct SwapSums {
   float est[16][2];
 };
 // weights of particle chunks at an odd stride (no bank conflicts for the lanes'
-// sequential sums): room for two buffers of 32 * (chunk | 1) floats
-constexpr int SWAP_WPAD = 64;
+// sequential sums): 32 * (chunk | 1) floats, two buffers of which exceed N
+// doubles by at most 504 bytes
 __host__ __device__ inline int swap_wstride(int N) { return 32 * (((N + 31) / 32) | 1); }
 
 // windows of a sweep's swap_sweep: at most SWAP_LANES links
@@ -96,37 +96,52 @@ constexpr int SWAP_LANES = 31, SWAP_BEADS = SWAP_LANES + 1;
 // shared scratch of the swap
 struct SwapScratch {
   double *w;                                   // N heat-bath weights (sweeps: two buffers of
-                                               // swap_wstride floats)
+                                               // swap_wstride floats, into z's first quarter)
   double *r1x, *r1y, *r2x, *r2y, *vb1, *vb2;   // WMAX+1 each
   double *z;                                   // 4*WMAX normals
   unsigned long long *q;                       // PQ_CAP neighbour queue per warp
   unsigned *q1, *q2;                           // WMAX+1 mirror words each
   int *iv;                                     // 4 ints: group broadcasts
-  uint4 *cq;                                   // mirror words per bead: old 1, new 1, old 2, new 2
-  SwapSums *sums;                              // a sweep's partial sums
-  SwapDraws *draws;                            // a sweep's next choices
+  // swap_sweep's, in the second halves of r1x .. vb2 (its windows have at most
+  // SWAP_LANES links): mirror words per bead (old 1, new 1, old 2, new 2), a
+  // sweep's next choices, partial sums
+  uint4 *cq;
+  SwapDraws *draws;
+  SwapSums *sums;
   static __host__ __device__ size_t bytes(int N, int nwarps) {
-    return sizeof(uint4) * SWAP_BEADS + sizeof(double) * ((((size_t)N + 1) & ~(size_t)1) + SWAP_WPAD + 6 * (WMAX + 1) + 4 * WMAX) +
+    return sizeof(double) * ((size_t)N + 6 * (WMAX + 1) + 4 * WMAX) +
            sizeof(unsigned long long) * PQ_CAP * (size_t)nwarps +
-           sizeof(unsigned) * 2 * (WMAX + 1) + sizeof(int) * 4 + sizeof(SwapDraws) +
-           sizeof(SwapSums);
+           sizeof(unsigned) * 2 * (WMAX + 1) + sizeof(int) * 4;
   }
   __device__ void carve(void *base, int N, int nwarps) {
-    cq = (uint4 *)base;
-    double *p = (double *)(cq + SWAP_BEADS);
-    w = p; p += ((N + 1) & ~1) + SWAP_WPAD;
-    r1x = p; p += WMAX + 1; r1y = p; p += WMAX + 1;
-    r2x = p; p += WMAX + 1; r2y = p; p += WMAX + 1;
-    vb1 = p; p += WMAX + 1; vb2 = p; p += WMAX + 1;
+    double *p = (double *)base;
+    double *r = p;  // first: 16-byte aligned
+    p += 6 * (WMAX + 1);
+    w = p; p += N;
     z = p; p += 4 * WMAX;
+    r1x = r; r1y = r + (WMAX + 1);
+    r2x = r + 2 * (WMAX + 1); r2y = r + 3 * (WMAX + 1);
+    vb1 = r + 4 * (WMAX + 1); vb2 = r + 5 * (WMAX + 1);
     q = (unsigned long long *)p;
     q1 = (unsigned *)(q + (size_t)PQ_CAP * nwarps);
     q2 = q1 + (WMAX + 1);
     iv = (int *)(q2 + (WMAX + 1));
-    sums = (SwapSums *)(iv + 4);  // 8-byte aligned: an even count of words above
+    cq = (uint4 *)r;
+    sums = (SwapSums *)(cq + SWAP_BEADS);
     draws = (SwapDraws *)(sums + 1);
   }
+  // the layout of swap_sweep: bead arrays of SWAP_BEADS after its own
+  // structures
+  __device__ void carve_sweep() {
+    double *r = (double *)(draws + 1);
+    r1x = r; r1y = r + SWAP_BEADS;
+    r2x = r + 2 * SWAP_BEADS; r2y = r + 3 * SWAP_BEADS;
+    vb1 = r + 4 * SWAP_BEADS; vb2 = r + 5 * SWAP_BEADS;
+  }
 };
+static_assert(sizeof(uint4) * SWAP_BEADS + sizeof(SwapSums) + sizeof(SwapDraws) + 48 * SWAP_BEADS <=
+                  sizeof(double) * 6 * (WMAX + 1) && sizeof(SwapSums) % 8 == 0 && sizeof(SwapDraws) % 8 == 0,
+              "swap_sweep's scratch fits swap_group's");
 
 // scratch of a centre-of-mass move: cycle members and their index, the
 // shifted single path (x, y, external potential, mirror words), and one
@@ -1015,18 +1030,6 @@ __device__ __forceinline__ void swap_draws(SwapDraws &D, const ChainDesc &d, uns
   }
 }
 
-// a bridge's end e taken to the start s's side of the periodic box; returns
-// s - e (out of line: rarely taken, five FP64 instructions otherwise)
-static __device__ __noinline__ double2 unwrap_end_far(double s, double e, double L) {
-  e += sgn(s) * (2.0 * L);
-  return make_double2(s - e, e);
-}
-__device__ __forceinline__ double unwrap_end(double s, double &e, double L) {
-  const double2 r = unwrap_end_far(s, e, L);
-  e = r.y;
-  return r.x;
-}
-
 template <bool WARP, int SPEC>
 __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, unsigned wmagic, SwapScratch &S,
                           double *red) {
@@ -1060,7 +1063,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
   const unsigned E1q = c.Q(e1p, se);
   GenDraws dr = gen_draws(ss);
   float *Sw = reinterpret_cast<float *>(S.w) + buf * wstride;
-  float *Sz = reinterpret_cast<float *>(S.z) + buf * (4 * WMAX);
+  float *Sz = reinterpret_cast<float *>(S.z) + 256 + buf * (4 * SWAP_BEADS);  // past the weights' excess
   // the bridges' normals depend on the move's stream alone
   for (int k = tid; k < 2 * (m - 1); k += nt) {
     float z0, z1;
@@ -1381,7 +1384,8 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
         if (level == 0) {
           scan_mirror<4>(c, j0, m, reinterpret_cast<const unsigned *>(S.cq), skip, warp, nwarps, e, lane, stop);
         } else {
-          uint2 *cf = reinterpret_cast<uint2 *>(Sz);  // the normals are spent
+          // both buffers' normals are spent
+          uint2 *cf = reinterpret_cast<uint2 *>(reinterpret_cast<float *>(S.z) + 256);
           for (int k = tid; k < 4 * (m + 1); k += nt) {
             double x, y;
             seg_of((k >> 1) & 1).cur(k & 1, k >> 2, x, y);

@@ -8,6 +8,12 @@
 
 namespace pimc {
 
+// counters of a chain's slots within one sweep's staging
+struct SlotTally {
+  unsigned long long beads;
+  unsigned att, acc;
+};
+
 struct SweepArgs {
   const ChainDesc *desc;
   ChainVar *var;
@@ -23,6 +29,13 @@ struct SweepArgs {
   int state_bytes;    // shared bytes reserved for staging a chain's state
   int warp_scratch_d; // doubles of scratch per warp
   int warp_bytes;     // warp-per-chain mode: scratch bytes of each warp
+  int slot_bytes;     // shared bytes a CTA's slot-wise staging may use (0: none)
+  int stage_par;      // staging by slots: 1 = only chains whose windows depend on
+                      // one another, 2 = every chain (k_stage_slots); the staging
+                      // kernel of whole chains skips those
+  int stage_phase;    // the staging phase that k_stage_slots runs
+  int stage_slots;    // slots per chain of its queue (the longest chain's)
+  struct SlotTally *tally;  // [chains] k_stage_slots' counters, zero between phases
   int teams;          // 1: staging slots walked by teams of warps (latency-bound
                       // launches whose chains all fit on the GPU at once)
 };
@@ -95,6 +108,14 @@ cudaError_t launch_sweep_phase(const SweepArgs &a, int phase, int warp, int spec
 cudaError_t sweep_phase_set_smem(int phase, int warp, int spec, int regs, size_t smem);
 cudaError_t sweep_phase_occupancy(int phase, int warp, int spec, int regs, int block, size_t smem,
                                   int *blocks_per_sm);
+// staging by (chain, slot) items from the work queue a.queue (a.order names
+// the chains), or without one a CTA per item; and the end of the phases
+cudaError_t launch_stage_slots(const SweepArgs &a, int grid, int block, size_t smem, cudaStream_t s);
+cudaError_t launch_stage_close(const SweepArgs &a, cudaStream_t s);
+cudaError_t stage_slots_set_smem(size_t smem);
+cudaError_t stage_slots_occupancy(int block, size_t smem, int *blocks_per_sm);
+// shared bytes of slot-wise staging for windows of at most ell slices
+size_t slot_scratch_bytes(int ell, int nwarps);
 size_t sweep_ctl_bytes();
 cudaError_t sweep_occupancy(int mode, int block, size_t smem, int *blocks_per_sm);
 cudaError_t launch_attempt(const AttemptArgs &a, size_t smem, cudaStream_t s);

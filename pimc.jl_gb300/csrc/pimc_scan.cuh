@@ -39,67 +39,70 @@ struct ScanSkip {
   }
 };
 
-// the lane's sums over the particles 32 (part, part + nparts, ...) + lane, from
-// the mirror: e.so / e.sn old and new sums of exp(-r_a^2/2s^2) +
-// exp(-r_b^2/2s^2) over the links and the partners within reach at the link's
-// start, e.bo / e.bn bounds on their distance from the exact sums (a mirror
-// distance is within kQErr units of the exact one; ChainDesc::est_a, est_b).
-// cq[t * NC + k]: mirror word of centre k at bead t, t = 0 .. m.  stop(e) ends
-// the scan early; it is asked after every block of particles.
+// a lane's sums over one particle, from the mirror: e.so / e.sn old and new
+// sums of exp(-r_a^2/2s^2) + exp(-r_b^2/2s^2) over the links whose start has
+// the particle within reach, e.bo / e.bn bounds on their distance from the
+// exact sums (a mirror distance is within kQErr units of the exact one;
+// ChainDesc::est_a, est_b).  cq[t * NC + k]: mirror word of centre k at bead t,
+// t = 0 .. m; word(t): the particle's; on(k): whether centre k counts it.
+template <int NC, class Word, class On>
+__device__ __forceinline__ void scan_block(const ChainDesc &d, int m, const unsigned *cq, const Word &word,
+                                           const On &on, PairEst &e) {
+  const float ca = d.est_a, cb = d.est_b, cx = d.est_x;
+  unsigned lo[NC], hi[NC];
+  float ep[NC], rp[NC], wp[NC], gp[NC];
+#pragma unroll
+  for (int k = 0; k < NC; ++k) {
+    lo[k] = on(k) ? d.q_lim_lo : 0u;
+    hi[k] = on(k) ? d.q_lim_hi + 1u : 0u;
+    ep[k] = rp[k] = wp[k] = gp[k] = 0.f;
+  }
+  // the slices' words four beads ahead: a step takes a few hundred cycles, a
+  // word from L2 up to a thousand
+  unsigned q0 = word(0), q1 = word(min(1, m)), q2 = word(min(2, m)), q3 = word(min(3, m));
+  for (int t = 0; t <= m; ++t) {
+    const unsigned q = q0;
+    q0 = q1;
+    q1 = q2;
+    q2 = q3;
+    if (t + 4 <= m) q3 = word(t + 4);
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      const unsigned d2 = qdist2(cq[t * NC + k], q);
+      const float f = (float)d2, x = ex2_approx(f * cx);
+      const float r = fmaf(x, fmaf(ca, f, cb), 1e-30f);
+      const float v = ep[k] + x, ve = rp[k] + r;
+      float &s = (k & 1) ? e.sn : e.so, &bd = (k & 1) ? e.bn : e.bo;
+      s = fmaf(wp[k], v, s);
+      bd = fmaf(wp[k], ve, bd);
+      bd = fmaf(gp[k], v + ve, bd);
+      ep[k] = x;
+      rp[k] = r;
+      // surely within reach: weight 1; unsettled: half the link, within half
+      const bool in = d2 < lo[k], may = d2 < hi[k];
+      gp[k] = may && !in ? 0.5f : 0.f;
+      wp[k] = in ? 1.f : gp[k];
+    }
+  }
+  e.ko += m * (NC / 2) * 3;
+  e.kn += m * (NC / 2) * 3;
+}
+
+// the lane's sums over the particles 32 (part, part + nparts, ...) + lane, the
+// block `leave` left out; stop(e) ends the scan early and is asked after every
+// block of particles
 template <int NC, class Stop>
 __device__ __forceinline__ bool scan_mirror(const CV &c, int j0, int m, const unsigned *cq,
                                             const ScanSkip<NC> &skip, int part, int nparts, PairEst &e,
-                                            int lane, const Stop &stop) {
-  const ChainDesc &d = *c.d;
+                                            int lane, const Stop &stop, int leave = -1) {
   const int N = c.N, M = c.M;
-  const float ca = d.est_a, cb = d.est_b, cx = d.est_x;
   const bool wraps = j0 + m >= M;
   for (int b0 = 32 * part; b0 < N; b0 += 32 * nparts) {
+    if (b0 == leave) continue;
     const int b = b0 + lane, bl = min(b, N - 1);
     const int nb = wraps ? c.next[bl] : bl;
-    unsigned lo[NC], hi[NC];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      const bool on = b < N && !skip(k, b);
-      lo[k] = on ? d.q_lim_lo : 0u;
-      hi[k] = on ? d.q_lim_hi + 1u : 0u;
-    }
-    float ep[NC], rp[NC], wp[NC], gp[NC];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) ep[k] = rp[k] = wp[k] = gp[k] = 0.f;
-    // the slices' words four beads ahead: a step takes a few hundred cycles, a
-    // word from L2 up to a thousand
-    auto word = [&](int t) -> unsigned {
-      const int a = j0 + min(t, m);
-      return a < M ? c.Q(bl, a) : c.Q(nb, a - M);
-    };
-    unsigned q0 = word(0), q1 = word(1), q2 = word(2), q3 = word(3);
-    for (int t = 0; t <= m; ++t) {
-      const unsigned q = q0;
-      q0 = q1;
-      q1 = q2;
-      q2 = q3;
-      if (t + 4 <= m) q3 = word(t + 4);
-#pragma unroll
-      for (int k = 0; k < NC; ++k) {
-        const unsigned d2 = qdist2(cq[t * NC + k], q);
-        const float f = (float)d2, x = ex2_approx(f * cx);
-        const float r = fmaf(x, fmaf(ca, f, cb), 1e-30f);
-        const float v = ep[k] + x, ve = rp[k] + r;
-        float &s = (k & 1) ? e.sn : e.so, &bd = (k & 1) ? e.bn : e.bo;
-        s = fmaf(wp[k], v, s);
-        bd = fmaf(wp[k], ve, bd);
-        bd = fmaf(gp[k], v + ve, bd);
-        ep[k] = x;
-        rp[k] = r;
-        // surely within reach: weight 1; unsettled: half the link, within half
-        const bool in = d2 < lo[k], may = d2 < hi[k];
-        gp[k] = may && !in ? 0.5f : 0.f;
-        wp[k] = in ? 1.f : gp[k];
-      }
-    }
-    e.ko += m * (NC / 2) * 3;
-    e.kn += m * (NC / 2) * 3;
+    scan_block<NC>(*c.d, m, cq, [&](int t) { return j0 + t < M ? c.Q(bl, j0 + t) : c.Q(nb, j0 + t - M); },
+                   [&](int k) { return b < N && !skip(k, b); }, e);
     if (stop(e)) return true;
   }
   return false;

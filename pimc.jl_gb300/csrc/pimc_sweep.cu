@@ -25,6 +25,156 @@ namespace pimc {
 __global__ void __launch_bounds__(512, 1) k_sweep_stage(SweepArgs a) { sweep_cta<SW_STAGE>(a); }
 __global__ void __launch_bounds__(512, 1) k_sweep_rest(SweepArgs a) { sweep_cta<SW_REST>(a); }
 
+// Staging with a CTA per (chain, slot): the slots of a phase share only their
+// fixed boundary slices, so they run on as many SMs as there are slots.  For
+// chains whose windows depend on one another (each slot a serial walk), and
+// for every chain of a launch too small to fill the GPU with whole chains.
+// Items in chain order (longest first), a.stage_slots per chain, the ones past
+// a chain's own slots empty.  The slots add their counts to the chain's tally;
+// k_stage_close adds them to the chain's counters and adapts the window length
+// (close_phase) once every slot is done -- in a launch of its own, because the
+// slots' items read the length.  A chain of 1024 particles (64 slices, four
+// slots) went from 57 to 7.9 ms of staging, 512 chains of 8 to 512 particles from
+// 72-89 to 8.4 ms.
+__global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ SmemCtl sc;
+  __shared__ double red[256];
+  __shared__ unsigned bits[(kMaxParticles + 31) / 32];
+  __shared__ int s_item;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int nitems = a.nchains * a.stage_slots;
+  for (int iter = 0;; ++iter) {
+    if (tid == 0) s_item = a.queue ? atomicAdd(a.queue, 1) : (iter == 0 ? (int)blockIdx.x : nitems);
+    __syncthreads();
+    const int item = s_item;
+    if (item >= nitems) break;
+    const int ci = item / a.stage_slots, s = item % a.stage_slots;
+    const int ch = a.order ? a.order[ci] : a.chain0 + ci;
+    for (int k = tid; k < (int)(sizeof(ChainDesc) / 4); k += blockDim.x)
+      reinterpret_cast<unsigned *>(&sc.d)[k] = reinterpret_cast<const unsigned *>(a.desc + ch)[k];
+    for (int k = tid; k < (int)(sizeof(MixDev) / 4); k += blockDim.x)
+      reinterpret_cast<unsigned *>(&sc.mix)[k] = reinterpret_cast<const unsigned *>(a.mix + ch)[k];
+    if (tid == 0) {
+      const ChainVar &v = a.var[ch];
+      sc.v.sweep = v.sweep;
+      sc.v.stage_m = v.stage_m;
+      sc.v.err = v.err;
+      sc.chain = ch;
+    }
+    __syncthreads();
+    const ChainDesc &d = sc.d;
+    const int N = d.N, M = d.M, ph = a.stage_phase;
+    const int ell = max(2, min(sc.v.stage_m, min(M - 1, WMAX))), k = (M + ell - 1) / ell;
+    const bool serial = chain_serial_local(d);
+    if (s >= k || ph >= sc.mix.staging_phases || (a.stage_par == 1 && !serial) || sc.v.err != 0) {
+      __syncthreads();
+      continue;
+    }
+    CV c = make_cv(&sc.d, a.dpool, a.ipool, a.upool);
+    const bool ok = next_is_permutation<false>(c.next, N, bits);
+    int n_att = 0, n_acc = 0;
+    long long n_bead = 0;
+    if (!ok) {
+      if (tid == 0) a.var[ch].err = DERR_STATE;
+    } else {
+      const unsigned long long sweep = sc.v.sweep;
+      const int o = min(M - 1, (int)(make_stream(d, sweep, PH_STAGE_OFF, (unsigned)ph).uni(0) * M));
+      const int budget = (int)dyn_smem_bytes();
+      // one slot, or several where a restored window length makes more slots
+      // than the launch counted on
+      for (int sl = s; sl < k; sl += a.stage_slots) {
+        const int len = sl < k - 1 ? ell : M - (k - 1) * ell, st = (o + sl * ell) % M;
+        const unsigned item0 = (unsigned)(ph * (N * k) + sl * N);
+        if (len < 2) continue;
+        if (stage_by_slots(d) && SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)budget) {
+          stage_slot(c, sweep, item0, ell, st, len, smem, red, n_att, n_acc, n_bead);
+        } else if (!serial && ell <= TWMAX) {
+          for (int n = tid; n < N; n += blockDim.x) {
+            GenDraws dr = gen_draws(make_stream(d, sweep, PH_STAGE, item0 + n));
+            const int m = min(len, 2 + (int)(dr.s.uni(DRAW_CHOICE) * (ell - 1)));
+            n_acc += window_thread(c, n, st, m, dr, false, nullptr);
+            n_att += 1;
+            n_bead += m - 1;
+          }
+        } else {
+          // a warp per window (pair-free), the first warp walking the slot (hard
+          // core), or the CTA as a team on each window (contact table, exact
+          // decisions)
+          double *wsb = (double *)smem + (size_t)warp * a.warp_scratch_d;
+          const bool team = serial && !(d.flags & PF_HARD) && nwarps > 1;
+          const Team tm{warp, nwarps, 1};
+          for (int n = serial ? 0 : warp; n < N; n += serial ? 1 : nwarps) {
+            if (serial && !team && warp > 0) break;
+            GenDraws dr = gen_draws(make_stream(d, sweep, PH_STAGE, item0 + n));
+            const int m = min(len, 2 + (int)(dr.s.uni(DRAW_CHOICE) * (ell - 1)));
+            const int r = team ? window_team(c, tm, n, st, m, dr, (double *)smem, a.warp_scratch_d)
+                               : window_warp(c, n, st, m, dr, false, wsb, nullptr);
+            if (lane == 0 && (!team || warp == 0)) {
+              n_att += 1;
+              n_acc += r == RES_ACCEPT;
+              if (r != RES_HARDCORE) n_bead += m - 1;
+            }
+          }
+          __syncthreads();
+        }
+      }
+    }
+    __syncwarp();
+    n_att = __reduce_add_sync(0xffffffffu, n_att);
+    n_acc = __reduce_add_sync(0xffffffffu, n_acc);
+    n_bead = __reduce_add_sync(0xffffffffu, (int)n_bead);
+    if (lane) n_att = 0;
+    if (n_att) {
+      SlotTally *t = a.tally + ch;
+      atomicAdd(&t->att, (unsigned)n_att);
+      atomicAdd(&t->acc, (unsigned)n_acc);
+      atomicAdd(&t->beads, (unsigned long long)n_bead);
+    }
+    __syncthreads();
+  }
+}
+
+// the end of the slots' staging phases: close_phase of every chain they served
+__global__ void k_stage_close(SweepArgs a) {
+  const int ci = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ci >= a.nchains) return;
+  const int ch = a.order ? a.order[ci] : a.chain0 + ci;
+  SlotTally *t = a.tally + ch;
+  if (t->att == 0u) return;
+  const MixDev &mix = a.mix[ch];
+  ChainVar &v = a.var[ch];
+  v.att[MV_STAGE] += t->att;
+  v.acc[MV_STAGE] += t->acc;
+  v.bead_updates += (double)t->beads;
+  v.beads_kind[MV_STAGE] += (double)t->beads;
+  if (mix.adapt) {
+    int m = v.stage_m;
+    adapt_slices(m, (double)t->acc / (double)t->att, mix.stage_min, mix.stage_max, mix.stage_minacc,
+                 mix.stage_maxacc);
+    v.stage_m = m;
+  }
+  *t = SlotTally{};
+}
+
+cudaError_t launch_stage_slots(const SweepArgs &a, int grid, int block, size_t smem, cudaStream_t s) {
+  k_stage_slots<<<grid, block, smem, s>>>(a);
+  return cudaGetLastError();
+}
+cudaError_t launch_stage_close(const SweepArgs &a, cudaStream_t s) {
+  k_stage_close<<<(a.nchains + 127) / 128, 128, 0, s>>>(a);
+  return cudaGetLastError();
+}
+cudaError_t stage_slots_set_smem(size_t smem) {
+  return cudaFuncSetAttribute(k_stage_slots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+cudaError_t stage_slots_occupancy(int block, size_t smem, int *blocks_per_sm) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_stage_slots, block, smem);
+}
+size_t slot_scratch_bytes(int ell, int nwarps) {
+  return (SlotScratch::bytes(ell + 1, nwarps) + 15) & ~(size_t)15;
+}
+
 // ---------------------------------------------------------------------------
 // state maintenance: layout transposes, init_world, cached links + mirror,
 // measurements

@@ -11,6 +11,7 @@
 
 #include "pimc_kernels.cuh"
 #include "pimc_launch.h"
+#include "pimc_stage.cuh"
 
 namespace pimc {
 
@@ -37,6 +38,12 @@ __device__ __forceinline__ CV make_cv(const ChainDesc *d, double *dpool, int *ip
 // moves whose acceptance depends on other paths at the same slice
 __device__ __forceinline__ bool chain_serial_local(const ChainDesc &d) {
   return ((d.flags & PF_PAIR) && (d.flags & PF_PHYS)) || (d.flags & PF_HARD);
+}
+
+// chains whose staging windows go by slots (stage_slot): pair action under the
+// physical rules, bounded decisions
+__device__ __forceinline__ bool stage_by_slots(const ChainDesc &d) {
+  return (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && !(d.flags & (PF_HARD | PF_CONTACT | PF_EXACT));
 }
 
 // next[] of a chain must be a permutation of 0..N-1: every value in range
@@ -155,7 +162,7 @@ __device__ void close_phase(SmemCtl &sc, double *red, int q, double (&t)[4]) {
 
 template <bool WARP, int PH, int SPEC = SWAP_ANY>
 __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *scratch,
-                          int warp_scratch_d, bool teams) {
+                          int warp_scratch_d, bool teams, int slot_bytes = 0) {
   using G = Group<WARP>;
   const ChainDesc &d = sc.d;
   const MixDev &mix = sc.mix;
@@ -203,9 +210,25 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
     const Stream so = make_stream(d, sweep, PH_STAGE_OFF, (unsigned)ph);
     const int o = min(M - 1, (int)(so.uni(0) * M));
     const int items = N * k;
-    const bool lists = serial_local && build_lists();
+    const bool slots = !WARP && slot_bytes > 0 && stage_by_slots(d) &&
+                       SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)slot_bytes;
+    const bool lists = serial_local && !slots && build_lists();
     const CV &cw = lists ? cq : c;
-    if (!serial_local) {
+    if (slots) {
+      int n_att = 0, n_acc = 0;
+      long long n_bead = 0;
+      for (int s = 0; s < k; ++s) {
+        const int len = s < k - 1 ? ell : M - (k - 1) * ell;
+        if (len >= 2)
+          stage_slot_call(c, sweep, (unsigned)(ph * items + s * N), ell, (o + s * ell) % M, len, scratch, red,
+                          n_att, n_acc, n_bead);
+      }
+      if (tid == 0) {
+        tal[0] += n_att;
+        tal[1] += n_acc;
+        tal[3] += (double)n_bead;
+      }
+    } else if (!serial_local) {
       // every window of the phase is independent: slot s of particle n moves
       // the beads strictly inside its slot; item order s*N + n makes
       // neighbouring threads touch neighbouring particles of one slice
@@ -288,6 +311,8 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
   if ((PH & SW_SWAP) && N > 1 && mix.swaps_per_sweep > 0) {
     SwapScratch S;
     S.carve(scratch, N, nwarps);
+    SwapScratch Sf = S;  // swap_sweep's layout of the same scratch
+    Sf.carve_sweep();
     const int mmax = max(2, min(mix.swap_max, min(M - 1, WMAX)));
     const int sm = max(2, sc.v.swap_m);
     const bool lists = (d.flags & (PF_PAIR | PF_HARD)) && build_lists();
@@ -299,23 +324,26 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
     // hold the leading warp up after every attempt
     int n_att = 0, n_acc = 0, n_skip = 0;
     long long n_bead = 0;
+    int drawn = -1;  // the first of the swaps whose choices are at hand
     for (int a = 0; a < mix.swaps_per_sweep; ++a) {
-      if ((a & (SWAP_DRAWS - 1)) == 0) {
+      if ((a & ~(SWAP_DRAWS - 1)) != drawn) {
+        drawn = a & ~(SWAP_DRAWS - 1);
         G::sync();
-        if (warp == 0) swap_draws(*S.draws, d, sweep, a, mix.swaps_per_sweep, M, N, mmax, sm);
+        if (warp == 0) swap_draws(*Sf.draws, d, sweep, drawn, mix.swaps_per_sweep, M, N, mmax, sm);
         G::sync();
       }
       const Stream ss = make_stream(d, sweep, PH_SWAP, (unsigned)a);
-      const int m = S.draws->m[a & (SWAP_DRAWS - 1)];
+      const int m = Sf.draws->m[a & (SWAP_DRAWS - 1)];
       int r;
       if (m <= SWAP_LANES && !(SPEC == SWAP_ANY && (d.flags & PF_HARD))) {
-        r = swap_sweep<WARP, SPEC>(cs, a, ss, wstride, wmagic, S, red);
+        r = swap_sweep<WARP, SPEC>(cs, a, ss, wstride, wmagic, Sf, red);
       } else {
+        const int j0 = Sf.draws->j0[a & (SWAP_DRAWS - 1)], n1 = Sf.draws->n1[a & (SWAP_DRAWS - 1)];
         const uint4 r1 = ss.at(DRAW_CHOICE + 1);
         G::sync();
-        r = swap_general<WARP, SPEC>(cs, S.draws->j0[a & (SWAP_DRAWS - 1)], m, S.draws->n1[a & (SWAP_DRAWS - 1)],
-                                     u53(r1.z, r1.w), ss, S, red);
+        r = swap_general<WARP, SPEC>(cs, j0, m, n1, u53(r1.z, r1.w), ss, S, red);
         G::sync();
+        drawn = -1;  // its beads overwrote the choices
       }
       if (r == RES_SKIP) {
         ++n_skip;
@@ -493,6 +521,10 @@ __device__ __forceinline__ void sweep_cta(const SweepArgs &a) {
     ++iter;
     if (sc.chain < 0) break;
     const ChainDesc &d = sc.d;
+    if (PH == SW_STAGE && a.stage_par == 1 && chain_serial_local(d)) {  // k_stage_slots'
+      __syncthreads();
+      continue;
+    }
     CV c = make_cv(&sc.d, a.dpool, a.ipool, a.upool);
     {
       __shared__ unsigned bits[(kMaxParticles + 31) / 32];
@@ -526,7 +558,7 @@ __device__ __forceinline__ void sweep_cta(const SweepArgs &a) {
     }
     unsigned char *scratch = smem + a.state_bytes;
     for (int s = 0; s < a.sweeps; ++s)
-      sweep_one<false, PH, SPEC>(sc, red, c, scratch, a.warp_scratch_d, a.teams != 0);
+      sweep_one<false, PH, SPEC>(sc, red, c, scratch, a.warp_scratch_d, a.teams != 0, a.slot_bytes);
     if (staged) {
       double *gx = a.dpool + d.x_off, *gV = a.dpool + d.V_off;
       unsigned *gq = (unsigned *)(a.dpool + d.xq_off);
