@@ -109,6 +109,8 @@ struct Handle {
     int n;
     bool given;
     double *d;
+    float4 *cells;  // the bracket's FP32 copy, or null
+    float neg;      // ChainDesc::ct_neg
   };
   std::vector<ContactTab> ctabs;
   unsigned long long *d_rdf = nullptr;  // pair-distance histograms of every chain
@@ -1127,7 +1129,10 @@ int pimc_destroy(void *handle) {
   for (cudaEvent_t e : h->io_ev) cudaEventDestroy(e);
   if (h->s_up) cudaStreamDestroy(h->s_up);
   if (h->s_down) cudaStreamDestroy(h->s_down);
-  for (auto &t : h->ctabs) cudaFree(t.d);
+  for (auto &t : h->ctabs) {
+    cudaFree(t.d);
+    cudaFree(t.cells);
+  }
   cudaFree(h->d_rdf);
   cudaFree(h->d_badj);
   cudaFree(h->d_tile_off);
@@ -2228,12 +2233,41 @@ int contact_targets(Handle *h, int chain, int *c0, int *c1) {
   return PIMC_OK;
 }
 
-void attach_contact(ChainDesc &d, const double *tab, int n, double range) {
+// the FP32 copy of table t for the sweeps' brackets (without room for it they
+// decide from exact sums) and the radius past which its terms are light, for
+// chains of imaginary-time step at most tau
+int contact_cells(Handle *h, Handle::ContactTab &t, double tau) {
+  t.cells = nullptr;
+  t.neg = 0.f;
+  if (cudaMalloc(&t.cells, sizeof(float4) * (size_t)(t.n - 1) * (t.n - 1)) != cudaSuccess) {
+    cudaGetLastError();
+    t.cells = nullptr;
+    return PIMC_OK;
+  }
+  int last = -1;
+  CK(cudaMemcpyAsync(h->d_iout, &last, sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  CK(launch_contact_cells(t.d, t.cells, t.n, 1e-9 / (12.566370614359172 * tau), h->d_iout, h->stream));
+  CK(cudaMemcpyAsync(&last, h->d_iout, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  if (sync_check(h)) return PIMC_ECUDA;
+  // no light terms in a table that does not decay: clamped radii lie past it
+  t.neg = last >= t.n - 1 ? INFINITY : (float)((last + 1) * (t.range / (t.n - 1)) * 1.00001);
+  return PIMC_OK;
+}
+
+void attach_contact(ChainDesc &d, const Handle::ContactTab &t) {
+  const double *tab = t.d;
+  const int n = t.n;
+  const double range = t.range;
   d.ct_tab = tab;
   d.ct_n = n;
   d.ct_r0 = kContactR0;
   d.ct_rmax = range;
   d.ct_h = (range - kContactR0) / (double)(n - 1);
+  d.ct_cells = t.cells;
+  d.ct_neg = t.neg;
+  d.ct_invh = (float)(1.0 / d.ct_h);
+  d.ct_c4 = (float)(1.4426950408889634 / (4.0 * d.tau));
+  d.ct_4pt = (float)(12.566370614359172 * d.tau);
   d.flags |= PF_CONTACT;
 }
 
@@ -2244,6 +2278,7 @@ void release_contact_tables(Handle *h) {
     for (const auto &d : h->desc) used = used || ((d.flags & PF_CONTACT) && d.ct_tab == h->ctabs[i].d);
     if (used) { ++i; continue; }
     cudaFree(h->ctabs[i].d);
+    cudaFree(h->ctabs[i].cells);
     h->ctabs.erase(h->ctabs.begin() + (long)i);
   }
 }
@@ -2265,17 +2300,20 @@ int pimc_set_contact_propagator(void *handle, int chain, double g0, double range
   CK(cudaStreamSynchronize(h->stream));
   for (int c = c0; c < c1; ++c) {
     const double tau = h->desc[c].tau;
-    const double *tab = nullptr;
-    for (const auto &t : h->ctabs)
-      if (!t.given && t.g0 == g0 && t.tau == tau && t.range == range && t.n == n) tab = t.d;
-    if (!tab) {
+    int at = -1;
+    for (size_t i = 0; i < h->ctabs.size(); ++i) {
+      const auto &t = h->ctabs[i];
+      if (!t.given && t.g0 == g0 && t.tau == tau && t.range == range && t.n == n) at = (int)i;
+    }
+    if (at < 0) {
       double *d = nullptr;
       CK(cudaMalloc(&d, sizeof(double) * (size_t)n * n));
-      h->ctabs.push_back({g0, tau, range, n, false, d});
+      at = (int)h->ctabs.size();
+      h->ctabs.push_back({g0, tau, range, n, false, d, nullptr, 0.f});
       CK(launch_contact_table(d, n, range, g0, tau, h->stream));
-      tab = d;
+      if (contact_cells(h, h->ctabs[at], tau)) return PIMC_ECUDA;
     }
-    attach_contact(h->desc[c], tab, n, range);
+    attach_contact(h->desc[c], h->ctabs[at]);
   }
   if (upload_desc(h)) return PIMC_ECUDA;
   int rc = sync_check(h);
@@ -2295,9 +2333,12 @@ int pimc_set_contact_table(void *handle, int chain, const double *tab, int n, do
   CK(cudaStreamSynchronize(h->stream));
   double *d = nullptr;
   CK(cudaMalloc(&d, sizeof(double) * cnt));
-  h->ctabs.push_back({0.0, 0.0, range, n, true, d});
-  CK(cudaMemcpy(d, tab, sizeof(double) * cnt, cudaMemcpyHostToDevice));
-  for (int c = c0; c < c1; ++c) attach_contact(h->desc[c], d, n, range);
+  h->ctabs.push_back({0.0, 0.0, range, n, true, d, nullptr, 0.f});
+  CK(cudaMemcpyAsync(d, tab, sizeof(double) * cnt, cudaMemcpyHostToDevice, h->stream));
+  double tau = 0.0;
+  for (int c = c0; c < c1; ++c) tau = std::max(tau, h->desc[c].tau);
+  if (contact_cells(h, h->ctabs.back(), tau)) return PIMC_ECUDA;
+  for (int c = c0; c < c1; ++c) attach_contact(h->desc[c], h->ctabs.back());
   if (upload_desc(h)) return PIMC_ECUDA;
   int rc = sync_check(h);
   release_contact_tables(h);
@@ -2333,6 +2374,7 @@ int pimc_clear_contact(void *handle, int chain) {
     ChainDesc &d = h->desc[c];
     d.flags &= ~PF_CONTACT;
     d.ct_tab = nullptr;
+    d.ct_cells = nullptr;
     d.ct_n = 0;
   }
   CK(cudaStreamSynchronize(h->stream));

@@ -1349,13 +1349,14 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
             w2[1] += lnU2(d, r2n, mi2(d, S.r1x[t + 1], S.r1y[t + 1], S.r2x[t + 1], S.r2y[t + 1]));
         }
       }
-    if (fast && !f_contact) {
+    if (fast && (!f_contact || d.ct_cells)) {
       // bracketed from the mirror, and where that straddles the threshold from
       // the positions in fixed point (pimc_scan.cuh); the warps split the
       // particles.  With rising pairs a warp whose own lower bound already
       // accepts raises a flag in shared memory, and every warp stops at its
       // next block
-      const float gh = (float)(-d.mhtau_g);  // tau g / 2, within 6e-8
+      // (contact chains: from fixed point alone)
+      const float gh = f_contact ? -1.f : (float)(-d.mhtau_g);  // tau g / 2, within 6e-8
       const float sgn_new = f_phys ? -1.f : 1.f;
       const float need = lu - pf + pfe + 1e-5f * (1.f + fabsf(lu)) + 1e-6f * (fabsf(lu) + fabsf(pf));
       const bool monotone = rising && d.g > 0.0 && lu > -3e38f;
@@ -1379,7 +1380,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
         xs = warp_sum((float)(w2[1] - w2[0]));
         xr = 2e-6f * warp_sum((float)(fabs(w2[0]) + fabs(w2[1])));
       }
-      for (int level = 0; level < 2 && dec == -1; ++level) {
+      for (int level = f_contact ? 1 : 0; level < 2 && dec == -1; ++level) {
         PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
         if (level == 0) {
           scan_mirror<4>(c, j0, m, reinterpret_cast<const unsigned *>(S.cq), skip, warp, nwarps, e, lane, stop);
@@ -1392,7 +1393,14 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
             cf[k] = make_uint2(fix32(d, x), fix32(d, y));
           }
           G::sync();
-          scan_fixed<4>(c, j0, m, cf, skip, warp, nwarps, e, lane);
+          if (f_contact)
+            scan_contact<4>(c, j0, m, cf, skip, warp, nwarps, e, lane,
+                            reinterpret_cast<unsigned *>(S.q + (size_t)warp * PQ_CAP),
+                            [&](int k, int t, double &x, double &y) {
+                              seg_of((k >> 1) & 1).cur(k & 1, t, x, y);
+                            });
+          else
+            scan_fixed<4>(c, j0, m, cf, skip, warp, nwarps, e, lane);
         }
         float t, r;
         est_lane(e, sgn_new, t, r);

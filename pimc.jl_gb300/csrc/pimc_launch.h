@@ -172,6 +172,9 @@ cudaError_t adjoint_static_scratch(double **ptr);
 // the contact-interaction propagator table T[n][n] for (range, g0, tau)
 cudaError_t launch_contact_table(double *dtab, int n, double range, double g0, double tau,
                                  cudaStream_t s);
+// the FP32 copy of a contact table, (n-1)^2 cells of four corners, and the last
+// index whose entries reach thr (*last set to -1 before)
+cudaError_t launch_contact_cells(const double *tab, float4 *cells, int n, double thr, int *last, cudaStream_t s);
 // measured FP64 FMA throughput of the current device (TFLOP/s)
 cudaError_t fp64_peak(int num_sms, cudaStream_t st, double *tflops);
 // the swap-phase kernels' translation unit (pimc_swap.cu): its kernel for a

@@ -182,6 +182,167 @@ __device__ __forceinline__ void scan_fixed(const CV &c, int j0, int m, const uin
   e.bn *= 1.001f;
 }
 
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// one contact term log(1 + T(|d1|, |d2|) / rel0) in FP32 from fixed-point
+// differences (a1x, a1y) at a slice and (a2x, a2y) at the next: its value and a
+// bound on the distance from contact_lnU; a negative bound: not settled here
+// (where 1 + T / rel0 is small), the FP64 form decides.  T's weights are off by
+// the radii's rounding (5e-7 and three units), bounded with the cell's slopes
+// (next to a kink of the bilinear table the neighbouring cells' too); rel0's
+// exponent by its own.  Lanes that do not count (act) read the first cell.
+__device__ __forceinline__ float2 contact_term(const ChainDesc &d, bool act, int a1x, int a1y, int a2x, int a2y) {
+  const float u = d.f_unit;
+  const float x1 = (float)a1x * u, y1 = (float)a1y * u, x2 = (float)a2x * u, y2 = (float)a2y * u;
+  const float r[2] = {sqrt_approx(fmaf(x1, x1, y1 * y1)), sqrt_approx(fmaf(x2, x2, y2 * y2))};
+  int cell[2];
+  float w[2], dp[2];
+  bool kink = false;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const float p = r[q] * d.ct_invh, last = (float)(d.ct_n - 1), f = fminf(floorf(p), last - 1.f);
+    const bool past = p * (1.f - 8e-7f) - 3.f * u * d.ct_invh > last;  // clamped
+    dp[q] = past ? 0.f : p * 8e-7f + 3.f * u * d.ct_invh;
+    cell[q] = (int)f;
+    w[q] = past ? 1.f : p - f;
+    kink = kink || (!past && ((w[q] < dp[q] && f > 0.f) || w[q] > 1.f - dp[q]));
+  }
+  const size_t at = act ? (size_t)cell[0] * (d.ct_n - 1) + cell[1] : 0;
+  const float4 g = __ldg(d.ct_cells + at);  // T at (i, j), (i, j+1), (i+1, j), (i+1, j+1)
+  const float s0 = fmaf(w[1], g.y - g.x, g.x), s1 = fmaf(w[1], g.w - g.z, g.z), T = fmaf(w[0], s1 - s0, s0);
+  const float big = fmaxf(fmaxf(fabsf(g.x), fabsf(g.y)), fmaxf(fabsf(g.z), fabsf(g.w)));
+  float gx = fmaxf(fabsf(g.z - g.x), fabsf(g.w - g.y)), gy = fmaxf(fabsf(g.y - g.x), fabsf(g.w - g.z));
+  if (act && kink)
+    for (int i = max(cell[0] - 1, 0); i <= min(cell[0] + 1, d.ct_n - 2); ++i)
+      for (int j = max(cell[1] - 1, 0); j <= min(cell[1] + 1, d.ct_n - 2); ++j) {
+        const float4 h = __ldg(d.ct_cells + (size_t)i * (d.ct_n - 1) + j);
+        gx = fmaxf(gx, fmaxf(fabsf(h.z - h.x), fabsf(h.w - h.y)));
+        gy = fmaxf(gy, fmaxf(fabsf(h.y - h.x), fabsf(h.w - h.z)));
+      }
+  const float dT = 2.f * (dp[0] * gx + dp[1] * gy) + 8e-7f * big;
+  // the physical rules take the signed difference of the two separations, the
+  // reference its components' absolute values
+  const bool phys = (d.flags & PF_PHYS) != 0;
+  const int ix = phys ? (int)((unsigned)a1x - (unsigned)a2x) : abs(a1x) - abs(a2x);
+  const int iy = phys ? (int)((unsigned)a1y - (unsigned)a2y) : abs(a1y) - abs(a2y);
+  const float ex = (float)ix * u, ey = (float)iy * u;
+  const float z = fmaf(ex, ex, ey * ey) * d.ct_c4;  // log2 of exp(dd / 4 tau)
+  const float dz = z * 8e-7f + 8.f * u * (fabsf(ex) + fabsf(ey) + u) * d.ct_c4;
+  const float K = ex2_approx(z) * d.ct_4pt, q = T * K, p1 = 1.f + q;
+  const float dq = dT * K * 1.00001f + fabsf(q) * (dz + 6e-7f);
+  // lg2.approx: within 2^-22 (about p1 = 1) or two ulp
+  const float v = __logf(p1), dv = __fdividef(1.31f * dq, p1) + 4e-7f * (1.f + fabsf(v));
+  const bool settled = z < 100.f && p1 > 1e-4f && dq < 0.2f * p1 && dv < 2e-3f;
+  return make_float2(v, settled ? dv : -1.f);
+}
+
+// the contact chains' bracket: per link the table's pair action itself over the
+// partners within reach at the link's start, from the positions in fixed
+// point; cur(k, t, x, y): centre k's position at bead t (terms settled in
+// FP64); ring: RING_C words of the warp.  The exact sums spend some 150 FP64
+// instructions a term.  Here the lanes test a term for weight -- past ct_neg at
+// both ends and with a small exponent it is below 1e-7, three of four terms
+// within reach of a dense cloud -- and queue the others, evaluated 32 at a time.
+constexpr int RING_C = 64;  // at most 31 + 32 in use
+template <int NC, class Cur>
+__device__ __forceinline__ void scan_contact(const CV &c, int j0, int m, const uint2 *cf,
+                                             const ScanSkip<NC> &skip, int part, int nparts, PairEst &e,
+                                             int lane, unsigned *ring, const Cur &cur) {
+  const ChainDesc &d = *c.d;
+  const int N = c.N, M = c.M;
+  const bool wraps = j0 + m >= M;
+  const float u = d.f_unit, rc2 = (float)d.rc2, neg2 = d.ct_neg * d.ct_neg;
+  const float r_lo = rc2 * (1.f - 2e-6f) - 8.f * u * (float)d.rc, r_hi = rc2 * (1.f + 2e-6f) + 8.f * u * (float)d.rc;
+  const unsigned lt = (1u << lane) - 1u;
+  int head = 0, tail = 0;
+  float sa = 0.f, na = 0.f, lo_o = 0.f, lo_n = 0.f;  // sum of magnitudes, terms left out
+  auto flush = [&](int cnt) {
+    if (lane < cnt) {
+      const unsigned w = ring[(head + lane) & (RING_C - 1)];
+      const int b = (int)(w & 0x1fffu), t = (int)((w >> 13) & 0x7fu), k = (int)((w >> 20) & 3u);
+      const float wt = (w >> 22) & 1u ? 0.5f : 1.f;
+      const int ap = j0 + t - 1, at = j0 + t;
+      const int nb = wraps ? c.next[b] : b;
+      const int jp = ap < M ? ap : ap - M, np = ap < M ? b : nb, j = at < M ? at : at - M, n = at < M ? b : nb;
+      const double px = c.X(0, np, jp), py = c.Xd(1, np, jp), qx = c.X(0, n, j), qy = c.Xd(1, n, j);
+      const uint2 cp = cf[(t - 1) * NC + k], ct = cf[t * NC + k];
+      float2 v = contact_term(d, true, (int)(cp.x - fix32(d, px)), (int)(cp.y - fix32(d, py)),
+                              (int)(ct.x - fix32(d, qx)), (int)(ct.y - fix32(d, qy)));
+      if (v.y < 0.f) {
+        double ax, ay, nx, ny;
+        cur(k, t - 1, ax, ay);
+        cur(k, t, nx, ny);
+        v.x = (float)contact_link(d, ax, ay, px, py, nx, ny, qx, qy);
+        v.y = 1e-7f * fabsf(v.x);
+      }
+      if (k & 1) two_sum(e.sn, lo_n, wt * v.x);
+      else two_sum(e.so, lo_o, wt * v.x);
+      sa += fabsf(v.x);
+      e.bo += v.y + (1.f - wt) * fabsf(v.x);
+    }
+    head += cnt;
+    __syncwarp();
+  };
+  for (int b0 = 32 * part; b0 < N; b0 += 32 * nparts) {
+    const int b = b0 + lane, bl = min(b, N - 1);
+    const int nb = wraps ? c.next[bl] : bl;
+    int px[NC], py[NC];
+    float wp[NC], rp[NC];  // reach at the slice before (1, 0.5 unsettled, 0), its r^2
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      px[k] = py[k] = 0;
+      wp[k] = rp[k] = 0.f;
+    }
+    double xn = c.X(0, bl, j0), yn = c.Xd(1, bl, j0);
+    for (int t = 0; t <= m; ++t) {
+      const unsigned qx = fix32(d, xn), qy = fix32(d, yn);
+      if (t < m) {  // the next slice's position
+        const int a = j0 + t + 1, j = a < M ? a : a - M, n = a < M ? bl : nb;
+        xn = c.X(0, n, j);
+        yn = c.Xd(1, n, j);
+      }
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        const uint2 ct = cf[t * NC + k];
+        const int ix = (int)(ct.x - qx), iy = (int)(ct.y - qy);
+        const float dx = (float)ix * u, dy = (float)iy * u, r2 = fmaf(dx, dx, dy * dy);
+        if (t > 0) {
+          // an upper bound of dd (either rule): the components' signed difference
+          const float ex = dx - (float)px[k] * u, ey = dy - (float)py[k] * u;
+          const bool light = fminf(rp[k], r2) > neg2 && fmaf(ex, ex, ey * ey) * d.ct_c4 < 6.6f;
+          const bool on = wp[k] != 0.f;
+          if (on && light) na += 1.f;
+          const bool push = on && !light;
+          const unsigned mk = __ballot_sync(0xffffffffu, push);
+          if (push)
+            ring[(tail + __popc(mk & lt)) & (RING_C - 1)] =
+                (unsigned)b | ((unsigned)t << 13) | ((unsigned)k << 20) | (wp[k] != 1.f ? 1u << 22 : 0u);
+          tail += __popc(mk);
+          __syncwarp();
+          if (tail - head >= 32) flush(32);
+        }
+        const bool cnt = b < N && !skip(k, b);
+        wp[k] = cnt && r2 < r_lo ? 1.f : (cnt && r2 <= r_hi ? 0.5f : 0.f);
+        rp[k] = r2;
+        px[k] = ix;
+        py[k] = iy;
+      }
+    }
+  }
+  if (tail > head) flush(tail - head);
+  e.so += lo_o;
+  e.sn += lo_n;
+  e.ko += 2;
+  e.kn += 2;
+  // the light terms, and for terms of either sign what est_lane and the sums
+  // over the warps need of the magnitudes
+  e.bo = (e.bo + 1.1e-7f * na + 3e-6f * sa) * 1.001f;
+}
+
 // a lane's contribution to the change of the action from its estimates, in
 // units of tau g / 2: the old terms raise it, the new ones raise (sgn_new = 1,
 // the reference's rules for a swap) or lower it, and a bound that covers the
@@ -189,7 +350,8 @@ __device__ __forceinline__ void scan_fixed(const CV &c, int j0, int m, const uin
 __device__ __forceinline__ void est_lane(const PairEst &q, float sgn_new, float &t, float &r) {
   t = fmaf(sgn_new, q.sn, q.so);
   const float ro = 2.4e-7f * (float)(q.ko + 1), rn = 2.4e-7f * (float)(q.kn + 1);
-  r = (q.bo * (1.f + ro) + ro * q.so + q.bn * (1.f + rn) + rn * q.sn + 2e-6f * (q.so + q.sn)) * 1.00001f + 1e-30f;
+  const float ao = fabsf(q.so), an = fabsf(q.sn);
+  r = (q.bo * (1.f + ro) + ro * ao + q.bn * (1.f + rn) + rn * an + 2e-6f * (ao + an)) * 1.00001f + 1e-30f;
 }
 
 // the Metropolis decision of a log ratio known to lie in [s - r, s + r], from

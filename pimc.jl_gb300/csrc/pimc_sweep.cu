@@ -1055,6 +1055,34 @@ __global__ void __launch_bounds__(256) k_contact_gather(const double *part, doub
   }
 }
 
+// the FP32 copy of a table (scan_contact): a cell's four corners together, one
+// read per term
+__global__ void k_contact_cells(const double *tab, float4 *cells, int n) {
+  const size_t cnt = (size_t)(n - 1) * (n - 1);
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < cnt; e += (size_t)gridDim.x * blockDim.x) {
+    const size_t i = e / (n - 1), j = e % (n - 1);
+    const double *t = tab + i * n + j;
+    cells[e] = make_float4((float)t[0], (float)t[1], (float)t[n], (float)t[n + 1]);
+  }
+}
+// *last: the largest index c such that an entry (c, j >= c) or (j, c) is not
+// below thr in magnitude (starts at -1)
+__global__ void k_contact_last(const double *tab, int n, double thr, int *last) {
+  int c = -1;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)n * n;
+       e += (size_t)gridDim.x * blockDim.x)
+    if (!(fabs(tab[e]) < thr)) c = max(c, min((int)(e / n), (int)(e % n)));
+  c = __reduce_max_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0 && c >= 0) atomicMax(last, c);
+}
+cudaError_t launch_contact_cells(const double *tab, float4 *cells, int n, double thr, int *last, cudaStream_t s) {
+  const size_t cnt = (size_t)(n - 1) * (n - 1);
+  const unsigned grid = (unsigned)std::min<size_t>((cnt + 255) / 256, 1024);
+  k_contact_cells<<<grid, 256, 0, s>>>(tab, cells, n);
+  k_contact_last<<<grid, 256, 0, s>>>(tab, n, thr, last);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_contact_table(double *dtab, int n, double range, double g0, double tau,
                                  cudaStream_t s) {
   ContactQuad q;

@@ -94,6 +94,15 @@ struct ChainDesc {
   const double *ct_tab;
   int ct_n, ct_pad_;
   double ct_r0, ct_h, ct_rmax;
+  // the bracket's FP32 copy of the table, four corners per cell (null: no room,
+  // exact sums alone), and 1 / ct_h, log2(e) / 4 tau, 4 pi tau
+#ifdef __CUDACC__
+  const float4 *ct_cells;
+#else
+  const void *ct_cells;
+#endif
+  float ct_invh, ct_c4, ct_4pt;
+  float ct_neg;  // with both radii past it, 4 pi tau |T| < 1e-9
   // pair-distance histogram (rdf_nb > 0): counts of unordered pairs per
   // slice with floor(r / rdf_dr) = k, k < rdf_nb
   unsigned long long *rdf;

@@ -133,3 +133,32 @@ def test_sweep_paths_decide_as_exact_sums(sem, ell, M, engine_lib):
         np.testing.assert_array_equal(xa, xb)
         np.testing.assert_array_equal(na, nb)
         assert aa == ab and np.isfinite(xa).all()
+
+
+@pytest.mark.parametrize("sem", [0, 1])
+@pytest.mark.parametrize("scale", [1.0, 6.0])
+def test_contact_sweeps_decide_as_exact_sums(sem, scale, engine_lib):
+    """contact chains, dense and sparse, with separations past a short table's
+    end and (scale 6) pairs on the -mu branch: bracketed decisions give the beads
+    and acceptance counts of exact FP64 ones, bit for bit"""
+    from pimc.engine import ChainParams, Engine, Mix, OPT_EXACT_DECISIONS, contact_table
+    M = 20
+    tab = scale * contact_table(1.16, 1.0 / M, 3.0, 200)
+    ps = [ChainParams(dim=dim, N=N, M=M, L=L, T=1.0, lam=0.5, mu=0.3, harmonic_omega=om, interactions=True,
+                      r_a=1.0, semantics=sem, seed=40 + i)
+          for i, (N, dim, L, om) in enumerate([(2, 2, 3.0, 2.0), (33, 2, 3.0, 1.5), (40, 1, 6.0, 1.0), (64, 2, 5.0, 1.0)])]
+    out = []
+    for exact in (0, 1):
+        e = Engine(ps)
+        e.set_contact_table(tab, 3.0)
+        for i, p in enumerate(ps):
+            e.set_mix(Mix(stage_slices=9, stage_max=9, stage_minacc=0.0, stage_maxacc=1.0, swaps_per_sweep=60,
+                          swap_slices=9, swap_max=9, swap_minacc=0.0, swap_maxacc=1.0, com_maxstep=2.0), chain=i)
+        e.set_option(OPT_EXACT_DECISIONS, exact)
+        e.run_batched(8)
+        out.append([(e.get_beads(c), e.get_next(c), e.stats(c).accepts) for c in range(len(ps))])
+        e.close()
+    for (xa, na, aa), (xb, nb, ab) in zip(*out):
+        np.testing.assert_array_equal(xa, xb)
+        np.testing.assert_array_equal(na, nb)
+        assert aa == ab and np.isfinite(xa).all()
