@@ -83,6 +83,10 @@ struct Handle {
   int *d_order = nullptr;
   int *d_iout = nullptr;
   SlotTally *d_tally = nullptr;  // k_stage_slots' counters per chain
+  // the measurement launches' slices per item, items, and their buffer: per item
+  // a row of 9 sums and a list entry, then two counters
+  int meas_group = 1, meas_items = 0;
+  double *d_meas = nullptr;
   double *d_buf = nullptr;
   size_t n_buf = 0;
   double *d_adj = nullptr;
@@ -390,13 +394,16 @@ Plan plan_smem(const Handle *h, int mode, int block, int spl, int state_cap) {
 
 // the chain descriptors to the device; the captured sweep graph is dropped,
 // since which kernels it launches depends on the chains' flags
-int upload_desc(Handle *h) {
-  CK(cudaMemcpyAsync(h->d_desc, h->desc.data(), sizeof(ChainDesc) * h->nchains,
-                     cudaMemcpyHostToDevice, h->stream));
+void drop_graph(Handle *h) {
   if (h->gexec) {
     cudaGraphExecDestroy(h->gexec);
     h->gexec = nullptr;
   }
+}
+int upload_desc(Handle *h) {
+  CK(cudaMemcpyAsync(h->d_desc, h->desc.data(), sizeof(ChainDesc) * h->nchains,
+                     cudaMemcpyHostToDevice, h->stream));
+  drop_graph(h);
   return PIMC_OK;
 }
 
@@ -495,6 +502,15 @@ int create_impl(const pimc_params *params, int nchains, void **out) {
     h->maxM = std::max(h->maxM, p.M);
     h->maxNM = std::max(h->maxNM, (int)NM);
   }
+  // slices per item of the measurement launches: eight where that still makes
+  // some thousand items, one for few chains
+  long long slices = 0;
+  for (const ChainDesc &d : h->desc) slices += d.M;
+  h->meas_group = slices >= 16384 ? 8 : 1;
+  for (ChainDesc &d : h->desc) {
+    d.meas_off = h->meas_items;
+    h->meas_items += (d.M + h->meas_group - 1) / h->meas_group;
+  }
   h->n_dpool = dp;
   h->n_ipool = std::max<size_t>(ip, 1);
   h->n_upool = std::max<size_t>(up, 1);
@@ -521,6 +537,7 @@ int create_impl(const pimc_params *params, int nchains, void **out) {
       cudaMalloc(&h->d_order, sizeof(int) * nchains) != cudaSuccess ||
       cudaMalloc(&h->d_iout, sizeof(int) * 16) != cudaSuccess ||
       cudaMalloc(&h->d_tally, sizeof(SlotTally) * nchains) != cudaSuccess ||
+      cudaMalloc(&h->d_meas, (9 * sizeof(double) + sizeof(int2)) * (size_t)h->meas_items + 16) != cudaSuccess ||
       cudaMalloc(&h->d_stage, sizeof(double) * std::max<size_t>(h->n_stage, 1)) != cudaSuccess)
     return cleanup(fail(PIMC_ENOMEM, "device allocation failed"));
   cudaMemsetAsync(h->d_dpool, 0, sizeof(double) * h->n_dpool, h->stream);
@@ -664,7 +681,26 @@ SweepArgs sweep_args(Handle *h, const Plan &p) {
   a.stage_phase = 0;
   a.stage_slots = 0;
   a.tally = h->d_tally;
+  a.measure_par = 0;
+  a.meas_group = h->meas_group;
+  a.meas_part = h->d_meas;
+  a.meas_list = reinterpret_cast<int2 *>(h->d_meas + 9 * (size_t)h->meas_items);
+  a.meas_cnt = reinterpret_cast<int *>(a.meas_list + h->meas_items);
   return a;
+}
+
+// whether any chain of [c0, c1) measures, and whether its measurement is worth
+// launches of its own: at least 2^18 pairs a measurement (about 30 us of one
+// SM; two or three launches take 5 to 8)
+bool measures(const Handle *h, int c0, int c1) {
+  for (int c = c0; c < c1; ++c)
+    if (h->mix[c].measure_every > 0) return true;
+  return false;
+}
+bool measure_large(const Handle *h, int c) {
+  const ChainDesc &d = h->desc[c];
+  const bool pairs = ((d.flags & PF_PAIR) && !(d.flags & PF_CONTACT)) || d.rdf_nb > 0;
+  return pairs && 0.5 * d.N * d.N * d.M >= 262144.0;
 }
 
 // chains whose windows depend on one another (chain_serial_local) and, of
@@ -771,8 +807,16 @@ int run_plain(Handle *h, long long n) {
         CK(launch_sweep_phase(a, 1, 0, spec[c], 0, 1, p.block, p.dyn_smem, h->stream));
         ++launches;
       }
+      a.measure_par = h->mix[c].measure_every > 0 && measure_large(h, c);
       CK(launch_sweep_phase(a, 2, 0, 0, 0, 1, p.block, p.dyn_smem, h->stream));
       ++launches;
+      if (a.measure_par) {
+        SweepArgs b = a;
+        b.meas_list = nullptr;
+        CK(launch_measure_sweep(b, (h->desc[c].M + h->meas_group - 1) / h->meas_group, h->num_sms, h->stream));
+        launches += 2;
+        a.measure_par = 0;
+      }
     }
   CK(cudaEventRecord(h->ev1, h->stream));
   int rc = sync_check(h);
@@ -870,11 +914,17 @@ cudaError_t issue_phase(Handle *h, const Plan &p, const SweepArgs &a, int ph, lo
     }
   }
   if (!whole) return cudaSuccess;
+  const bool meas = ph == 2 && measures(h, 0, h->nchains);
+  b.measure_par = meas;
   cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
   if (e == cudaSuccess)
     e = launch_sweep_phase(b, ph, p.pwarp[ph], swap_spec(h), p.pregs[ph], grid_for(h, p, ph, a.nchains),
                            phase_block(p, ph), phase_smem(p, ph), h->stream);
   if (launches) *launches += 1;
+  if (meas && e == cudaSuccess) {
+    e = launch_measure_sweep(b, h->meas_items, h->num_sms, h->stream);
+    if (launches) *launches += 3;
+  }
   return e;
 }
 
@@ -888,10 +938,16 @@ cudaError_t issue_sweeps(Handle *h, const Plan &p, SweepArgs a, int n, long long
     a.sweeps = n;
     const size_t smem = fused_smem(h, p);
     if (p.mode == 0) a.slot_bytes = (int)(smem - p.state_bytes);
+    if (p.mode == 0 && n == 1 && measures(h, 0, h->nchains))
+      for (int c = 0; c < h->nchains && !a.measure_par; ++c) a.measure_par = measure_large(h, c);
     cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
     if (e == cudaSuccess)
       e = launch_sweep(a, p.mode, grid_for(h, p, -1, a.nchains), p.block, smem, h->stream);
     if (launches) *launches += 1;
+    if (a.measure_par && e == cudaSuccess) {
+      e = launch_measure_sweep(a, h->meas_items, h->num_sms, h->stream);
+      if (launches) *launches += 3;
+    }
     return e;
   }
   for (int s = 0; s < n; ++s)
@@ -1123,6 +1179,7 @@ int pimc_destroy(void *handle) {
   cudaFree(h->d_order);
   cudaFree(h->d_iout);
   cudaFree(h->d_tally);
+  cudaFree(h->d_meas);
   cudaFree(h->d_buf);
   cudaFree(h->d_adj);
   cudaFree(h->d_stage);
@@ -1421,13 +1478,7 @@ int pimc_set_move_mix(void *handle, int chain, const pimc_move_mix *mix) {
   }
   CK(cudaMemcpyAsync(h->d_var, v.data(), sizeof(ChainVar) * h->nchains, cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->d_mix, h->mix.data(), sizeof(MixDev) * h->nchains, cudaMemcpyHostToDevice, h->stream));
-  // the captured launches depend on the mixes where chains are staged by slots
-  bool slots = false;
-  for (const auto &d : h->desc) slots = slots || desc_serial(d);
-  if (slots && h->gexec) {
-    cudaGraphExecDestroy(h->gexec);
-    h->gexec = nullptr;
-  }
+  drop_graph(h);  // the captured launches depend on the mixes
   return sync_check(h);
 }
 
@@ -1600,8 +1651,10 @@ int pimc_batch_tune(void *handle, int sweeps_per_trial, pimc_launch *chosen) {
   for (MixDev &m : h->mix) m.measure_every = 0;
   CK(cudaMemcpyAsync(h->d_mix, h->mix.data(), sizeof(MixDev) * h->nchains, cudaMemcpyHostToDevice,
                      h->stream));
+  drop_graph(h);
   const int rc = tune_impl(h, sweeps_per_trial, chosen);
   h->mix = saved;
+  drop_graph(h);
   CK(cudaMemcpyAsync(h->d_mix, h->mix.data(), sizeof(MixDev) * h->nchains, cudaMemcpyHostToDevice,
                      h->stream));
   const int rs = sync_check(h);

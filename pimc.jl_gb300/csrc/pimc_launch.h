@@ -36,6 +36,11 @@ struct SweepArgs {
   int stage_phase;    // the staging phase that k_stage_slots runs
   int stage_slots;    // slots per chain of its queue (the longest chain's)
   struct SlotTally *tally;  // [chains] k_stage_slots' counters, zero between phases
+  int measure_par;    // 1: the sweep leaves its measurement to launch_measure_sweep
+  int meas_group;     // slices per item of it
+  int2 *meas_list;    // its items (chain, group), or null: chain0's groups alone
+  int *meas_cnt;      // [2] items, next item
+  double *meas_part;  // [items][9] partial sums (ChainDesc::meas_off)
   int teams;          // 1: staging slots walked by teams of warps (latency-bound
                       // launches whose chains all fit on the GPU at once)
 };
@@ -114,6 +119,10 @@ cudaError_t launch_stage_slots(const SweepArgs &a, int grid, int block, size_t s
 cudaError_t launch_stage_close(const SweepArgs &a, cudaStream_t s);
 cudaError_t stage_slots_set_smem(size_t smem);
 cudaError_t stage_slots_occupancy(int block, size_t smem, int *blocks_per_sm);
+// the measurement of the chains whose sweep calls for one, by (chain, slice
+// group) items: of a.nchains chains in a.order, or (meas_list null) of chain
+// chain0, ngroups its groups
+cudaError_t launch_measure_sweep(const SweepArgs &a, int ngroups, int num_sms, cudaStream_t s);
 // shared bytes of slot-wise staging for windows of at most ell slices
 size_t slot_scratch_bytes(int ell, int nwarps);
 size_t sweep_ctl_bytes();

@@ -1,0 +1,190 @@
+// pimc_measure.cuh -- the sweeps' measurements (src/measurement.jl:45-55,
+// 92-122, and the radial distribution and superfluid estimators its TODOs
+// name, 125-127): E_th, E_v, pair energy, pair virial, winding, area, sum r^2,
+// the density and the pair-distance histogram.
+//
+// A link's pair within reach at its start: FP64 separations and exact reach,
+// FP32 expf of both ends' squared distances (relative error about 1e-7 per
+// term, far below any Monte Carlo error).  The sums of a lane's terms are exact
+// to FP64 (two floats for at most 16 terms, then a double), so launch shapes
+// agree to rounding.  pimc_measure keeps every term in FP64 (measure_group).
+#pragma once
+#include "pimc_kernels.cuh"
+
+namespace pimc {
+
+// a thread's sums: link, potential, virial of the external potential, pair
+// energy, pair virial; winding x, y, area, sum r^2
+struct MeasureSums {
+  double s[5], f[4];
+  __device__ void clear() {
+    for (int k = 0; k < 5; ++k) s[k] = 0.0;
+    for (int k = 0; k < 4; ++k) f[k] = 0.0;
+  }
+};
+
+// the beads k = j N + i of k0, k0 + nt, ... below k1
+__device__ __forceinline__ void measure_beads(const CV &c, int k0, int k1, int nt, bool density, double inv_bw,
+                                              MeasureSums &a) {
+  const ChainDesc &d = *c.d;
+  const int N = c.N, M = c.M, dim = c.dim;
+  for (int k = k0; k < k1; k += nt) {
+    const int j = k / N, i = k % N, jn = j + 1 == M ? 0 : j + 1, in = j == M - 1 ? c.next[i] : i;
+    const double ax = c.X(0, i, j), ay = c.Xd(1, i, j);
+    const double dx = mi1(c.X(0, in, jn), ax, d.L, d.L2);
+    const double dy = dim > 1 ? mi1(c.X(1, in, jn), ay, d.L, d.L2) : 0.0;
+    a.s[0] += dim > 1 ? fma(dy, dy, dx * dx) : dx * dx;
+    // every bead is the start of one link and the end of another
+    a.s[1] += 2.0 * vext(d, ax, ay);
+    double gx, gy;
+    grad_vext(d, ax, ay, gx, gy);
+    a.s[2] += ax * gx + (dim > 1 ? ay * gy : 0.0);
+    a.f[0] += dx;
+    a.f[1] += dy;
+    a.f[2] += 0.5 * __dsub_rn(__dmul_rn(ax, dy), __dmul_rn(ay, dx));
+    a.f[3] += __dadd_rn(__dmul_rn(ax, ax), __dmul_rn(ay, ay));
+    if (density) {
+      const long long ib = bin_floor(ax, d.L, d.dens_bw, inv_bw);
+      bool ok = ib >= 1 && ib <= d.dens_nb;
+      long long idx = ib - 1;
+      if (dim > 1) {
+        const long long jb = bin_floor(ay, d.L, d.dens_bw, inv_bw);
+        ok = ok && jb >= 1 && jb <= d.dens_nb;
+        idx += (jb - 1) * d.dens_nb;
+      }
+      if (ok) atomicAdd(c.hist + idx, 1ull);
+    }
+  }
+}
+
+// the pairs of a warp: rows (j, i) k = j N + i of k0, k0 + dk, ... below k1 (rows
+// shorten with i: dealt to the warps in turn), the links of particles i < b that
+// start at slice j.  Lanes test 32 partners on the mirror; survivors go onto a
+// ring and are evaluated 32 at a time.  Bound by the FP64 separations (six
+// instructions and three conversions per 32 pairs, 16 cycles of the SM each) and
+// the scan's issue; sums in FP64 instead of two floats cost four more.
+constexpr int MEAS_RING = 64;  // at most 31 + 32 in use
+__device__ __forceinline__ void measure_pairs(const CV &c, int k0, int k1, int dk, unsigned long long *ring,
+                                              MeasureSums &a) {
+  const ChainDesc &d = *c.d;
+  const int N = c.N, M = c.M, dim = c.dim, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u, lim = d.q_lim_hi;
+  const float cg = (float)d.inv2s2;
+  int head = 0, tail = 0, nf = 0;
+  float e0 = 0.f, e1 = 0.f, v0 = 0.f, v1 = 0.f;  // running sums, high and low parts
+  auto spill = [&]() {
+    a.s[3] += (double)e0 + (double)e1;
+    a.s[4] += (double)v0 + (double)v1;
+    e0 = e1 = v0 = v1 = 0.f;
+    nf = 0;
+  };
+  auto flush = [&](int cnt) {
+    if (lane < cnt) {
+      const unsigned long long w = ring[(head + lane) & (MEAS_RING - 1)];  // i | b << 13 | j << 26
+      const int i = (int)(w & 0x1fffu), b = (int)((w >> 13) & 0x1fffu), j = (int)(w >> 26);
+      const double r2 = mi2(d, c.X(0, i, j), c.Xd(1, i, j), c.X(0, b, j), c.Xd(1, b, j));
+      if (__double_as_longlong(r2) <= __double_as_longlong(d.rc2)) {
+        const int jn = j + 1 == M ? 0 : j + 1, in = j == M - 1 ? c.next[i] : i, bn = j == M - 1 ? c.next[b] : b;
+        const float dx = (float)mi1(c.X(0, in, jn), c.X(0, bn, jn), d.L, d.L2);
+        const float dy = dim > 1 ? (float)mi1(c.X(1, in, jn), c.X(1, bn, jn), d.L, d.L2) : 0.f;
+        // the pair exponentials e = exp(x), x = -r^2/(2 s^2), and x e; the factors
+        // g tau/2 are applied once at the end
+        const float xa = -(float)r2 * cg, xb = -fmaf(dx, dx, dy * dy) * cg;
+        const float ea = expf(xa), eb = expf(xb);
+        two_sum(e0, e1, ea + eb);
+        two_sum(v0, v1, fmaf(xa, ea, xb * eb));
+      }
+    }
+    head += cnt;
+    __syncwarp();
+    if (++nf == 16) spill();
+  };
+  for (int k = k0; k < k1; k += dk) {
+    const int j = k / N, i = k % N;
+    const unsigned *row = c.xq + (size_t)j * c.ldn;
+    const unsigned ci = row[i];
+    for (int b0 = i + 1; b0 < N; b0 += 32) {
+      const int b = b0 + lane;
+      const bool in = b < N && qdist2(ci, row[b]) <= lim;
+      const unsigned mk = __ballot_sync(0xffffffffu, in);
+      if (in)
+        ring[(tail + __popc(mk & lt)) & (MEAS_RING - 1)] =
+            (unsigned long long)((unsigned)i | ((unsigned)b << 13)) | ((unsigned long long)j << 26);
+      tail += __popc(mk);
+      __syncwarp();
+      if (tail - head >= 32) flush(32);
+    }
+  }
+  if (tail > head) flush(tail - head);
+  spill();
+}
+
+// the pair-distance histogram of slices [j0, j1): warps gw, gw + ngw, ... over
+// the beads, lanes the partners of higher index; lanes with the same bin add
+// once (match_any)
+__device__ __forceinline__ void measure_radial(const CV &c, int j0, int j1, int gw, int ngw) {
+  const ChainDesc &d = *c.d;
+  const int N = c.N, dim = c.dim, lane = threadIdx.x & 31;
+  for (int kk = j0 * N + gw; kk < j1 * N; kk += ngw) {
+    const int j = kk / N, i = kk % N;
+    const double ax = c.X(0, i, j), ay = c.Xd(1, i, j);
+    for (int b0 = i + 1; b0 < N; b0 += 32) {
+      const int b = b0 + lane;
+      int bin = -1;
+      if (b < N) {
+        const double dx = fabs(mi1(ax, c.X(0, b, j), d.L, d.L2));
+        const double dy = dim > 1 ? fabs(mi1(ay, c.Xd(1, b, j), d.L, d.L2)) : 0.0;
+        const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+        const double f = floor(r / d.rdf_dr);
+        if (f < (double)d.rdf_nb) bin = (int)f;
+      }
+      const unsigned act = __ballot_sync(0xffffffffu, bin >= 0);
+      if (bin >= 0) {
+        const unsigned peers = __match_any_sync(act, bin);
+        if (lane == __ffs(peers) - 1) atomicAdd(d.rdf + bin, (unsigned long long)__popc(peers));
+      }
+    }
+  }
+}
+
+// the observables of one measurement from the chain's summed s and f
+__device__ __forceinline__ void measure_out(const ChainDesc &d, const double *s, const double *f, double *out) {
+  const double tau = d.tau;
+  const int M = d.M;
+  const bool pair = (d.flags & PF_PAIR) != 0 && !(d.flags & PF_CONTACT);
+  out[4] = f[0] * f[0] + f[1] * f[1];
+  out[5] = f[2];
+  out[6] = f[3] / M;
+  out[7] = 0.0;
+  out[0] = (double)(d.dim * d.N) / (2.0 * tau) - 1.0 / (4.0 * d.lambda * (tau * tau) * M) * s[0] +
+           1.0 / (2.0 * M) * s[1];
+  out[1] = 1.0 / (2.0 * M) * s[2] + 1.0 / (2.0 * M) * s[1];
+  // pair energy sum (tau/2) g (e_a + e_b) / (M tau) and its virial part
+  // sum (tau/2) g (-2 r^2/(2 s^2)) (e_a, e_b) / (2 M tau)
+  out[2] = pair ? d.g * s[3] / (2.0 * M) : 0.0;
+  out[3] = pair ? out[2] + d.g * s[4] / (2.0 * M) : 0.0;
+}
+
+// a sweep's measurement by the group that sweeps the chain; qbuf: one
+// PQ_CAP-entry queue per warp
+template <bool WARP>
+__device__ void measure_sweep(const CV &c, double *red, double *out, bool density, unsigned long long *qbuf) {
+  using G = Group<WARP>;
+  const ChainDesc &d = *c.d;
+  const int N = c.N, M = c.M, tid = G::rank(), nt = G::size();
+  const int warp = WARP ? 0 : (int)(threadIdx.x >> 5), nwarps = WARP ? 1 : (int)(blockDim.x >> 5);
+  MeasureSums a;
+  a.clear();
+  const double inv_bw = density ? 1.0 / d.dens_bw : 0.0;
+  measure_beads(c, tid, N * M, nt, density, inv_bw, a);
+  __syncwarp();
+  if ((d.flags & PF_PAIR) && !(d.flags & PF_CONTACT)) {
+    measure_pairs(c, warp, N * M, nwarps, qbuf + (size_t)warp * PQ_CAP, a);
+  }
+  if (d.rdf_nb > 0) measure_radial(c, 0, M, warp, nwarps);
+  G::template sum<5>(a.s, red);
+  G::template sum<4>(a.f, red);
+  if (tid == 0) measure_out(d, a.s, a.f, out);
+}
+
+}  // namespace pimc

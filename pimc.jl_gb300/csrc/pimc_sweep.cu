@@ -176,6 +176,101 @@ size_t slot_scratch_bytes(int ell, int nwarps) {
 }
 
 // ---------------------------------------------------------------------------
+// The measurement of a sweep in launches of its own, after the sweep: items of
+// meas_group slices, so that a few long chains' N^2 M / 2 pairs spread over the
+// GPU (measured in the sweep's own CTA, 17 ms of a 1024-particle chain's sweep
+// and 50 of a batch of 512 chains').  k_measure_plan lists the items of the chains
+// that measure now (their sweep counter has just advanced), the items' sums go
+// to their rows, and k_measure_close adds a chain's rows in order and records.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool measures_now(const SweepArgs &a, int ch) {
+  const int every = a.mix[ch].measure_every;
+  const unsigned long long sw = a.var[ch].sweep;
+  return every > 0 && a.var[ch].err == 0 && sw > 0 && sw % (unsigned long long)every == 0;
+}
+__global__ void k_measure_plan(SweepArgs a) {
+  const int ci = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ci >= a.nchains) return;
+  const int ch = a.order ? a.order[ci] : ci;
+  if (!measures_now(a, ch)) return;
+  const int ng = (a.desc[ch].M + a.meas_group - 1) / a.meas_group, at = atomicAdd(a.meas_cnt, ng);
+  for (int g = 0; g < ng; ++g) a.meas_list[at + g] = make_int2(ch, g);
+}
+
+__global__ void __launch_bounds__(128) k_measure_slices(SweepArgs a) {
+  __shared__ ChainDesc d;
+  __shared__ double red[256];
+  __shared__ unsigned long long qbuf[4 * MEAS_RING];
+  __shared__ int s_it;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if (!a.meas_list && !measures_now(a, a.chain0)) return;
+  const int nit = a.meas_list ? a.meas_cnt[0] : (int)gridDim.x;
+  for (int iter = 0;; ++iter) {
+    if (tid == 0) s_it = a.meas_list ? atomicAdd(a.meas_cnt + 1, 1) : (iter ? nit : (int)blockIdx.x);
+    __syncthreads();
+    const int it = s_it;
+    if (it >= nit) break;
+    const int2 item = a.meas_list ? a.meas_list[it] : make_int2(a.chain0, it);
+    for (int k = tid; k < (int)(sizeof(ChainDesc) / 4); k += blockDim.x)
+      reinterpret_cast<unsigned *>(&d)[k] = reinterpret_cast<const unsigned *>(a.desc + item.x)[k];
+    __syncthreads();
+    const CV c = make_cv(&d, a.dpool, a.ipool, a.upool);
+    const int N = c.N, j0 = item.y * a.meas_group, j1 = min(c.M, j0 + a.meas_group);
+    MeasureSums m;
+    m.clear();
+    const bool density = c.hist != nullptr;
+    const double inv_bw = density ? 1.0 / d.dens_bw : 0.0;
+    measure_beads(c, j0 * N + tid, j1 * N, 128, density, inv_bw, m);
+    __syncwarp();
+    if ((d.flags & PF_PAIR) && !(d.flags & PF_CONTACT)) {
+      measure_pairs(c, j0 * N + warp, j1 * N, 4, qbuf + warp * MEAS_RING, m);
+    }
+    if (d.rdf_nb > 0) measure_radial(c, j0, j1, warp, 4);
+    block_sum_k<5>(m.s, red);
+    block_sum_k<4>(m.f, red);
+    if (tid == 0) {
+      double *o = a.meas_part + 9 * (size_t)(d.meas_off + item.y);
+      for (int k = 0; k < 5; ++k) o[k] = m.s[k];
+      for (int k = 0; k < 4; ++k) o[5 + k] = m.f[k];
+    }
+    __syncthreads();
+  }
+}
+
+// a warp per chain
+__global__ void __launch_bounds__(128) k_measure_close(SweepArgs a) {
+  const int ci = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (ci >= a.nchains) return;
+  const int ch = a.order ? a.order[ci] : a.chain0 + ci;
+  if (!measures_now(a, ch)) return;
+  const ChainDesc &d = a.desc[ch];
+  const int ng = (d.M + a.meas_group - 1) / a.meas_group;
+  const double *p = a.meas_part + 9 * (size_t)d.meas_off;
+  double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int g = lane; g < ng; g += 32)
+    for (int k = 0; k < 9; ++k) v[k] += p[9 * (size_t)g + k];
+  for (int k = 0; k < 9; ++k) v[k] = warp_sum(v[k]);
+  if (lane == 0) {
+    const CV c = make_cv(&d, a.dpool, a.ipool, a.upool);
+    double out[NOBS];
+    measure_out(d, v, v + 5, out);
+    record_measurement(d, a.var[ch], c, out, c.hist != nullptr);
+  }
+}
+
+cudaError_t launch_measure_sweep(const SweepArgs &a, int ngroups, int num_sms, cudaStream_t s) {
+  if (a.meas_list) {
+    cudaError_t e = cudaMemsetAsync(a.meas_cnt, 0, 2 * sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    k_measure_plan<<<(a.nchains + 127) / 128, 128, 0, s>>>(a);
+    ngroups = std::min(ngroups, 5 * num_sms);
+  }
+  k_measure_slices<<<ngroups, 128, 0, s>>>(a);
+  k_measure_close<<<(a.nchains + 3) / 4, 128, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
 // state maintenance: layout transposes, init_world, cached links + mirror,
 // measurements
 // ---------------------------------------------------------------------------

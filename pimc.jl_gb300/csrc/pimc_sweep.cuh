@@ -11,6 +11,7 @@
 
 #include "pimc_kernels.cuh"
 #include "pimc_launch.h"
+#include "pimc_measure.cuh"
 #include "pimc_stage.cuh"
 
 namespace pimc {
@@ -162,7 +163,7 @@ __device__ void close_phase(SmemCtl &sc, double *red, int q, double (&t)[4]) {
 
 template <bool WARP, int PH, int SPEC = SWAP_ANY>
 __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *scratch,
-                          int warp_scratch_d, bool teams, int slot_bytes = 0) {
+                          int warp_scratch_d, bool teams, int slot_bytes = 0, bool measure_par = false) {
   using G = Group<WARP>;
   const ChainDesc &d = sc.d;
   const MixDev &mix = sc.mix;
@@ -434,9 +435,8 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
   if (mix.polymer_com_phases > 0) close_phase<WARP>(sc, red, MV_PCOM, tlp);
 
   // ---- measurement cadence (measurement_Z_sector)
-  if (mix.measure_every > 0 && ((sweep + 1) % (unsigned long long)mix.measure_every) == 0) {
-    const bool lists = (d.flags & PF_PAIR) && !(d.flags & PF_CONTACT) && build_lists();
-    measure_group<WARP, true>(lists ? cq : c, red, sc.e4, c.hist != nullptr, (unsigned long long *)scratch);
+  if (!measure_par && mix.measure_every > 0 && ((sweep + 1) % (unsigned long long)mix.measure_every) == 0) {
+    measure_sweep<WARP>(c, red, sc.e4, c.hist != nullptr, (unsigned long long *)scratch);
     if (tid == 0) record_measurement(d, sc.v, c, sc.e4, c.hist != nullptr);
   }
   if (tid == 0) {
@@ -558,7 +558,7 @@ __device__ __forceinline__ void sweep_cta(const SweepArgs &a) {
     }
     unsigned char *scratch = smem + a.state_bytes;
     for (int s = 0; s < a.sweeps; ++s)
-      sweep_one<false, PH, SPEC>(sc, red, c, scratch, a.warp_scratch_d, a.teams != 0, a.slot_bytes);
+      sweep_one<false, PH, SPEC>(sc, red, c, scratch, a.warp_scratch_d, a.teams != 0, a.slot_bytes, a.measure_par != 0);
     if (staged) {
       double *gx = a.dpool + d.x_off, *gV = a.dpool + d.V_off;
       unsigned *gq = (unsigned *)(a.dpool + d.xq_off);

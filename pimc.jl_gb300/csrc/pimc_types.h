@@ -84,6 +84,7 @@ struct ChainDesc {
   int cl_nc, cl_cap, cl_mode;
   float cl_frac;
   int eser_cap;
+  int meas_off;         // first item (slice group) of the chain in the measurement's rows
   int smem_bytes;       // bytes to stage x, V, mirror, next in shared memory
   unsigned key0, key1;  // Philox key
   unsigned chain_tag;   // chain id (low 24 bits of counter word 3)

@@ -162,3 +162,40 @@ def test_contact_sweeps_decide_as_exact_sums(sem, scale, engine_lib):
         np.testing.assert_array_equal(xa, xb)
         np.testing.assert_array_equal(na, nb)
         assert aa == ab and np.isfinite(xa).all()
+
+
+@pytest.mark.parametrize("N,M,dim", [(2, 4, 2), (31, 9, 2), (33, 20, 1), (200, 17, 2), (300, 24, 2)])
+def test_measurement_launches_agree(N, M, dim, engine_lib):
+    """a sweep's measurement in its own CTA, in launches of its own (a split
+    sweep; a lone large chain) and by pimc_measure after the sweep: the same
+    observables, density counts and pair histogram; the pair columns within the
+    FP32 terms' 2e-7, the rest to rounding"""
+    from pimc.engine import ChainParams, Engine, Mix
+    kw = dict(dim=dim, N=N, M=M, L=5.0, T=0.5, lam=0.5, harmonic_omega=1.0, interactions=True, pair_g=1.0,
+              pair_sigma=0.5, r_a=1.5, density_nbins=16, energy_capacity=4, seed=5)
+    mix = Mix(stage_slices=3, stage_max=3, swaps_per_sweep=N, swap_slices=3, swap_max=3, com_maxstep=2.0,
+              measure_every=2)
+    out = []
+    for shape in ("plain", "fused", "split"):
+        e = Engine([ChainParams(**kw), ChainParams(**dict(kw, N=3, seed=6))], mix)
+        e.set_radial(12)
+        if shape == "plain":
+            e.run_plain(4)
+        else:
+            e.set_launch(128, split_phases=int(shape == "split"))
+            e.run_batched(4)
+        out.append((e.observables(), e.density()[0], e.radial()[0], e.get_beads()))
+        if shape == "split":
+            e.reset_measurements()
+            e.measure()
+            exact = e.observables()[0]
+        e.close()
+    for o in out[1:]:
+        np.testing.assert_array_equal(o[3], out[0][3])
+        np.testing.assert_allclose(o[0], out[0][0], rtol=1e-12, atol=1e-12)
+        np.testing.assert_array_equal(o[1], out[0][1])
+        np.testing.assert_array_equal(o[2], out[0][2])
+    last = out[2][0][-1]
+    scale = np.maximum(np.abs(exact), 1.0)
+    assert np.all(np.abs(last - exact)[[0, 1, 4, 5, 6]] <= 1e-10 * scale[[0, 1, 4, 5, 6]])
+    assert np.all(np.abs(last - exact)[[2, 3]] <= 2e-7 * scale[[2, 3]])
