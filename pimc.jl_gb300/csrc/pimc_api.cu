@@ -213,11 +213,17 @@ ChainDesc make_desc(const pimc_params &p, int chain) {
       // 2 d <= d^2 / s + s with s the reach; the exponential turns an argument
       // error D into expm1(D) <= D exp(D), D at three reaches (beyond, the terms
       // are below exp(-9 y(s))); the FP32 product and ex2.approx add 5e-7 (1 + y)
-      const double u2i = u * u * d.inv2s2, sr = std::sqrt((double)d.q_lim_hi) + 1.0;
+      const double u2i = std::max(u * u * d.inv2s2, 1e-300), sr = std::sqrt((double)d.q_lim_hi) + 1.0;
       const double fac = 1.01 * std::exp(std::min(60.0, u2i * e * (6.0 * sr + e)));
-      d.est_a = (float)(fac * u2i * e / sr + 5e-7 * u2i);
-      d.est_b = (float)(fac * u2i * e * (sr + e) + 5e-7);
-      d.est_x = (float)(-u2i * 1.4426950408889634);
+      // at the reach y(s) = u2i s^2 = yh: relative error eps; past it the bound is
+      // at most eps (y / yh) exp(-y), which falls from y = 1 on
+      const double yh = u2i * sr * sr, w16 = 65536.0 * 65536.0;
+      d.est_eps = (float)(fac * u2i * e * (2.0 * sr + e) + 5e-7 * (1.0 + yh));
+      d.est_far = (float)(1.001 * (yh >= 1.0 ? std::exp(-yh) : std::exp(-1.0) / yh) + 1e-30);
+      d.est_x = (float)(-u2i * 1.4426950408889634 / w16);
+      // the FP32 squares and sums are within 2e-7
+      d.est_lo = d.q_lim_lo > 0u ? (float)(d.q_lim_lo * w16 * (1.0 - 4e-7)) : -1.f;
+      d.est_hi = (float)((d.q_lim_hi + 1.0) * w16 * (1.0 + 4e-7));
       d.f_scale = 4294967296.0 / (2.0 * p.L);
       const double fu = 1.0 / d.f_scale;
       d.f_unit = (float)fu;
@@ -781,7 +787,10 @@ int run_plain(Handle *h, long long n) {
   }
   if (any_fused) CK(sweep_set_smem(0, p.dyn_smem));
   CK(stage_slots_set_smem(stage_smem));
-  for (int sc = 0; sc < 2; ++sc) CK(sweep_phase_set_smem(1, 0, sc, 0, p.dyn_smem));
+  // the swaps of a long interacting chain: twice the warps for its pair scans
+  Plan wide = plan_smem(h, 0, 512, 1, kStateBudget);
+  if (h->max_dyn_smem > 0 && wide.dyn_smem > (size_t)h->max_dyn_smem) wide = p;
+  for (int sc = 0; sc < 2; ++sc) CK(sweep_phase_set_smem(1, 0, sc, 0, std::max(wide.dyn_smem, p.dyn_smem)));
   CK(sweep_phase_set_smem(2, 0, 0, 0, p.dyn_smem));
   SweepArgs a = sweep_args(h, p);
   a.nchains = 1;
@@ -804,7 +813,10 @@ int run_plain(Handle *h, long long n) {
       if (sp[c].phases > 0) CK(launch_stage_close(a, h->stream));
       launches += sp[c].phases + (sp[c].phases > 0);
       if (h->mix[c].swaps_per_sweep > 0 && h->desc[c].N > 1) {
-        CK(launch_sweep_phase(a, 1, 0, spec[c], 0, 1, p.block, p.dyn_smem, h->stream));
+        const Plan &w = (h->desc[c].flags & PF_PAIR) && h->desc[c].N >= 512 ? wide : p;
+        a.state_bytes = w.state_bytes;
+        CK(launch_sweep_phase(a, 1, 0, spec[c], 0, 1, w.block, w.dyn_smem, h->stream));
+        a.state_bytes = p.state_bytes;
         ++launches;
       }
       a.measure_par = h->mix[c].measure_every > 0 && measure_large(h, c);

@@ -1542,6 +1542,7 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
       __syncwarp();
       PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
       scan_mirror<2>(c, j0, m, cq, skip, 0, 1, e, lane, NoStop());
+      scan_bounds(d, e);
       __syncwarp();
       float t, r;
       est_lane(e, -1.f, t, r);

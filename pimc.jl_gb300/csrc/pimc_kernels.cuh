@@ -1111,8 +1111,20 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
     const int i0 = min(N, lane * chunk), i1 = min(N, i0 + chunk);
     float *mine = Sw + lane * (chunk | 1);
     const int len = i1 - i0;
-    float ls = 0.f;
-    for (int k = 0; k < len; ++k) ls += mine[k];
+    // eight weights read at a time, added one by one (zeros past the chunk add
+    // nothing)
+    auto chunk_sum = [&]() {
+      float t = 0.f;
+      for (int k0 = 0; k0 < len; k0 += 8) {
+        float w[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) w[q] = k0 + q < len ? mine[k0 + q] : 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t += w[q];
+      }
+      return t;
+    };
+    float ls = chunk_sum();
     ssum = warp_sum(ls);
     if (!(ssum > 0.f)) {
       // every weight underflowed: exponents shifted by their largest.  One warp
@@ -1133,17 +1145,22 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
       }
       G::sync();
       wmax = S.sums->pf[0];
-      ls = 0.f;
-      for (int k = 0; k < len; ++k) ls += mine[k];
+      ls = chunk_sum();
       ssum = warp_sum(ls);
       G::sync();
     }
     const float target = S.draws->up[slot] * ssum;
     float cw = warp_exclusive_scan(ls);
     int cand = 0x7fffffff;
-    for (int k = 0; k < len; ++k) {
-      cw += mine[k];
-      if (cw >= target) { cand = i0 + k; break; }
+    for (int k0 = 0; k0 < len && cand == 0x7fffffff; k0 += 8) {
+      float w[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) w[q] = k0 + q < len ? mine[k0 + q] : 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        cw += w[q];
+        if (cw >= target && k0 + q < len) cand = min(cand, i0 + k0 + q);
+      }
     }
     n2 = __reduce_min_sync(0xffffffffu, (unsigned)cand);
     if (n2 >= N || n2 < 0) n2 = N - 1;
@@ -1164,25 +1181,48 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
   float mx3[3] = {0.f, 0.f, 0.f}, s34[4] = {0.f, 0.f, 0.f, 0.f};
   float lrf = 0.f, lre = 0.f;
   if (f_phys) {
-    const HBead A{0.0, 0.0, Aq}, E1{0.0, 0.0, E1q};
-    const HBead B{0.0, 0.0, c.Q(n2, j0)}, E2{0.0, 0.0, c.Q(e2p, se)};
-    auto expo_p = [&](int i, const HBead &s_, const HBead &f_) {
-      if (i != n1 && i != n2) return hb.expo(i, s_, f_);
-      return hb.expo(i, s_, f_, i == n1 ? &E2 : &E1);
+    const unsigned Bq = c.Q(n2, j0), E2q = c.Q(e2p, se);
+    // expo(i; B, E2), then with the ends of n1 and n2 exchanged expo(i; A, E2) and
+    // expo(i; B, E1): minus the squared distances from the start to i's end and
+    // from i's start to the end (swap_group's, in its arithmetic); the exponents
+    // stay in registers between the maxima and the sums.  At most 256 threads:
+    // the sums are then the same in larger CTAs
+    constexpr int U = 4;
+    const int np = min(nt, 256);
+    auto expos = [&](int i, float (&x)[3]) {
+      const unsigned qa = c.Q(i, j0), qe = c.Q(hb.endp(i), se);
+      const unsigned qx = i == n1 ? E2q : (i == n2 ? E1q : qe);  // the exchanged end
+      const float f2 = (float)qdist2(qa, E2q);
+      x[0] = -((float)qdist2(Bq, qe) + f2) * hb.inv_denf;
+      x[1] = -((float)qdist2(Aq, qx) + f2) * hb.inv_denf;
+      x[2] = -((float)qdist2(Bq, qx) + (float)qdist2(qa, E1q)) * hb.inv_denf;
     };
-    float mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = tid; i < N; i += nt) {
-      const float a0 = hb.expo(i, B, E2), a1 = expo_p(i, A, E2), a2 = expo_p(i, B, E1);
-      mx[0] = a0 > mx[0] ? a0 : mx[0];
-      mx[1] = a1 > mx[1] ? a1 : mx[1];
-      mx[2] = a2 > mx[2] ? a2 : mx[2];
+    float mx[3] = {-INFINITY, -INFINITY, -INFINITY}, kept[U][3];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const int i = tid + q * np;
+      if (tid < np && i < N) {
+        expos(i, kept[q]);
+        for (int k = 0; k < 3; ++k) mx[k] = kept[q][k] > mx[k] ? kept[q][k] : mx[k];
+      }
     }
+    if (tid < np)
+      for (int i = tid + U * np; i < N; i += np) {
+        float x[3];
+        expos(i, x);
+        for (int k = 0; k < 3; ++k) mx[k] = x[k] > mx[k] ? x[k] : mx[k];
+      }
     G::template max<3>(mx, red);
-    for (int i = tid; i < N; i += nt) {
-      s34[0] += hb.ex_(hb.expo(i, B, E2) - mx[0]);
-      s34[1] += hb.ex_(expo_p(i, A, E2) - mx[1]);
-      s34[2] += hb.ex_(expo_p(i, B, E1) - mx[2]);
-    }
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+      if (tid < np && tid + q * np < N)
+        for (int k = 0; k < 3; ++k) s34[k] += hb.ex_(kept[q][k] - mx[k]);
+    if (tid < np)
+      for (int i = tid + U * np; i < N; i += np) {
+        float x[3];
+        expos(i, x);
+        for (int k = 0; k < 3; ++k) s34[k] += hb.ex_(x[k] - mx[k]);
+      }
     // S_1 rides along in the fourth slot
     s34[3] = tid == 0 ? ssum : 0.f;
     G::template sum<4>(s34, red);
@@ -1365,7 +1405,9 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
         if (!monotone) return false;
         if (*flag) return true;
         float t, r;
-        est_lane(q, sgn_new, t, r);
+        PairEst qb = q;
+        scan_bounds(d, qb);
+        est_lane(qb, sgn_new, t, r);
         const float lb = warp_sum(t - r);
         if (gh * lb * (lb > 0.f ? 0.99999f : 1.00001f) > need) {
           if (lane == 0) *flag = 1;
@@ -1384,6 +1426,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
         PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
         if (level == 0) {
           scan_mirror<4>(c, j0, m, reinterpret_cast<const unsigned *>(S.cq), skip, warp, nwarps, e, lane, stop);
+          scan_bounds(d, e);
         } else {
           // both buffers' normals are spent
           uint2 *cf = reinterpret_cast<uint2 *>(reinterpret_cast<float *>(S.z) + 256);

@@ -39,53 +39,67 @@ struct ScanSkip {
   }
 };
 
-// a lane's sums over one particle, from the mirror: e.so / e.sn old and new
-// sums of exp(-r_a^2/2s^2) + exp(-r_b^2/2s^2) over the links whose start has
-// the particle within reach, e.bo / e.bn bounds on their distance from the
-// exact sums (a mirror distance is within kQErr units of the exact one;
-// ChainDesc::est_a, est_b).  cq[t * NC + k]: mirror word of centre k at bead t,
-// t = 0 .. m; word(t): the particle's; on(k): whether centre k counts it.
+// a lane's sums over one particle, from the mirror, added to e: old and new
+// sums of exp(-r_a^2/2s^2) + exp(-r_b^2/2s^2) over the links whose start surely
+// has the particle within reach (PairEst so, sn) and over those where it may
+// (bo, bn: scan_bounds turns both into a sum and a bound).  cq[t * NC + k]:
+// mirror word of centre k at bead t, t = 0 .. m; word(t): the particle's; on(k):
+// whether centre k counts it.  Sixteen instructions per bead and centre bound
+// the scan: coordinates as the upper halves of words, so that a difference
+// wraps by itself and converts exactly.
 template <int NC, class Word, class On>
 __device__ __forceinline__ void scan_block(const ChainDesc &d, int m, const unsigned *cq, const Word &word,
                                            const On &on, PairEst &e) {
-  const float ca = d.est_a, cb = d.est_b, cx = d.est_x;
-  unsigned lo[NC], hi[NC];
-  float ep[NC], rp[NC], wp[NC], gp[NC];
+  const float cx = d.est_x;
+  float lo[NC], hi[NC], ep[NC], wi[NC], wm[NC];
 #pragma unroll
   for (int k = 0; k < NC; ++k) {
-    lo[k] = on(k) ? d.q_lim_lo : 0u;
-    hi[k] = on(k) ? d.q_lim_hi + 1u : 0u;
-    ep[k] = rp[k] = wp[k] = gp[k] = 0.f;
+    lo[k] = on(k) ? d.est_lo : -1.f;
+    hi[k] = on(k) ? d.est_hi : -1.f;
+    ep[k] = wi[k] = wm[k] = 0.f;
   }
   // the slices' words four beads ahead: a step takes a few hundred cycles, a
   // word from L2 up to a thousand
   unsigned q0 = word(0), q1 = word(min(1, m)), q2 = word(min(2, m)), q3 = word(min(3, m));
   for (int t = 0; t <= m; ++t) {
-    const unsigned q = q0;
+    const unsigned qx = q0 << 16, qy = q0 & 0xffff0000u;
     q0 = q1;
     q1 = q2;
     q2 = q3;
     if (t + 4 <= m) q3 = word(t + 4);
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      const unsigned d2 = qdist2(cq[t * NC + k], q);
-      const float f = (float)d2, x = ex2_approx(f * cx);
-      const float r = fmaf(x, fmaf(ca, f, cb), 1e-30f);
-      const float v = ep[k] + x, ve = rp[k] + r;
-      float &s = (k & 1) ? e.sn : e.so, &bd = (k & 1) ? e.bn : e.bo;
-      s = fmaf(wp[k], v, s);
-      bd = fmaf(wp[k], ve, bd);
-      bd = fmaf(gp[k], v + ve, bd);
+      const unsigned w = cq[t * NC + k];
+      const float dx = (float)(int)((w << 16) - qx), dy = (float)(int)((w & 0xffff0000u) - qy);
+      const float f = fmaf(dx, dx, dy * dy), x = ex2_approx(f * cx), v = ep[k] + x;
+      if (k & 1) {
+        e.sn = fmaf(wi[k], v, e.sn);
+        e.bn = fmaf(wm[k], v, e.bn);
+      } else {
+        e.so = fmaf(wi[k], v, e.so);
+        e.bo = fmaf(wm[k], v, e.bo);
+      }
       ep[k] = x;
-      rp[k] = r;
-      // surely within reach: weight 1; unsettled: half the link, within half
-      const bool in = d2 < lo[k], may = d2 < hi[k];
-      gp[k] = may && !in ? 0.5f : 0.f;
-      wp[k] = in ? 1.f : gp[k];
+      wi[k] = f < lo[k] ? 1.f : 0.f;
+      wm[k] = f < hi[k] ? 1.f : 0.f;
     }
   }
-  e.ko += m * (NC / 2) * 3;
-  e.kn += m * (NC / 2) * 3;
+  e.ko += m * (NC / 2);
+  e.kn += m * (NC / 2);
+}
+
+// the lane's sums [sure, may] of scan_block as the middle of the interval that
+// holds the exact sum, and its half width.  An end within reach is off by at
+// most est_eps of its value; one beyond by at most est_eps times est_far (the
+// error bound grows with d^2, but x d^2 falls past the reach), once per link
+// (ko, kn).
+__device__ __forceinline__ void scan_bounds(const ChainDesc &d, PairEst &e) {
+  const float far = d.est_eps * d.est_far;
+  const float mo = 0.5f * (e.so + e.bo), mn = 0.5f * (e.sn + e.bn);
+  e.bo = 0.5f * (e.bo - e.so) + d.est_eps * e.bo + far * (float)e.ko;
+  e.bn = 0.5f * (e.bn - e.sn) + d.est_eps * e.bn + far * (float)e.kn;
+  e.so = mo;
+  e.sn = mn;
 }
 
 // the lane's sums over the particles 32 (part, part + nparts, ...) + lane, the
@@ -107,6 +121,7 @@ __device__ __forceinline__ bool scan_mirror(const CV &c, int j0, int m, const un
   }
   return false;
 }
+// (stop sees the raw sums; the caller applies scan_bounds)
 
 // 32-bit fixed point of a coordinate on the periodic box (a wrapped difference
 // is the minimum image), one FP64 instruction

@@ -145,6 +145,7 @@ __device__ __forceinline__ void stage_slot(const CV &c, unsigned long long sweep
       const ScanSkip<2> skip{n, -1, true};
       PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
       scan_mirror<2>(c, st, m, cq, skip, 0, 1, e, lane, NoStop(), n0);
+      scan_bounds(d, e);
       float t, r, tb, rb;
       est_lane(e, -1.f, t, r);
       // the batch's paths: in place, and for earlier windows as proposed
@@ -154,6 +155,7 @@ __device__ __forceinline__ void stage_slot(const CV &c, unsigned long long sweep
       auto word = [&](int q) { return st + q < M ? c.Q(bl, st + q) : c.Q(nxb, st + q - M); };
       PairEst o = {0.f, 0.f, 0.f, 0.f, 0, 0}, p = {0.f, 0.f, 0.f, 0.f, 0, 0};
       scan_block<2>(d, m, cq, word, [&](int) { return b < N && b != n; }, o);
+      scan_bounds(d, o);
       est_lane(o, -1.f, tb, rb);
       if (lane > i) {  // a later window's path stays in place
         t += tb;
@@ -171,6 +173,7 @@ __device__ __forceinline__ void stage_slot(const CV &c, unsigned long long sweep
         const uint2 *cb = S.cq + (size_t)ib * E;
         scan_block<2>(d, m, cq, [&](int q) { return q >= 1 && q < mb ? cb[q].y : word(q); },
                       [&](int) { return lane < i; }, p);
+        scan_bounds(d, p);
         est_lane(p, -1.f, w.z, w.w);
       }
       S.pt[i * SLOT_B + lane] = w;

@@ -56,10 +56,12 @@ struct ChainDesc {
   // which it is surely beyond (kQErr units of mirror error on a distance)
   float q_u2i;
   unsigned q_lim_lo, q_lim_hi;
-  // scan_mirror's exponential at squared mirror distance d2: ex2(est_x d2),
-  // relative error at most est_a d2 + est_b; scan_fixed's fixed point: 2^32 / 2L,
-  // its unit, and the constant part of its exponentials' relative error
-  float est_a, est_b, est_x;
+  // scan_mirror's exponential at squared mirror distance f (in units 2^-16 of the
+  // mirror's): ex2(est_x f), relative error at most est_eps within reach, and
+  // est_eps est_far in absolute terms beyond; reach bounds surely within and
+  // surely beyond.  scan_fixed's fixed point: 2^32 / 2L, its unit, and the
+  // constant part of its exponentials' relative error
+  float est_eps, est_far, est_x, est_lo, est_hi;
   float f_unit, est2;
   double f_scale;
   // the sweeps' FP32 heat-bath exponent scale per window length m:
