@@ -790,7 +790,8 @@ int run_plain(Handle *h, long long n) {
   // the swaps of a long interacting chain: twice the warps for its pair scans
   Plan wide = plan_smem(h, 0, 512, 1, kStateBudget);
   if (h->max_dyn_smem > 0 && wide.dyn_smem > (size_t)h->max_dyn_smem) wide = p;
-  for (int sc = 0; sc < 2; ++sc) CK(sweep_phase_set_smem(1, 0, sc, 0, std::max(wide.dyn_smem, p.dyn_smem)));
+  for (int sc = 0; sc < 2; ++sc)
+    for (int rg : {0, SWAP_LONE}) CK(sweep_phase_set_smem(1, 0, sc, rg, std::max(wide.dyn_smem, p.dyn_smem)));
   CK(sweep_phase_set_smem(2, 0, 0, 0, p.dyn_smem));
   SweepArgs a = sweep_args(h, p);
   a.nchains = 1;
@@ -801,7 +802,7 @@ int run_plain(Handle *h, long long n) {
     for (int c = 0; c < h->nchains; ++c) {
       a.chain0 = c;
       if (fused[c]) {
-        CK(launch_sweep(a, 0, 1, p.block, p.dyn_smem, h->stream));
+        CK(launch_sweep(a, 2, 1, p.block, p.dyn_smem, h->stream));
         ++launches;
         continue;
       }
@@ -813,9 +814,10 @@ int run_plain(Handle *h, long long n) {
       if (sp[c].phases > 0) CK(launch_stage_close(a, h->stream));
       launches += sp[c].phases + (sp[c].phases > 0);
       if (h->mix[c].swaps_per_sweep > 0 && h->desc[c].N > 1) {
-        const Plan &w = (h->desc[c].flags & PF_PAIR) && h->desc[c].N >= 512 ? wide : p;
+        const bool two = (h->desc[c].flags & PF_PAIR) && h->desc[c].N >= 512 && wide.block > 256;
+        const Plan &w = two ? wide : p;
         a.state_bytes = w.state_bytes;
-        CK(launch_sweep_phase(a, 1, 0, spec[c], 0, 1, w.block, w.dyn_smem, h->stream));
+        CK(launch_sweep_phase(a, 1, 0, spec[c], two ? 0 : SWAP_LONE, 1, w.block, w.dyn_smem, h->stream));
         a.state_bytes = p.state_bytes;
         ++launches;
       }
@@ -840,6 +842,18 @@ int run_plain(Handle *h, long long n) {
   return PIMC_OK;
 }
 
+// the fused kernel of a plan: in CTAs of up to 256 threads the one with 255
+// registers where as many CTAs (or all chains) are resident with it (contact
+// batch of 256 chains, one CTA per SM by shared memory: 25.4 -> 21.9 ms)
+int fused_mode(const Handle *h, const Plan &p) {
+  if (p.mode != 0 || p.block > 256) return p.mode;
+  const size_t smem = fused_smem(h, p);
+  int narrow = 0, wide = 0;
+  if (sweep_occupancy(0, p.block, smem, &narrow) != cudaSuccess || sweep_occupancy(2, p.block, smem, &wide) != cudaSuccess)
+    return 0;
+  return wide >= narrow || (long long)wide * h->num_sms >= h->nchains ? 2 : 0;
+}
+
 // persistent grid: every resident CTA (CTA mode) or resident warp (warp mode)
 // pulls chains from the work queue
 // 1 when every chain follows the reference's rules without a hard core or
@@ -851,14 +865,23 @@ int swap_spec(const Handle *h) {
   return 1;
 }
 
+// register variant of a phase's kernel: the plan's, or for swaps in CTAs of 64
+// threads the one with the most registers that still holds every chain at once
+// (128 registers, eight CTAs per SM, spill in the pair scans: 512 physical
+// chains end to end 34.5 ms, with 255 registers and four CTAs 28.3)
+int phase_regs(const Handle *h, const Plan &p, int ph) {
+  if (p.pregs[ph] || ph != 1 || p.pwarp[1] || phase_block(p, 1) > 64) return p.pregs[ph];
+  return h->nchains <= 4 * h->num_sms ? 255 : (h->nchains <= 6 * h->num_sms ? 170 : 0);
+}
+
 // resident CTAs (or warps) for a launch of the plan's kernel; phase >= 0
 // names a phase kernel of a split plan
 int grid_for(Handle *h, const Plan &p, int phase = -1, int nch = -1) {
   int per_sm = 0;
   const cudaError_t e = phase >= 0
-                            ? sweep_phase_occupancy(phase, p.pwarp[phase], swap_spec(h), p.pregs[phase],
+                            ? sweep_phase_occupancy(phase, p.pwarp[phase], swap_spec(h), phase_regs(h, p, phase),
                                                     phase_block(p, phase), phase_smem(p, phase), &per_sm)
-                            : sweep_occupancy(p.mode, p.block, fused_smem(h, p), &per_sm);
+                            : sweep_occupancy(fused_mode(h, p), p.block, fused_smem(h, p), &per_sm);
   if (e != cudaSuccess || per_sm < 1) per_sm = 1;
   const bool warp = phase >= 0 ? p.pwarp[phase] != 0 : p.mode == 1;
   const int units_per_cta = warp ? phase_block(p, phase >= 0 ? phase : 0) / 32 : 1;
@@ -888,7 +911,7 @@ cudaError_t plan_set_smem(const Handle *h, const Plan &p) {
     if (e != cudaSuccess) return e;
   }
   for (int ph = 0; ph < 3; ++ph) {
-    const cudaError_t e = sweep_phase_set_smem(ph, p.pwarp[ph], swap_spec(h), p.pregs[ph], phase_smem(p, ph));
+    const cudaError_t e = sweep_phase_set_smem(ph, p.pwarp[ph], swap_spec(h), phase_regs(h, p, ph), phase_smem(p, ph));
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -930,7 +953,7 @@ cudaError_t issue_phase(Handle *h, const Plan &p, const SweepArgs &a, int ph, lo
   b.measure_par = meas;
   cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
   if (e == cudaSuccess)
-    e = launch_sweep_phase(b, ph, p.pwarp[ph], swap_spec(h), p.pregs[ph], grid_for(h, p, ph, a.nchains),
+    e = launch_sweep_phase(b, ph, p.pwarp[ph], swap_spec(h), phase_regs(h, p, ph), grid_for(h, p, ph, a.nchains),
                            phase_block(p, ph), phase_smem(p, ph), h->stream);
   if (launches) *launches += 1;
   if (meas && e == cudaSuccess) {
@@ -954,7 +977,7 @@ cudaError_t issue_sweeps(Handle *h, const Plan &p, SweepArgs a, int n, long long
       for (int c = 0; c < h->nchains && !a.measure_par; ++c) a.measure_par = measure_large(h, c);
     cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
     if (e == cudaSuccess)
-      e = launch_sweep(a, p.mode, grid_for(h, p, -1, a.nchains), p.block, smem, h->stream);
+      e = launch_sweep(a, fused_mode(h, p), grid_for(h, p, -1, a.nchains), p.block, smem, h->stream);
     if (launches) *launches += 1;
     if (a.measure_par && e == cudaSuccess) {
       e = launch_measure_sweep(a, h->meas_items, h->num_sms, h->stream);

@@ -1367,7 +1367,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
     };
     // the pair of the two moving paths, old and new (physical rules), exact
     double w2[2] = {0.0, 0.0};  // pair parts of w_initial, w_update
-    if (f_phys)
+    auto cross_exact = [&]() {
       for (int t = tid; t < m; t += nt) {
         const int j = slc(t), jn = slc(t + 1);
         const int o1 = own(0, t), o1n = own(0, t + 1), o2 = own(1, t), o2n = own(1, t + 1);
@@ -1389,6 +1389,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
             w2[1] += lnU2(d, r2n, mi2(d, S.r1x[t + 1], S.r1y[t + 1], S.r2x[t + 1], S.r2y[t + 1]));
         }
       }
+    };
     if (fast && (!f_contact || d.ct_cells)) {
       // bracketed from the mirror, and where that straddles the threshold from
       // the positions in fixed point (pimc_scan.cuh); the warps split the
@@ -1416,18 +1417,35 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
         return false;
       };
       const ScanSkip<4> skip{n1, n2, f_phys};
-      // the exact cross term rides along (its lanes' float sums)
-      float xs = 0.f, xr = 0.f;
-      if (f_phys) {
-        xs = warp_sum((float)(w2[1] - w2[0]));
-        xr = 2e-6f * warp_sum((float)(fabs(w2[0]) + fabs(w2[1])));
-      }
+      float xs = 0.f, xr = 0.f;  // the exact cross term's float sums
       for (int level = f_contact ? 1 : 0; level < 2 && dec == -1; ++level) {
         PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
         if (level == 0) {
+          if (f_phys && warp == 0) {
+            // the two moving paths' own pair, a lane per bead (the exact form's 64
+            // FP64 instructions wait for the next level)
+            const uint4 w = S.cq[min(lane, m)];
+            const float ox = (float)(int)((w.x << 16) - (w.z << 16)), oy = (float)(int)((w.x & 0xffff0000u) - (w.z & 0xffff0000u));
+            const float nx = (float)(int)((w.y << 16) - (w.w << 16)), ny = (float)(int)((w.y & 0xffff0000u) - (w.w & 0xffff0000u));
+            const float fo = fmaf(ox, ox, oy * oy), fn = fmaf(nx, nx, ny * ny);
+            const float xo = ex2_approx(fo * d.est_x), xn = ex2_approx(fn * d.est_x);
+            const float vo = xo + __shfl_down_sync(0xffffffffu, xo, 1), vn = xn + __shfl_down_sync(0xffffffffu, xn, 1);
+            if (lane < m) {
+              e.so = fo < d.est_lo ? vo : 0.f;
+              e.bo = fo < d.est_hi ? vo : 0.f;
+              e.sn = fn < d.est_lo ? vn : 0.f;
+              e.bn = fn < d.est_hi ? vn : 0.f;
+            }
+            e.ko = e.kn = 1;
+          }
           scan_mirror<4>(c, j0, m, reinterpret_cast<const unsigned *>(S.cq), skip, warp, nwarps, e, lane, stop);
           scan_bounds(d, e);
         } else {
+          if (f_phys) {
+            cross_exact();
+            xs = warp_sum((float)(w2[1] - w2[0]));
+            xr = 2e-6f * warp_sum((float)(fabs(w2[0]) + fabs(w2[1])));
+          }
           // both buffers' normals are spent
           uint2 *cf = reinterpret_cast<uint2 *>(reinterpret_cast<float *>(S.z) + 256);
           for (int k = tid; k < 4 * (m + 1); k += nt) {
@@ -1474,6 +1492,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
     PROF_MARK(6);
     if (dec == -1) {
       PROF_COUNT(4);
+      if (f_phys && !(fast && (!f_contact || d.ct_cells))) cross_exact();  // not at hand yet
       for (int b = 0; b < 2; ++b) {
         const int t0 = max(a0 - b * m, 0), t1 = min(a1 - b * m, m);
         if (t0 >= t1) continue;

@@ -97,7 +97,8 @@ inline long long adjoint_ctas(int N, int M, int ib) {
   return ((long long)M * ((N + ib - 1) / ib) + 3) / 4;
 }
 
-// mode 0: one CTA per chain (k_sweep); mode 1: one warp per chain (k_sweep_warp)
+// mode 0: one CTA per chain (k_sweep); mode 1: one warp per chain (k_sweep_warp);
+// mode 2: one CTA of up to 256 threads per chain, compiled for 255 registers
 cudaError_t launch_sweep(const SweepArgs &a, int mode, int grid, int block, size_t smem,
                          cudaStream_t s);
 cudaError_t sweep_set_smem(int mode, size_t smem);
@@ -186,17 +187,22 @@ cudaError_t launch_contact_table(double *dtab, int n, double range, double g0, d
 cudaError_t launch_contact_cells(const double *tab, float4 *cells, int n, double thr, int *last, cudaStream_t s);
 // measured FP64 FMA throughput of the current device (TFLOP/s)
 cudaError_t fp64_peak(int num_sms, cudaStream_t st, double *tflops);
+constexpr int SWAP_LONE = 256;  // swap kernel variant for lone chains (regs)
 // the swap-phase kernels' translation unit (pimc_swap.cu): its kernel for a
 // launch shape and its launcher
 const void *swap_kernel(int warp, int spec, int regs);
 cudaError_t launch_swap(const SweepArgs &a, int warp, int spec, int regs, int grid, int block,
                         size_t smem, cudaStream_t s);
-// accessors of each kernel unit's device globals (swap_, fused_, attempt_)
+const void *swap_any_kernel(int warp, int regs);
+cudaError_t launch_swap_any(const SweepArgs &a, int warp, int regs, int grid, int block, size_t smem,
+                            cudaStream_t s);
+// accessors of each kernel unit's device globals (swap_, swap_any_, fused_, attempt_)
 #define PIMC_UNIT_DECL(unit)                                                              \
   cudaError_t unit##_upload_exp_table(const double *tab, size_t bytes);                   \
   cudaError_t unit##_profile_take(unsigned long long *out, bool reset, cudaStream_t s);  \
   cudaError_t unit##_check_word_take(cudaStream_t s, unsigned long long *w);
 PIMC_UNIT_DECL(swap)
+PIMC_UNIT_DECL(swap_any)
 PIMC_UNIT_DECL(fused)
 PIMC_UNIT_DECL(attempt)
 #undef PIMC_UNIT_DECL

@@ -1,51 +1,46 @@
-// pimc_swap.cu -- the swap-phase kernels of the split sweep, in a
-// translation unit of their own so that they compile in parallel with the
-// rest (pimc_sweep.cu); the host reaches them through the launchers below.
+// pimc_swap.cu -- the swap-phase kernels of the split sweep for the reference's
+// rules, and the launchers of all swap kernels; the generic ones are
+// pimc_swap_any.cu's (translation units of their own compile in parallel).
 #include <cuda_runtime.h>
 
 #include "pimc_sweep.cuh"
 
 namespace pimc {
 
-// one CTA per chain (the generic swap)
-__global__ void __launch_bounds__(512, 1) k_sweep_swap(SweepArgs a) { sweep_cta<SW_SWAP>(a); }
 // the swap launch for batches whose every chain follows the reference's
-// rules without a hard core or a contact table (swap_group SWAP_REF)
+// rules without a hard core or a contact table (SWAP_REF), one CTA per chain
 __global__ void __launch_bounds__(512, 1) k_sweep_swap_ref(SweepArgs a) {
   sweep_cta<SW_SWAP, SWAP_REF>(a);
 }
-// both for CTAs of at most 64 threads, compiled for 6 and 4 resident CTAs
-// per SM: up to 170 and 255 registers a thread instead of 128 (fewer
-// spills, fewer chains in flight)
-__global__ void __launch_bounds__(64, 6) k_sweep_swap_r170(SweepArgs a) { sweep_cta<SW_SWAP>(a); }
-__global__ void __launch_bounds__(64, 4) k_sweep_swap_r255(SweepArgs a) { sweep_cta<SW_SWAP>(a); }
+// for CTAs of at most 64 threads, compiled for 6 and 4 resident CTAs per SM: up
+// to 170 and 255 registers a thread instead of 128 (fewer spills, fewer chains
+// in flight); and for lone chains in CTAs of up to 256 threads
 __global__ void __launch_bounds__(64, 6) k_sweep_swap_ref_r170(SweepArgs a) {
   sweep_cta<SW_SWAP, SWAP_REF>(a);
 }
 __global__ void __launch_bounds__(64, 4) k_sweep_swap_ref_r255(SweepArgs a) {
   sweep_cta<SW_SWAP, SWAP_REF>(a);
 }
-// one warp per chain: twice the chains in flight of a two-warp CTA per chain
-// at the same registers per SM
-__global__ void __launch_bounds__(256, 2) k_sweep_swap_warp(SweepArgs a) { sweep_warp<SW_SWAP>(a); }
+__global__ void __launch_bounds__(256, 1) k_sweep_swap_ref_lone(SweepArgs a) {
+  sweep_cta<SW_SWAP, SWAP_REF>(a);
+}
 
-// regs: 0 (the 128-register kernels), 170 or 255
+// regs: 0 (the 128-register kernels), 170 or 255 (CTAs of 64 threads), SWAP_LONE
 const void *swap_kernel(int warp, int spec, int regs) {
-  if (warp) return (const void *)k_sweep_swap_warp;
-  if (regs == 170) return spec ? (const void *)k_sweep_swap_ref_r170 : (const void *)k_sweep_swap_r170;
-  if (regs == 255) return spec ? (const void *)k_sweep_swap_ref_r255 : (const void *)k_sweep_swap_r255;
-  return spec ? (const void *)k_sweep_swap_ref : (const void *)k_sweep_swap;
+  if (warp || !spec) return swap_any_kernel(warp, regs);
+  if (regs == SWAP_LONE) return (const void *)k_sweep_swap_ref_lone;
+  if (regs == 170) return (const void *)k_sweep_swap_ref_r170;
+  if (regs == 255) return (const void *)k_sweep_swap_ref_r255;
+  return (const void *)k_sweep_swap_ref;
 }
 
 cudaError_t launch_swap(const SweepArgs &a, int warp, int spec, int regs, int grid, int block,
                         size_t smem, cudaStream_t s) {
-  if (warp) k_sweep_swap_warp<<<grid, block, smem, s>>>(a);
-  else if (regs == 170 && spec) k_sweep_swap_ref_r170<<<grid, block, smem, s>>>(a);
-  else if (regs == 170) k_sweep_swap_r170<<<grid, block, smem, s>>>(a);
-  else if (regs == 255 && spec) k_sweep_swap_ref_r255<<<grid, block, smem, s>>>(a);
-  else if (regs == 255) k_sweep_swap_r255<<<grid, block, smem, s>>>(a);
-  else if (spec) k_sweep_swap_ref<<<grid, block, smem, s>>>(a);
-  else k_sweep_swap<<<grid, block, smem, s>>>(a);
+  if (warp || !spec) return launch_swap_any(a, warp, regs, grid, block, smem, s);
+  if (regs == SWAP_LONE) k_sweep_swap_ref_lone<<<grid, block, smem, s>>>(a);
+  else if (regs == 170) k_sweep_swap_ref_r170<<<grid, block, smem, s>>>(a);
+  else if (regs == 255) k_sweep_swap_ref_r255<<<grid, block, smem, s>>>(a);
+  else k_sweep_swap_ref<<<grid, block, smem, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -928,6 +928,7 @@ cudaError_t upload_exp_table() {
   for (int k = 0; k <= EXPTAB_N; ++k) tab[k] = std::exp(-k / 64.0);
   cudaError_t e = tu_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = swap_upload_exp_table(tab, sizeof(tab));
+  if (e == cudaSuccess) e = swap_any_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = fused_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = attempt_upload_exp_table(tab, sizeof(tab));
   return e;
@@ -1327,6 +1328,7 @@ cudaError_t profile_take(unsigned long long *out, bool reset, cudaStream_t s) {
   for (int k = 0; k < 32; ++k) out[k] = 0;
   cudaError_t e = tu_profile_take(out, reset, s);
   if (e == cudaSuccess) e = swap_profile_take(out, reset, s);
+  if (e == cudaSuccess) e = swap_any_profile_take(out, reset, s);
   if (e == cudaSuccess) e = fused_profile_take(out, reset, s);
   if (e == cudaSuccess) e = attempt_profile_take(out, reset, s);
   return e;
@@ -1342,10 +1344,10 @@ cudaError_t profile_take(unsigned long long *out, bool reset, cudaStream_t s) {
 // nonzero): read and cleared (0 in the default build, which has no bounds
 // checks)
 cudaError_t check_word_take(cudaStream_t s, unsigned long long *w) {
-  cudaError_t (*const take[3])(cudaStream_t, unsigned long long *) = {
-      swap_check_word_take, fused_check_word_take, attempt_check_word_take};
+  cudaError_t (*const take[4])(cudaStream_t, unsigned long long *) = {
+      swap_check_word_take, swap_any_check_word_take, fused_check_word_take, attempt_check_word_take};
   cudaError_t e = tu_check_word_take(s, w);
-  for (int u = 0; u < 3 && e == cudaSuccess; ++u) {
+  for (int u = 0; u < 4 && e == cudaSuccess; ++u) {
     unsigned long long w2 = 0;
     e = take[u](s, &w2);
     if (*w == 0) *w = w2;

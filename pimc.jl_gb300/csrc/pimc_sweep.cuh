@@ -2,7 +2,7 @@
 // and the persistent drivers that pull chains from the batch's work queue,
 // shared by the kernel translation units, compiled in parallel:
 // pimc_sweep.cu (the staging and rest phases and the other kernels),
-// pimc_swap.cu (the swap phase), pimc_fused.cu (whole sweeps in one launch)
+// pimc_swap.cu and pimc_swap_any.cu (the swap phase), pimc_fused.cu (whole sweeps in one launch)
 // and pimc_attempt.cu (single moves with injected draws).  Device globals of
 // the headers are per translation unit (static); each unit gives the host
 // its own accessors (tu_* below, exported by PIMC_UNIT_ACCESSORS).
