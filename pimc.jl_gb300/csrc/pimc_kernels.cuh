@@ -1184,7 +1184,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
     const unsigned Bq = c.Q(n2, j0), E2q = c.Q(e2p, se);
     // expo(i; B, E2), then with the ends of n1 and n2 exchanged expo(i; A, E2) and
     // expo(i; B, E1): minus the squared distances from the start to i's end and
-    // from i's start to the end (swap_group's, in its arithmetic); the exponents
+    // from i's start to the end (swap_group's, in its arithmetic); the distances
     // stay in registers between the maxima and the sums.  At most 256 threads:
     // the sums are then the same in larger CTAs
     constexpr int U = 4;
@@ -1193,35 +1193,38 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
       const unsigned qa = c.Q(i, j0), qe = c.Q(hb.endp(i), se);
       const unsigned qx = i == n1 ? E2q : (i == n2 ? E1q : qe);  // the exchanged end
       const float f2 = (float)qdist2(qa, E2q);
-      x[0] = -((float)qdist2(Bq, qe) + f2) * hb.inv_denf;
-      x[1] = -((float)qdist2(Aq, qx) + f2) * hb.inv_denf;
-      x[2] = -((float)qdist2(Bq, qx) + (float)qdist2(qa, E1q)) * hb.inv_denf;
+      x[0] = (float)qdist2(Bq, qe) + f2;
+      x[1] = (float)qdist2(Aq, qx) + f2;
+      x[2] = (float)qdist2(Bq, qx) + (float)qdist2(qa, E1q);
     };
+    // the exponent rounds once with its shift, as swap_group's fused form does:
+    // the ratio is a function of the configuration to its last bit
+    const float ninv = -hb.inv_denf;
     float mx[3] = {-INFINITY, -INFINITY, -INFINITY}, kept[U][3];
 #pragma unroll
     for (int q = 0; q < U; ++q) {
       const int i = tid + q * np;
       if (tid < np && i < N) {
         expos(i, kept[q]);
-        for (int k = 0; k < 3; ++k) mx[k] = kept[q][k] > mx[k] ? kept[q][k] : mx[k];
+        for (int k = 0; k < 3; ++k) mx[k] = fmaxf(mx[k], __fmul_rn(kept[q][k], ninv));
       }
     }
     if (tid < np)
       for (int i = tid + U * np; i < N; i += np) {
         float x[3];
         expos(i, x);
-        for (int k = 0; k < 3; ++k) mx[k] = x[k] > mx[k] ? x[k] : mx[k];
+        for (int k = 0; k < 3; ++k) mx[k] = fmaxf(mx[k], __fmul_rn(x[k], ninv));
       }
     G::template max<3>(mx, red);
 #pragma unroll
     for (int q = 0; q < U; ++q)
       if (tid < np && tid + q * np < N)
-        for (int k = 0; k < 3; ++k) s34[k] += hb.ex_(kept[q][k] - mx[k]);
+        for (int k = 0; k < 3; ++k) s34[k] += hb.ex_(fmaf(kept[q][k], ninv, -mx[k]));
     if (tid < np)
       for (int i = tid + U * np; i < N; i += np) {
         float x[3];
         expos(i, x);
-        for (int k = 0; k < 3; ++k) s34[k] += hb.ex_(x[k] - mx[k]);
+        for (int k = 0; k < 3; ++k) s34[k] += hb.ex_(fmaf(x[k], ninv, -mx[k]));
       }
     // S_1 rides along in the fourth slot
     s34[3] = tid == 0 ? ssum : 0.f;
