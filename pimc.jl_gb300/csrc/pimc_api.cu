@@ -1311,7 +1311,8 @@ int pimc_batch_set_beads_all(void *handle, const double *x_all) {
   }
   CK(launch_transpose_tiles(true, h->d_desc, h->d_dpool, src, h->d_tile_off, 0, h->nchains,
                             h->ntiles, 8 * h->num_sms, h->stream));
-  if (refresh_links(h, 0, h->nchains)) return PIMC_ECUDA;
+  CK(launch_links_tiles(h->d_desc, h->d_dpool, h->d_ipool, h->d_tile_off, 0, h->nchains, h->ntiles,
+                        8 * h->num_sms, h->stream));
   return sync_check(h);
 }
 
@@ -1352,7 +1353,8 @@ int pimc_batch_run_io(void *handle, const double *x_in, double *x_out, long long
     CK(cudaEventRecord(h->ev0, h->stream));
     CK(launch_transpose_tiles(true, h->d_desc, h->d_dpool, vin, h->d_tile_off, 0, h->nchains,
                               h->ntiles, 8 * h->num_sms, h->stream));
-    CK(launch_links(h->d_desc, h->d_dpool, h->d_ipool, 0, h->nchains, h->maxNM, h->stream));
+    CK(launch_links_tiles(h->d_desc, h->d_dpool, h->d_ipool, h->d_tile_off, 0, h->nchains, h->ntiles,
+                          8 * h->num_sms, h->stream));
     launches += 2;
     if (n_sweeps > 0 && (rc = issue_batched(h, n_sweeps, &launches))) return rc;
     CK(launch_transpose_tiles(false, h->d_desc, h->d_dpool, vout, h->d_tile_off, 0, h->nchains,
@@ -1390,7 +1392,7 @@ int pimc_batch_run_io(void *handle, const double *x_in, double *x_out, long long
     CK(cudaStreamWaitEvent(h->stream, h->io_ev[2 * k], 0));
     CK(launch_transpose_tiles(true, h->d_desc, h->d_dpool, h->d_stage, h->d_tile_off, c0, c1, nt,
                               8 * h->num_sms, h->stream));
-    CK(launch_links(h->d_desc, h->d_dpool, h->d_ipool, c0, c1 - c0, h->maxNM, h->stream));
+    CK(launch_links_tiles(h->d_desc, h->d_dpool, h->d_ipool, h->d_tile_off, c0, c1, nt, 8 * h->num_sms, h->stream));
     launches += 2;
   }
   if (n_sweeps > 0 && (rc = issue_batched(h, n_sweeps, &launches))) return rc;

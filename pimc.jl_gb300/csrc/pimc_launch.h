@@ -139,6 +139,9 @@ cudaError_t launch_init_world_hard(const ChainDesc *desc, ChainVar *var, double 
                                    int chain0, int nchains, cudaStream_t s);
 cudaError_t launch_links(const ChainDesc *desc, double *dpool, int *ipool, int chain0, int nchains,
                          int maxNM, cudaStream_t s);
+// the same for chains [c_lo, c_hi) over the batch's tiles (launch_transpose_tiles)
+cudaError_t launch_links_tiles(const ChainDesc *desc, double *dpool, int *ipool, const int *tile_off, int c_lo,
+                               int c_hi, int ntiles, int grid, cudaStream_t s);
 cudaError_t launch_import(const ChainDesc *desc, double *dpool, const double *src, int chain0,
                           int nchains, size_t maxn, cudaStream_t s);
 cudaError_t launch_export(const ChainDesc *desc, const double *dpool, double *dst, int chain0,

@@ -484,6 +484,35 @@ __global__ void k_links(const ChainDesc *desc, double *dpool, int *ipool, int ch
   }
 }
 
+// the same over the batch's 32 x 32 (particle, slice) tiles: a warp takes four
+// slices of a tile, a lane a particle, and carries the potential from slice to
+// slice (five evaluations for four links instead of eight).  One grid over the
+// tiles: the grid of k_links, sized by the longest chain, is three quarters
+// empty blocks on uneven batches (4096 chains, upload with links 7.67 -> 6.55 ms).
+__global__ void __launch_bounds__(256) k_links_tiles(const ChainDesc *desc, double *dpool, int *ipool,
+                                                      const int *tile_off, int c_lo, int c_hi) {
+  const int t_end = tile_off[c_hi], lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int t = tile_off[c_lo] + blockIdx.x; t < t_end; t += gridDim.x) {
+    const int ch = tile_chain(tile_off, c_lo, c_hi, t);
+    const ChainDesc &d = desc[ch];
+    const int M = d.M, tj = (M + 31) >> 5, lt = t - tile_off[ch];
+    const int n = (lt / tj) * 32 + lane, j0 = (lt % tj) * 32 + 4 * w, j1 = min(M, j0 + 4);
+    if (n >= d.N || j0 >= M) continue;
+    const CV c = make_cv(&d, dpool, ipool, nullptr);
+    const double mhtau = -0.5 * d.tau;
+    double x = c.X(0, n, j0), y = c.Xd(1, n, j0), v = vext(d, x, y);
+    for (int j = j0; j < j1; ++j) {
+      const int in = j == M - 1 ? c.next[n] : n, jn = j + 1 == M ? 0 : j + 1;
+      const double xn = c.X(0, in, jn), yn = c.Xd(1, in, jn), vn = vext(d, xn, yn);
+      c.Vl(n, j) = mhtau * (v + vn);
+      c.xq[(size_t)j * c.ldn + n] = qpos(d, x, y);
+      x = xn;
+      y = yn;
+      v = vn;
+    }
+  }
+}
+
 // the 16-bit mirror alone (after verbatim state uploads)
 __global__ void k_mirror(const ChainDesc *desc, double *dpool, int chain0) {
   const ChainDesc &d = desc[chain0 + blockIdx.y];
@@ -996,6 +1025,11 @@ cudaError_t launch_links(const ChainDesc *desc, double *dpool, int *ipool, int c
                          int maxNM, cudaStream_t s) {
   dim3 g((unsigned)std::min((maxNM + 255) / 256, 1024), nchains);
   k_links<<<g, 256, 0, s>>>(desc, dpool, ipool, chain0);
+  return cudaGetLastError();
+}
+cudaError_t launch_links_tiles(const ChainDesc *desc, double *dpool, int *ipool, const int *tile_off, int c_lo,
+                               int c_hi, int ntiles, int grid, cudaStream_t s) {
+  k_links_tiles<<<std::max(1, std::min(grid, ntiles)), 256, 0, s>>>(desc, dpool, ipool, tile_off, c_lo, c_hi);
   return cudaGetLastError();
 }
 cudaError_t launch_mirror(const ChainDesc *desc, double *dpool, int chain0, int nchains, int maxNM,
