@@ -689,6 +689,7 @@ SweepArgs sweep_args(Handle *h, const Plan &p) {
   a.tally = h->d_tally;
   a.measure_par = 0;
   a.meas_group = h->meas_group;
+  a.meas_staged = std::min(h->maxN, 2048);
   a.meas_part = h->d_meas;
   a.meas_list = reinterpret_cast<int2 *>(h->d_meas + 9 * (size_t)h->meas_items);
   a.meas_cnt = reinterpret_cast<int *>(a.meas_list + h->meas_items);
@@ -773,10 +774,13 @@ int run_plain(Handle *h, long long n) {
   const Plan &p = h->one;
   std::vector<StagePlan> sp(h->nchains);
   std::vector<char> spec(h->nchains), fused(h->nchains);
+  std::vector<int> sblock(h->nchains);
   bool any_fused = false;
   size_t stage_smem = 0;
   for (int c = 0; c < h->nchains; ++c) {
-    sp[c] = stage_plan(h, 2, p.block, c, c + 1);
+    // a serial chain's slot walks on all the warps a CTA can have
+    sblock[c] = desc_slots(h->desc[c]) && h->desc[c].N >= 256 ? 512 : p.block;
+    sp[c] = stage_plan(h, 2, sblock[c], c, c + 1);
     stage_smem = std::max(stage_smem, sp[c].smem);
     spec[c] = !(h->desc[c].flags & (PF_PHYS | PF_HARD | PF_CONTACT));
     const MixDev &m = h->mix[c];
@@ -809,7 +813,7 @@ int run_plain(Handle *h, long long n) {
       a.stage_slots = sp[c].slots;
       for (int ph = 0; ph < sp[c].phases; ++ph) {
         a.stage_phase = ph;
-        CK(launch_stage_slots(a, sp[c].slots, p.block, sp[c].smem, h->stream));
+        CK(launch_stage_slots(a, sp[c].slots, sblock[c], sp[c].smem, h->stream));
       }
       if (sp[c].phases > 0) CK(launch_stage_close(a, h->stream));
       launches += sp[c].phases + (sp[c].phases > 0);

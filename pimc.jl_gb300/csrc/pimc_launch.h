@@ -38,6 +38,7 @@ struct SweepArgs {
   struct SlotTally *tally;  // [chains] k_stage_slots' counters, zero between phases
   int measure_par;    // 1: the sweep leaves its measurement to launch_measure_sweep
   int meas_group;     // slices per item of it
+  int meas_staged;    // chains of up to so many particles stage their slices
   int2 *meas_list;    // its items (chain, group), or null: chain0's groups alone
   int *meas_cnt;      // [2] items, next item
   double *meas_part;  // [items][9] partial sums (ChainDesc::meas_off)

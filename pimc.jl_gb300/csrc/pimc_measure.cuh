@@ -119,6 +119,102 @@ __device__ __forceinline__ void measure_pairs(const CV &c, int k0, int k1, int d
   spill();
 }
 
+// ---------------------------------------------------------------------------
+// the same pairs with the separations in two floats (48 bits), from slices
+// staged in shared memory as (x hi, x lo, y hi, y lo): an FP64 instruction takes
+// one of the SM's four pipes for 64 cycles, the six of a pair's separations and
+// its three conversions some 500 of a warp's 600 cycles; the two-float form takes
+// about fifty FP32 instructions.  Its squared distance is within 2^-45, so the
+// float that exp takes is the FP64 form's but for ties; a pair within 1e-6 of
+// the cut-off is settled in FP64.
+// ---------------------------------------------------------------------------
+struct FF {
+  float h, l;
+};
+// a - b folded to the minimum image, normalised
+__device__ __forceinline__ FF ff_sep(float ah, float al, float bh, float bl, float Lh, float L2h, float L2l) {
+  const float s = ah - bh, z = s - ah, e = (ah - (s - z)) - (bh + z), l = e + (al - bl);
+  FF r;
+  r.h = s + l;
+  r.l = l - (r.h - s);
+  if (fabsf(r.h) >= Lh) {
+    // past half the box (or within rounding of it, where the fold changes
+    // nothing a pair within reach sees)
+    const float f = copysignf(1.f, r.h), t = r.h - f * L2h, y = t - r.h, q = (r.h - (t - y)) + (-f * L2h - y);
+    const float w = q + (r.l - f * L2l);
+    r.h = t + w;
+    r.l = w - (r.h - t);
+  }
+  return r;
+}
+
+// bead (i, j) as two floats per coordinate
+__device__ __forceinline__ float4 ff_bead(double x, double y) {
+  const float xh = (float)x, yh = (float)y;
+  return make_float4(xh, (float)(x - (double)xh), yh, (float)(y - (double)yh));
+}
+
+// the pairs of slice j by a CTA of `nw` warps: cur and nxt the staged slice and
+// the next along the paths; this warp takes rows w, w + nw, ...
+__device__ __forceinline__ void measure_pairs_ff(const CV &c, int j, const float4 *cur, const float4 *nxt, int w,
+                                                 int nw, unsigned *ring, MeasureSums &a) {
+  const ChainDesc &d = *c.d;
+  const int N = c.N, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u, lim = d.q_lim_hi;
+  const float cg = (float)d.inv2s2;
+  const float Lh = (float)d.L, L2h = (float)d.L2, L2l = (float)(d.L2 - (double)L2h);
+  const float r_lo = (float)d.rc2 * (1.f - 1e-6f), r_hi = (float)d.rc2 * (1.f + 1e-6f);
+  int head = 0, tail = 0, nf = 0;
+  float e0 = 0.f, e1 = 0.f, v0 = 0.f, v1 = 0.f;  // running sums, high and low parts
+  auto spill = [&]() {
+    a.s[3] += (double)e0 + (double)e1;
+    a.s[4] += (double)v0 + (double)v1;
+    e0 = e1 = v0 = v1 = 0.f;
+    nf = 0;
+  };
+  auto flush = [&](int cnt) {
+    if (lane < cnt) {
+      const unsigned q = ring[(head + lane) & (MEAS_RING - 1)];  // i | b << 13
+      const int i = (int)(q & 0x1fffu), b = (int)(q >> 13);
+      const float4 p = cur[i], r = cur[b];
+      const FF dx = ff_sep(p.x, p.y, r.x, r.y, Lh, L2h, L2l), dy = ff_sep(p.z, p.w, r.z, r.w, Lh, L2h, L2l);
+      // dx^2 + dy^2 in two floats
+      const float xx = dx.h * dx.h, yy = dy.h * dy.h;
+      const float ex = fmaf(dx.h, dx.h, -xx) + 2.f * dx.h * dx.l, ey = fmaf(dy.h, dy.h, -yy) + 2.f * dy.h * dy.l;
+      const float s = xx + yy, z = s - xx, r2 = s + (((xx - (s - z)) + (yy - z)) + (ex + ey));
+      bool in = r2 < r_lo;
+      if (!in && r2 <= r_hi) in = mi2(d, c.X(0, i, j), c.Xd(1, i, j), c.X(0, b, j), c.Xd(1, b, j)) <= d.rc2;
+      if (in) {
+        const float4 pn = nxt[i], rn = nxt[b];
+        const float nx = ff_sep(pn.x, pn.y, rn.x, rn.y, Lh, L2h, L2l).h;
+        const float ny = ff_sep(pn.z, pn.w, rn.z, rn.w, Lh, L2h, L2l).h;
+        const float xa = -r2 * cg, xb = -fmaf(nx, nx, ny * ny) * cg;
+        const float ea = expf(xa), eb = expf(xb);
+        two_sum(e0, e1, ea + eb);
+        two_sum(v0, v1, fmaf(xa, ea, xb * eb));
+      }
+    }
+    head += cnt;
+    __syncwarp();
+    if (++nf == 16) spill();
+  };
+  const unsigned *row = c.xq + (size_t)j * c.ldn;
+  for (int i = w; i < N; i += nw) {
+    const unsigned ci = row[i];
+    for (int b0 = i + 1; b0 < N; b0 += 32) {
+      const int b = b0 + lane;
+      const bool in = b < N && qdist2(ci, row[b]) <= lim;
+      const unsigned mk = __ballot_sync(0xffffffffu, in);
+      if (in) ring[(tail + __popc(mk & lt)) & (MEAS_RING - 1)] = (unsigned)i | ((unsigned)b << 13);
+      tail += __popc(mk);
+      __syncwarp();
+      if (tail - head >= 32) flush(32);
+    }
+  }
+  if (tail > head) flush(tail - head);
+  spill();
+}
+
 // the pair-distance histogram of slices [j0, j1): warps gw, gw + ngw, ... over
 // the beads, lanes the partners of higher index; lanes with the same bin add
 // once (match_any)

@@ -179,7 +179,8 @@ size_t slot_scratch_bytes(int ell, int nwarps) {
 // The measurement of a sweep in launches of its own, after the sweep: items of
 // meas_group slices, so that a few long chains' N^2 M / 2 pairs spread over the
 // GPU (measured in the sweep's own CTA, 17 ms of a 1024-particle chain's sweep
-// and 50 of a batch of 512 chains').  k_measure_plan lists the items of the chains
+// and 50 of a batch of 512 chains');
+// the pairs in two floats where two slices fit 64 KB of shared memory.  k_measure_plan lists the items of the chains
 // that measure now (their sweep counter has just advanced), the items' sums go
 // to their rows, and k_measure_close adds a chain's rows in order and records.
 // ---------------------------------------------------------------------------
@@ -198,6 +199,7 @@ __global__ void k_measure_plan(SweepArgs a) {
 }
 
 __global__ void __launch_bounds__(128) k_measure_slices(SweepArgs a) {
+  extern __shared__ __align__(16) float4 slices[];  // two staged slices of a.meas_staged beads, or none
   __shared__ ChainDesc d;
   __shared__ double red[256];
   __shared__ unsigned long long qbuf[4 * MEAS_RING];
@@ -223,7 +225,21 @@ __global__ void __launch_bounds__(128) k_measure_slices(SweepArgs a) {
     measure_beads(c, j0 * N + tid, j1 * N, 128, density, inv_bw, m);
     __syncwarp();
     if ((d.flags & PF_PAIR) && !(d.flags & PF_CONTACT)) {
-      measure_pairs(c, j0 * N + warp, j1 * N, 4, qbuf + warp * MEAS_RING, m);
+      if (N <= a.meas_staged) {
+        for (int j = j0; j < j1; ++j) {
+          const bool wrap = j == c.M - 1;
+          __syncthreads();  // the last slice's pairs are done
+          for (int i = tid; i < N; i += 128) {
+            const int in = wrap ? c.next[i] : i, jn = wrap ? 0 : j + 1;
+            slices[i] = ff_bead(c.X(0, i, j), c.Xd(1, i, j));
+            slices[N + i] = ff_bead(c.X(0, in, jn), c.Xd(1, in, jn));
+          }
+          __syncthreads();
+          measure_pairs_ff(c, j, slices, slices + N, warp, 4, reinterpret_cast<unsigned *>(qbuf + warp * MEAS_RING), m);
+        }
+      } else {
+        measure_pairs(c, j0 * N + warp, j1 * N, 4, qbuf + warp * MEAS_RING, m);
+      }
     }
     if (d.rdf_nb > 0) measure_radial(c, j0, j1, warp, 4);
     block_sum_k<5>(m.s, red);
@@ -265,7 +281,10 @@ cudaError_t launch_measure_sweep(const SweepArgs &a, int ngroups, int num_sms, c
     k_measure_plan<<<(a.nchains + 127) / 128, 128, 0, s>>>(a);
     ngroups = std::min(ngroups, 5 * num_sms);
   }
-  k_measure_slices<<<ngroups, 128, 0, s>>>(a);
+  const size_t smem = 32 * (size_t)a.meas_staged;
+  const cudaError_t es = cudaFuncSetAttribute(k_measure_slices, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (es != cudaSuccess) return es;
+  k_measure_slices<<<ngroups, 128, smem, s>>>(a);
   k_measure_close<<<(a.nchains + 3) / 4, 128, 0, s>>>(a);
   return cudaGetLastError();
 }
