@@ -590,9 +590,10 @@ __global__ void __launch_bounds__(256) k_measure(const ChainDesc *desc, ChainVar
 // cut-off.  Before, one thread per bead scanned its partners (5.6 of 32 lanes
 // active in the FP64 branch) and a batch's CTA per slice added forces through
 // FP64 shared atomics (compare-and-swap loops).  Whole calls: one chain of N =
-// 1024, M = 64 (lattice, trap, pair) 5.97 -> 0.42 ms; 60 chains of 8 to 512
-// particles with every bead's force 29.3 -> 5.9 ms, of which k_adjoint_slices
-// takes 5.2 at 85 % of the FP64 pipe.
+// 1024, M = 64 (lattice, trap, pair) 5.97 -> 0.39 ms; 60 chains of 8 to 512
+// particles with every bead's force 29.4 -> 5.3 ms, of which k_adjoint_slices
+// takes 4.6 (its rare parts out of line and the weight at one rounding less: 5.9
+// -> 5.3).
 //
 // Partial sums per CTA: part[cta][9] = S_ext, dV0, domega, S_pair, dg, pair
 // virial, r.g_ext, 0, r.dS/dr.
@@ -640,6 +641,40 @@ __device__ __forceinline__ bool adjoint_reach(unsigned ci, unsigned pi, unsigned
   return d2c <= lim_hi || st;
 }
 
+// The rarely taken parts of a pair, out of line: an FP64 instruction that is
+// predicated off, or that the compiler evaluates ahead of a select, costs the
+// pipe as much as one that runs (inline, they took 5 of a pair's 26).
+static __device__ __noinline__ double adjoint_wrap(double dx, double L2) { return dx - copysign(L2, dx); }
+__device__ __forceinline__ double adjoint_sep(double a, double b, double L, double L2) {  // as mi1
+  const double dx = a - b;
+  return abs_gt(dx, L) ? adjoint_wrap(dx, L2) : dx;
+}
+static __device__ __noinline__ int adjoint_near(CV c, int i, int b, int jp, const int *inv) {
+  const int ip = inv ? inv[i] : i, bp = inv ? inv[b] : b;
+  return mi2(*c.d, c.X(0, ip, jp), c.Xd(1, ip, jp), c.X(0, bp, jp), c.Xd(1, bp, jp)) <= c.d->rc2;
+}
+static __device__ __noinline__ double adjoint_weight_far(double r2, double cg, int uses) {
+  return (double)uses * exp(-r2 * cg);
+}
+// uses exp(-cg r2) by exp_neg's table and polynomial: the product goes into both
+// its roundings (to k / 64 by adding 1.5 2^46, and to the rest, then exact but
+// for one rounding), the doubling into the exponent of the table's entry.  far:
+// the bits of the r2 from which the library's exp takes over.
+__device__ __forceinline__ double adjoint_weight(double r2, double cg, long long far, int uses) {
+  if ((unsigned long long)__double_as_longlong(r2) > (unsigned long long)far) return adjoint_weight_far(r2, cg, uses);
+  const double t = fma(r2, -cg, 105553116266496.0);
+  const unsigned k = min((unsigned)-__double2loint(t), (unsigned)EXPTAB_N);
+  const double f = fma(r2, -cg, 105553116266496.0 - t);
+  double p = fma(f, 1.0 / 120.0, 1.0 / 24.0);
+  p = fma(p, f, 1.0 / 6.0);
+  p = fma(p, f, 0.5);
+  p = fma(p, f, 1.0);
+  p = fma(p, f, 1.0);
+  const double e = __ldg(&g_exptab[k]);
+  return __hiloint2double(__double2hiint(e) + ((uses - 1) << 20), __double2loint(e)) * p;
+}
+__device__ __forceinline__ long long adjoint_far(double cg) { return __double_as_longlong(39.99 / cg); }
+
 // the uses of a pair at slice j -- the link it starts (r2 within reach) and the
 // link it ends (the earlier beads' reach, settled by the entry or exactly)
 __device__ __forceinline__ int adjoint_uses(const CV &c, const ChainDesc &d, unsigned e, double r2, int i, int b,
@@ -649,8 +684,7 @@ __device__ __forceinline__ int adjoint_uses(const CV &c, const ChainDesc &d, uns
   if (st == 1u) {
     ++uses;
   } else if (st == 2u) {
-    const int ip = inv ? inv[i] : i, bp = inv ? inv[b] : b;
-    if (mi2(d, c.X(0, ip, jp), c.Xd(1, ip, jp), c.X(0, bp, jp), c.Xd(1, bp, jp)) <= d.rc2) ++uses;
+    uses += adjoint_near(c, i, b, jp, inv);
   }
   return uses;
 }
@@ -745,6 +779,7 @@ __global__ void __launch_bounds__(128) k_adjoint_gather(AdjArgs a) {
     }
     if ((d.flags & PF_PAIR) && N > 1) {
       const double cg = d.inv2s2, h = 0.5 * d.tau;
+      const long long far = adjoint_far(cg);
       const double kf = -2.0 * cg * h * d.g;  // the force's factor
       const unsigned lim_lo = d.q_lim_lo, lim_hi = d.q_lim_hi, lt = (1u << lane) - 1u;
       unsigned *ring = ring_s[warp];
@@ -759,14 +794,13 @@ __global__ void __launch_bounds__(128) k_adjoint_gather(AdjArgs a) {
           if (lane < k) {
             const unsigned e = ring[(head + lane) & (ADJ_RING - 1)];
             const int b = (int)(e & 0xffffu);
-            const double dx = mi1(px, c.X(0, b, j), d.L, d.L2);
-            const double dy = dim > 1 ? mi1(py, c.X(1, b, j), d.L, d.L2) : 0.0;
+            const double dx = adjoint_sep(px, c.X(0, b, j), d.L, d.L2);
+            const double dy = dim > 1 ? adjoint_sep(py, c.X(1, b, j), d.L, d.L2) : 0.0;
             double r2 = dx * dx;
             if (dim > 1) r2 = fma(dy, dy, r2);
             const int uses = adjoint_uses(c, d, e, r2, i, b, jp, inv);
             if (uses) {
-              double w = exp_neg(-r2 * cg);
-              if (uses == 2) w += w;
+              const double w = adjoint_weight(r2, cg, far, uses);
               se += w;
               sr = fma(r2, w, sr);
               fx = fma(w, dx, fx);
@@ -848,6 +882,7 @@ __global__ void __launch_bounds__(128) k_adjoint_slices(AdjArgs a) {
   const bool pair = (d.flags & PF_PAIR) && N > 1;
   double v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, rg = 0.0;
   const double cg = d.inv2s2, h = 0.5 * d.tau;
+  const long long far = adjoint_far(cg);
   const double kf = -2.0 * cg * h * d.g;  // the force's factor
   if (pair) {
     for (int b = lane; b < N; b += 32) acc[b] = make_double2(0.0, 0.0);
@@ -864,14 +899,13 @@ __global__ void __launch_bounds__(128) k_adjoint_slices(AdjArgs a) {
         if (lane < k) {
           const unsigned e = ring[(head + lane) & (ADJ_RING - 1)];
           const int b = (int)(e & 0xffffu);
-          const double dx = mi1(px, c.X(0, b, j), d.L, d.L2);
-          const double dy = dim > 1 ? mi1(py, c.X(1, b, j), d.L, d.L2) : 0.0;
+          const double dx = adjoint_sep(px, c.X(0, b, j), d.L, d.L2);
+          const double dy = dim > 1 ? adjoint_sep(py, c.X(1, b, j), d.L, d.L2) : 0.0;
           double r2 = dx * dx;
           if (dim > 1) r2 = fma(dy, dy, r2);
           const int uses = adjoint_uses(c, d, e, r2, i, b, jp, inv);
           if (uses) {
-            double w = exp_neg(-r2 * cg);
-            if (uses == 2) w += w;
+            const double w = adjoint_weight(r2, cg, far, uses);
             se += w;
             sr = fma(r2, w, sr);
             fx = fma(w, dx, fx);
