@@ -2528,8 +2528,9 @@ int pimc_set_beams(void *handle, int chain, const double *angles, int nangles, d
     ChainDesc &d = h->desc[c];
     d.nbeam = nangles;
     d.beam_helical = helical ? 1 : 0;
-    d.beam_scale = scale;
     d.beam_depth = depth;
+    d.beam_s2 = 2.0 * scale;
+    d.beam_inv = nangles > 0 ? 1.0 / nangles : 0.0;
     for (int k = 0; k < MAX_BEAMS; ++k) {
       d.beam_sin[k] = k < nangles ? std::sin(angles[k]) : 0.0;
       d.beam_cos[k] = k < nangles ? std::cos(angles[k]) : 0.0;

@@ -604,45 +604,81 @@ __device__ __forceinline__ double unwrap_end(double s, double &e, double L) {
   return r.x;
 }
 
+// The host's tables, one copy per kernel translation unit (static): exp(-k/64)
+// for exp_neg, then (sin, cos)(pi k / 128) of a whole turn for sincos_turn.
+constexpr int EXPTAB_N = 2560, TURN_N = 256, TURN_AT = EXPTAB_N + 2, TABLE_N = TURN_AT + 2 * TURN_N;
+static __device__ __align__(16) double g_exptab[TABLE_N];
+
+// phases of 2^40 half turns and beyond (and no numbers), where the rounding
+// below would lose the low bits
+static __device__ __noinline__ double2 sincos_turn_far(double z) {
+  double2 r;
+  sincospi(z, &r.x, &r.y);
+  return r;
+}
+// (sin, cos)(pi z): the nearest table entry at k / 128 (adding 1.5 2^45 leaves k
+// in the low word, exactly), turned by f = z - k / 128, |f| <= 1/256, with the
+// Taylor polynomials of sin(pi f) and cos(pi f) - 1: truncation 8e-18 and
+// 1.3e-20.  16 FP64 operations.
+__device__ __forceinline__ double2 sincos_turn(double z) {
+  if ((unsigned)__double2hiint(z) << 1 >= 0x427u << 21) return sincos_turn_far(z);  // |z| >= 2^40
+  const double t = z + 52776558133248.0;
+  const double2 w = __ldg(reinterpret_cast<const double2 *>(g_exptab + TURN_AT) + (__double2loint(t) & (TURN_N - 1)));
+  const double f = z - (t - 52776558133248.0), q = f * f;
+  double sn = fma(q, 2.5501640398773455, -5.167712780049970);
+  sn = fma(sn, q, 3.141592653589793) * f;
+  double cm = fma(q, -1.3352627688545893, 4.058712126416768);
+  cm = fma(cm, q, -4.934802200544679) * q;
+  // the small terms first: one rounding less of the large ones
+  return make_double2(w.x + fma(w.y, sn, w.x * cm), w.y + fma(-w.x, sn, w.y * cm));
+}
+
 // engine-known external potential: hcoef |r|^2 + V0 sum sin^2(pi r_d / a)
 // the optical lattice's normalized intensity (examples/tools/potentialtools.jl:1-16):
 // with phi_k = 2 pi scale (x sin a_k + y cos a_k) (+ a_k when helical),
-// S = (1/K) sum sin phi_k, C = (1/K) sum cos phi_k, I = S^2 + C^2; optionally
-// the gradient of I
-static __device__ __noinline__ double beam_intensity(const ChainDesc &d, double x, double y, double *gx,
-                                              double *gy) {
+// S = (1/K) sum sin phi_k, C = (1/K) sum cos phi_k, I = S^2 + C^2.  Bound by the
+// FP64 pipe, 21 operations a beam (38 with the library's sincospi and the
+// gradient's sums in the same function): out of line, the gradient apart.
+__device__ __forceinline__ double2 beam_phase(const ChainDesc &d, double x, double y, double sa, double ca) {
+  double2 w = sincos_turn(d.beam_s2 * fma(x, sa, y * ca));
+  if (d.beam_helical)  // rotate by the beam's own angle a_k
+    w = make_double2(fma(w.x, ca, w.y * sa), fma(w.y, ca, -(w.x * sa)));
+  return w;
+}
+static __device__ __noinline__ double beam_intensity(const ChainDesc &d, double x, double y) {
+  double S = 0.0, Cc = 0.0;
+  for (int k = 0; k < d.nbeam; ++k) {
+    const double2 w = beam_phase(d, x, y, d.beam_sin[k], d.beam_cos[k]);
+    S += w.x;
+    Cc += w.y;
+  }
+  S *= d.beam_inv;
+  Cc *= d.beam_inv;
+  return S * S + Cc * Cc;
+}
+static __device__ __noinline__ double beam_gradient(const ChainDesc &d, double x, double y, double *gx, double *gy) {
   double S = 0.0, Cc = 0.0, sx = 0.0, sy = 0.0, cx = 0.0, cy = 0.0;
   for (int k = 0; k < d.nbeam; ++k) {
     const double sa = d.beam_sin[k], ca = d.beam_cos[k];
-    double s, c;
-    sincospi(2.0 * d.beam_scale * (x * sa + y * ca), &s, &c);
-    if (d.beam_helical) {  // rotate by the beam's own angle a_k
-      const double s2 = s * ca + c * sa, c2 = c * ca - s * sa;
-      s = s2;
-      c = c2;
-    }
-    S += s;
-    Cc += c;
+    const double2 w = beam_phase(d, x, y, sa, ca);
+    S += w.x;
+    Cc += w.y;
     // d(sin phi) = cos phi dphi, d(cos phi) = -sin phi dphi, dphi/dx = 2 pi scale sin a_k
-    sx += c * sa;
-    sy += c * ca;
-    cx -= s * sa;
-    cy -= s * ca;
+    sx = fma(w.y, sa, sx);
+    sy = fma(w.y, ca, sy);
+    cx = fma(-w.x, sa, cx);
+    cy = fma(-w.x, ca, cy);
   }
-  const double inv = 1.0 / d.nbeam;
-  S *= inv;
-  Cc *= inv;
-  if (gx) {
-    const double w = 2.0 * 3.141592653589793 * d.beam_scale * inv;
-    *gx = 2.0 * w * (S * sx + Cc * cx);
-    *gy = 2.0 * w * (S * sy + Cc * cy);
-  }
+  const double g = 2.0 * 3.141592653589793 * d.beam_s2 * d.beam_inv;
+  S *= d.beam_inv;
+  Cc *= d.beam_inv;
+  *gx = g * (S * sx + Cc * cx);
+  *gy = g * (S * sy + Cc * cy);
   return S * S + Cc * Cc;
 }
 
-__device__ __forceinline__ double vext(const ChainDesc &d, double x, double y) {
-  double v = 0.0;
-  if (d.flags & PF_BEAM) v += d.beam_depth * beam_intensity(d, x, y, nullptr, nullptr);
+// v plus the separable terms
+__device__ __forceinline__ double vext_sep(const ChainDesc &d, double x, double y, double v) {
   if (d.flags & PF_HARM) {
     double s = x * x;
     if (d.dim > 1) s += y * y;
@@ -659,6 +695,12 @@ __device__ __forceinline__ double vext(const ChainDesc &d, double x, double y) {
   }
   return v;
 }
+__device__ __forceinline__ double vext(const ChainDesc &d, double x, double y) {
+  double v = 0.0;
+  if (d.flags & PF_BEAM) v += d.beam_depth * beam_intensity(d, x, y);
+  v = vext_sep(d, x, y, v);
+  return v;
+}
 
 // gradient of vext along one coordinate, separable terms only
 __device__ __forceinline__ double dvext(const ChainDesc &d, double x) {
@@ -668,17 +710,19 @@ __device__ __forceinline__ double dvext(const ChainDesc &d, double x) {
   return g;
 }
 
-// full gradient of vext (the optical lattice is not separable)
-__device__ __forceinline__ void grad_vext(const ChainDesc &d, double x, double y, double &gx,
-                                          double &gy) {
+// vext and its full gradient (the optical lattice is not separable, and its
+// beams give both at once)
+__device__ __forceinline__ double vext_grad(const ChainDesc &d, double x, double y, double &gx, double &gy) {
+  double v = 0.0, bx = 0.0, by = 0.0;
+  if (d.flags & PF_BEAM) v += d.beam_depth * beam_gradient(d, x, y, &bx, &by);
+  v = vext_sep(d, x, y, v);
   gx = dvext(d, x);
   gy = d.dim > 1 ? dvext(d, y) : 0.0;
   if (d.flags & PF_BEAM) {
-    double bx, by;
-    beam_intensity(d, x, y, &bx, &by);
     gx += d.beam_depth * bx;
     gy += d.beam_depth * by;
   }
+  return v;
 }
 
 // exp(x) for x <= 0 by a table of exp(-k/64), k = 0..2560 (filled from the
@@ -687,10 +731,6 @@ __device__ __forceinline__ void grad_vext(const ChainDesc &d, double x, double y
 // truncation <= (1/128)^6/720 = 3.2e-16 relative, about 9 FP64 operations
 // against the library's longer range reduction and polynomial.  Arguments
 // below -40 (pair terms of far-away next beads) go to the library exp.
-constexpr int EXPTAB_N = 2560;
-// one per kernel translation unit (static), both filled by the host
-static __device__ double g_exptab[EXPTAB_N + 1];
-
 __device__ __forceinline__ double exp_neg(double x) {
   // -x > 40 on the bits (x <= 0): a compare or a conversion costs the FP64
   // pipe as much as a product, so the rounding to k goes through the low word

@@ -1833,10 +1833,9 @@ __device__ void measure_group(const CV &c, double *red, double *out, bool densit
     const double ax = c.X(0, i, j), ay = c.Xd(1, i, j);
     const double bx = c.X(0, in, jn), by = c.Xd(1, in, jn);
     s[0] += mi2(d, ax, ay, bx, by);
-    s[1] += vext(d, ax, ay) + vext(d, bx, by);
     {
       double gx, gy;
-      grad_vext(d, ax, ay, gx, gy);
+      s[1] += vext_grad(d, ax, ay, gx, gy) + vext(d, bx, by);
       s[2] += ax * gx + (dim > 1 ? ay * gy : 0.0);
     }
     {

@@ -35,9 +35,8 @@ __device__ __forceinline__ void measure_beads(const CV &c, int k0, int k1, int n
     const double dy = dim > 1 ? mi1(c.X(1, in, jn), ay, d.L, d.L2) : 0.0;
     a.s[0] += dim > 1 ? fma(dy, dy, dx * dx) : dx * dx;
     // every bead is the start of one link and the end of another
-    a.s[1] += 2.0 * vext(d, ax, ay);
     double gx, gy;
-    grad_vext(d, ax, ay, gx, gy);
+    a.s[1] += 2.0 * vext_grad(d, ax, ay, gx, gy);
     a.s[2] += ax * gx + (dim > 1 ? ay * gy : 0.0);
     a.f[0] += dx;
     a.f[1] += dy;

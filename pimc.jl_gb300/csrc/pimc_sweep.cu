@@ -695,10 +695,9 @@ __device__ __forceinline__ void adjoint_ext(const ChainDesc &d, double ax, doubl
                                             double (&v)[8]) {
   const double tau = d.tau;
   double ge[2];
-  grad_vext(d, ax, ay, ge[0], ge[1]);
+  v[0] += tau * vext_grad(d, ax, ay, ge[0], ge[1]);
   gx = ge[0] * tau;
   gy = ge[1] * tau;
-  v[0] += tau * vext(d, ax, ay);
   if (d.flags & PF_LATT) {
     const double sx = sinpi(ax * d.lat_k), sy = d.dim > 1 ? sinpi(ay * d.lat_k) : 0.0;
     v[1] += tau * (sx * sx + sy * sy);
@@ -1004,10 +1003,18 @@ size_t swap_scratch_bytes(int N, int nwarps) { return SwapScratch::bytes(N, nwar
 size_t com_scratch_bytes(int N, int M, int nwarps) { return ComScratch::bytes(N, M, nwarps); }
 int window_scratch_doubles() { return WARP_SCRATCH_D; }
 
-// the exp table of exp_neg for the current device, in every kernel unit
+// the tables of exp_neg and sincos_turn for the current device, in every kernel
+// unit
 cudaError_t upload_exp_table() {
-  static double tab[EXPTAB_N + 1];
+  static double tab[TABLE_N];
   for (int k = 0; k <= EXPTAB_N; ++k) tab[k] = std::exp(-k / 64.0);
+  for (int k = 0; k < TURN_N; ++k) {  // a quarter turn, and exactly 0 and 1 at its ends
+    const int r = k % (TURN_N / 4), q = k / (TURN_N / 4);
+    const long double a = 3.14159265358979323846264338327950288L * r / (TURN_N / 2);
+    const double sn = (double)sinl(a), cs = (double)cosl(a);
+    tab[TURN_AT + 2 * k] = q == 0 ? sn : (q == 1 ? cs : (q == 2 ? -sn : -cs));
+    tab[TURN_AT + 2 * k + 1] = q == 0 ? cs : (q == 1 ? -sn : (q == 2 ? -cs : sn));
+  }
   cudaError_t e = tu_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = swap_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = swap_any_upload_exp_table(tab, sizeof(tab));

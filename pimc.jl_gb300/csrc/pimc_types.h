@@ -115,7 +115,7 @@ struct ChainDesc {
   // a_k when helical; V = depth |(1/K) sum exp(i phi_k)|^2, phi_k =
   // 2 pi scale (x sin a_k + y cos a_k) (+ a_k)
   int nbeam, beam_helical;
-  double beam_depth, beam_scale;
+  double beam_depth, beam_s2, beam_inv;  // 2 scale, 1 / nbeam
   double beam_sin[MAX_BEAMS], beam_cos[MAX_BEAMS];
 };
 

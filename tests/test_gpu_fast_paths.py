@@ -199,3 +199,43 @@ def test_measurement_launches_agree(N, M, dim, engine_lib):
     scale = np.maximum(np.abs(exact), 1.0)
     assert np.all(np.abs(last - exact)[[0, 1, 4, 5, 6]] <= 1e-10 * scale[[0, 1, 4, 5, 6]])
     assert np.all(np.abs(last - exact)[[2, 3]] <= 2e-7 * scale[[2, 3]])
+
+
+@pytest.mark.parametrize("helical", [False, True])
+@pytest.mark.parametrize("scale,K", [(0.5, 1), (0.6, 12), (3.0, 16), (1e15, 5)])
+def test_beam_phases_around_the_table(scale, K, helical, engine_lib):
+    """links of beads whose phases lie on, halfway between and beside the entries
+    of the table of a turn, across many turns and beyond the table's range,
+    against extended precision from the same rounded half turns z.  An entry,
+    the polynomials and the turn by them are a few roundings of numbers below
+    1, z two of its last places: I within 8 ulp + 4 pi |z| ulp"""
+    from pimc.engine import ChainParams, Engine
+    if np.finfo(np.longdouble).nmant < 63:
+        pytest.skip("no extended precision")
+    N, M, L = 16, 16, 4.0
+    ang = np.linspace(0.0, 2.0, K) if K > 1 else np.array([0.0])
+    k = np.arange(N * M)
+    y = ((k % 9 - 4) / 512.0 + (k * 37 % 256 - 128) / 128.0) / (2.0 * scale) * (1.0 + (k % 5 - 2) * 2.0 ** -40)
+    y[np.abs(y) > L * 0.99] *= 0.25
+    x = np.zeros((2, N, M))
+    x[1] = y.reshape(N, M)
+    if K > 1:
+        x[0] = np.random.default_rng(4).uniform(-3.9, 3.9, (N, M))
+    e = Engine(ChainParams(dim=2, N=N, M=M, L=L, T=1.0, lam=0.5, semantics=1))
+    e.set_beams(ang, scale, 1.0, helical)
+    e.set_beads(x)
+    got = np.asarray(e.get_links())  # -tau/2 (I_j + I_j+1)
+    e.close()
+    if scale > 1e6:  # the phases themselves carry no digits: finite and in range
+        assert np.all(np.isfinite(got)) and np.all(got <= 0.0) and np.all(got >= -1.0 / M * (1 + 1e-12))
+        return
+    q = np.longdouble
+    ph = [2 * q(scale) * (q(1) * x[0] * np.sin(q(a)) + q(1) * x[1] * np.cos(q(a))) for a in ang]
+    off = [q(a) if helical else q(0) for a in ang]
+    pi = q("3.14159265358979323846264338327950288")
+    S = sum(np.sin(pi * np.fmod(z, 2) + o) for z, o in zip(ph, off)) / K
+    Cc = sum(np.cos(pi * np.fmod(z, 2) + o) for z, o in zip(ph, off)) / K
+    I = S * S + Cc * Cc
+    want = np.asarray(-0.5 / M * (I + np.roll(I, -1, axis=1)), dtype=float)
+    zmax = float(max(np.abs(z).max() for z in ph))
+    np.testing.assert_allclose(got.reshape(want.shape), want, rtol=0, atol=(8 + 4 * np.pi * zmax) * 2.0 ** -52 / M)
