@@ -3,8 +3,8 @@
 // name, 125-127): E_th, E_v, pair energy, pair virial, winding, area, sum r^2,
 // the density and the pair-distance histogram.
 //
-// A link's pair within reach at its start: FP64 separations and exact reach,
-// FP32 expf of both ends' squared distances (relative error about 1e-7 per
+// A link's pair within reach at its start: separations in two floats and exact
+// reach, FP32 expf of both ends' squared distances (relative error about 1e-7 per
 // term, far below any Monte Carlo error).  The sums of a lane's terms are exact
 // to FP64 (two floats for at most 16 terms, then a double), so launch shapes
 // agree to rounding.  pimc_measure keeps every term in FP64 (measure_group).
@@ -56,19 +56,96 @@ __device__ __forceinline__ void measure_beads(const CV &c, int k0, int k1, int n
   }
 }
 
+// ---------------------------------------------------------------------------
+// The pairs' separations in two floats (48 bits): an FP64 instruction takes one of
+// the SM's four pipes for 64 cycles, the six of a pair's separations and its
+// three conversions some 500 of a warp's 600 cycles; the two-float form takes
+// about fifty FP32 instructions.  Its squared distance is within 2^-45, so the
+// float that exp takes is the FP64 form's but for ties; a pair within 1e-6 of
+// the cut-off is settled in FP64.  A measuring sweep of 4096 chains (measurement
+// launches) 148 -> 51 ms.
+// ---------------------------------------------------------------------------
+struct FF {
+  float h, l;
+};
+// a - b folded to the minimum image, normalised
+__device__ __forceinline__ FF ff_sep(float ah, float al, float bh, float bl, float Lh, float L2h, float L2l) {
+  const float s = ah - bh, z = s - ah, e = (ah - (s - z)) - (bh + z), l = e + (al - bl);
+  FF r;
+  r.h = s + l;
+  r.l = l - (r.h - s);
+  if (fabsf(r.h) >= Lh) {
+    // past half the box (or within rounding of it, where the fold changes
+    // nothing a pair within reach sees)
+    const float f = copysignf(1.f, r.h), t = r.h - f * L2h, y = t - r.h, q = (r.h - (t - y)) + (-f * L2h - y);
+    const float w = q + (r.l - f * L2l);
+    r.h = t + w;
+    r.l = w - (r.h - t);
+  }
+  return r;
+}
+
+// x as two floats, the first truncated, on the integer pipe: conversions between
+// the formats take the FP64 pipe's time.  Below 2^-74 it is 0.
+__device__ __forceinline__ float2 ff_bits(double x) {
+  const unsigned hi = __double2hiint(x), lo = __double2loint(x), s = hi & 0x80000000u, e = hi & 0x7fffffffu;
+  const float h = __uint_as_float(s | __funnelshift_l(lo, e - (896u << 20), 3));
+  const float u = __uint_as_float(s | (((e >> 20) - 948u) << 23));  // sign and weight of the word's last bit
+  return e < (950u << 20) ? make_float2(0.f, 0.f) : make_float2(h, u * (float)(lo & 0x1fffffffu));
+}
+
+// what a chain's pairs are measured against
+struct FFBox {
+  float cg, Lh, L2h, L2l, r_lo, r_hi;
+  __device__ __forceinline__ explicit FFBox(const ChainDesc &d)
+      : cg((float)d.inv2s2), Lh((float)d.L), L2h((float)d.L2), L2l((float)(d.L2 - (double)L2h)),
+        r_lo((float)d.rc2 * (1.f - 1e-6f)), r_hi((float)d.rc2 * (1.f + 1e-6f)) {}
+  // the squared distance of beads p and r
+  __device__ __forceinline__ float dist2(const float4 &p, const float4 &r) const {
+    const FF dx = ff_sep(p.x, p.y, r.x, r.y, Lh, L2h, L2l), dy = ff_sep(p.z, p.w, r.z, r.w, Lh, L2h, L2l);
+    const float xx = dx.h * dx.h, yy = dy.h * dy.h;
+    const float ex = fmaf(dx.h, dx.h, -xx) + 2.f * dx.h * dx.l, ey = fmaf(dy.h, dy.h, -yy) + 2.f * dy.h * dy.l;
+    const float s = xx + yy, z = s - xx;
+    return s + (((xx - (s - z)) + (yy - z)) + (ex + ey));
+  }
+  // the terms of a pair within reach at r2 whose next beads are p and r: the pair
+  // exponentials e = exp(x), x = -r^2/(2 s^2), and x e; the factors g tau/2 are
+  // applied once at the end
+  __device__ __forceinline__ void terms(float r2, const float4 &p, const float4 &r, float &e0, float &e1, float &v0,
+                                        float &v1) const {
+    const float nx = ff_sep(p.x, p.y, r.x, r.y, Lh, L2h, L2l).h, ny = ff_sep(p.z, p.w, r.z, r.w, Lh, L2h, L2l).h;
+    const float xa = -r2 * cg, xb = -fmaf(nx, nx, ny * ny) * cg;
+    const float ea = expf(xa), eb = expf(xb);
+    two_sum(e0, e1, ea + eb);
+    two_sum(v0, v1, fmaf(xa, ea, xb * eb));
+  }
+};
+
+// a bead as two floats per coordinate
+__device__ __forceinline__ float4 ff_bead(double x, double y) {
+  const float2 a = ff_bits(x), b = ff_bits(y);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// a pair next to the cut-off, in FP64 (out of line: a predicated FP64 instruction
+// costs the pipe as much as one that runs)
+static __device__ __noinline__ bool measure_near(CV c, int i, int b, int j) {
+  return mi2(*c.d, c.X(0, i, j), c.Xd(1, i, j), c.X(0, b, j), c.Xd(1, b, j)) <= c.d->rc2;
+}
+
 // the pairs of a warp: rows (j, i) k = j N + i of k0, k0 + dk, ... below k1 (rows
 // shorten with i: dealt to the warps in turn), the links of particles i < b that
 // start at slice j.  Lanes test 32 partners on the mirror; survivors go onto a
-// ring and are evaluated 32 at a time.  Bound by the FP64 separations (six
-// instructions and three conversions per 32 pairs, 16 cycles of the SM each) and
-// the scan's issue; sums in FP64 instead of two floats cost four more.
+// ring and are evaluated 32 at a time.  768 replicas of 8 to 48
+// particles measured in every sweep: 3.92 -> 3.83 ms (four sweeps) by the
+// separations in two floats.
 constexpr int MEAS_RING = 64;  // at most 31 + 32 in use
 __device__ __forceinline__ void measure_pairs(const CV &c, int k0, int k1, int dk, unsigned long long *ring,
                                               MeasureSums &a) {
   const ChainDesc &d = *c.d;
-  const int N = c.N, M = c.M, dim = c.dim, lane = threadIdx.x & 31;
+  const int N = c.N, M = c.M, lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u, lim = d.q_lim_hi;
-  const float cg = (float)d.inv2s2;
+  const FFBox box(d);
   int head = 0, tail = 0, nf = 0;
   float e0 = 0.f, e1 = 0.f, v0 = 0.f, v1 = 0.f;  // running sums, high and low parts
   auto spill = [&]() {
@@ -81,17 +158,13 @@ __device__ __forceinline__ void measure_pairs(const CV &c, int k0, int k1, int d
     if (lane < cnt) {
       const unsigned long long w = ring[(head + lane) & (MEAS_RING - 1)];  // i | b << 13 | j << 26
       const int i = (int)(w & 0x1fffu), b = (int)((w >> 13) & 0x1fffu), j = (int)(w >> 26);
-      const double r2 = mi2(d, c.X(0, i, j), c.Xd(1, i, j), c.X(0, b, j), c.Xd(1, b, j));
-      if (__double_as_longlong(r2) <= __double_as_longlong(d.rc2)) {
+      auto bead = [&](int n, int t) { return ff_bead(c.X(0, n, t), c.Xd(1, n, t)); };
+      const float r2 = box.dist2(bead(i, j), bead(b, j));
+      bool in = r2 < box.r_lo;
+      if (!in && r2 <= box.r_hi) in = measure_near(c, i, b, j);
+      if (in) {
         const int jn = j + 1 == M ? 0 : j + 1, in = j == M - 1 ? c.next[i] : i, bn = j == M - 1 ? c.next[b] : b;
-        const float dx = (float)mi1(c.X(0, in, jn), c.X(0, bn, jn), d.L, d.L2);
-        const float dy = dim > 1 ? (float)mi1(c.X(1, in, jn), c.X(1, bn, jn), d.L, d.L2) : 0.f;
-        // the pair exponentials e = exp(x), x = -r^2/(2 s^2), and x e; the factors
-        // g tau/2 are applied once at the end
-        const float xa = -(float)r2 * cg, xb = -fmaf(dx, dx, dy * dy) * cg;
-        const float ea = expf(xa), eb = expf(xb);
-        two_sum(e0, e1, ea + eb);
-        two_sum(v0, v1, fmaf(xa, ea, xb * eb));
+        box.terms(r2, bead(in, jn), bead(bn, jn), e0, e1, v0, v1);
       }
     }
     head += cnt;
@@ -118,40 +191,6 @@ __device__ __forceinline__ void measure_pairs(const CV &c, int k0, int k1, int d
   spill();
 }
 
-// ---------------------------------------------------------------------------
-// the same pairs with the separations in two floats (48 bits), from slices
-// staged in shared memory as (x hi, x lo, y hi, y lo): an FP64 instruction takes
-// one of the SM's four pipes for 64 cycles, the six of a pair's separations and
-// its three conversions some 500 of a warp's 600 cycles; the two-float form takes
-// about fifty FP32 instructions.  Its squared distance is within 2^-45, so the
-// float that exp takes is the FP64 form's but for ties; a pair within 1e-6 of
-// the cut-off is settled in FP64.
-// ---------------------------------------------------------------------------
-struct FF {
-  float h, l;
-};
-// a - b folded to the minimum image, normalised
-__device__ __forceinline__ FF ff_sep(float ah, float al, float bh, float bl, float Lh, float L2h, float L2l) {
-  const float s = ah - bh, z = s - ah, e = (ah - (s - z)) - (bh + z), l = e + (al - bl);
-  FF r;
-  r.h = s + l;
-  r.l = l - (r.h - s);
-  if (fabsf(r.h) >= Lh) {
-    // past half the box (or within rounding of it, where the fold changes
-    // nothing a pair within reach sees)
-    const float f = copysignf(1.f, r.h), t = r.h - f * L2h, y = t - r.h, q = (r.h - (t - y)) + (-f * L2h - y);
-    const float w = q + (r.l - f * L2l);
-    r.h = t + w;
-    r.l = w - (r.h - t);
-  }
-  return r;
-}
-
-// bead (i, j) as two floats per coordinate
-__device__ __forceinline__ float4 ff_bead(double x, double y) {
-  const float xh = (float)x, yh = (float)y;
-  return make_float4(xh, (float)(x - (double)xh), yh, (float)(y - (double)yh));
-}
 
 // the pairs of slice j by a CTA of `nw` warps: cur and nxt the staged slice and
 // the next along the paths; this warp takes rows w, w + nw, ...
@@ -160,9 +199,7 @@ __device__ __forceinline__ void measure_pairs_ff(const CV &c, int j, const float
   const ChainDesc &d = *c.d;
   const int N = c.N, lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u, lim = d.q_lim_hi;
-  const float cg = (float)d.inv2s2;
-  const float Lh = (float)d.L, L2h = (float)d.L2, L2l = (float)(d.L2 - (double)L2h);
-  const float r_lo = (float)d.rc2 * (1.f - 1e-6f), r_hi = (float)d.rc2 * (1.f + 1e-6f);
+  const FFBox box(d);
   int head = 0, tail = 0, nf = 0;
   float e0 = 0.f, e1 = 0.f, v0 = 0.f, v1 = 0.f;  // running sums, high and low parts
   auto spill = [&]() {
@@ -176,22 +213,10 @@ __device__ __forceinline__ void measure_pairs_ff(const CV &c, int j, const float
       const unsigned q = ring[(head + lane) & (MEAS_RING - 1)];  // i | b << 13
       const int i = (int)(q & 0x1fffu), b = (int)(q >> 13);
       const float4 p = cur[i], r = cur[b];
-      const FF dx = ff_sep(p.x, p.y, r.x, r.y, Lh, L2h, L2l), dy = ff_sep(p.z, p.w, r.z, r.w, Lh, L2h, L2l);
-      // dx^2 + dy^2 in two floats
-      const float xx = dx.h * dx.h, yy = dy.h * dy.h;
-      const float ex = fmaf(dx.h, dx.h, -xx) + 2.f * dx.h * dx.l, ey = fmaf(dy.h, dy.h, -yy) + 2.f * dy.h * dy.l;
-      const float s = xx + yy, z = s - xx, r2 = s + (((xx - (s - z)) + (yy - z)) + (ex + ey));
-      bool in = r2 < r_lo;
-      if (!in && r2 <= r_hi) in = mi2(d, c.X(0, i, j), c.Xd(1, i, j), c.X(0, b, j), c.Xd(1, b, j)) <= d.rc2;
-      if (in) {
-        const float4 pn = nxt[i], rn = nxt[b];
-        const float nx = ff_sep(pn.x, pn.y, rn.x, rn.y, Lh, L2h, L2l).h;
-        const float ny = ff_sep(pn.z, pn.w, rn.z, rn.w, Lh, L2h, L2l).h;
-        const float xa = -r2 * cg, xb = -fmaf(nx, nx, ny * ny) * cg;
-        const float ea = expf(xa), eb = expf(xb);
-        two_sum(e0, e1, ea + eb);
-        two_sum(v0, v1, fmaf(xa, ea, xb * eb));
-      }
+      const float r2 = box.dist2(p, r);
+      bool in = r2 < box.r_lo;
+      if (!in && r2 <= box.r_hi) in = measure_near(c, i, b, j);
+      if (in) box.terms(r2, nxt[i], nxt[b], e0, e1, v0, v1);
     }
     head += cnt;
     __syncwarp();
