@@ -159,7 +159,7 @@ __global__ void k_eval_weights(EvalArgs a) {
 }
 
 cudaError_t launch_attempt(const AttemptArgs &a, size_t smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_attempt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem((const void *)k_attempt, smem);
   if (e != cudaSuccess) return e;
   k_attempt<<<1, 128, smem, s>>>(a);
   return cudaGetLastError();

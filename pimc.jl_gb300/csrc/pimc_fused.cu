@@ -25,10 +25,10 @@ cudaError_t launch_sweep(const SweepArgs &a, int mode, int grid, int block, size
 }
 cudaError_t sweep_set_smem(int mode, size_t smem) {
   if (mode == 1)
-    return cudaFuncSetAttribute(k_sweep_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const cudaError_t e = cudaFuncSetAttribute(k_sweep_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return allow_smem((const void *)k_sweep_warp, smem);
+  const cudaError_t e = allow_smem((const void *)k_sweep_wide, smem);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return allow_smem((const void *)k_sweep, smem);
 }
 cudaError_t sweep_occupancy(int mode, int block, size_t smem, int *blocks_per_sm) {
   if (mode == 1)

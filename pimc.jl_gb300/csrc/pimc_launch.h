@@ -215,4 +215,20 @@ size_t swap_scratch_bytes(int N, int nwarps);
 size_t com_scratch_bytes(int N, int M, int nwarps);
 int window_scratch_doubles();
 
+// lets kernel f take `smem` bytes of dynamic shared memory.  The limit belongs to
+// the function, not to a launch or a handle: it is only ever raised, and to all
+// that the device offers, so handles on other threads never find it lowered
+// between their own call and their launch.
+inline cudaError_t allow_smem(const void *f, size_t smem) {
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, f);
+  if (e != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= smem) return e;
+  int dev = 0, most = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  most -= (int)fa.sharedSizeBytes;
+  if (smem > (size_t)std::max(most, 0)) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 }  // namespace pimc

@@ -166,7 +166,7 @@ cudaError_t launch_stage_close(const SweepArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t stage_slots_set_smem(size_t smem) {
-  return cudaFuncSetAttribute(k_stage_slots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return allow_smem((const void *)k_stage_slots, smem);
 }
 cudaError_t stage_slots_occupancy(int block, size_t smem, int *blocks_per_sm) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_stage_slots, block, smem);
@@ -282,7 +282,7 @@ cudaError_t launch_measure_sweep(const SweepArgs &a, int ngroups, int num_sms, c
     ngroups = std::min(ngroups, 5 * num_sms);
   }
   const size_t smem = 32 * (size_t)a.meas_staged;
-  const cudaError_t es = cudaFuncSetAttribute(k_measure_slices, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t es = allow_smem((const void *)k_measure_slices, smem);
   if (es != cudaSuccess) return es;
   k_measure_slices<<<ngroups, 128, smem, s>>>(a);
   k_measure_close<<<(a.nchains + 3) / 4, 128, 0, s>>>(a);
@@ -1039,8 +1039,7 @@ cudaError_t launch_sweep_phase(const SweepArgs &a, int phase, int warp, int spec
 }
 
 cudaError_t sweep_phase_set_smem(int phase, int warp, int spec, int regs, size_t smem) {
-  return cudaFuncSetAttribute(phase_kernel(phase, warp, spec, regs),
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return allow_smem(phase_kernel(phase, warp, spec, regs), smem);
 }
 
 cudaError_t sweep_phase_occupancy(int phase, int warp, int spec, int regs, int block, size_t smem,
@@ -1466,7 +1465,7 @@ cudaError_t launch_adjoint(const AdjArgs &a, int maxN, const int *tile_off, int 
   k_adjoint_inv<<<dim3((maxN + 255) / 256, nc), 256, 0, s>>>(a);
   if (a.ib == ADJ_SLICES) {
     const size_t sm = 64 * (size_t)maxN;
-    const cudaError_t e = cudaFuncSetAttribute(k_adjoint_slices, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = allow_smem((const void *)k_adjoint_slices, sm);
     if (e != cudaSuccess) return e;
     k_adjoint_slices<<<a.nctas, 128, sm, s>>>(a);
   } else {
