@@ -57,7 +57,7 @@ PER_BEAD = {
     # the swap launch of the split sweep, the kernel compiled for the
     # reference's rules alone, row scans (its bead updates are the swaps'
     # 2(m-1) per attempt; every attempt also reads the N heat-bath candidates)
-    ("c4", "reference", "k_sweep_swap_ref"): {"dram_bytes": 1036.0, "fp64_flops": 330.0},  # 3.15 GB, 1.00 G / 3.037 M
+    ("c4", "reference", "k_sweep_swap_ref"): {"dram_bytes": 1034.0, "fp64_flops": 92.2},  # 3.14 GB, 0.280 G / 3.037 M
 }
 ROOF_SWEEPS = 2  # sweeps of the per-phase timing pass
 
@@ -577,7 +577,7 @@ def run_ours(args):
                                "pimc_batch_get_beads_all + pimc_batch_energy_sums_all"),
                       "calls_apart_ms": {"set_beads_all": tb[0], "sweep": tb[1],
                                          "get_beads_all": tb[2], "energy_sums_all": tb[3]}}
-    # the adjoint of every chain of the batch in one call (four launches),
+    # the adjoint of every chain of the batch in one call (three or four launches),
     # device time by CUDA events; a step of "batched + adjoint" is one sweep
     # of every chain followed by the adjoint of every chain
     if batched and not args.no_adjoint:

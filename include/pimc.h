@@ -163,7 +163,7 @@ int pimc_run(void *handle, long long n_sweeps);
 /* all chains, one persistent launch per sweep block from a device work
  * queue, captured in a CUDA graph */
 int pimc_batch_run(void *handle, long long n_sweeps);
-/* the same sweeps issued as one plain launch per chain (no queue, no graph) */
+/* the same sweeps issued chain by chain in plain launches (no queue, no graph) */
 int pimc_batch_run_plain(void *handle, long long n_sweeps);
 /* pimc_batch_set_beads_all(x_in), pimc_batch_run(n_sweeps),
  * pimc_batch_get_beads_all(x_out) as one call with no host round trip in
@@ -188,7 +188,7 @@ typedef struct {
   int sweeps_per_launch;
   int state_smem_bytes;
   /* 0: every phase of a sweep in one launch; 1 (one CTA per chain only):
-   * staging, swaps and the rest as three launches per sweep, each phase
+   * staging, swaps and the rest as launches of their own, each phase
    * finished by every chain before the next starts */
   int split_phases;
   /* with split_phases: CTA size of the staging, swap and remaining launches
@@ -313,12 +313,12 @@ int pimc_adjoint(void *handle, int chain, double *dSdr, double *dSdtheta, double
  * any handles of one device) race on it. */
 int pimc_adjoint_noalloc(void *handle, int chain, double *dSdr, double *dSdtheta,
                          double *extra);
-/* pimc_adjoint for every chain of the batch at once (four launches over all
- * chains, scratch carved from a pool the handle allocates on the first call
- * and keeps): dSdtheta[c][3], extra[c][4] as pimc_adjoint per chain c, and
+/* pimc_adjoint for every chain of the batch at once (three launches over all
+ * chains, a fourth for dSdr_all, scratch carved from a pool the handle allocates
+ * on the first call and keeps): dSdtheta[c][3], extra[c][4] as pimc_adjoint per chain c, and
  * dSdr_all (optional) in the layout of pimc_batch_get_beads_all, each
  * chain's [dim][N][M] in chain order.  pimc_last_run_ms then gives the
- * device time of the four launches.  No reference counterpart (PIMC.jl has
+ * device time of the launches.  No reference counterpart (PIMC.jl has
  * no adjoint); the examples' pmap over systems is what it batches. */
 int pimc_batch_adjoint(void *handle, double *dSdtheta, double *extra, double *dSdr_all);
 /* change (V0, omega, g) in place; cached links are recomputed */
