@@ -2348,6 +2348,29 @@ int contact_cells(Handle *h, Handle::ContactTab &t, double tau) {
   return PIMC_OK;
 }
 
+// fills table t (its key given, d and cells null): tab's values, or with tab
+// null the propagator's.  On failure t owns nothing: a table is either whole or
+// in no list.
+int make_contact_table(Handle *h, Handle::ContactTab &t, const double *tab, double tau) {
+  auto build = [&]() -> int {
+    const size_t bytes = sizeof(double) * (size_t)t.n * t.n;
+    CK(cudaMalloc(&t.d, bytes));
+    if (tab) CK(cudaMemcpyAsync(t.d, tab, bytes, cudaMemcpyHostToDevice, h->stream));
+    else CK(launch_contact_table(t.d, t.n, t.range, t.g0, tau, h->stream));
+    return contact_cells(h, t, tau);
+  };
+  const int rc = build();
+  if (rc) {
+    cudaGetLastError();  // an allocation's error is reported once
+    cudaStreamSynchronize(h->stream);
+    cudaFree(t.d);
+    cudaFree(t.cells);
+    t.d = nullptr;
+    t.cells = nullptr;
+  }
+  return rc;
+}
+
 void attach_contact(ChainDesc &d, const Handle::ContactTab &t) {
   const double *tab = t.d;
   const int n = t.n;
@@ -2392,23 +2415,25 @@ int pimc_set_contact_propagator(void *handle, int chain, double g0, double range
   if (!(g0 != 0.0) || !std::isfinite(g0)) return fail(PIMC_EARG, "contact propagator needs g0 != 0");
   if (contact_args(range, n)) return PIMC_EARG;
   CK(cudaStreamSynchronize(h->stream));
+  // every table of the call first, then the chains: a call that fails changes none
+  std::vector<int> at(c1 - c0, -1);
   for (int c = c0; c < c1; ++c) {
     const double tau = h->desc[c].tau;
-    int at = -1;
+    int &k = at[c - c0];
     for (size_t i = 0; i < h->ctabs.size(); ++i) {
       const auto &t = h->ctabs[i];
-      if (!t.given && t.g0 == g0 && t.tau == tau && t.range == range && t.n == n) at = (int)i;
+      if (!t.given && t.g0 == g0 && t.tau == tau && t.range == range && t.n == n) k = (int)i;
     }
-    if (at < 0) {
-      double *d = nullptr;
-      CK(cudaMalloc(&d, sizeof(double) * (size_t)n * n));
-      at = (int)h->ctabs.size();
-      h->ctabs.push_back({g0, tau, range, n, false, d, nullptr, 0.f});
-      CK(launch_contact_table(d, n, range, g0, tau, h->stream));
-      if (contact_cells(h, h->ctabs[at], tau)) return PIMC_ECUDA;
+    if (k >= 0) continue;
+    Handle::ContactTab t{g0, tau, range, n, false, nullptr, nullptr, 0.f};
+    if (const int rc = make_contact_table(h, t, nullptr, tau)) {
+      release_contact_tables(h);
+      return rc;
     }
-    attach_contact(h->desc[c], h->ctabs[at]);
+    k = (int)h->ctabs.size();
+    h->ctabs.push_back(t);
   }
+  for (int c = c0; c < c1; ++c) attach_contact(h->desc[c], h->ctabs[at[c - c0]]);
   if (upload_desc(h)) return PIMC_ECUDA;
   int rc = sync_check(h);
   release_contact_tables(h);
@@ -2425,14 +2450,12 @@ int pimc_set_contact_table(void *handle, int chain, const double *tab, int n, do
   for (size_t i = 0; i < cnt; ++i)
     if (std::isnan(tab[i])) return fail(PIMC_EARG, "contact table holds NaN");
   CK(cudaStreamSynchronize(h->stream));
-  double *d = nullptr;
-  CK(cudaMalloc(&d, sizeof(double) * cnt));
-  h->ctabs.push_back({0.0, 0.0, range, n, true, d, nullptr, 0.f});
-  CK(cudaMemcpyAsync(d, tab, sizeof(double) * cnt, cudaMemcpyHostToDevice, h->stream));
   double tau = 0.0;
   for (int c = c0; c < c1; ++c) tau = std::max(tau, h->desc[c].tau);
-  if (contact_cells(h, h->ctabs.back(), tau)) return PIMC_ECUDA;
-  for (int c = c0; c < c1; ++c) attach_contact(h->desc[c], h->ctabs.back());
+  Handle::ContactTab t{0.0, 0.0, range, n, true, nullptr, nullptr, 0.f};
+  if (const int rc = make_contact_table(h, t, tab, tau)) return rc;
+  h->ctabs.push_back(t);
+  for (int c = c0; c < c1; ++c) attach_contact(h->desc[c], t);
   if (upload_desc(h)) return PIMC_ECUDA;
   int rc = sync_check(h);
   release_contact_tables(h);

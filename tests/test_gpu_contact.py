@@ -234,3 +234,26 @@ def test_contact_system_api(engine_lib):
            (1, pimc.SingleCenterOfMass(s, 1.0))]
     pimc.run(s, 30, ups)
     assert np.isfinite(s.engine.get_beads()).all()
+
+
+def test_refused_contact_propagator_changes_nothing(engine_lib):
+    """a propagator whose table cannot be made for one of the chains (its time
+    step asks for more quadrature nodes than an int counts) is refused every
+    time, and the chains, the first of which has a table that can be made, sweep
+    on as before"""
+    from pimc.engine import ChainParams, Engine, Mix, OPT_EXACT_DECISIONS, PimcError
+    ps = [ChainParams(dim=2, N=6, M=10, L=3.0, T=T, lam=0.5, harmonic_omega=1.0, interactions=True,
+                      pair_g=1.0, pair_sigma=0.5, r_a=1.0, semantics=1, seed=3) for T in (1.0, 1e13)]
+    out = []
+    for refused in (0, 2):
+        e = Engine(ps, Mix(stage_slices=4, stage_max=4, swaps_per_sweep=6, swap_slices=4, swap_max=4))
+        for _ in range(refused):
+            with pytest.raises(PimcError):
+                e.set_contact_propagator(G0, 40.0)
+            assert all(e.contact_table(c)[0] is None for c in range(2))
+        e.set_option(OPT_EXACT_DECISIONS, 0)  # the descriptors go to the device again
+        e.run_batched(4)
+        out.append([e.get_beads(c) for c in range(2)])
+        e.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
