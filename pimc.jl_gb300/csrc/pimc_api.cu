@@ -1004,15 +1004,24 @@ int build_graph(Handle *h) {
   a.order = h->d_order;
   a.queue = h->d_queue;
   a.teams = launch_teams(h, p);
-  cudaGraph_t g;
+  cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   long long nl = 0;
-  issue_sweeps(h, p, a, p.spl, &nl);
+  const cudaError_t ei = issue_sweeps(h, p, a, p.spl, &nl);
+  const cudaError_t ec = cudaStreamEndCapture(h->stream, &g);
+  if (ei != cudaSuccess || ec != cudaSuccess) {
+    // what was captured up to an error is not a sweep
+    cudaGetLastError();
+    if (g) cudaGraphDestroy(g);
+    return fail(PIMC_ECUDA, std::string("graph capture: ") + cudaGetErrorString(ei != cudaSuccess ? ei : ec));
+  }
   h->graph_launches = nl;
-  CK(cudaStreamEndCapture(h->stream, &g));
   cudaError_t e = cudaGraphInstantiate(&h->gexec, g, 0);
   cudaGraphDestroy(g);
-  if (e != cudaSuccess) return fail(PIMC_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    h->gexec = nullptr;
+    return fail(PIMC_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  }
   return PIMC_OK;
 }
 
