@@ -1134,10 +1134,10 @@ struct ContactQuad {
 };
 
 // node q of the rule: the wave number and its weight
-__device__ __forceinline__ void contact_node(const ContactQuad &c, int q, double &k, double &w) {
+__device__ __forceinline__ void contact_node(const ContactQuad &c, long long q, double &k, double &w) {
   const double xs[4] = {0.18343464249564978, 0.525532409916329, 0.7966664774136267, 0.9602898564975362};
   const double ws[4] = {0.36268378337836166, 0.3137066458778869, 0.22238103445337443, 0.10122853629037706};
-  const int p = q >> 3, i = (q >> 1) & 3;
+  const int p = (int)(q >> 3), i = (int)(q >> 1) & 3;
   double a, b;
   if (p < c.ngraded) {
     a = ldexp(1e-10, p);
@@ -1152,7 +1152,7 @@ __device__ __forceinline__ void contact_node(const ContactQuad &c, int q, double
 }
 
 // rows of the product for nodes [q0, q0 + kc): f[r][kc][ld], r = Y, J, U, V
-__global__ void __launch_bounds__(128) k_contact_nodes(double *f, int n, int ld, int q0, int kc, double r0,
+__global__ void __launch_bounds__(128) k_contact_nodes(double *f, int n, int ld, long long q0, int kc, double r0,
                                                         double h, ContactQuad c) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ld) return;
@@ -1284,15 +1284,15 @@ cudaError_t launch_contact_table(double *dtab, int n, double range, double g0, d
   // periods per panel
   const double period = 2.0 * 3.141592653589793 / (2.0 * range);
   const double nu = ceil((q.K - q.k0) / (0.25 * period));
-  if (!(nu < (1 << 27))) return cudaErrorInvalidValue;  // more nodes than an int counts
+  if (!(nu < 2147483600.0)) return cudaErrorInvalidValue;  // more panels than an int counts
   q.nuniform = nu < 1.0 ? 1 : (int)nu;
   q.du = (q.K - q.k0) / q.nuniform;
   const double r0 = 1e-20, h = (range - r0) / (n - 1);
-  const int nodes = 8 * (q.ngraded + q.nuniform);
+  const long long nodes = 8 * ((long long)q.ngraded + q.nuniform);
   const int ld = (n + CT_T - 1) / CT_T * CT_T, nt = ld / CT_T, ntile = nt * (nt + 1) / 2;
   // about 3000 tile products in flight (ten CTAs of 64 threads per SM and a
   // second wave), never fewer than 64 nodes each
-  const int nsplit = std::max(1, std::min({3000 / ntile, (nodes + 63) / 64, 64}));
+  const int nsplit = std::max(1, std::min({3000 / ntile, (int)std::min<long long>((nodes + 63) / 64, 64)}));
   const size_t npart = (size_t)nsplit * ntile * CT_T * CT_T;
   // ranges of nodes whose four rows fit a scratch of 128 MB, less when the
   // device has no such room left
@@ -1300,14 +1300,14 @@ cudaError_t launch_contact_table(double *dtab, int n, double range, double g0, d
   int kc = 0;
   cudaError_t e = cudaErrorMemoryAllocation;
   for (size_t room = (size_t)128 << 20; room >= ((size_t)1 << 18) && e == cudaErrorMemoryAllocation; room >>= 1) {
-    kc = (int)std::min<size_t>(nodes, std::max<size_t>(CT_K, room / (32 * (size_t)ld)));
+    kc = (int)std::min<size_t>((size_t)nodes, std::max<size_t>(CT_K, room / (32 * (size_t)ld)));
     e = cudaMalloc(&ws, 8 * (4 * (size_t)kc * ld + npart));
     if (e == cudaErrorMemoryAllocation) cudaGetLastError();
   }
   if (e != cudaSuccess) return e;
   double *part = ws + 4 * (size_t)kc * ld;
-  for (int q0 = 0; q0 < nodes && e == cudaSuccess; q0 += kc) {
-    const int m = std::min(kc, nodes - q0);
+  for (long long q0 = 0; q0 < nodes && e == cudaSuccess; q0 += kc) {
+    const int m = (int)std::min<long long>(kc, nodes - q0);
     const int per = ((m + nsplit - 1) / nsplit + CT_K - 1) / CT_K * CT_K;
     k_contact_nodes<<<dim3((ld + 127) / 128, std::min(m, 4096)), 128, 0, s>>>(ws, n, ld, q0, m, r0, h, q);
     k_contact_product<<<dim3(ntile, nsplit), 64, 0, s>>>(ws, part, ld, m, per);

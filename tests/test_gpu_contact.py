@@ -238,7 +238,7 @@ def test_contact_system_api(engine_lib):
 
 def test_refused_contact_propagator_changes_nothing(engine_lib):
     """a propagator whose table cannot be made for one of the chains (its time
-    step asks for more quadrature nodes than an int counts) is refused every
+    step asks for more quadrature panels than an int counts) is refused every
     time, and the chains, the first of which has a table that can be made, sweep
     on as before"""
     from pimc.engine import ChainParams, Engine, Mix, OPT_EXACT_DECISIONS, PimcError
