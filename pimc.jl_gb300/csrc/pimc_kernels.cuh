@@ -1556,13 +1556,40 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
   return RES_ACCEPT;
 }
 
-// swaps that swap_sweep does not take (windows past SWAP_LANES links, hard
-// cores), out of line: their code stays out of its way
+// swap a of a sweep that swap_sweep does not take (windows past SWAP_LANES
+// links, hard cores), out of line: its code stays out of swap_sweep's way.  Its
+// beads overlie the sweep's choices D, which the first warp keeps, a lane each:
+// drawn again after every such swap, they cost a hard-core chain 8 % of its
+// swaps.
 template <bool WARP, int SPEC>
-static __device__ __noinline__ int swap_general(CV c, int j0, int m, int n1, double u_pick, Stream ss,
-                                                SwapScratch S, double *red) {
+static __device__ __noinline__ int swap_general(CV c, int a, Stream ss, SwapScratch S, SwapDraws &D,
+                                                double *red) {
+  using G = Group<WARP>;
+  const int k = a & (SWAP_DRAWS - 1), lane = threadIdx.x & 31;
+  const int j0 = D.j0[k], m = D.m[k], n1 = D.n1[k];
+  const double up = (double)D.up[k];
+  const bool keep = WARP || threadIdx.x < 32;
+  int kj = 0, km = 0, kn = 0;
+  float ku = 0.f, kl = 0.f;
+  if (keep) {
+    kj = D.j0[lane];
+    km = D.m[lane];
+    kn = D.n1[lane];
+    ku = D.up[lane];
+    kl = D.lu[lane];
+  }
+  G::sync();
   GenDraws dr = gen_draws(ss);
-  return swap_group<WARP, true, GenDraws, SPEC>(c, j0, m, n1, u_pick, dr, S, red, nullptr, nullptr);
+  const int r = swap_group<WARP, true, GenDraws, SPEC>(c, j0, m, n1, up, dr, S, red, nullptr, nullptr);
+  if (keep) {  // swap_group's last reads of its beads lie before its last barrier
+    D.j0[lane] = kj;
+    D.m[lane] = km;
+    D.n1[lane] = kn;
+    D.up[lane] = ku;
+    D.lu[lane] = kl;
+  }
+  G::sync();
+  return r;
 }
 
 // ---------------------------------------------------------------------------

@@ -325,12 +325,10 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
     // hold the leading warp up after every attempt
     int n_att = 0, n_acc = 0, n_skip = 0;
     long long n_bead = 0;
-    int drawn = -1;  // the first of the swaps whose choices are at hand
     for (int a = 0; a < mix.swaps_per_sweep; ++a) {
-      if ((a & ~(SWAP_DRAWS - 1)) != drawn) {
-        drawn = a & ~(SWAP_DRAWS - 1);
+      if ((a & (SWAP_DRAWS - 1)) == 0) {
         G::sync();
-        if (warp == 0) swap_draws(*Sf.draws, d, sweep, drawn, mix.swaps_per_sweep, M, N, mmax, sm);
+        if (warp == 0) swap_draws(*Sf.draws, d, sweep, a, mix.swaps_per_sweep, M, N, mmax, sm);
         G::sync();
       }
       const Stream ss = make_stream(d, sweep, PH_SWAP, (unsigned)a);
@@ -339,12 +337,7 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
       if (m <= SWAP_LANES && !(SPEC == SWAP_ANY && (d.flags & PF_HARD))) {
         r = swap_sweep<WARP, SPEC>(cs, a, ss, wstride, wmagic, Sf, red);
       } else {
-        const int j0 = Sf.draws->j0[a & (SWAP_DRAWS - 1)], n1 = Sf.draws->n1[a & (SWAP_DRAWS - 1)];
-        const uint4 r1 = ss.at(DRAW_CHOICE + 1);
-        G::sync();
-        r = swap_general<WARP, SPEC>(cs, j0, m, n1, u53(r1.z, r1.w), ss, S, red);
-        G::sync();
-        drawn = -1;  // its beads overwrote the choices
+        r = swap_general<WARP, SPEC>(cs, a, ss, S, *Sf.draws, red);
       }
       if (r == RES_SKIP) {
         ++n_skip;
