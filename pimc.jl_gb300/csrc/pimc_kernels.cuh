@@ -1392,6 +1392,9 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
             w2[1] += lnU2(d, r2n, mi2(d, S.r1x[t + 1], S.r1y[t + 1], S.r2x[t + 1], S.r2y[t + 1]));
         }
       }
+      // the lanes without a link would otherwise run the pair sums' loop apart from
+      // the others between its votes (exact decisions: swaps twice as slow)
+      __syncwarp();
     };
     if (fast && (!f_contact || d.ct_cells)) {
       // bracketed from the mirror, and where that straddles the threshold from
