@@ -1465,6 +1465,44 @@ __device__ __forceinline__ void bridge_beads(const CV &c, int m, const D &dr, do
   }
 }
 
+// the same beads with a hard core, by one warp: sequential retries in the
+// reference's draw order (lane 0 draws, the warp scans the slice); the reference
+// excludes the start particle (fpcycle of the wrapped slice) in its find_nn, the
+// physical semantics the true owner.  Returns 1 when a bead could not be placed.
+template <class D>
+__device__ __forceinline__ int hard_bridge(const CV &c, int n, int nx, int j0, int m, D &dr, double sx, double sy,
+                                           double ex, double ey, double *X, double *Y, int lane) {
+  const ChainDesc &d = *c.d;
+  const int M = c.M, dim = c.dim;
+  double px = sx, py = sy;
+  for (int t = 1; t < m; ++t) {
+    const double2 ab = bridge_coef(c, m, t);
+    const int a = j0 + t, j = a < M ? a : a - M;
+    const int exc = (d.flags & PF_PHYS) ? (a < M ? n : nx) : n;
+    int tries = 0;
+    while (true) {
+      if (++tries > d.ctr) return 1;
+      double qx = 0.0, qy = 0.0;
+      if (lane == 0) {
+        const double z0 = dr.normal(), z1 = dim > 1 ? dr.normal() : 0.0;
+        qx = ab.x * px + (1.0 - ab.x) * ex + z0 * ab.y;
+        qy = dim > 1 ? ab.x * py + (1.0 - ab.x) * ey + z1 * ab.y : 0.0;
+      }
+      qx = __shfl_sync(0xffffffffu, qx, 0);
+      qy = __shfl_sync(0xffffffffu, qy, 0);
+      const double tx = teleport_s<D::kSweep>(qx, d.L, d.inv2L);
+      const double ty = dim > 1 ? teleport_s<D::kSweep>(qy, d.L, d.inv2L) : 0.0;
+      const bool hit = __any_sync(0xffffffffu, hard_hit_lanes(c, tx, ty, j, exc, -1, lane, 32));
+      if (!hit) { px = qx; py = qy; break; }
+    }
+    if (lane == 0) {
+      X[t] = px;
+      Y[t] = py;
+    }
+  }
+  return 0;
+}
+
 // ---------------------------------------------------------------------------
 // Levy staging window, one warp: pair terms (physical semantics) and the
 // hard-core retry loop.  sb: per-warp shared scratch of 5*(WMAX+1) doubles
@@ -1515,35 +1553,7 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
       }
     }
   } else {
-    // sequential retries in the reference's draw order (lane 0 draws, the warp
-    // scans the slice); the reference excludes the start particle (fpcycle of
-    // the wrapped slice) in its find_nn, the physical semantics the true owner
-    double px = sx, py = sy;
-    for (int t = 1; t < m && !fail; ++t) {
-      const double2 ab = bridge_coef(c, m, t);
-      const int a = j0 + t, j = a < M ? a : a - M;
-      const int exc = (d.flags & PF_PHYS) ? (a < M ? n : nx) : n;
-      int tries = 0;
-      while (true) {
-        if (++tries > d.ctr) { fail = 1; break; }
-        double qx = 0.0, qy = 0.0;
-        if (lane == 0) {
-          const double z0 = dr.normal(), z1 = dim > 1 ? dr.normal() : 0.0;
-          qx = ab.x * px + (1.0 - ab.x) * ex + z0 * ab.y;
-          qy = dim > 1 ? ab.x * py + (1.0 - ab.x) * ey + z1 * ab.y : 0.0;
-        }
-        qx = __shfl_sync(0xffffffffu, qx, 0);
-        qy = __shfl_sync(0xffffffffu, qy, 0);
-        const double tx = teleport_s<D::kSweep>(qx, L, inv2L);
-        const double ty = dim > 1 ? teleport_s<D::kSweep>(qy, L, inv2L) : 0.0;
-        const bool hit = __any_sync(0xffffffffu, hard_hit_lanes(c, tx, ty, j, exc, -1, lane, 32));
-        if (!hit) { px = qx; py = qy; break; }
-      }
-      if (lane == 0) {
-        sx_[t] = px;
-        sy_[t] = py;
-      }
-    }
+    fail = hard_bridge(c, n, nx, j0, m, dr, sx, sy, ex, ey, sx_, sy_, lane);
   }
   __syncwarp();
   if (fail) return RES_HARDCORE;
@@ -1631,7 +1641,7 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
 }
 
 // ---------------------------------------------------------------------------
-// a staging window by a team of warps (pair action, no hard core): the warps
+// a staging window by a team of warps (pair action): the warps
 // of the team split the window's links for the pair scans, each with its own
 // neighbour queue; the first warp draws the bridge and decides.  Warp w of
 // the team has the scratch tb + w * tstride (the first warp's holds the
@@ -1675,8 +1685,20 @@ __device__ int window_team(const CV &c, const Team &tm, int n, int j0, int m, D 
   double ex = c.X(0, oe, je), ey = c.Xd(1, oe, je);
   if (fabs(sx - ex) > L) ex += sgn(sx) * (2.0 * L);
   if (dim > 1 && fabs(sy - ey) > L) ey += sgn(sy) * (2.0 * L);
-  if (tm.w == 0) bridge_beads(c, m, dr, sx, sy, ex, ey, sx_, sy_, lane);
+  const bool hard = (d.flags & PF_HARD) != 0;
+  if (tm.w == 0) {
+    if (!hard) {
+      bridge_beads(c, m, dr, sx, sy, ex, ey, sx_, sy_, lane);
+    } else {
+      const int fail = hard_bridge(c, n, nx, j0, m, dr, sx, sy, ex, ey, sx_, sy_, lane);
+      if (lane == 0) b0[TEAM_SLOT_D + 3] = fail;
+    }
+  }
   tm.sync();
+  if (hard && b0[TEAM_SLOT_D + 3] != 0.0) {
+    tm.sync();  // read before the next window's
+    return RES_HARDCORE;
+  }
   for (int t = tid; t <= m; t += nt) {
     double qx = t == 0 ? sx : (t == m ? ex : sx_[t]);
     double qy = t == 0 ? sy : (t == m ? ey : sy_[t]);

@@ -280,8 +280,10 @@ struct Group {
 // slice) is marked for the row scan.  nusable (shared) counts the slices
 // whose lists are usable.
 // ---------------------------------------------------------------------------
+// The slices st, st + 1, ... (past slice M - 1 from 0), len of them; len 0: all.
 template <bool WARP>
-__device__ void cells_build(const CV &c, const CellLists &L, int *ws, int ws_ints, int *nusable) {
+__device__ void cells_build(const CV &c, const CellLists &L, int *ws, int ws_ints, int *nusable, int st = 0,
+                            int len = 0) {
   const ChainDesc &d = *c.d;
   const int lane = threadIdx.x & 31, warp = WARP ? 0 : (int)(threadIdx.x >> 5);
   const int nwarps = WARP ? 1 : (int)(blockDim.x >> 5);
@@ -292,7 +294,9 @@ __device__ void cells_build(const CV &c, const CellLists &L, int *ws, int ws_int
   const int nb = local ? min(nwarps, ws_ints / ne) : nwarps;
   if (warp >= nb) return;
   int *E = local ? ws + (size_t)warp * ne : nullptr;
-  for (int j = warp; j < M; j += nb) {
+  if (len == 0) len = M;
+  for (int q = warp; q < len; q += nb) {
+    const int j = st + q < M ? st + q : st + q - M;
     int *Eg = L.end + (size_t)j * ne;
     if (!local) E = Eg;
     for (int k = lane; k < ne; k += 32) E[k] = 0;

@@ -36,6 +36,14 @@ __global__ void __launch_bounds__(512, 1) k_sweep_rest(SweepArgs a) { sweep_cta<
 // slots' items read the length.  A chain of 1024 particles (64 slices, four
 // slots) went from 57 to 7.9 ms of staging, 512 chains of 8 to 512 particles from
 // 72-89 to 8.4 ms.
+// whether a slot that is walked window by window (hard core, contact table, exact
+// decisions) builds cell lists first.  Sparse chains, staging of a sweep with
+// lists / with row scans: 256 particles 5.16 / 5.03 ms, 512 12.9 / 13.3 (hard core
+// alone 9.44 / 9.33), 1024 37.0 / 41.3, 2048 116 / 141
+constexpr int SLOT_LISTS_N = 512;
+__device__ __forceinline__ bool slot_lists(const ChainDesc &d) {
+  return d.cl_nc > 0 && d.cl_mode > 0 && d.N >= SLOT_LISTS_N;
+}
 __global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ SmemCtl sc;
@@ -60,10 +68,12 @@ __global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
       sc.v.sweep = v.sweep;
       sc.v.stage_m = v.stage_m;
       sc.v.err = v.err;
+      sc.v.cl_hold = v.cl_hold;
       sc.chain = ch;
     }
     __syncthreads();
     const ChainDesc &d = sc.d;
+    if (tid == 0 && d.cl_nc > 0) sc.cl.bind(sc.d, a.ipool);  // used past the barriers below
     const int N = d.N, M = d.M, ph = a.stage_phase;
     const int ell = max(2, min(sc.v.stage_m, min(M - 1, WMAX))), k = (M + ell - 1) / ell;
     const bool serial = chain_serial_local(d);
@@ -99,17 +109,30 @@ __global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
           }
         } else {
           // a warp per window (pair-free), the first warp walking the slot (hard
-          // core), or the CTA as a team on each window (contact table, exact
-          // decisions)
+          // core alone), or the CTA as a team on each window (pair action with
+          // a hard core, a contact table or exact decisions; 1024 hard spheres
+          // with a pair action, staging 58.6 -> 41.3 ms)
+          CV cw = c;
+          if (serial && slot_lists(d) && sc.v.cl_hold == 0) {
+            // the slot's own cell lists: its windows query the slices st .. st + len
+            // - 1 and no other slot's do
+            if (tid == 0) sc.iflag[5] = 0;
+            __syncthreads();
+            cells_build<false>(c, sc.cl, (int *)smem, budget / 4, &sc.iflag[5], st, len);
+            __syncthreads();
+            if (2 * sc.iflag[5] >= len) cw.cl = &sc.cl;
+            else if (tid == 0) atomicMax(&a.var[ch].cl_hold, kCellHold);  // as build_lists holds them off
+            __syncthreads();
+          }
           double *wsb = (double *)smem + (size_t)warp * a.warp_scratch_d;
-          const bool team = serial && !(d.flags & PF_HARD) && nwarps > 1;
+          const bool team = serial && (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && nwarps > 1;
           const Team tm{warp, nwarps, 1};
           for (int n = serial ? 0 : warp; n < N; n += serial ? 1 : nwarps) {
             if (serial && !team && warp > 0) break;
             GenDraws dr = gen_draws(make_stream(d, sweep, PH_STAGE, item0 + n));
             const int m = min(len, 2 + (int)(dr.s.uni(DRAW_CHOICE) * (ell - 1)));
-            const int r = team ? window_team(c, tm, n, st, m, dr, (double *)smem, a.warp_scratch_d)
-                               : window_warp(c, n, st, m, dr, false, wsb, nullptr);
+            const int r = team ? window_team(cw, tm, n, st, m, dr, (double *)smem, a.warp_scratch_d)
+                               : window_warp(cw, n, st, m, dr, false, wsb, nullptr);
             if (lane == 0 && (!team || warp == 0)) {
               n_att += 1;
               n_acc += r == RES_ACCEPT;

@@ -90,3 +90,36 @@ def test_cell_lists_auto_and_plain_launches():
     for c in range(len(ps)):
         np.testing.assert_array_equal(a[0][c], b[0][c])
     np.testing.assert_allclose(a[2], b[2], rtol=1e-12, atol=1e-9)
+
+
+@pytest.mark.parametrize("hard,pair,exact,contact", [
+    (0.2, False, 0, False), (0.2, True, 0, False), (0.0, True, 1, False), (0.0, True, 0, True),
+    (0.1, True, 0, True)])
+def test_slots_build_their_own_lists(hard, pair, exact, contact):
+    """staging slots walked window by window (hard core, exact decisions, contact
+    table), chains long enough for lists of the slot's own slices and windows
+    that wrap around the last slice: lone chains and split sweeps with lists and
+    with row scans move as whole chains in one launch do"""
+    from pimc.engine import ChainParams, Engine, Mix, OPT_EXACT_DECISIONS
+    p = ChainParams(dim=2, N=530, M=11, L=16.0, T=0.5, lam=0.5, interactions=pair, pair_g=1.0, pair_sigma=0.4,
+                    r_a=1.0, hardcore_a=hard, semantics=1, seed=77, retry_cap=100)
+    out = []
+    for how, mode in (("fused", 0), ("plain", 0), ("plain", 1), ("split", 0), ("split", 2)):
+        e = Engine(p, Mix(stage_slices=4, stage_max=4, stage_minacc=0.0, stage_maxacc=1.0, swaps_per_sweep=40,
+                          swap_slices=4, swap_max=4, swap_minacc=0.0, swap_maxacc=1.0, com_phases=0))
+        e.set_cells(mode)
+        e.set_option(OPT_EXACT_DECISIONS, exact)
+        if contact:
+            e.set_contact_propagator(1.16, 5.0, 100)
+        if how == "plain":
+            e.run_plain(3)
+        else:
+            e.set_launch(128, split_phases=int(how == "split"))
+            e.run_batched(3)
+        out.append((e.get_beads(), e.get_next(), e.stats(0).accepts, e.stats(0).bead_updates))
+        e.close()
+    assert out[0][2][0] > 100
+    for x, n, acc, beads in out[1:]:
+        np.testing.assert_array_equal(x, out[0][0])
+        np.testing.assert_array_equal(n, out[0][1])
+        assert acc == out[0][2] and beads == out[0][3]
