@@ -1018,15 +1018,17 @@ __device__ int swap_warp(const CV &c, int j0, int m, int n1, double u_pick, D &d
 // one chain of 64 free particles under the physical rules 22 k -> 7.3 k, 4.26
 // -> 1.81 ms.
 // ---------------------------------------------------------------------------
-// choices of swaps a0 .. a0 + 31 of a sweep, by one warp
+// choices of swaps a0 .. a0 + 31 of a sweep, by one warp; tag: added to the window
+// lengths (SWAP_GENERAL: none of them for the inlined swap_sweep)
+constexpr int SWAP_GENERAL = 256;
 __device__ __forceinline__ void swap_draws(SwapDraws &D, const ChainDesc &d, unsigned long long sweep, int a0,
-                                           int n, int M, int N, int mmax, int sm) {
+                                           int n, int M, int N, int mmax, int sm, int tag) {
   const int lane = threadIdx.x & 31;
   if (a0 + lane < n) {
     const Stream ss = make_stream(d, sweep, PH_SWAP, (unsigned)(a0 + lane));
     const uint4 r0 = ss.at(DRAW_CHOICE), r1 = ss.at(DRAW_CHOICE + 1);
     D.j0[lane] = min(M - 1, (int)(u53(r0.x, r0.y) * M));
-    D.m[lane] = min(mmax, 2 + (int)(u53(r0.z, r0.w) * (sm - 1)));
+    D.m[lane] = min(mmax, 2 + (int)(u53(r0.z, r0.w) * (sm - 1))) + tag;
     D.n1[lane] = min(N - 1, (int)(u53(r1.x, r1.y) * N));
     D.up[lane] = (float)u53(r1.z, r1.w);
     const double u = ss.uni(DRAW_ACCEPT);
@@ -1034,7 +1036,8 @@ __device__ __forceinline__ void swap_draws(SwapDraws &D, const ChainDesc &d, uns
   }
 }
 
-template <bool WARP, int SPEC>
+// LISTS: the first bracket from the cell lists
+template <bool WARP, int SPEC, bool LISTS = false>
 __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, unsigned wmagic, SwapScratch &S,
                           double *red) {
   using G = Group<WARP>;
@@ -1046,7 +1049,8 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
   const int tid = G::rank(), nt = G::size();
   const int warp = WARP ? 0 : (int)(threadIdx.x >> 5), nwarps = WARP ? 1 : (int)(blockDim.x >> 5);
   const int slot = a & (SWAP_DRAWS - 1), buf = a & 1;
-  const int j0 = S.draws->j0[slot], m = S.draws->m[slot], n1 = S.draws->n1[slot];
+  const int j0 = S.draws->j0[slot], n1 = S.draws->n1[slot];
+  const int m = LISTS ? S.draws->m[slot] & (SWAP_GENERAL - 1) : S.draws->m[slot];
   const float lu = S.draws->lu[slot];
   if (!check_ok(m >= 2 && m <= SWAP_LANES && m < M && j0 >= 0 && j0 < M, DERR_WINDOW, d) ||
       !check_ok(n1 >= 0 && n1 < N, DERR_INDEX, d))
@@ -1448,8 +1452,23 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
             }
             e.ko = e.kn = 1;
           }
-          scan_mirror<4>(c, j0, m, reinterpret_cast<const unsigned *>(S.cq), skip, warp, nwarps, e, lane, stop);
+          if (!LISTS)
+            scan_mirror<4>(c, j0, m, reinterpret_cast<const unsigned *>(S.cq), skip, warp, nwarps, e, lane, stop);
           scan_bounds(d, e);
+          if (LISTS) {
+            // segment_estimate's sums come with their bounds: the warp's links
+            PairEst l = {0.f, 0.f, 0.f, 0.f, 0, 0};
+            for (int b = 0; b < 2; ++b) {
+              const int t0 = max(a0 - b * m, 0), t1 = min(a1 - b * m, m);
+              if (t0 < t1) segment_estimate(c, seg_of(b), t0, t1, l, lane);
+            }
+            e.so += l.so;
+            e.bo += l.bo;
+            e.sn += l.sn;
+            e.bn += l.bn;
+            e.ko += l.ko + 1;
+            e.kn += l.kn + 1;
+          }
         } else {
           if (f_phys) {
             cross_exact();
@@ -1563,8 +1582,22 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
   return RES_ACCEPT;
 }
 
-// swap a of a sweep that swap_sweep does not take (windows past SWAP_LANES
-// links, hard cores), out of line: its code stays out of swap_sweep's way.  Its
+// whether a chain's swaps take their first bracket from the cell lists (c.cl not
+// null): a scan of
+// every particle costs less per particle but grows with N.  Physical chains, swaps
+// of a sweep by scans / from the lists, CTAs of 64 threads: 768 particles 12.4 /
+// 12.0 ms, 1024 22.4 / 18.5, 2048 116 / 62, 4096 614 / 250 (sparse: 0.6 a unit
+// square); a lone chain with 256 threads: 1024 10.5 / 9.5, 2048 41.8 / 27.4, 4096
+// 196 / 89, and 2.5 times as dense 1024 13.1 / 13.9, 1536 27.7 / 25.8
+constexpr int SWAP_LISTS_N = 1280;
+__device__ __forceinline__ bool swap_listed(const CV &c) {
+  const int f = c.d->flags;
+  return c.cl && c.N >= SWAP_LISTS_N && (f & PF_PHYS) && (f & PF_PAIR) && !(f & (PF_HARD | PF_CONTACT | PF_EXACT));
+}
+
+// swap a of a sweep that the inlined swap_sweep does not take (windows past SWAP_LANES
+// links, hard cores, brackets from the cell lists), out of line: its code stays out of
+// swap_sweep's way (the lists' bracket called from beside it cost 512 physical chains 3 %).  swap_group's
 // beads overlie the sweep's choices D, which the first warp keeps, a lane each:
 // drawn again after every such swap, they cost a hard-core chain 8 % of its
 // swaps.
@@ -1573,7 +1606,13 @@ static __device__ __noinline__ int swap_general(CV c, int a, Stream ss, SwapScra
                                                 double *red) {
   using G = Group<WARP>;
   const int k = a & (SWAP_DRAWS - 1), lane = threadIdx.x & 31;
-  const int j0 = D.j0[k], m = D.m[k], n1 = D.n1[k];
+  const int j0 = D.j0[k], m = D.m[k] & (SWAP_GENERAL - 1), n1 = D.n1[k];
+  if (SPEC == SWAP_ANY && swap_listed(c) && m <= SWAP_LANES) {
+    S.carve_sweep();
+    const int chunk = (c.N + 31) / 32;
+    return swap_sweep<WARP, SPEC, SPEC == SWAP_ANY>(c, a, ss, swap_wstride(c.N), 0xffffffffu / (unsigned)chunk + 1u, S,
+                                                    red);
+  }
   const double up = (double)D.up[k];
   const bool keep = WARP || threadIdx.x < 32;
   int kj = 0, km = 0, kn = 0;

@@ -328,13 +328,15 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
     for (int a = 0; a < mix.swaps_per_sweep; ++a) {
       if ((a & (SWAP_DRAWS - 1)) == 0) {
         G::sync();
-        if (warp == 0) swap_draws(*Sf.draws, d, sweep, a, mix.swaps_per_sweep, M, N, mmax, sm);
+        if (warp == 0)
+          swap_draws(*Sf.draws, d, sweep, a, mix.swaps_per_sweep, M, N, mmax, sm,
+                     SPEC == SWAP_ANY && ((d.flags & PF_HARD) || swap_listed(cs)) ? SWAP_GENERAL : 0);
         G::sync();
       }
       const Stream ss = make_stream(d, sweep, PH_SWAP, (unsigned)a);
       const int m = Sf.draws->m[a & (SWAP_DRAWS - 1)];
       int r;
-      if (m <= SWAP_LANES && !(SPEC == SWAP_ANY && (d.flags & PF_HARD))) {
+      if (m <= SWAP_LANES) {
         r = swap_sweep<WARP, SPEC>(cs, a, ss, wstride, wmagic, Sf, red);
       } else {
         r = swap_general<WARP, SPEC>(cs, a, ss, S, *Sf.draws, red);
@@ -344,7 +346,7 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
       } else {
         ++n_att;
         n_acc += r == RES_ACCEPT;
-        if (r != RES_HARDCORE) n_bead += 2 * (m - 1);
+        if (r != RES_HARDCORE) n_bead += 2 * ((m & (SWAP_GENERAL - 1)) - 1);
       }
     }
     G::sync();

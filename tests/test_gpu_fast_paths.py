@@ -239,3 +239,34 @@ def test_beam_phases_around_the_table(scale, K, helical, engine_lib):
     want = np.asarray(-0.5 / M * (I + np.roll(I, -1, axis=1)), dtype=float)
     zmax = float(max(np.abs(z).max() for z in ph))
     np.testing.assert_allclose(got.reshape(want.shape), want, rtol=0, atol=(8 + 4 * np.pi * zmax) * 2.0 ** -52 / M)
+
+
+@pytest.mark.parametrize("sem", [0, 1])
+@pytest.mark.parametrize("N,L", [(257, 9.0), (513, 9.0), (1100, 16.0), (1300, 20.0)])
+def test_long_chains_decide_as_exact_sums(N, L, sem, engine_lib):
+    """lone chains and split sweeps with swaps in CTAs of 64 threads at lengths
+    where the kernels change over (staging in CTAs of 512 threads, the partner
+    ratio's particles past the kept ones, swaps bracketed from the cell lists):
+    bracketed decisions, with lists and with row scans, give the beads,
+    permutations and acceptance counts of exact FP64 ones, bit for bit"""
+    from pimc.engine import ChainParams, Engine, Mix, OPT_EXACT_DECISIONS
+    p = ChainParams(dim=2, N=N, M=9, L=L, T=1.0, lam=0.5, harmonic_omega=0.3, interactions=True, pair_g=1.0,
+                    pair_sigma=0.4, r_a=1.0, semantics=sem, seed=61)
+    out = []
+    for exact, mode, split in ((1, 0, 0), (0, 0, 0), (0, 2, 0), (0, 0, 1), (0, 2, 1)):
+        e = Engine(p, Mix(stage_slices=4, stage_max=4, stage_minacc=0.0, stage_maxacc=1.0, swaps_per_sweep=200,
+                          swap_slices=5, swap_max=5, swap_minacc=0.0, swap_maxacc=1.0, com_maxstep=2.0))
+        e.set_option(OPT_EXACT_DECISIONS, exact)
+        e.set_cells(mode)
+        if split:
+            e.set_launch(64, split_phases=1)
+            e.run_batched(3)
+        else:
+            e.run_plain(3)
+        out.append((e.get_beads(), e.get_next(), e.stats(0).accepts))
+        e.close()
+    assert out[0][2][1] > 20
+    for x, n, acc in out[1:]:
+        np.testing.assert_array_equal(x, out[0][0])
+        np.testing.assert_array_equal(n, out[0][1])
+        assert acc == out[0][2]
