@@ -765,6 +765,18 @@ size_t fused_smem(const Handle *h, const Plan &p) {
   return want > p.dyn_smem && (h->max_dyn_smem <= 0 || want <= (size_t)h->max_dyn_smem) ? want : p.dyn_smem;
 }
 
+// whether a lone chain's swaps go in CTAs of 512 threads (128 registers) instead of
+// 256 (255 registers, SWAP_LONE): where the contact bracket's scan of a long chain
+// outweighs the other parts.  512 threads / 256, swaps of a sweep: contact 512
+// particles 8.6 / 8.5 ms, 768 15.1 / 14.4, 1024 20.5 / 21.4 (a whole sweep of 1000
+// under the reference's rules 14.6 / 15.6), 2048 56.7 / 64.5;
+// Gaussian pair, physical rules 512 4.1 / 3.3, 1024 10.9 / 10.0, from 1280 on (the
+// lists' bracket) 2048 29.8 / 27.4; reference rules 1024 6.5 / 5.5; exact decisions
+// 512 15.2 / 9.5; hard core 512 22.4 / 15.3
+bool lone_swap_wide(const ChainDesc &d) {
+  return (d.flags & PF_CONTACT) && !(d.flags & (PF_HARD | PF_EXACT)) && d.N >= 896;
+}
+
 // plain path: each chain's sweep as its own launches, no queue, no graph.  A
 // chain of at most block / 4 pair-free windows sweeps in one launch of one CTA
 // (10 particles, 20 slices, 30 windows: 143 us a sweep, 147 in four launches);
@@ -791,7 +803,6 @@ int run_plain(Handle *h, long long n) {
   }
   if (any_fused) CK(sweep_set_smem(0, p.dyn_smem));
   CK(stage_slots_set_smem(stage_smem));
-  // the swaps of a long interacting chain: twice the warps for its pair scans
   Plan wide = plan_smem(h, 0, 512, 1, kStateBudget);
   if (h->max_dyn_smem > 0 && wide.dyn_smem > (size_t)h->max_dyn_smem) wide = p;
   for (int sc = 0; sc < 2; ++sc)
@@ -818,7 +829,7 @@ int run_plain(Handle *h, long long n) {
       if (sp[c].phases > 0) CK(launch_stage_close(a, h->stream));
       launches += sp[c].phases + (sp[c].phases > 0);
       if (h->mix[c].swaps_per_sweep > 0 && h->desc[c].N > 1) {
-        const bool two = (h->desc[c].flags & PF_PAIR) && h->desc[c].N >= 512 && wide.block > 256;
+        const bool two = lone_swap_wide(h->desc[c]) && wide.block > 256;
         const Plan &w = two ? wide : p;
         a.state_bytes = w.state_bytes;
         CK(launch_sweep_phase(a, 1, 0, spec[c], two ? 0 : SWAP_LONE, 1, w.block, w.dyn_smem, h->stream));
