@@ -711,12 +711,24 @@ bool measure_large(const Handle *h, int c) {
 }
 
 // chains whose windows depend on one another (chain_serial_local) and, of
-// those, the ones that stage_slot takes (stage_by_slots)
+// those, the ones that stage_slot takes (stage_by_slots) and the long ones of the
+// others (stage_long)
 bool desc_serial(const ChainDesc &d) {
   return ((d.flags & PF_PAIR) && (d.flags & PF_PHYS)) || (d.flags & PF_HARD);
 }
 bool desc_slots(const ChainDesc &d) {
   return (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && !(d.flags & (PF_HARD | PF_CONTACT | PF_EXACT));
+}
+
+bool desc_long(const ChainDesc &d) {
+  const bool pairs = (d.flags & PF_PAIR) && (d.flags & PF_PHYS);
+  return desc_serial(d) && !desc_slots(d) &&
+         d.N >= (!pairs ? kLongHard : ((d.flags & PF_HARD) ? kLongPairs : kLongTeam));
+}
+// chains whose swaps may take the cell lists' bracket (swap_listed)
+bool desc_listed(const ChainDesc &d) {
+  return d.cl_nc > 0 && d.cl_mode > 0 && d.N >= kSwapLists && (d.flags & PF_PHYS) && (d.flags & PF_PAIR) &&
+         !(d.flags & (PF_HARD | PF_CONTACT | PF_EXACT));
 }
 
 // what the slot-wise staging of chains [c0, c1) needs under their current
@@ -726,6 +738,7 @@ struct StagePlan {
   int slots = 0, phases = 0;
   size_t smem = 0;
   bool whole = false;  // some chain is staged by the whole-chain kernel
+  bool lng[2] = {false, false};  // some chain by k_stage_slots, by k_stage_slots_long
 };
 StagePlan stage_plan(const Handle *h, int par, int block, int c0, int c1) {
   StagePlan s;
@@ -742,6 +755,7 @@ StagePlan stage_plan(const Handle *h, int par, int block, int c0, int c1) {
     const int lo = std::max(2, std::min({m.stage_min, h->umix[c].stage_slices, h->umix[c].stage_max, d.M - 1}));
     s.slots = std::max(s.slots, (d.M + lo - 1) / lo);
     s.phases = std::max(s.phases, m.staging_phases);
+    if (m.staging_phases > 0) s.lng[desc_long(d)] = true;
     if (desc_slots(d)) ell = std::max(ell, std::min({std::max(m.stage_max, lo), d.M - 1, 64}));
   }
   const int nw = block / 32;
@@ -794,7 +808,7 @@ int run_plain(Handle *h, long long n) {
     sblock[c] = desc_slots(h->desc[c]) && h->desc[c].N >= 256 ? 512 : p.block;
     sp[c] = stage_plan(h, 2, sblock[c], c, c + 1);
     stage_smem = std::max(stage_smem, sp[c].smem);
-    spec[c] = !(h->desc[c].flags & (PF_PHYS | PF_HARD | PF_CONTACT));
+    spec[c] = desc_listed(h->desc[c]) ? 2 : !(h->desc[c].flags & (PF_PHYS | PF_HARD | PF_CONTACT));
     const MixDev &m = h->mix[c];
     const int ell = std::max(2, std::min({h->umix[c].stage_slices, m.stage_max, h->desc[c].M - 1, 64}));
     fused[c] = !desc_serial(h->desc[c]) && ell <= 32 &&
@@ -805,7 +819,7 @@ int run_plain(Handle *h, long long n) {
   CK(stage_slots_set_smem(stage_smem));
   Plan wide = plan_smem(h, 0, 512, 1, kStateBudget);
   if (h->max_dyn_smem > 0 && wide.dyn_smem > (size_t)h->max_dyn_smem) wide = p;
-  for (int sc = 0; sc < 2; ++sc)
+  for (int sc = 0; sc < 3; ++sc)
     for (int rg : {0, SWAP_LONE}) CK(sweep_phase_set_smem(1, 0, sc, rg, std::max(wide.dyn_smem, p.dyn_smem)));
   CK(sweep_phase_set_smem(2, 0, 0, 0, p.dyn_smem));
   SweepArgs a = sweep_args(h, p);
@@ -824,7 +838,7 @@ int run_plain(Handle *h, long long n) {
       a.stage_slots = sp[c].slots;
       for (int ph = 0; ph < sp[c].phases; ++ph) {
         a.stage_phase = ph;
-        CK(launch_stage_slots(a, sp[c].slots, sblock[c], sp[c].smem, h->stream));
+        CK(launch_stage_slots(a, desc_long(h->desc[c]), sp[c].slots, sblock[c], sp[c].smem, h->stream));
       }
       if (sp[c].phases > 0) CK(launch_stage_close(a, h->stream));
       launches += sp[c].phases + (sp[c].phases > 0);
@@ -873,11 +887,15 @@ int fused_mode(const Handle *h, const Plan &p) {
 // pulls chains from the work queue
 // 1 when every chain follows the reference's rules without a hard core or
 // a contact table: the swap phase then runs the kernel compiled for those
-// rules alone (the CUDA graph is rebuilt whenever a chain's flags change)
+// rules alone; 2 when some chain's swaps take the cell lists' bracket (the CUDA
+// graph is rebuilt whenever a chain's flags or list mode change)
 int swap_spec(const Handle *h) {
-  for (const auto &d : h->desc)
-    if (d.flags & (PF_PHYS | PF_HARD | PF_CONTACT)) return 0;
-  return 1;
+  int spec = 1;
+  for (const auto &d : h->desc) {
+    if (desc_listed(d)) return 2;
+    if (d.flags & (PF_PHYS | PF_HARD | PF_CONTACT)) spec = 0;
+  }
+  return spec;
 }
 
 // register variant of a phase's kernel: the plan's, or for swaps in CTAs of 64
@@ -947,15 +965,17 @@ cudaError_t issue_phase(Handle *h, const Plan &p, const SweepArgs &a, int ph, lo
     whole = sp.whole;
     if (sp.slots > 0 && sp.phases > 0) {
       b.stage_slots = sp.slots;
-      int per_sm = 0;
-      if (stage_slots_occupancy(block, sp.smem, &per_sm) != cudaSuccess || per_sm < 1) per_sm = 1;
       const long long items = (long long)sp.slots * a.nchains;
-      const int grid = (int)std::min<long long>(items, (long long)per_sm * h->num_sms);
       cudaError_t e = cudaSuccess;
-      for (int q = 0; q < sp.phases && e == cudaSuccess; ++q) {
-        b.stage_phase = q;
+      for (int q = 0; q < 2 * sp.phases && e == cudaSuccess; ++q) {
+        const bool lng = q & 1;
+        if (!sp.lng[lng]) continue;
+        b.stage_phase = q >> 1;
+        int per_sm = 0;
+        if (stage_slots_occupancy(lng, block, sp.smem, &per_sm) != cudaSuccess || per_sm < 1) per_sm = 1;
+        const int grid = (int)std::min<long long>(items, (long long)per_sm * h->num_sms);
         e = cudaMemsetAsync(a.queue, 0, sizeof(int), h->stream);
-        if (e == cudaSuccess) e = launch_stage_slots(b, grid, block, sp.smem, h->stream);
+        if (e == cudaSuccess) e = launch_stage_slots(b, lng, grid, block, sp.smem, h->stream);
         if (launches) *launches += 1;
       }
       if (e == cudaSuccess) e = launch_stage_close(b, h->stream);

@@ -1474,14 +1474,16 @@ __device__ __forceinline__ int hard_bridge(const CV &c, int n, int nx, int j0, i
                                            double ex, double ey, double *X, double *Y, int lane) {
   const ChainDesc &d = *c.d;
   const int M = c.M, dim = c.dim;
+  const double L = d.L, inv2L = d.inv2L;
   double px = sx, py = sy;
-  for (int t = 1; t < m; ++t) {
+  int fail = 0;  // (a return from the loops costs the walk 5 %)
+  for (int t = 1; t < m && !fail; ++t) {
     const double2 ab = bridge_coef(c, m, t);
     const int a = j0 + t, j = a < M ? a : a - M;
     const int exc = (d.flags & PF_PHYS) ? (a < M ? n : nx) : n;
     int tries = 0;
     while (true) {
-      if (++tries > d.ctr) return 1;
+      if (++tries > d.ctr) { fail = 1; break; }
       double qx = 0.0, qy = 0.0;
       if (lane == 0) {
         const double z0 = dr.normal(), z1 = dim > 1 ? dr.normal() : 0.0;
@@ -1490,8 +1492,8 @@ __device__ __forceinline__ int hard_bridge(const CV &c, int n, int nx, int j0, i
       }
       qx = __shfl_sync(0xffffffffu, qx, 0);
       qy = __shfl_sync(0xffffffffu, qy, 0);
-      const double tx = teleport_s<D::kSweep>(qx, d.L, d.inv2L);
-      const double ty = dim > 1 ? teleport_s<D::kSweep>(qy, d.L, d.inv2L) : 0.0;
+      const double tx = teleport_s<D::kSweep>(qx, L, inv2L);
+      const double ty = dim > 1 ? teleport_s<D::kSweep>(qy, L, inv2L) : 0.0;
       const bool hit = __any_sync(0xffffffffu, hard_hit_lanes(c, tx, ty, j, exc, -1, lane, 32));
       if (!hit) { px = qx; py = qy; break; }
     }
@@ -1500,7 +1502,7 @@ __device__ __forceinline__ int hard_bridge(const CV &c, int n, int nx, int j0, i
       Y[t] = py;
     }
   }
-  return 0;
+  return fail;
 }
 
 // ---------------------------------------------------------------------------
@@ -1667,7 +1669,8 @@ struct Team {
   }
 };
 
-template <class D>
+// HARD: chains with a hard core may come
+template <bool HARD, class D>
 __device__ int window_team(const CV &c, const Team &tm, int n, int j0, int m, D &dr, double *tb,
                            int tstride) {
   auto sb = [&](int w) { return tb + (size_t)w * tstride; };
@@ -1685,7 +1688,7 @@ __device__ int window_team(const CV &c, const Team &tm, int n, int j0, int m, D 
   double ex = c.X(0, oe, je), ey = c.Xd(1, oe, je);
   if (fabs(sx - ex) > L) ex += sgn(sx) * (2.0 * L);
   if (dim > 1 && fabs(sy - ey) > L) ey += sgn(sy) * (2.0 * L);
-  const bool hard = (d.flags & PF_HARD) != 0;
+  const bool hard = HARD && (d.flags & PF_HARD);
   if (tm.w == 0) {
     if (!hard) {
       bridge_beads(c, m, dr, sx, sy, ex, ey, sx_, sy_, lane);

@@ -8,11 +8,11 @@
 namespace pimc {
 
 // one CTA per chain, every phase of the sweep in one launch
-__global__ void __launch_bounds__(512, 1) k_sweep(SweepArgs a) { sweep_cta<SW_ALL>(a); }
+__global__ void __launch_bounds__(512, 1) k_sweep(SweepArgs a) { sweep_cta<SW_ALL, SWAP_LISTS>(a); }
 // the same for CTAs of up to 256 threads with up to 255 registers a thread: no
 // spills in the pair scans, where shared memory or the number of chains keeps
 // a second CTA off the SM anyway
-__global__ void __launch_bounds__(256, 1) k_sweep_wide(SweepArgs a) { sweep_cta<SW_ALL>(a); }
+__global__ void __launch_bounds__(256, 1) k_sweep_wide(SweepArgs a) { sweep_cta<SW_ALL, SWAP_LISTS>(a); }
 // one warp per chain, every phase
 __global__ void __launch_bounds__(256, 2) k_sweep_warp(SweepArgs a) { sweep_warp<SW_ALL>(a); }
 

@@ -438,14 +438,16 @@ struct HeatBath {
 // the other rules' code is compiled out, so the kernel needs fewer registers
 // and less instruction cache (the host picks it when the whole batch
 // qualifies)
-constexpr int SWAP_ANY = 0, SWAP_REF = 1;
+// SPEC = SWAP_LISTS: any rules, and the swaps of long chains with cell lists
+// (swap_listed); the kernels without it keep the registers of shorter chains'
+constexpr int SWAP_ANY = 0, SWAP_REF = 1, SWAP_LISTS = 2;
 
 template <bool WARP, bool FAST, class D, int SPEC = SWAP_ANY>
 __device__ int swap_group(const CV &c, int j0, int m, int n1, double u_pick, D &dr,
                           SwapScratch &S, double *red, double *prop, int *n2_out) {
   using G = Group<WARP>;
   const ChainDesc &d = *c.d;
-  constexpr bool GEN = SPEC == SWAP_ANY;
+  constexpr bool GEN = SPEC != SWAP_REF;
   const bool f_phys = GEN && (d.flags & PF_PHYS), f_hard = GEN && (d.flags & PF_HARD);
   const bool f_contact = GEN && (d.flags & PF_CONTACT);
   const int N = c.N, M = c.M, dim = c.dim, lane = threadIdx.x & 31;
@@ -1042,7 +1044,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
                           double *red) {
   using G = Group<WARP>;
   const ChainDesc &d = *c.d;
-  constexpr bool GEN = SPEC == SWAP_ANY;
+  constexpr bool GEN = SPEC != SWAP_REF;
   const bool f_phys = GEN && (d.flags & PF_PHYS), f_contact = GEN && (d.flags & PF_CONTACT);
   const bool pair = (d.flags & PF_PAIR) != 0;
   const int N = c.N, M = c.M, dim = c.dim, lane = threadIdx.x & 31;
@@ -1589,15 +1591,22 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
 // 12.0 ms, 1024 22.4 / 18.5, 2048 116 / 62, 4096 614 / 250 (sparse: 0.6 a unit
 // square); a lone chain with 256 threads: 1024 10.5 / 9.5, 2048 41.8 / 27.4, 4096
 // 196 / 89, and 2.5 times as dense 1024 13.1 / 13.9, 1536 27.7 / 25.8
-constexpr int SWAP_LISTS_N = 1280;
 __device__ __forceinline__ bool swap_listed(const CV &c) {
   const int f = c.d->flags;
-  return c.cl && c.N >= SWAP_LISTS_N && (f & PF_PHYS) && (f & PF_PAIR) && !(f & (PF_HARD | PF_CONTACT | PF_EXACT));
+  return c.cl && c.N >= kSwapLists && (f & PF_PHYS) && (f & PF_PAIR) && !(f & (PF_HARD | PF_CONTACT | PF_EXACT));
+}
+
+template <bool WARP>
+static __device__ __noinline__ int swap_by_lists(CV c, int a, Stream ss, SwapScratch S, double *red) {
+  S.carve_sweep();
+  const int chunk = (c.N + 31) / 32;
+  return swap_sweep<WARP, SWAP_LISTS, true>(c, a, ss, swap_wstride(c.N), 0xffffffffu / (unsigned)chunk + 1u, S, red);
 }
 
 // swap a of a sweep that the inlined swap_sweep does not take (windows past SWAP_LANES
 // links, hard cores, brackets from the cell lists), out of line: its code stays out of
-// swap_sweep's way (the lists' bracket called from beside it cost 512 physical chains 3 %).  swap_group's
+// swap_sweep's way (the lists' bracket called from beside it cost 512 physical chains
+// 3 %, and in kernels of chains that have none hard-core swaps 4 %).  swap_group's
 // beads overlie the sweep's choices D, which the first warp keeps, a lane each:
 // drawn again after every such swap, they cost a hard-core chain 8 % of its
 // swaps.
@@ -1607,12 +1616,7 @@ static __device__ __noinline__ int swap_general(CV c, int a, Stream ss, SwapScra
   using G = Group<WARP>;
   const int k = a & (SWAP_DRAWS - 1), lane = threadIdx.x & 31;
   const int j0 = D.j0[k], m = D.m[k] & (SWAP_GENERAL - 1), n1 = D.n1[k];
-  if (SPEC == SWAP_ANY && swap_listed(c) && m <= SWAP_LANES) {
-    S.carve_sweep();
-    const int chunk = (c.N + 31) / 32;
-    return swap_sweep<WARP, SPEC, SPEC == SWAP_ANY>(c, a, ss, swap_wstride(c.N), 0xffffffffu / (unsigned)chunk + 1u, S,
-                                                    red);
-  }
+  if (SPEC == SWAP_LISTS && swap_listed(c) && m <= SWAP_LANES) return swap_by_lists<WARP>(c, a, ss, S, red);
   const double up = (double)D.up[k];
   const bool keep = WARP || threadIdx.x < 32;
   int kj = 0, km = 0, kn = 0;

@@ -105,7 +105,8 @@ cudaError_t launch_sweep(const SweepArgs &a, int mode, int grid, int block, size
 cudaError_t sweep_set_smem(int mode, size_t smem);
 // the sweep as three launches per sweep (phase 0 staging, 1 swaps, 2 the
 // rest), one CTA per chain, or for the swaps (warp = 1) one warp per chain;
-// spec = 1 selects the swap kernel compiled for the reference's rules alone
+// spec = 2 selects the swap kernels with the cell lists' bracket (swap_listed),
+// spec = 1 those compiled for the reference's rules alone
 // (every chain of the launch without physical rules, hard core or contact
 // table); a.sweeps must be 1
 // regs (swap phase in CTA mode): 0 the 128-register kernel, 170 or 255 the
@@ -116,11 +117,12 @@ cudaError_t sweep_phase_set_smem(int phase, int warp, int spec, int regs, size_t
 cudaError_t sweep_phase_occupancy(int phase, int warp, int spec, int regs, int block, size_t smem,
                                   int *blocks_per_sm);
 // staging by (chain, slot) items from the work queue a.queue (a.order names
-// the chains), or without one a CTA per item; and the end of the phases
-cudaError_t launch_stage_slots(const SweepArgs &a, int grid, int block, size_t smem, cudaStream_t s);
+// the chains), or without one a CTA per item; lng: the chains of desc_long, else
+// the others; and the end of the phases
+cudaError_t launch_stage_slots(const SweepArgs &a, bool lng, int grid, int block, size_t smem, cudaStream_t s);
 cudaError_t launch_stage_close(const SweepArgs &a, cudaStream_t s);
 cudaError_t stage_slots_set_smem(size_t smem);
-cudaError_t stage_slots_occupancy(int block, size_t smem, int *blocks_per_sm);
+cudaError_t stage_slots_occupancy(bool lng, int block, size_t smem, int *blocks_per_sm);
 // the measurement of the chains whose sweep calls for one, by (chain, slice
 // group) items: of a.nchains chains in a.order, or (meas_list null) of chain
 // chain0, ngroups its groups
@@ -198,15 +200,15 @@ const void *swap_kernel(int warp, int spec, int regs);
 cudaError_t launch_swap(const SweepArgs &a, int warp, int spec, int regs, int grid, int block,
                         size_t smem, cudaStream_t s);
 const void *swap_any_kernel(int warp, int regs);
-cudaError_t launch_swap_any(const SweepArgs &a, int warp, int regs, int grid, int block, size_t smem,
-                            cudaStream_t s);
-// accessors of each kernel unit's device globals (swap_, swap_any_, fused_, attempt_)
+const void *swap_lists_kernel(int regs);
+// accessors of each kernel unit's device globals (swap_, swap_any_, swap_lists_, fused_, attempt_)
 #define PIMC_UNIT_DECL(unit)                                                              \
   cudaError_t unit##_upload_exp_table(const double *tab, size_t bytes);                   \
   cudaError_t unit##_profile_take(unsigned long long *out, bool reset, cudaStream_t s);  \
   cudaError_t unit##_check_word_take(cudaStream_t s, unsigned long long *w);
 PIMC_UNIT_DECL(swap)
 PIMC_UNIT_DECL(swap_any)
+PIMC_UNIT_DECL(swap_lists)
 PIMC_UNIT_DECL(fused)
 PIMC_UNIT_DECL(attempt)
 #undef PIMC_UNIT_DECL

@@ -1,6 +1,7 @@
 // pimc_swap.cu -- the swap-phase kernels of the split sweep for the reference's
-// rules, and the launchers of all swap kernels; the generic ones are
-// pimc_swap_any.cu's (translation units of their own compile in parallel).
+// rules, and the launcher of all swap kernels; the generic ones are
+// pimc_swap_any.cu's and pimc_swap_lists.cu's (translation units of their own
+// compile in parallel).
 #include <cuda_runtime.h>
 
 #include "pimc_sweep.cuh"
@@ -28,6 +29,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_swap_ref_lone(SweepArgs a) {
 // regs: 0 (the 128-register kernels), 170 or 255 (CTAs of 64 threads), SWAP_LONE
 const void *swap_kernel(int warp, int spec, int regs) {
   if (warp || !spec) return swap_any_kernel(warp, regs);
+  if (spec == 2) return swap_lists_kernel(regs);
   if (regs == SWAP_LONE) return (const void *)k_sweep_swap_ref_lone;
   if (regs == 170) return (const void *)k_sweep_swap_ref_r170;
   if (regs == 255) return (const void *)k_sweep_swap_ref_r255;
@@ -36,12 +38,9 @@ const void *swap_kernel(int warp, int spec, int regs) {
 
 cudaError_t launch_swap(const SweepArgs &a, int warp, int spec, int regs, int grid, int block,
                         size_t smem, cudaStream_t s) {
-  if (warp || !spec) return launch_swap_any(a, warp, regs, grid, block, smem, s);
-  if (regs == SWAP_LONE) k_sweep_swap_ref_lone<<<grid, block, smem, s>>>(a);
-  else if (regs == 170) k_sweep_swap_ref_r170<<<grid, block, smem, s>>>(a);
-  else if (regs == 255) k_sweep_swap_ref_r255<<<grid, block, smem, s>>>(a);
-  else k_sweep_swap_ref<<<grid, block, smem, s>>>(a);
-  return cudaGetLastError();
+  SweepArgs args = a;
+  void *ptr[] = {&args};
+  return cudaLaunchKernel(swap_kernel(warp, spec, regs), dim3(grid), dim3(block), ptr, smem, s);
 }
 
 PIMC_UNIT_ACCESSORS(swap)

@@ -1,6 +1,6 @@
 // pimc_swap_any.cu -- the swap-phase kernels for any rules (physical ratio, hard
 // core, contact table), in a translation unit of their own; reached through
-// pimc_swap.cu's launchers.
+// pimc_swap.cu's launcher.
 #include <cuda_runtime.h>
 
 #include "pimc_sweep.cuh"
@@ -23,16 +23,6 @@ const void *swap_any_kernel(int warp, int regs) {
   if (regs == 170) return (const void *)k_sweep_swap_r170;
   if (regs == 255) return (const void *)k_sweep_swap_r255;
   return (const void *)k_sweep_swap;
-}
-
-cudaError_t launch_swap_any(const SweepArgs &a, int warp, int regs, int grid, int block, size_t smem,
-                            cudaStream_t s) {
-  if (warp) k_sweep_swap_warp<<<grid, block, smem, s>>>(a);
-  else if (regs == SWAP_LONE) k_sweep_swap_lone<<<grid, block, smem, s>>>(a);
-  else if (regs == 170) k_sweep_swap_r170<<<grid, block, smem, s>>>(a);
-  else if (regs == 255) k_sweep_swap_r255<<<grid, block, smem, s>>>(a);
-  else k_sweep_swap<<<grid, block, smem, s>>>(a);
-  return cudaGetLastError();
 }
 
 PIMC_UNIT_ACCESSORS(swap_any)

@@ -25,6 +25,49 @@ namespace pimc {
 __global__ void __launch_bounds__(512, 1) k_sweep_stage(SweepArgs a) { sweep_cta<SW_STAGE>(a); }
 __global__ void __launch_bounds__(512, 1) k_sweep_rest(SweepArgs a) { sweep_cta<SW_REST>(a); }
 
+// A slot of a long chain walked window by window (hard core, contact table, exact
+// decisions; stage_long), with cell lists of the slot's own slices: its windows
+// query the slices st .. st + len - 1 and no other slot's do.  Every window with a
+// pair action goes to the CTA as a team, hard cores too.  Sparse chains with a hard
+// core and a pair action, staging of a sweep by the short chains' walk / by this:
+// 256 particles 4.80 / 5.16 ms, 512 15.0 / 12.1 (kLongPairs), 1024 58.6 / 37.0; exact
+// decisions 512 4.90 / 5.15, 1024 14.4 / 13.5 (kLongTeam); hard core alone 512 8.2 / 8.7,
+// 1024 24.0 / 24.3, 2048 77.7 / 76.6 (kLongHard).  Returns the calling thread's attempts,
+// accepts and beads.
+static __device__ __forceinline__ int3 walk_long_slot(CV c, SmemCtl &sc, ChainVar *var, unsigned long long sweep,
+                                                   unsigned item0, int ell, int st, int len, unsigned char *smem,
+                                                   int budget, int warp_scratch_d, int *ipool) {
+  const ChainDesc &d = *c.d;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  if (d.cl_nc > 0 && d.cl_mode > 0 && sc.v.cl_hold == 0) {
+    if (tid == 0) {
+      sc.iflag[5] = 0;
+      sc.cl.bind(d, ipool);
+    }
+    __syncthreads();
+    cells_build<false>(c, sc.cl, (int *)smem, budget / 4, &sc.iflag[5], st, len);
+    __syncthreads();
+    if (2 * sc.iflag[5] >= len) c.cl = &sc.cl;
+    else if (tid == 0) atomicMax(&var->cl_hold, kCellHold);  // as build_lists holds them off
+    __syncthreads();
+  }
+  const bool team = (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && nwarps > 1;
+  const Team tm{warp, nwarps, 1};
+  int3 t = make_int3(0, 0, 0);
+  for (int n = 0; n < c.N && (team || warp == 0); ++n) {
+    GenDraws dr = gen_draws(make_stream(d, sweep, PH_STAGE, item0 + n));
+    const int m = min(len, 2 + (int)(dr.s.uni(DRAW_CHOICE) * (ell - 1)));
+    const int r = team ? window_team<true>(c, tm, n, st, m, dr, (double *)smem, warp_scratch_d)
+                       : window_warp(c, n, st, m, dr, false, (double *)smem, nullptr);
+    if (tid == 0) {
+      t.x += 1;
+      t.y += r == RES_ACCEPT;
+      if (r != RES_HARDCORE) t.z += m - 1;
+    }
+  }
+  return t;
+}
+
 // Staging with a CTA per (chain, slot): the slots of a phase share only their
 // fixed boundary slices, so they run on as many SMs as there are slots.  For
 // chains whose windows depend on one another (each slot a serial walk), and
@@ -36,15 +79,10 @@ __global__ void __launch_bounds__(512, 1) k_sweep_rest(SweepArgs a) { sweep_cta<
 // slots' items read the length.  A chain of 1024 particles (64 slices, four
 // slots) went from 57 to 7.9 ms of staging, 512 chains of 8 to 512 particles from
 // 72-89 to 8.4 ms.
-// whether a slot that is walked window by window (hard core, contact table, exact
-// decisions) builds cell lists first.  Sparse chains, staging of a sweep with
-// lists / with row scans: 256 particles 5.16 / 5.03 ms, 512 12.9 / 13.3 (hard core
-// alone 9.44 / 9.33), 1024 37.0 / 41.3, 2048 116 / 141
-constexpr int SLOT_LISTS_N = 512;
-__device__ __forceinline__ bool slot_lists(const ChainDesc &d) {
-  return d.cl_nc > 0 && d.cl_mode > 0 && d.N >= SLOT_LISTS_N;
-}
-__global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
+// k_stage_slots_long: the chains of stage_long, the other kernel's without them (in
+// one kernel their lists' code cost the short chains' walks 5 to 12 %)
+template <bool LONG>
+__device__ __forceinline__ void stage_slots(const SweepArgs &a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ SmemCtl sc;
   __shared__ double red[256];
@@ -73,11 +111,11 @@ __global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
     }
     __syncthreads();
     const ChainDesc &d = sc.d;
-    if (tid == 0 && d.cl_nc > 0) sc.cl.bind(sc.d, a.ipool);  // used past the barriers below
     const int N = d.N, M = d.M, ph = a.stage_phase;
     const int ell = max(2, min(sc.v.stage_m, min(M - 1, WMAX))), k = (M + ell - 1) / ell;
     const bool serial = chain_serial_local(d);
-    if (s >= k || ph >= sc.mix.staging_phases || (a.stage_par == 1 && !serial) || sc.v.err != 0) {
+    if (s >= k || ph >= sc.mix.staging_phases || (a.stage_par == 1 && !serial) || stage_long(d) != LONG ||
+        sc.v.err != 0) {
       __syncthreads();
       continue;
     }
@@ -97,7 +135,14 @@ __global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
         const int len = sl < k - 1 ? ell : M - (k - 1) * ell, st = (o + sl * ell) % M;
         const unsigned item0 = (unsigned)(ph * (N * k) + sl * N);
         if (len < 2) continue;
-        if (stage_by_slots(d) && SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)budget) {
+        if (LONG) {
+          const int3 w = walk_long_slot(c, sc, a.var + ch, sweep, item0, ell, st, len, smem, budget, a.warp_scratch_d,
+                                        a.ipool);
+          n_att += w.x;
+          n_acc += w.y;
+          n_bead += w.z;
+          __syncthreads();
+        } else if (stage_by_slots(d) && SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)budget) {
           stage_slot(c, sweep, item0, ell, st, len, smem, red, n_att, n_acc, n_bead);
         } else if (!serial && ell <= TWMAX) {
           for (int n = tid; n < N; n += blockDim.x) {
@@ -109,30 +154,17 @@ __global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
           }
         } else {
           // a warp per window (pair-free), the first warp walking the slot (hard
-          // core alone), or the CTA as a team on each window (pair action with
-          // a hard core, a contact table or exact decisions; 1024 hard spheres
-          // with a pair action, staging 58.6 -> 41.3 ms)
-          CV cw = c;
-          if (serial && slot_lists(d) && sc.v.cl_hold == 0) {
-            // the slot's own cell lists: its windows query the slices st .. st + len
-            // - 1 and no other slot's do
-            if (tid == 0) sc.iflag[5] = 0;
-            __syncthreads();
-            cells_build<false>(c, sc.cl, (int *)smem, budget / 4, &sc.iflag[5], st, len);
-            __syncthreads();
-            if (2 * sc.iflag[5] >= len) cw.cl = &sc.cl;
-            else if (tid == 0) atomicMax(&a.var[ch].cl_hold, kCellHold);  // as build_lists holds them off
-            __syncthreads();
-          }
+          // core), or the CTA as a team on each window (contact table, exact
+          // decisions)
           double *wsb = (double *)smem + (size_t)warp * a.warp_scratch_d;
-          const bool team = serial && (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && nwarps > 1;
+          const bool team = serial && !(d.flags & PF_HARD) && nwarps > 1;
           const Team tm{warp, nwarps, 1};
           for (int n = serial ? 0 : warp; n < N; n += serial ? 1 : nwarps) {
             if (serial && !team && warp > 0) break;
             GenDraws dr = gen_draws(make_stream(d, sweep, PH_STAGE, item0 + n));
             const int m = min(len, 2 + (int)(dr.s.uni(DRAW_CHOICE) * (ell - 1)));
-            const int r = team ? window_team(cw, tm, n, st, m, dr, (double *)smem, a.warp_scratch_d)
-                               : window_warp(cw, n, st, m, dr, false, wsb, nullptr);
+            const int r = team ? window_team<false>(c, tm, n, st, m, dr, (double *)smem, a.warp_scratch_d)
+                               : window_warp(c, n, st, m, dr, false, wsb, nullptr);
             if (lane == 0 && (!team || warp == 0)) {
               n_att += 1;
               n_acc += r == RES_ACCEPT;
@@ -158,6 +190,9 @@ __global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) {
   }
 }
 
+__global__ void __launch_bounds__(512, 1) k_stage_slots(SweepArgs a) { stage_slots<false>(a); }
+__global__ void __launch_bounds__(512, 1) k_stage_slots_long(SweepArgs a) { stage_slots<true>(a); }
+
 // the end of the slots' staging phases: close_phase of every chain they served
 __global__ void k_stage_close(SweepArgs a) {
   const int ci = blockIdx.x * blockDim.x + threadIdx.x;
@@ -180,8 +215,9 @@ __global__ void k_stage_close(SweepArgs a) {
   *t = SlotTally{};
 }
 
-cudaError_t launch_stage_slots(const SweepArgs &a, int grid, int block, size_t smem, cudaStream_t s) {
-  k_stage_slots<<<grid, block, smem, s>>>(a);
+cudaError_t launch_stage_slots(const SweepArgs &a, bool lng, int grid, int block, size_t smem, cudaStream_t s) {
+  if (lng) k_stage_slots_long<<<grid, block, smem, s>>>(a);
+  else k_stage_slots<<<grid, block, smem, s>>>(a);
   return cudaGetLastError();
 }
 cudaError_t launch_stage_close(const SweepArgs &a, cudaStream_t s) {
@@ -189,10 +225,12 @@ cudaError_t launch_stage_close(const SweepArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t stage_slots_set_smem(size_t smem) {
-  return allow_smem((const void *)k_stage_slots, smem);
+  const cudaError_t e = allow_smem((const void *)k_stage_slots, smem);
+  return e != cudaSuccess ? e : allow_smem((const void *)k_stage_slots_long, smem);
 }
-cudaError_t stage_slots_occupancy(int block, size_t smem, int *blocks_per_sm) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_stage_slots, block, smem);
+cudaError_t stage_slots_occupancy(bool lng, int block, size_t smem, int *blocks_per_sm) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      blocks_per_sm, lng ? (const void *)k_stage_slots_long : (const void *)k_stage_slots, block, smem);
 }
 size_t slot_scratch_bytes(int ell, int nwarps) {
   return (SlotScratch::bytes(ell + 1, nwarps) + 15) & ~(size_t)15;
@@ -1041,6 +1079,7 @@ cudaError_t upload_exp_table() {
   cudaError_t e = tu_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = swap_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = swap_any_upload_exp_table(tab, sizeof(tab));
+  if (e == cudaSuccess) e = swap_lists_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = fused_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = attempt_upload_exp_table(tab, sizeof(tab));
   return e;
@@ -1445,6 +1484,7 @@ cudaError_t profile_take(unsigned long long *out, bool reset, cudaStream_t s) {
   cudaError_t e = tu_profile_take(out, reset, s);
   if (e == cudaSuccess) e = swap_profile_take(out, reset, s);
   if (e == cudaSuccess) e = swap_any_profile_take(out, reset, s);
+  if (e == cudaSuccess) e = swap_lists_profile_take(out, reset, s);
   if (e == cudaSuccess) e = fused_profile_take(out, reset, s);
   if (e == cudaSuccess) e = attempt_profile_take(out, reset, s);
   return e;
@@ -1460,10 +1500,11 @@ cudaError_t profile_take(unsigned long long *out, bool reset, cudaStream_t s) {
 // nonzero): read and cleared (0 in the default build, which has no bounds
 // checks)
 cudaError_t check_word_take(cudaStream_t s, unsigned long long *w) {
-  cudaError_t (*const take[4])(cudaStream_t, unsigned long long *) = {
-      swap_check_word_take, swap_any_check_word_take, fused_check_word_take, attempt_check_word_take};
+  cudaError_t (*const take[5])(cudaStream_t, unsigned long long *) = {
+      swap_check_word_take, swap_any_check_word_take, swap_lists_check_word_take, fused_check_word_take,
+      attempt_check_word_take};
   cudaError_t e = tu_check_word_take(s, w);
-  for (int u = 0; u < 4 && e == cudaSuccess; ++u) {
+  for (int u = 0; u < 5 && e == cudaSuccess; ++u) {
     unsigned long long w2 = 0;
     e = take[u](s, &w2);
     if (*w == 0) *w = w2;

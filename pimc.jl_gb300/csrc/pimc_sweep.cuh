@@ -2,7 +2,8 @@
 // and the persistent drivers that pull chains from the batch's work queue,
 // shared by the kernel translation units, compiled in parallel:
 // pimc_sweep.cu (the staging and rest phases and the other kernels),
-// pimc_swap.cu and pimc_swap_any.cu (the swap phase), pimc_fused.cu (whole sweeps in one launch)
+// pimc_swap.cu, pimc_swap_any.cu and pimc_swap_lists.cu (the swap phase),
+// pimc_fused.cu (whole sweeps in one launch)
 // and pimc_attempt.cu (single moves with injected draws).  Device globals of
 // the headers are per translation unit (static); each unit gives the host
 // its own accessors (tu_* below, exported by PIMC_UNIT_ACCESSORS).
@@ -45,6 +46,14 @@ __device__ __forceinline__ bool chain_serial_local(const ChainDesc &d) {
 // physical rules, bounded decisions
 __device__ __forceinline__ bool stage_by_slots(const ChainDesc &d) {
   return (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && !(d.flags & (PF_HARD | PF_CONTACT | PF_EXACT));
+}
+
+// of the other chains whose windows depend on one another, the long ones
+// (k_stage_slots_long)
+__device__ __forceinline__ bool stage_long(const ChainDesc &d) {
+  const bool pairs = (d.flags & PF_PAIR) && (d.flags & PF_PHYS);
+  return chain_serial_local(d) && !stage_by_slots(d) &&
+         d.N >= (!pairs ? kLongHard : ((d.flags & PF_HARD) ? kLongPairs : kLongTeam));
 }
 
 // next[] of a chain must be a permutation of 0..N-1: every value in range
@@ -275,7 +284,7 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
           for (int n = 0; n < N; ++n) {
             GenDraws dr = gen_draws(make_stream(d, sweep, PH_STAGE, (unsigned)(ph * items + team * N + n)));
             const int m = min(len, 2 + (int)(dr.s.uni(DRAW_CHOICE) * (ell - 1)));
-            const int r = window_team(cw, tm, n, st, m, dr, tb, warp_scratch_d);
+            const int r = window_team<false>(cw, tm, n, st, m, dr, tb, warp_scratch_d);
             if (tm.w == 0 && lane == 0) {
               tal[0] += 1.0;
               tal[1] += r == RES_ACCEPT;
@@ -330,7 +339,8 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
         G::sync();
         if (warp == 0)
           swap_draws(*Sf.draws, d, sweep, a, mix.swaps_per_sweep, M, N, mmax, sm,
-                     SPEC == SWAP_ANY && ((d.flags & PF_HARD) || swap_listed(cs)) ? SWAP_GENERAL : 0);
+                     SPEC != SWAP_REF && ((d.flags & PF_HARD) || (SPEC == SWAP_LISTS && swap_listed(cs))) ? SWAP_GENERAL
+                                                                                                          : 0);
         G::sync();
       }
       const Stream ss = make_stream(d, sweep, PH_SWAP, (unsigned)a);
@@ -481,7 +491,7 @@ __device__ __forceinline__ void sweep_warp(const SweepArgs &a) {
     if (!ok && lane == 0 && sc.v.err == 0) sc.v.err = DERR_STATE;
     __syncwarp();
     if (ok)
-      for (int s = 0; s < a.sweeps; ++s) sweep_one<true, PH>(sc, nullptr, c, scratch, a.warp_scratch_d, false);
+      for (int s = 0; s < a.sweeps; ++s) sweep_one<true, PH, SWAP_LISTS>(sc, nullptr, c, scratch, a.warp_scratch_d, false);
     if (lane == 0) a.var[sc.chain] = sc.v;
     __syncwarp();
   }

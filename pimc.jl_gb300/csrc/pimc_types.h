@@ -18,6 +18,9 @@ enum : int {
 
 constexpr int MAX_BEAMS = 16;  // laser beams of an optical-lattice potential
 constexpr int kMaxParticles = 8192;  // particles per chain (pimc_params.N)
+// cell lists where a chain's moves would otherwise scan its rows: staging slots
+// walked window by window (stage_long), swaps (swap_listed)
+constexpr int kLongPairs = 512, kLongTeam = 1024, kLongHard = 2048, kSwapLists = 1280;
 
 // observables of one measurement (a row of the series): E_th, E_v, pair
 // energy, pair virial energy, squared winding W^2, signed area A_z, sum r^2/M,

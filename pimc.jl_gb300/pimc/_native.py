@@ -30,8 +30,8 @@ INCLUDE = os.path.join(REPO_DIR, "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", INCLUDE]
-SOURCES = ["pimc_sweep.cu", "pimc_swap.cu", "pimc_swap_any.cu", "pimc_fused.cu", "pimc_attempt.cu", "pimc_api.cu",
-           "pimc_io.cpp"]
+SOURCES = ["pimc_sweep.cu", "pimc_swap.cu", "pimc_swap_any.cu", "pimc_swap_lists.cu", "pimc_fused.cu",
+           "pimc_attempt.cu", "pimc_api.cu", "pimc_io.cpp"]
 
 
 class PimcError(RuntimeError):
