@@ -720,9 +720,10 @@ bool desc_slots(const ChainDesc &d) {
   return (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && !(d.flags & (PF_HARD | PF_CONTACT | PF_EXACT));
 }
 
-bool desc_long(const ChainDesc &d) {
+bool desc_long(const ChainDesc &d, int block) {
   const bool pairs = (d.flags & PF_PAIR) && (d.flags & PF_PHYS);
-  return desc_serial(d) && !desc_slots(d) &&
+  if (desc_slots(d)) return d.N >= kLongSlots && block < 512 && d.cl_nc > 0 && d.cl_mode > 0;
+  return desc_serial(d) &&
          d.N >= (!pairs ? kLongHard : ((d.flags & PF_HARD) ? kLongPairs : kLongTeam));
 }
 // chains whose swaps may take the cell lists' bracket (swap_listed)
@@ -755,7 +756,7 @@ StagePlan stage_plan(const Handle *h, int par, int block, int c0, int c1) {
     const int lo = std::max(2, std::min({m.stage_min, h->umix[c].stage_slices, h->umix[c].stage_max, d.M - 1}));
     s.slots = std::max(s.slots, (d.M + lo - 1) / lo);
     s.phases = std::max(s.phases, m.staging_phases);
-    if (m.staging_phases > 0) s.lng[desc_long(d)] = true;
+    if (m.staging_phases > 0) s.lng[desc_long(d, block)] = true;
     if (desc_slots(d)) ell = std::max(ell, std::min({std::max(m.stage_max, lo), d.M - 1, 64}));
   }
   const int nw = block / 32;
@@ -838,7 +839,7 @@ int run_plain(Handle *h, long long n) {
       a.stage_slots = sp[c].slots;
       for (int ph = 0; ph < sp[c].phases; ++ph) {
         a.stage_phase = ph;
-        CK(launch_stage_slots(a, desc_long(h->desc[c]), sp[c].slots, sblock[c], sp[c].smem, h->stream));
+        CK(launch_stage_slots(a, desc_long(h->desc[c], sblock[c]), sp[c].slots, sblock[c], sp[c].smem, h->stream));
       }
       if (sp[c].phases > 0) CK(launch_stage_close(a, h->stream));
       launches += sp[c].phases + (sp[c].phases > 0);

@@ -25,32 +25,35 @@ namespace pimc {
 __global__ void __launch_bounds__(512, 1) k_sweep_stage(SweepArgs a) { sweep_cta<SW_STAGE>(a); }
 __global__ void __launch_bounds__(512, 1) k_sweep_rest(SweepArgs a) { sweep_cta<SW_REST>(a); }
 
-// A slot of a long chain walked window by window (hard core, contact table, exact
-// decisions; stage_long), with cell lists of the slot's own slices: its windows
-// query the slices st .. st + len - 1 and no other slot's do.  Every window with a
-// pair action goes to the CTA as a team, hard cores too.  Sparse chains with a hard
-// core and a pair action, staging of a sweep by the short chains' walk / by this:
+// Slots of long chains (stage_long), with cell lists of the slot's own slices: its
+// windows query the slices st .. st + len - 1 and no other slot's do.  Every window
+// with a pair action goes to the CTA as a team, hard cores too.  Sparse chains with a
+// hard core and a pair action, staging of a sweep by the short chains' walk / by this:
 // 256 particles 4.80 / 5.16 ms, 512 15.0 / 12.1 (kLongPairs), 1024 58.6 / 37.0; exact
 // decisions 512 4.90 / 5.15, 1024 14.4 / 13.5 (kLongTeam); hard core alone 512 8.2 / 8.7,
-// 1024 24.0 / 24.3, 2048 77.7 / 76.6 (kLongHard).  Returns the calling thread's attempts,
-// accepts and beads.
-static __device__ __forceinline__ int3 walk_long_slot(CV c, SmemCtl &sc, ChainVar *var, unsigned long long sweep,
-                                                   unsigned item0, int ell, int st, int len, unsigned char *smem,
-                                                   int budget, int warp_scratch_d, int *ipool) {
+// 1024 24.0 / 24.3, 2048 77.7 / 76.6 (kLongHard); kLongSlots beside its figures.
+// slot_lists: whether the slot's lists are usable (built by the CTA in smem).
+static __device__ __forceinline__ bool slot_lists(const CV &c, SmemCtl &sc, ChainVar *var, int st, int len,
+                                                  unsigned char *smem, int budget, int *ipool) {
   const ChainDesc &d = *c.d;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  if (d.cl_nc > 0 && d.cl_mode > 0 && sc.v.cl_hold == 0) {
-    if (tid == 0) {
-      sc.iflag[5] = 0;
-      sc.cl.bind(d, ipool);
-    }
-    __syncthreads();
-    cells_build<false>(c, sc.cl, (int *)smem, budget / 4, &sc.iflag[5], st, len);
-    __syncthreads();
-    if (2 * sc.iflag[5] >= len) c.cl = &sc.cl;
-    else if (tid == 0) atomicMax(&var->cl_hold, kCellHold);  // as build_lists holds them off
-    __syncthreads();
+  if (d.cl_nc <= 0 || d.cl_mode <= 0 || sc.v.cl_hold > 0) return false;
+  if (threadIdx.x == 0) {
+    sc.iflag[5] = 0;
+    sc.cl.bind(d, ipool);
   }
+  __syncthreads();
+  cells_build<false>(c, sc.cl, (int *)smem, budget / 4, &sc.iflag[5], st, len);
+  __syncthreads();
+  const bool use = 2 * sc.iflag[5] >= len;
+  if (!use && threadIdx.x == 0) atomicMax(&var->cl_hold, kCellHold);  // as build_lists holds them off
+  __syncthreads();
+  return use;
+}
+// the walk; returns the calling thread's attempts, accepts and beads
+static __device__ __forceinline__ int3 walk_long_slot(const CV &c, unsigned long long sweep, unsigned item0, int ell,
+                                                      int st, int len, unsigned char *smem, int warp_scratch_d) {
+  const ChainDesc &d = *c.d;
+  const int tid = threadIdx.x, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const bool team = (d.flags & PF_PAIR) && (d.flags & PF_PHYS) && nwarps > 1;
   const Team tm{warp, nwarps, 1};
   int3 t = make_int3(0, 0, 0);
@@ -114,7 +117,7 @@ __device__ __forceinline__ void stage_slots(const SweepArgs &a) {
     const int N = d.N, M = d.M, ph = a.stage_phase;
     const int ell = max(2, min(sc.v.stage_m, min(M - 1, WMAX))), k = (M + ell - 1) / ell;
     const bool serial = chain_serial_local(d);
-    if (s >= k || ph >= sc.mix.staging_phases || (a.stage_par == 1 && !serial) || stage_long(d) != LONG ||
+    if (s >= k || ph >= sc.mix.staging_phases || (a.stage_par == 1 && !serial) || stage_long(d, blockDim.x) != LONG ||
         sc.v.err != 0) {
       __syncthreads();
       continue;
@@ -135,14 +138,20 @@ __device__ __forceinline__ void stage_slots(const SweepArgs &a) {
         const int len = sl < k - 1 ? ell : M - (k - 1) * ell, st = (o + sl * ell) % M;
         const unsigned item0 = (unsigned)(ph * (N * k) + sl * N);
         if (len < 2) continue;
-        if (LONG) {
-          const int3 w = walk_long_slot(c, sc, a.var + ch, sweep, item0, ell, st, len, smem, budget, a.warp_scratch_d,
-                                        a.ipool);
+        // (short of memory for its scratch, a long chain of stage_slot's is walked)
+        const bool slot = stage_by_slots(d) && SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)budget;
+        const bool listed = LONG && slot_lists(c, sc, a.var + ch, st, len, smem, budget, a.ipool);
+        if (LONG && (listed || !slot)) {
+          CV cw = c;
+          if (listed) cw.cl = &sc.cl;
+          const int3 w = walk_long_slot(cw, sweep, item0, ell, st, len, smem, a.warp_scratch_d);
           n_att += w.x;
           n_acc += w.y;
           n_bead += w.z;
           __syncthreads();
-        } else if (stage_by_slots(d) && SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)budget) {
+        } else if (LONG) {
+          stage_slot_call(c, sweep, item0, ell, st, len, smem, red, n_att, n_acc, n_bead);
+        } else if (slot) {
           stage_slot(c, sweep, item0, ell, st, len, smem, red, n_att, n_acc, n_bead);
         } else if (!serial && ell <= TWMAX) {
           for (int n = tid; n < N; n += blockDim.x) {

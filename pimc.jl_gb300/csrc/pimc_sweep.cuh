@@ -50,9 +50,10 @@ __device__ __forceinline__ bool stage_by_slots(const ChainDesc &d) {
 
 // of the other chains whose windows depend on one another, the long ones
 // (k_stage_slots_long)
-__device__ __forceinline__ bool stage_long(const ChainDesc &d) {
+__device__ __forceinline__ bool stage_long(const ChainDesc &d, int block) {
   const bool pairs = (d.flags & PF_PAIR) && (d.flags & PF_PHYS);
-  return chain_serial_local(d) && !stage_by_slots(d) &&
+  if (stage_by_slots(d)) return d.N >= kLongSlots && block < 512 && d.cl_nc > 0 && d.cl_mode > 0;
+  return chain_serial_local(d) &&
          d.N >= (!pairs ? kLongHard : ((d.flags & PF_HARD) ? kLongPairs : kLongTeam));
 }
 
@@ -220,9 +221,12 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
     const Stream so = make_stream(d, sweep, PH_STAGE_OFF, (unsigned)ph);
     const int o = min(M - 1, (int)(so.uni(0) * M));
     const int items = N * k;
-    const bool slots = !WARP && slot_bytes > 0 && stage_by_slots(d) &&
-                       SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)slot_bytes;
-    const bool lists = serial_local && !slots && build_lists();
+    const bool fits = !WARP && slot_bytes > 0 && stage_by_slots(d) &&
+                      SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)slot_bytes;
+    // fewer slots than warps: a team of T warps walks each slot
+    const bool by_teams = !WARP && teams && !(d.flags & PF_HARD) && 2 * k <= nwarps && k <= kMaxTeams;
+    const bool lists = serial_local && (!fits || (by_teams && N >= kLongFused)) && build_lists();
+    const bool slots = fits && !lists;
     const CV &cw = lists ? cq : c;
     if (slots) {
       int n_att = 0, n_acc = 0;
@@ -271,9 +275,8 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
           }
         }
       }
-    } else if (!WARP && teams && !(d.flags & PF_HARD) && 2 * k <= nwarps && k <= kMaxTeams) {
-      // fewer slots than warps: a team of T warps walks each slot, the
-      // warps splitting every window's links (named barrier 1 + team)
+    } else if (by_teams) {
+      // the warps of a team split every window's links (named barrier 1 + team)
       const int T = min(nwarps / k, 8), team = warp / T;
       if (team < k) {
         const Team tm{warp - team * T, T, 1 + team};

@@ -21,6 +21,14 @@ constexpr int kMaxParticles = 8192;  // particles per chain (pimc_params.N)
 // cell lists where a chain's moves would otherwise scan its rows: staging slots
 // walked window by window (stage_long), swaps (swap_listed)
 constexpr int kLongPairs = 512, kLongTeam = 1024, kLongHard = 2048, kSwapLists = 1280;
+// and windows that stage_slot would take, whose scans of every particle grow with N:
+// in (chain, slot) CTAs of fewer than 512 threads, and in the fused kernel, whose CTA
+// has all the slots.  Staging of a sweep by stage_slot / from the lists, sparse to
+// dense: (chain, slot) CTAs of 128 threads 4096 particles 227 / 157, 175 / 183,
+// 154 / 207 ms, 8192 1179 / 700, 1023 / 729, 923 / 764; of 256 8192 629 / 461, 553 /
+// 492, 491 / 531; of 512 8192 384 / 401, 336 / 429, 297 / 472; fused 2048 58.6 / 42.5,
+// 48.9 / 48.2, 45.5 / 62.0, 4096 334 / 151, 252 / 178, 217 / 218
+constexpr int kLongSlots = 6144, kLongFused = 2560;
 
 // observables of one measurement (a row of the series): E_th, E_v, pair
 // energy, pair virial energy, squared winding W^2, signed area A_z, sum r^2/M,

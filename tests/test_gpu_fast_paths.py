@@ -270,3 +270,28 @@ def test_long_chains_decide_as_exact_sums(N, L, sem, engine_lib):
         np.testing.assert_array_equal(x, out[0][0])
         np.testing.assert_array_equal(n, out[0][1])
         assert acc == out[0][2]
+
+
+def test_longest_chains_stage_alike(engine_lib):
+    """a chain past the lengths where staging goes from stage_slot to the cell lists
+    (split sweeps, the fused kernel): lists and row scans, in split sweeps, whole
+    sweeps in one launch and lone launches, move the same beads"""
+    from pimc.engine import ChainParams, Engine, Mix
+    p = ChainParams(dim=2, N=6200, M=6, L=48.0, T=1.0, lam=0.5, interactions=True, pair_g=1.0, pair_sigma=0.4,
+                    r_a=1.0, semantics=1, seed=29)
+    out = []
+    for how, mode in (("plain", 0), ("split", 0), ("split", 2), ("fused", 0), ("fused", 2)):
+        e = Engine(p, Mix(stage_slices=3, stage_max=3, stage_minacc=0.0, stage_maxacc=1.0, swaps_per_sweep=20,
+                          swap_slices=3, swap_max=3, swap_minacc=0.0, swap_maxacc=1.0, com_phases=0))
+        e.set_cells(mode)
+        if how == "plain":
+            e.run_plain(1)
+        else:
+            e.set_launch(256, split_phases=int(how == "split"))
+            e.run_batched(1)
+        out.append((e.get_beads(), e.stats(0).accepts, e.stats(0).bead_updates))
+        e.close()
+    assert out[0][1][0] > 6200
+    for x, acc, beads in out[1:]:
+        np.testing.assert_array_equal(x, out[0][0])
+        assert acc == out[0][1] and beads == out[0][2]
