@@ -199,8 +199,10 @@ typedef struct {
    * phase (index 1) only */
   int phase_warp[3];
   /* with split_phases, the swap phase (index 1) with one CTA of at most 64
-   * threads per chain: its kernel compiled for at most 170 or 255 registers
-   * a thread (6 or 4 resident CTAs per SM) instead of 128 (0 or 128) */
+   * threads per chain: its kernel compiled for at most 128, 170 or 255
+   * registers a thread (8, 6 or 4 resident CTAs per SM); 0: the one with the
+   * most registers that still holds every chain at once.  Elsewhere 0 or 128,
+   * which pimc_batch_get_launch then reports as 0 */
   int phase_regs[3];
   /* the neighbour queries' candidates: 0 leaves PIMC_OPT_CELL_LISTS as it
    * is; 1 + a value of it (1 off, 2 auto, 3 always) sets it for every chain.

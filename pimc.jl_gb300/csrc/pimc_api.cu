@@ -55,7 +55,7 @@ struct Plan {
   size_t psmem[3] = {0, 0, 0}; // split: dynamic shared bytes per phase
   int pwarp[3] = {0, 0, 0};    // split: 1 = that phase with one warp per chain
   int pwarp_bytes[3] = {0, 0, 0};  // ... and the scratch bytes of each warp
-  int pregs[3] = {0, 0, 0};    // split, swap phase: register variant (0, 170, 255)
+  int pregs[3] = {0, 0, 0};    // split, swap phase: register variant (0: by residency, 128, 170, 255)
 };
 
 // CTA size and dynamic shared bytes of phase ph of a plan
@@ -899,12 +899,13 @@ int swap_spec(const Handle *h) {
   return spec;
 }
 
-// register variant of a phase's kernel: the plan's, or for swaps in CTAs of 64
-// threads the one with the most registers that still holds every chain at once
+// register variant of a phase's kernel (0: the 128-register one): the plan's, or
+// left open (0) for swaps in CTAs of 64 threads the one with the most registers that still holds every chain at once
 // (128 registers, eight CTAs per SM, spill in the pair scans: 512 physical
 // chains end to end 34.5 ms, with 255 registers and four CTAs 28.3)
 int phase_regs(const Handle *h, const Plan &p, int ph) {
-  if (p.pregs[ph] || ph != 1 || p.pwarp[1] || phase_block(p, 1) > 64) return p.pregs[ph];
+  if (p.pregs[ph]) return p.pregs[ph] == 128 ? 0 : p.pregs[ph];
+  if (ph != 1 || p.pwarp[1] || phase_block(p, 1) > 64) return 0;
   return h->nchains <= 4 * h->num_sms ? 255 : (h->nchains <= 6 * h->num_sms ? 170 : 0);
 }
 
@@ -1607,10 +1608,12 @@ int check_launch(const Handle *h, const pimc_launch &l, Plan *out) {
   for (int ph = 0; ph < 3; ++ph) {
     const int b = l.phase_block[ph];
     const int w = l.phase_warp[ph];
-    const int rg = l.phase_regs[ph] == 128 ? 0 : l.phase_regs[ph];
+    // 128 is every kernel's default; a choice where the variants are offered
+    const bool offered = l.split_phases && ph == 1 && !w && (b > 0 ? b : l.block) <= 64;
+    const int rg = l.phase_regs[ph] == 128 && !offered ? 0 : l.phase_regs[ph];
     if (w != 0 && w != 1) return fail(PIMC_EARG, "phase_warp must be 0 or 1");
-    if (rg != 0 && rg != 170 && rg != 255) return fail(PIMC_EARG, "phase_regs must be 0, 128, 170 or 255");
-    if (rg && (!l.split_phases || ph != 1 || w || (b > 0 ? b : l.block) > 64))
+    if (rg != 0 && rg != 128 && rg != 170 && rg != 255) return fail(PIMC_EARG, "phase_regs must be 0, 128, 170 or 255");
+    if (rg && !offered)
       return fail(PIMC_EARG,
                   "phase_regs: 170 and 255 are offered for the swap phase of a split sweep in CTAs of 64 threads");
     p.pregs[ph] = rg;
@@ -1838,9 +1841,9 @@ static int tune_impl(Handle *h, int sweeps_per_trial, pimc_launch *chosen) {
         ref.phase_regs[1] = 0;
       }
     }
-    // the swap phase in CTAs of 64 threads with the kernels compiled for 170
+    // the swap phase in CTAs of 64 threads with the kernels compiled for 128, 170
     // and 255 registers a thread (fewer spills, fewer chains per SM)
-    for (int rg : {170, 255}) {
+    for (int rg : {128, 170, 255}) {
       pimc_launch l = keep;
       for (int ph = 0; ph < 3; ++ph) l.phase_block[ph] = l.phase_warp[ph] = l.phase_regs[ph] = 0;
       l.phase_block[1] = 64;

@@ -295,3 +295,23 @@ def test_longest_chains_stage_alike(engine_lib):
     for x, acc, beads in out[1:]:
         np.testing.assert_array_equal(x, out[0][0])
         assert acc == out[0][1] and beads == out[0][2]
+
+
+def test_128_register_swaps_stay_a_choice(engine_lib):
+    """phase_regs 128 names a kernel: it is reported as chosen, unlike 0, which
+    leaves the choice open, and where no other is offered it is 0; all give the
+    same chains"""
+    from pimc.engine import ChainParams, Engine, Mix
+    ps = [ChainParams(dim=2, N=N, M=12, L=5.0, T=1.0, lam=0.5, harmonic_omega=1.0, interactions=True, pair_g=1.0,
+                      pair_sigma=0.4, r_a=1.0, semantics=1, seed=N) for N in (9, 40, 300)]
+    out = []
+    for block, regs in ((64, 128), (64, 0), (64, 170), (64, 255), (128, 128)):
+        e = Engine(ps, Mix(stage_slices=4, stage_max=4, swaps_per_sweep=40, swap_slices=4, swap_max=4))
+        e.set_launch(block, split_phases=1, state_smem_bytes=0, phase_regs=(0, regs, 0))
+        assert e.launch["phase_regs"] == [0, regs if block == 64 else 0, 0]
+        e.run_batched(3)
+        out.append([e.get_beads(c) for c in range(3)])
+        e.close()
+    for o in out[1:]:
+        for a, b in zip(o, out[0]):
+            np.testing.assert_array_equal(a, b)
