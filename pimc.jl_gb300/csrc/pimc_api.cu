@@ -79,6 +79,7 @@ struct Handle {
   size_t n_ipool = 0;
   unsigned long long *d_upool = nullptr;
   size_t n_upool = 0;
+  unsigned char *d_small = nullptr;  // one allocation for the next five
   int *d_queue = nullptr;
   int *d_order = nullptr;
   int *d_iout = nullptr;
@@ -533,19 +534,23 @@ int create_impl(const pimc_params *params, int nchains, void **out) {
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
     return cleanup(fail(PIMC_ECUDA, "stream/event creation failed"));
+  // the measurement rows and lists, tallies, order, queue and small results
+  const size_t meas = (9 * sizeof(double) + sizeof(int2)) * (size_t)h->meas_items + 16;
+  const size_t small = meas + sizeof(SlotTally) * (size_t)nchains + sizeof(int) * ((size_t)nchains + 4 + 16);
   if (cudaMalloc(&h->d_desc, sizeof(ChainDesc) * nchains) != cudaSuccess ||
       cudaMalloc(&h->d_var, sizeof(ChainVar) * nchains) != cudaSuccess ||
       cudaMalloc(&h->d_mix, sizeof(MixDev) * nchains) != cudaSuccess ||
       cudaMalloc(&h->d_dpool, sizeof(double) * h->n_dpool) != cudaSuccess ||
       cudaMalloc(&h->d_ipool, sizeof(int) * h->n_ipool) != cudaSuccess ||
       cudaMalloc(&h->d_upool, sizeof(unsigned long long) * h->n_upool) != cudaSuccess ||
-      cudaMalloc(&h->d_queue, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&h->d_order, sizeof(int) * nchains) != cudaSuccess ||
-      cudaMalloc(&h->d_iout, sizeof(int) * 16) != cudaSuccess ||
-      cudaMalloc(&h->d_tally, sizeof(SlotTally) * nchains) != cudaSuccess ||
-      cudaMalloc(&h->d_meas, (9 * sizeof(double) + sizeof(int2)) * (size_t)h->meas_items + 16) != cudaSuccess ||
+      cudaMalloc(&h->d_small, small) != cudaSuccess ||
       cudaMalloc(&h->d_stage, sizeof(double) * std::max<size_t>(h->n_stage, 1)) != cudaSuccess)
     return cleanup(fail(PIMC_ENOMEM, "device allocation failed"));
+  h->d_meas = (double *)h->d_small;
+  h->d_tally = (SlotTally *)(h->d_small + meas);
+  h->d_order = (int *)(h->d_tally + nchains);
+  h->d_queue = h->d_order + nchains;
+  h->d_iout = h->d_queue + 4;
   cudaMemsetAsync(h->d_dpool, 0, sizeof(double) * h->n_dpool, h->stream);
   cudaMemsetAsync(h->d_tally, 0, sizeof(SlotTally) * nchains, h->stream);
   cudaMemsetAsync(h->d_upool, 0, sizeof(unsigned long long) * h->n_upool, h->stream);
@@ -1258,11 +1263,7 @@ int pimc_destroy(void *handle) {
   cudaFree(h->d_dpool);
   cudaFree(h->d_ipool);
   cudaFree(h->d_upool);
-  cudaFree(h->d_queue);
-  cudaFree(h->d_order);
-  cudaFree(h->d_iout);
-  cudaFree(h->d_tally);
-  cudaFree(h->d_meas);
+  cudaFree(h->d_small);
   cudaFree(h->d_buf);
   cudaFree(h->d_adj);
   cudaFree(h->d_stage);

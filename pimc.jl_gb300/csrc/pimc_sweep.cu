@@ -1073,18 +1073,26 @@ size_t swap_scratch_bytes(int N, int nwarps) { return SwapScratch::bytes(N, nwar
 size_t com_scratch_bytes(int N, int M, int nwarps) { return ComScratch::bytes(N, M, nwarps); }
 int window_scratch_doubles() { return WARP_SCRATCH_D; }
 
-// the tables of exp_neg and sincos_turn for the current device, in every kernel
-// unit
-cudaError_t upload_exp_table() {
-  static double tab[TABLE_N];
-  for (int k = 0; k <= EXPTAB_N; ++k) tab[k] = std::exp(-k / 64.0);
-  for (int k = 0; k < TURN_N; ++k) {  // a quarter turn, and exactly 0 and 1 at its ends
-    const int r = k % (TURN_N / 4), q = k / (TURN_N / 4);
-    const long double a = 3.14159265358979323846264338327950288L * r / (TURN_N / 2);
-    const double sn = (double)sinl(a), cs = (double)cosl(a);
-    tab[TURN_AT + 2 * k] = q == 0 ? sn : (q == 1 ? cs : (q == 2 ? -sn : -cs));
-    tab[TURN_AT + 2 * k + 1] = q == 0 ? cs : (q == 1 ? -sn : (q == 2 ? -cs : sn));
+// the tables of exp_neg and sincos_turn, made once for the process (the sines in
+// extended precision take longer than the rest of a small handle's creation)
+struct HostTables {
+  double tab[TABLE_N];
+  HostTables() {
+    for (int k = 0; k <= EXPTAB_N; ++k) tab[k] = std::exp(-k / 64.0);
+    tab[EXPTAB_N + 1] = 0.0;
+    for (int k = 0; k < TURN_N; ++k) {  // a quarter turn, and exactly 0 and 1 at its ends
+      const int r = k % (TURN_N / 4), q = k / (TURN_N / 4);
+      const long double a = 3.14159265358979323846264338327950288L * r / (TURN_N / 2);
+      const double sn = (double)sinl(a), cs = (double)cosl(a);
+      tab[TURN_AT + 2 * k] = q == 0 ? sn : (q == 1 ? cs : (q == 2 ? -sn : -cs));
+      tab[TURN_AT + 2 * k + 1] = q == 0 ? cs : (q == 1 ? -sn : (q == 2 ? -cs : sn));
+    }
   }
+};
+// to the current device, in every kernel unit
+cudaError_t upload_exp_table() {
+  static const HostTables made;
+  const double (&tab)[TABLE_N] = made.tab;
   cudaError_t e = tu_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = swap_upload_exp_table(tab, sizeof(tab));
   if (e == cudaSuccess) e = swap_any_upload_exp_table(tab, sizeof(tab));
