@@ -114,7 +114,7 @@ struct Handle {
     int n;
     bool given;
     double *d;
-    float4 *cells;  // the bracket's FP32 copy, or null
+    float4 *cells;  // the bracket's FP32 copy, in d's allocation, or null
     float neg;      // ChainDesc::ct_neg
   };
   std::vector<ContactTab> ctabs;
@@ -1271,10 +1271,7 @@ int pimc_destroy(void *handle) {
   for (cudaEvent_t e : h->io_ev) cudaEventDestroy(e);
   if (h->s_up) cudaStreamDestroy(h->s_up);
   if (h->s_down) cudaStreamDestroy(h->s_down);
-  for (auto &t : h->ctabs) {
-    cudaFree(t.d);
-    cudaFree(t.cells);
-  }
+  for (auto &t : h->ctabs) cudaFree(t.d);
   cudaFree(h->d_rdf);
   cudaFree(h->d_badj);
   cudaFree(h->d_tile_off);
@@ -2384,19 +2381,14 @@ int contact_targets(Handle *h, int chain, int *c0, int *c1) {
   return PIMC_OK;
 }
 
-// the FP32 copy of table t for the sweeps' brackets (without room for it they
-// decide from exact sums) and the radius past which its terms are light, for
+// the FP32 copy of table t for the sweeps' brackets (where it has room for one;
+// without, they decide from exact sums) and the radius past which its terms are light, for
 // chains of imaginary-time step at most tau
 int contact_cells(Handle *h, Handle::ContactTab &t, double tau) {
-  t.cells = nullptr;
   t.neg = 0.f;
-  if (cudaMalloc(&t.cells, sizeof(float4) * (size_t)(t.n - 1) * (t.n - 1)) != cudaSuccess) {
-    cudaGetLastError();
-    t.cells = nullptr;
-    return PIMC_OK;
-  }
+  if (!t.cells) return sync_check(h);
   int last = -1;
-  CK(cudaMemcpyAsync(h->d_iout, &last, sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemsetAsync(h->d_iout, 0xff, sizeof(int), h->stream));  // -1
   CK(launch_contact_cells(t.d, t.cells, t.n, 1e-9 / (12.566370614359172 * tau), h->d_iout, h->stream));
   CK(cudaMemcpyAsync(&last, h->d_iout, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   if (sync_check(h)) return PIMC_ECUDA;
@@ -2410,8 +2402,15 @@ int contact_cells(Handle *h, Handle::ContactTab &t, double tau) {
 // in no list.
 int make_contact_table(Handle *h, Handle::ContactTab &t, const double *tab, double tau) {
   auto build = [&]() -> int {
-    const size_t bytes = sizeof(double) * (size_t)t.n * t.n;
-    CK(cudaMalloc(&t.d, bytes));
+    // one allocation for the table and the FP32 copy, or for the table alone
+    const size_t bytes = sizeof(double) * (size_t)t.n * t.n, at = (bytes + 15) & ~(size_t)15;
+    if (cudaMalloc(&t.d, at + sizeof(float4) * (size_t)(t.n - 1) * (t.n - 1)) == cudaSuccess) {
+      t.cells = (float4 *)((unsigned char *)t.d + at);
+    } else {
+      cudaGetLastError();
+      t.d = nullptr;
+      CK(cudaMalloc(&t.d, bytes));
+    }
     if (tab) CK(cudaMemcpyAsync(t.d, tab, bytes, cudaMemcpyHostToDevice, h->stream));
     else CK(launch_contact_table(t.d, t.n, t.range, t.g0, tau, h->stream));
     return contact_cells(h, t, tau);
@@ -2421,7 +2420,6 @@ int make_contact_table(Handle *h, Handle::ContactTab &t, const double *tab, doub
     cudaGetLastError();  // an allocation's error is reported once
     cudaStreamSynchronize(h->stream);
     cudaFree(t.d);
-    cudaFree(t.cells);
     t.d = nullptr;
     t.cells = nullptr;
   }
@@ -2452,7 +2450,6 @@ void release_contact_tables(Handle *h) {
     for (const auto &d : h->desc) used = used || ((d.flags & PF_CONTACT) && d.ct_tab == h->ctabs[i].d);
     if (used) { ++i; continue; }
     cudaFree(h->ctabs[i].d);
-    cudaFree(h->ctabs[i].cells);
     h->ctabs.erase(h->ctabs.begin() + (long)i);
   }
 }
