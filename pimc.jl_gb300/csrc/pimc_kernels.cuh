@@ -869,7 +869,7 @@ __device__ int swap_group(const CV &c, int j0, int m, int n1, double u_pick, D &
     // early accept is always one the exact sums would make
     auto stop = [&](const PairEst &pe) -> bool {
       if (!monotone) return false;
-      if (*flag) return true;
+      if (__any_sync(0xffffffffu, *flag)) return true;  // the warp decides as one
       const float ro = 2.4e-7f * (float)(pe.ko + 1), rn = 2.4e-7f * (float)(pe.kn + 1);
       const float lf = (pe.so * (1.f - ro) - pe.bo * (1.f + ro)) + (pe.sn * (1.f - rn) - pe.bn * (1.f + rn));
       const float af = (pe.so + pe.bo) + (pe.sn + pe.bn);
@@ -1420,7 +1420,7 @@ __device__ int swap_sweep(const CV &c, int a, const Stream &ss, int wstride, uns
       volatile int *flag = S.iv + 3;
       auto stop = [&](const PairEst &q) -> bool {
         if (!monotone) return false;
-        if (*flag) return true;
+        if (__any_sync(0xffffffffu, *flag)) return true;  // the warp decides as one
         float t, r;
         PairEst qb = q;
         scan_bounds(d, qb);
