@@ -115,7 +115,7 @@ struct Handle {
     bool given;
     double *d;
     float4 *cells;  // the bracket's FP32 copy, in d's allocation, or null
-    float neg;      // ChainDesc::ct_neg
+    double neg;     // the radius of ChainDesc::ct_neg
   };
   std::vector<ContactTab> ctabs;
   unsigned long long *d_rdf = nullptr;  // pair-distance histograms of every chain
@@ -228,10 +228,20 @@ ChainDesc make_desc(const pimc_params &p, int chain) {
       d.est_hi = (float)((d.q_lim_hi + 1.0) * w16 * (1.0 + 4e-7));
       d.f_scale = 4294967296.0 / (2.0 * p.L);
       const double fu = 1.0 / d.f_scale;
-      d.f_unit = (float)fu;
+      d.len_e = std::max(-900, std::min(900, std::ilogb(p.L)));
+      const double sc = std::ldexp(1.0, -d.len_e);
+      d.f_unit = (float)(fu * sc);
+      d.rc_s = (float)(d.rc * sc);
+      d.rc2_s = (float)(d.rc2 * sc * sc);
+      d.inv2s2_s = (float)(d.inv2s2 / sc / sc);
+      d.L_s = (float)(p.L * sc);
+      d.L2_s = (float)(2.0 * p.L * sc);
+      d.L2_sl = (float)(2.0 * p.L * sc - (double)d.L2_s);
       d.est2 = (float)(1e-6 + 8.0 * d.rc * fu * d.inv2s2);
     }
-    d.hb_unit = (float)((double)d.q_unit2 / (4.0 * d.tau * d.lambda));
+    // (as a float where it is one)
+    const double u2 = std::isnormal(d.q_unit2) ? (double)d.q_unit2 : u * u;
+    d.hb_unit = (float)(u2 / (4.0 * d.tau * d.lambda));
     d.q_Lf = (float)p.L;
     d.q_scalef = (float)d.q_scale;
   }
@@ -2385,7 +2395,7 @@ int contact_targets(Handle *h, int chain, int *c0, int *c1) {
 // without, they decide from exact sums) and the radius past which its terms are light, for
 // chains of imaginary-time step at most tau
 int contact_cells(Handle *h, Handle::ContactTab &t, double tau) {
-  t.neg = 0.f;
+  t.neg = 0.0;
   if (!t.cells) return sync_check(h);
   int last = -1;
   CK(cudaMemsetAsync(h->d_iout, 0xff, sizeof(int), h->stream));  // -1
@@ -2393,7 +2403,7 @@ int contact_cells(Handle *h, Handle::ContactTab &t, double tau) {
   CK(cudaMemcpyAsync(&last, h->d_iout, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   if (sync_check(h)) return PIMC_ECUDA;
   // no light terms in a table that does not decay: clamped radii lie past it
-  t.neg = last >= t.n - 1 ? INFINITY : (float)((last + 1) * (t.range / (t.n - 1)) * 1.00001);
+  t.neg = last >= t.n - 1 ? INFINITY : (last + 1) * (t.range / (t.n - 1)) * 1.00001;
   return PIMC_OK;
 }
 
@@ -2436,9 +2446,10 @@ void attach_contact(ChainDesc &d, const Handle::ContactTab &t) {
   d.ct_rmax = range;
   d.ct_h = (range - kContactR0) / (double)(n - 1);
   d.ct_cells = t.cells;
-  d.ct_neg = t.neg;
-  d.ct_invh = (float)(1.0 / d.ct_h);
-  d.ct_c4 = (float)(1.4426950408889634 / (4.0 * d.tau));
+  const double sc = std::ldexp(1.0, -d.len_e);
+  d.ct_neg = (float)(t.neg * sc);
+  d.ct_invh = (float)(1.0 / (d.ct_h * sc));
+  d.ct_c4 = (float)(1.4426950408889634 / (4.0 * d.tau) / sc / sc);
   d.ct_4pt = (float)(12.566370614359172 * d.tau);
   d.flags |= PF_CONTACT;
 }
@@ -2479,7 +2490,7 @@ int pimc_set_contact_propagator(void *handle, int chain, double g0, double range
       if (!t.given && t.g0 == g0 && t.tau == tau && t.range == range && t.n == n) k = (int)i;
     }
     if (k >= 0) continue;
-    Handle::ContactTab t{g0, tau, range, n, false, nullptr, nullptr, 0.f};
+    Handle::ContactTab t{g0, tau, range, n, false, nullptr, nullptr, 0.0};
     if (const int rc = make_contact_table(h, t, nullptr, tau)) {
       release_contact_tables(h);
       return rc;
@@ -2506,7 +2517,7 @@ int pimc_set_contact_table(void *handle, int chain, const double *tab, int n, do
   CK(cudaStreamSynchronize(h->stream));
   double tau = 0.0;
   for (int c = c0; c < c1; ++c) tau = std::max(tau, h->desc[c].tau);
-  Handle::ContactTab t{0.0, 0.0, range, n, true, nullptr, nullptr, 0.f};
+  Handle::ContactTab t{0.0, 0.0, range, n, true, nullptr, nullptr, 0.0};
   if (const int rc = make_contact_table(h, t, tab, tau)) return rc;
   h->ctabs.push_back(t);
   for (int c = c0; c < c1; ++c) attach_contact(h->desc[c], t);

@@ -85,10 +85,12 @@ __device__ __forceinline__ FF ff_sep(float ah, float al, float bh, float bl, flo
   return r;
 }
 
-// x as two floats, the first truncated, on the integer pipe: conversions between
-// the formats take the FP64 pipe's time.  Below 2^-74 it is 0.
-__device__ __forceinline__ float2 ff_bits(double x) {
-  const unsigned hi = __double2hiint(x), lo = __double2loint(x), s = hi & 0x80000000u, e = hi & 0x7fffffffu;
+// x 2^-len_e as two floats, the first truncated, on the integer pipe: conversions
+// between the formats take the FP64 pipe's time.  Below 2^-73 of 2^len_e (which is
+// no more than L, and a separation within reach is summed at L's precision) it is 0.
+__device__ __forceinline__ float2 ff_bits(double x, int len_e) {
+  const unsigned hi = __double2hiint(x), lo = __double2loint(x), s = hi & 0x80000000u;
+  const unsigned e = (unsigned)max((int)(hi & 0x7fffffffu) - (len_e << 20), 0);
   const float h = __uint_as_float(s | __funnelshift_l(lo, e - (896u << 20), 3));
   const float u = __uint_as_float(s | (((e >> 20) - 948u) << 23));  // sign and weight of the word's last bit
   return e < (950u << 20) ? make_float2(0.f, 0.f) : make_float2(h, u * (float)(lo & 0x1fffffffu));
@@ -97,9 +99,10 @@ __device__ __forceinline__ float2 ff_bits(double x) {
 // what a chain's pairs are measured against
 struct FFBox {
   float cg, Lh, L2h, L2l, r_lo, r_hi;
+  int len_e;
   __device__ __forceinline__ explicit FFBox(const ChainDesc &d)
-      : cg((float)d.inv2s2), Lh((float)d.L), L2h((float)d.L2), L2l((float)(d.L2 - (double)L2h)),
-        r_lo((float)d.rc2 * (1.f - 1e-6f)), r_hi((float)d.rc2 * (1.f + 1e-6f)) {}
+      : cg(d.inv2s2_s), Lh(d.L_s), L2h(d.L2_s), L2l(d.L2_sl), r_lo(d.rc2_s * (1.f - 1e-6f)),
+        r_hi(d.rc2_s * (1.f + 1e-6f)), len_e(d.len_e) {}
   // the squared distance of beads p and r
   __device__ __forceinline__ float dist2(const float4 &p, const float4 &r) const {
     const FF dx = ff_sep(p.x, p.y, r.x, r.y, Lh, L2h, L2l), dy = ff_sep(p.z, p.w, r.z, r.w, Lh, L2h, L2l);
@@ -122,8 +125,8 @@ struct FFBox {
 };
 
 // a bead as two floats per coordinate
-__device__ __forceinline__ float4 ff_bead(double x, double y) {
-  const float2 a = ff_bits(x), b = ff_bits(y);
+__device__ __forceinline__ float4 ff_bead(double x, double y, int len_e) {
+  const float2 a = ff_bits(x, len_e), b = ff_bits(y, len_e);
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
@@ -158,7 +161,7 @@ __device__ __forceinline__ void measure_pairs(const CV &c, int k0, int k1, int d
     if (lane < cnt) {
       const unsigned long long w = ring[(head + lane) & (MEAS_RING - 1)];  // i | b << 13 | j << 26
       const int i = (int)(w & 0x1fffu), b = (int)((w >> 13) & 0x1fffu), j = (int)(w >> 26);
-      auto bead = [&](int n, int t) { return ff_bead(c.X(0, n, t), c.Xd(1, n, t)); };
+      auto bead = [&](int n, int t) { return ff_bead(c.X(0, n, t), c.Xd(1, n, t), box.len_e); };
       const float r2 = box.dist2(bead(i, j), bead(b, j));
       bool in = r2 < box.r_lo;
       if (!in && r2 <= box.r_hi) in = measure_near(c, i, b, j);

@@ -146,9 +146,9 @@ __device__ __forceinline__ void scan_fixed(const CV &c, int j0, int m, const uin
   const ChainDesc &d = *c.d;
   const int N = c.N, M = c.M;
   const bool wraps = j0 + m >= M;
-  const float u = d.f_unit, rc2 = (float)d.rc2;
-  const float r_lo = rc2 * (1.f - 2e-6f) - 8.f * u * (float)d.rc, r_hi = rc2 * (1.f + 2e-6f) + 8.f * u * (float)d.rc;
-  const float cy = (float)d.inv2s2;
+  const float u = d.f_unit, rc2 = d.rc2_s;
+  const float r_lo = rc2 * (1.f - 2e-6f) - 8.f * u * d.rc_s, r_hi = rc2 * (1.f + 2e-6f) + 8.f * u * d.rc_s;
+  const float cy = d.inv2s2_s;
   float lo_s[2] = {0.f, 0.f};
   for (int b0 = 32 * part; b0 < N; b0 += 32 * nparts) {
     const int b = b0 + lane, bl = min(b, N - 1);
@@ -270,8 +270,8 @@ __device__ __forceinline__ void scan_contact(const CV &c, int j0, int m, const u
   const ChainDesc &d = *c.d;
   const int N = c.N, M = c.M;
   const bool wraps = j0 + m >= M;
-  const float u = d.f_unit, rc2 = (float)d.rc2, neg2 = d.ct_neg * d.ct_neg;
-  const float r_lo = rc2 * (1.f - 2e-6f) - 8.f * u * (float)d.rc, r_hi = rc2 * (1.f + 2e-6f) + 8.f * u * (float)d.rc;
+  const float u = d.f_unit, rc2 = d.rc2_s, neg2 = d.ct_neg * d.ct_neg;
+  const float r_lo = rc2 * (1.f - 2e-6f) - 8.f * u * d.rc_s, r_hi = rc2 * (1.f + 2e-6f) + 8.f * u * d.rc_s;
   const unsigned lt = (1u << lane) - 1u;
   int head = 0, tail = 0;
   float sa = 0.f, na = 0.f, lo_o = 0.f, lo_n = 0.f;  // sum of magnitudes, terms left out

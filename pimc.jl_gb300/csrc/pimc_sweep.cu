@@ -301,8 +301,8 @@ __global__ void __launch_bounds__(128) k_measure_slices(SweepArgs a) {
           __syncthreads();  // the last slice's pairs are done
           for (int i = tid; i < N; i += 128) {
             const int in = wrap ? c.next[i] : i, jn = wrap ? 0 : j + 1;
-            slices[i] = ff_bead(c.X(0, i, j), c.Xd(1, i, j));
-            slices[N + i] = ff_bead(c.X(0, in, jn), c.Xd(1, in, jn));
+            slices[i] = ff_bead(c.X(0, i, j), c.Xd(1, i, j), d.len_e);
+            slices[N + i] = ff_bead(c.X(0, in, jn), c.Xd(1, in, jn), d.len_e);
           }
           __syncthreads();
           measure_pairs_ff(c, j, slices, slices + N, warp, 4, reinterpret_cast<unsigned *>(qbuf + warp * MEAS_RING), m);

@@ -71,9 +71,14 @@ struct ChainDesc {
   // mirror's): ex2(est_x f), relative error at most est_eps within reach, and
   // est_eps est_far in absolute terms beyond; reach bounds surely within and
   // surely beyond.  scan_fixed's fixed point: 2^32 / 2L, its unit, and the
-  // constant part of its exponentials' relative error
+  // constant part of its exponentials' relative error.  Lengths in FP32 are in
+  // units of 2^len_e, the power of two below L, so that their squares stay in
+  // range whatever the chain's units: the unit, rc, rc^2 and inv2s2 there, L and 2L
+  // (in two floats)
   float est_eps, est_far, est_x, est_lo, est_hi;
   float f_unit, est2;
+  float rc_s, rc2_s, inv2s2_s, L_s, L2_s, L2_sl;
+  int len_e;
   double f_scale;
   // the sweeps' FP32 heat-bath exponent scale per window length m:
   // hb_unit / m = (squared mirror unit) / (4 lambda m tau)
@@ -109,7 +114,8 @@ struct ChainDesc {
   int ct_n, ct_pad_;
   double ct_r0, ct_h, ct_rmax;
   // the bracket's FP32 copy of the table, four corners per cell (null: no room,
-  // exact sums alone), and 1 / ct_h, log2(e) / 4 tau, 4 pi tau
+  // exact sums alone), and (lengths in units of 2^len_e) 1 / ct_h, log2(e) / 4
+  // tau, 4 pi tau
 #ifdef __CUDACC__
   const float4 *ct_cells;
 #else

@@ -315,3 +315,33 @@ def test_128_register_swaps_stay_a_choice(engine_lib):
     for o in out[1:]:
         for a, b in zip(o, out[0]):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("sem", [0, 1])
+@pytest.mark.parametrize("e", [-90, 80])
+def test_chains_in_any_unit_of_length(e, sem, engine_lib):
+    """the same chains with every length times 2^e (beyond the square roots of
+    FP32's range): positions times 2^e and the same decisions and observables,
+    bit for bit, since a power of two scales every product exactly"""
+    from pimc.engine import ChainParams, Engine, Mix
+    out = []
+    for k in (0, e):
+        u = 2.0 ** k
+        kw = dict(dim=2, M=16, L=4.0 * u, T=1.0, lam=0.5 * u * u, harmonic_omega=1.0 / u, interactions=True,
+                  pair_g=1.0, pair_sigma=0.5 * u, r_a=1.0 * u, semantics=sem, seed=3)
+        eng = Engine([ChainParams(N=N, **kw) for N in (7, 40, 160)],
+                     Mix(stage_slices=6, stage_max=6, swaps_per_sweep=60, swap_slices=6, swap_max=6,
+                         com_step=0.5 * u, com_minstep=0.1 * u, com_maxstep=2.0 * u, measure_every=1))
+        eng.run_batched(4)
+        s, _, cnt = eng.energy_sums_all()
+        eng.set_launch(64, split_phases=1)
+        eng.run_batched(2)
+        s2, _, _ = eng.energy_sums_all()
+        out.append(([eng.get_beads(c) / u for c in range(3)], [eng.stats(c).accepts for c in range(3)], s, s2, cnt))
+        eng.close()
+    for a, b in zip(out[0][0], out[1][0]):
+        np.testing.assert_array_equal(a, b)
+    assert out[0][1] == out[1][1]
+    for k in (2, 3, 4):
+        np.testing.assert_array_equal(out[0][k], out[1][k])
+    assert np.all(out[0][2][:, 2] != 0.0)
