@@ -944,14 +944,13 @@ int grid_for(Handle *h, const Plan &p, int phase = -1, int nch = -1) {
   return std::max(1, std::min(need, per_sm * h->num_sms));
 }
 
-// teams of warps pay off only when every chain of the launch is resident at
-// once (the launch is latency-bound); with more chains than resident CTAs
+// fused sweeps: teams of warps pay off only when every chain of the launch is resident
+// at once (the launch is latency-bound); with more chains than resident CTAs
 // the idle warps' issue slots are used by other chains anyway
 bool launch_teams(Handle *h, const Plan &p) {
   int per_sm = 0;
-  if (p.mode != 0) return false;
-  const cudaError_t e = p.split ? sweep_phase_occupancy(0, 0, 0, 0, phase_block(p, 0), phase_smem(p, 0), &per_sm)
-                                : sweep_occupancy(p.mode, p.block, fused_smem(h, p), &per_sm);
+  if (p.mode != 0 || p.split) return false;
+  const cudaError_t e = sweep_occupancy(p.mode, p.block, fused_smem(h, p), &per_sm);
   if (e != cudaSuccess) return false;
   return h->nchains <= per_sm * h->num_sms;
 }

@@ -242,7 +242,6 @@ struct InjDraws {
       z[d] = i < n_nrm ? nrm[i] : 0.0;
     }
   }
-  __device__ __forceinline__ void bead_normals_f(int, float &a, float &b) const { a = b = 0.f; }  // sweeps only
   __device__ __forceinline__ void consumed(int cnt) { pn += cnt; }
   __device__ __forceinline__ double normal() {
     if (pn < n_nrm) return nrm[pn++];
@@ -1534,7 +1533,7 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
   if (dim > 1 && fabs(sy - ey) > L) ey += sgn(sy) * (2.0 * L);
   int fail = 0;
   if (!hard && D::kSweep) {
-    bridge_beads(c, m, dr, sx, sy, ex, ey, sx_, sy_, lane);
+    if constexpr (D::kSweep) bridge_beads(c, m, dr, sx, sy, ex, ey, sx_, sy_, lane);
   } else if (!hard) {
     for (int t = 1 + lane; t < m; t += 32) {
       double z[2];

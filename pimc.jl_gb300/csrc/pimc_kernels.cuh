@@ -1890,14 +1890,12 @@ __device__ __forceinline__ long long bin_floor(double x, double L, double w, dou
 // Every term in FP64 (pimc_measure); the sweeps' measurements are
 // pimc_measure.cuh's.
 // ---------------------------------------------------------------------------
-template <bool WARP>
-__device__ void measure_group(const CV &c, double *red, double *out, bool density,
+static __device__ __forceinline__ void measure_group(const CV &c, double *red, double *out, bool density,
                               unsigned long long *qbuf) {
-  using G = Group<WARP>;
   const ChainDesc &d = *c.d;
-  const int N = c.N, M = c.M, dim = c.dim, tid = G::rank(), nt = G::size();
-  const int lane = threadIdx.x & 31, warp = WARP ? 0 : (int)(threadIdx.x >> 5);
-  const int nwarps = WARP ? 1 : (int)(blockDim.x >> 5);
+  const int N = c.N, M = c.M, dim = c.dim, tid = threadIdx.x, nt = blockDim.x;
+  const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5);
+  const int nwarps = (int)(blockDim.x >> 5);
   // the contact table carries no tau derivative: no pair energy for it
   const bool pair = (d.flags & PF_PAIR) != 0 && !(d.flags & PF_CONTACT);
   const double rc2 = d.rc * d.rc, cg = d.inv2s2;
@@ -2028,7 +2026,7 @@ __device__ void measure_group(const CV &c, double *red, double *out, bool densit
     // pair-distance histogram: warps split the beads, lanes the partners of
     // higher index; lanes with the same bin add once (match_any)
     const int tot = N * M;
-    const int gw = WARP ? 0 : warp, ngw = WARP ? 1 : nwarps;
+    const int gw = warp, ngw = nwarps;
     const int ib_max = d.rdf_nb;
     for (int kk = gw; kk < tot; kk += ngw) {
       const int j = kk / N, i = kk % N;
@@ -2051,8 +2049,8 @@ __device__ void measure_group(const CV &c, double *red, double *out, bool densit
       }
     }
   }
-  G::template sum<5>(s, red);
-  G::template sum<4>(sf, red);
+  block_sum_k<5>(s, red);
+  block_sum_k<4>(sf, red);
   if (tid == 0) {
     const double tau = d.tau;
     out[4] = sf[0] * sf[0] + sf[1] * sf[1];

@@ -30,9 +30,9 @@ struct SweepArgs {
   int warp_scratch_d; // doubles of scratch per warp
   int warp_bytes;     // warp-per-chain mode: scratch bytes of each warp
   int slot_bytes;     // shared bytes a CTA's slot-wise staging may use (0: none)
-  int stage_par;      // staging by slots: 1 = only chains whose windows depend on
-                      // one another, 2 = every chain (k_stage_slots); the staging
-                      // kernel of whole chains skips those
+  int stage_par;      // k_stage_slots: 1 = only chains whose windows depend on one
+                      // another (the staging kernel of whole chains has the others),
+                      // 2 = every chain (lone chains, which have no such launch)
   int stage_phase;    // the staging phase that k_stage_slots runs
   int stage_slots;    // slots per chain of its queue (the longest chain's)
   struct SlotTally *tally;  // [chains] k_stage_slots' counters, zero between phases

@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(256) k_measure(const ChainDesc *desc, ChainVar
     }
     return;
   }
-  measure_group<false>(c, red, sc.e4, c.hist != nullptr, qbuf);
+  measure_group(c, red, sc.e4, c.hist != nullptr, qbuf);
   if (threadIdx.x == 0) {
     record_measurement(sc.d, sc.v, c, sc.e4, c.hist != nullptr);
     var[ch] = sc.v;

@@ -180,7 +180,8 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
   const int tid = G::rank(), nt = G::size(), lane = threadIdx.x & 31;
   const int warp = WARP ? 0 : (int)(threadIdx.x >> 5), nwarps = WARP ? 1 : (int)(blockDim.x >> 5);
   const int N = c.N, M = c.M;
-  const bool serial_local = chain_serial_local(d);
+  // (the staging kernel's chains have none: sweep_cta leaves them to k_stage_slots)
+  const bool serial_local = PH != SW_STAGE && chain_serial_local(d);
   const unsigned long long sweep = sc.v.sweep;
   // the view with the chain's cell lists: a phase that queries neighbours
   // builds them at its start and its moves keep them current; the phases
@@ -221,7 +222,7 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
     const Stream so = make_stream(d, sweep, PH_STAGE_OFF, (unsigned)ph);
     const int o = min(M - 1, (int)(so.uni(0) * M));
     const int items = N * k;
-    const bool fits = !WARP && slot_bytes > 0 && stage_by_slots(d) &&
+    const bool fits = !WARP && PH != SW_STAGE && slot_bytes > 0 && stage_by_slots(d) &&
                       SlotScratch::bytes(min(ell, M - 1) + 1, nwarps) <= (size_t)slot_bytes;
     // fewer slots than warps: a team of T warps walks each slot
     const bool by_teams = !WARP && teams && !(d.flags & PF_HARD) && 2 * k <= nwarps && k <= kMaxTeams;
@@ -529,7 +530,7 @@ __device__ __forceinline__ void sweep_cta(const SweepArgs &a) {
     ++iter;
     if (sc.chain < 0) break;
     const ChainDesc &d = sc.d;
-    if (PH == SW_STAGE && a.stage_par == 1 && chain_serial_local(d)) {  // k_stage_slots'
+    if (PH == SW_STAGE && chain_serial_local(d)) {  // k_stage_slots'
       __syncthreads();
       continue;
     }

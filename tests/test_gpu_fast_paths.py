@@ -345,3 +345,48 @@ def test_chains_in_any_unit_of_length(e, sem, engine_lib):
     for k in (2, 3, 4):
         np.testing.assert_array_equal(out[0][k], out[1][k])
     assert np.all(out[0][2][:, 2] != 0.0)
+
+
+def test_measurement_of_chains_too_long_to_stage(engine_lib):
+    """a chain of more particles than the measurement launches stage: a split
+    sweep's and a lone chain's observables as pimc_measure's, within the bounds of
+    test_measurement_launches_agree (the sums of 2100 particles' positive terms
+    round within 1e-10 as well)"""
+    from pimc.engine import ChainParams, Engine, Mix
+    p = ChainParams(dim=2, N=2100, M=4, L=20.0, T=0.5, lam=0.5, harmonic_omega=0.2, interactions=True, pair_g=1.0,
+                    pair_sigma=0.5, r_a=1.5, energy_capacity=4, seed=5)
+    for split in (0, 1):
+        e = Engine(p, Mix(stage_slices=2, stage_max=2, swaps_per_sweep=20, swap_slices=2, swap_max=2, com_maxstep=2.0,
+                          measure_every=1))
+        if split:
+            e.set_launch(128, split_phases=1)
+            e.run_batched(1)
+        else:
+            e.run_plain(1)
+        got = e.observables()[-1]
+        e.reset_measurements()
+        e.measure()
+        want = e.observables()[0]
+        e.close()
+        scale = np.maximum(np.abs(want), 1.0)
+        assert np.all(np.abs(got - want)[[0, 1, 4, 5, 6]] <= 1e-10 * scale[[0, 1, 4, 5, 6]])
+        assert np.all(np.abs(got - want)[[2, 3]] <= 2e-7 * scale[[2, 3]]) and want[2] > 0.0
+
+
+def test_adjoint_of_one_chain_by_slices(engine_lib):
+    """a lone chain of enough slices for a CTA each, against FP64 numpy with the
+    bound of test_adjoint_gather_edges"""
+    from pimc.engine import ChainParams, Engine
+    N, M = 9, 700
+    rng = np.random.default_rng(8)
+    x = np.clip(rng.normal(scale=1.0, size=(2, N, M)), -3.99, 3.99)
+    nxt = rng.permutation(N).astype(np.int32)
+    e = Engine(ChainParams(dim=2, N=N, M=M, L=4.0, T=0.5, lam=0.5, harmonic_omega=0.7, lattice_V0=1.5, lattice_a=1.0,
+                           interactions=True, pair_g=1.3, pair_sigma=0.5, r_a=1.2, semantics=1))
+    e.set_beads(x)
+    e.set_next(nxt)
+    g, th, _ = e.adjoint()
+    e.close()
+    want, th_want = _adjoint_reference(x, nxt, 0.5, 4.0, 0.7, 1.5, 1.3, 0.5, 1.2, True)
+    np.testing.assert_allclose(g, want, rtol=0, atol=1e-12 * np.abs(want).max())
+    np.testing.assert_allclose(th, th_want, rtol=1e-12, atol=1e-13)
