@@ -14,9 +14,10 @@ launch path on the same chains, the CPU oracle on the machine's host cores, the
 end-to-end rate through host buffers, the roofline of the sweep kernel and
 the SM clocks seen during the timed region.
 
---impl reference times the CPU restatement of the reference's own sweep
-(reference semantics, run!-style random move selection, one chain per host
-thread) on a bounded sample of the same workload.
+--impl reference reports that the reference (a Julia package) cannot run here;
+the CPU restatement of its sweep (reference semantics, run!-style random move
+selection, one chain per host thread, a bounded sample of the same workload) is
+the cpu_baseline of the line.
 """
 from __future__ import annotations
 
@@ -295,38 +296,14 @@ def cpu_contact_table_rate(g0, chain, range_, budget_s=4.0):
 
 # --------------------------------------------------------------------- arms
 def run_reference(args):
-    ws, rank, local, pg = dist_setup()
-    if rank != 0:
-        return 0
-    if args.workload == "contact":
+    """the reference itself cannot run: it is a Julia package, and there is no Julia
+    runtime to install it into.  Its C restatement on the host cores is the
+    cpu_baseline of the engine's line, not a run of the reference"""
+    _, rank, _, _ = dist_setup()
+    if rank == 0:
         print(json.dumps({"impl": "reference", "unavailable": (
-            "the contact workload's 600x600 table is built on the device (a CPU build by "
-            "adaptive quadrature takes hours); its CPU sweep rate is the cpu_baseline of "
-            "the engine's line")}))
-        return 0
-    chains, mixes, desc = workload(args.workload, 0)
-    rates = []
-    cores = os.cpu_count() or 1
-    sample = ""
-    # each step a bounded sample; the whole run stays within a few minutes
-    budget = max(1.0, min(args.ref_budget, 120.0 / max(args.steps, 1)))
-    for _ in range(args.warmup):
-        cpu_oracle_rate(chains, mixes, 0, budget_s=0.5)
-    for _ in range(args.steps):
-        r, cores, sample = cpu_oracle_rate(chains, mixes, 0, budget_s=budget)
-        rates.append(r)
-    v = float(np.median(rates))
-    line = {
-        "impl": "reference", "metric": METRIC, "value": v, "unit": UNIT, "n_gpus": ws,
-        "steps": args.steps, "warmup": args.warmup, "ms_per_step": None, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
-        "config": {"workload": desc, "semantics": "reference (bug-compatible)"},
-        "cpu_baseline": {"value": v, "unit": UNIT, "cores": cores, "kind": "port",
-                         "sample": "C restatement of PIMC.jl's sweep, not Julia (no Julia "
-                                   "toolchain on the box); " + sample},
-        "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-    }
-    print(json.dumps(line))
+            "the reference is a Julia package and no Julia runtime is installed; the C "
+            "restatement's CPU rate is the cpu_baseline of the engine's own line")}))
     return 0
 
 
@@ -674,7 +651,7 @@ def main():
                          "the host buffer is not page-locked (0: 4)")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--cpu-budget", type=float, default=6.0)
-    ap.add_argument("--ref-budget", type=float, default=8.0)
+    ap.add_argument("--ref-budget", type=float, default=8.0, help="no effect: the reference cannot run here")
     ap.add_argument("--traffic-per-bead", type=float, default=None,
                     help="DRAM bytes per bead update of the sweep kernel (ncu)")
     ap.add_argument("--fp64-peak", type=float, default=None, help="TFLOP/s (default: measured)")

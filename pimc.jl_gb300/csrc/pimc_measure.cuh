@@ -140,7 +140,7 @@ static __device__ __noinline__ bool measure_near(CV c, int i, int b, int j) {
 // shorten with i: dealt to the warps in turn), the links of particles i < b that
 // start at slice j.  Lanes test 32 partners on the mirror; survivors go onto a
 // ring and are evaluated 32 at a time.  768 replicas of 8 to 48
-// particles measured in every sweep: 3.92 -> 3.83 ms (four sweeps) by the
+// particles measured in every sweep: 3.92 -> 3.81 ms (four sweeps) by the
 // separations in two floats.
 constexpr int MEAS_RING = 64;  // at most 31 + 32 in use
 __device__ __forceinline__ void measure_pairs(const CV &c, int k0, int k1, int dk, unsigned long long *ring,
