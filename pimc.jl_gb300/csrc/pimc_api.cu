@@ -812,10 +812,12 @@ bool lone_swap_wide(const ChainDesc &d) {
 }
 
 // plain path: each chain's sweep as its own launches, no queue, no graph.  A
-// chain of at most block / 4 pair-free windows sweeps in one launch of one CTA
-// (10 particles, 20 slices, 30 windows: 143 us a sweep, 147 in four launches);
-// others get a CTA per staging slot, then one CTA each for the swaps and the
-// rest (64 particles, 32 slices, 128 windows: 0.40 ms a sweep against 0.45).
+// chain of at most 3 block / 4 pair-free windows sweeps in one launch of one CTA,
+// others get a CTA per staging slot, then one CTA each for the swaps and the rest.
+// One launch / apart, 20 sweeps of ideal particles with three windows each: 12
+// particles 1.88 / 2.13 ms, 32 3.29 / 3.45, 64 5.62 / 5.65, 85 7.18 / 7.14, 128 10.5 /
+// 10.1; with pairs, measured, 64 7.91 / 7.83, 128 16.5 / 15.8; 64 free particles of
+// 32 slices under the physical rules 6.36 / 6.69.
 int run_plain(Handle *h, long long n) {
   const Plan &p = h->one;
   std::vector<StagePlan> sp(h->nchains);
@@ -824,15 +826,17 @@ int run_plain(Handle *h, long long n) {
   bool any_fused = false;
   size_t stage_smem = 0;
   for (int c = 0; c < h->nchains; ++c) {
-    // a serial chain's slot walks on all the warps a CTA can have
-    sblock[c] = desc_slots(h->desc[c]) && h->desc[c].N >= 256 ? 512 : p.block;
+    // a serial chain's slot walks on all the warps a CTA can have: 512 threads / 256,
+    // four sweeps' staging, 16 particles 0.19 / 0.20 ms, 64 0.42 / 0.46, 256 1.73 /
+    // 2.12, 1024 18.5 / 25.2
+    sblock[c] = desc_slots(h->desc[c]) ? 512 : p.block;
     sp[c] = stage_plan(h, 2, sblock[c], c, c + 1);
     stage_smem = std::max(stage_smem, sp[c].smem);
     spec[c] = desc_listed(h->desc[c]) ? 2 : !(h->desc[c].flags & (PF_PHYS | PF_HARD | PF_CONTACT));
     const MixDev &m = h->mix[c];
     const int ell = std::max(2, std::min({h->umix[c].stage_slices, m.stage_max, h->desc[c].M - 1, 64}));
     fused[c] = !desc_serial(h->desc[c]) && ell <= 32 &&
-               h->desc[c].N * ((h->desc[c].M + ell - 1) / ell) <= p.block / 4;
+               h->desc[c].N * ((h->desc[c].M + ell - 1) / ell) <= 3 * p.block / 4;
     any_fused = any_fused || fused[c];
   }
   if (any_fused) CK(sweep_set_smem(0, p.dyn_smem));
