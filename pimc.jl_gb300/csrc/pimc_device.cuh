@@ -1509,7 +1509,9 @@ __device__ __forceinline__ int hard_bridge(const CV &c, int n, int nx, int j0, i
 // hard-core retry loop.  sb: per-warp shared scratch of 5*(WMAX+1) doubles
 // followed by a PQ_CAP-entry neighbour queue.
 // ---------------------------------------------------------------------------
-template <class D>
+// LISTS: long chains take the first bracket from the cell lists (a warp per chain:
+// one chain of 2048 sparse particles 689 -> 322 ms a sweep)
+template <bool LISTS = false, class D>
 __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrite_start,
                            double *sb, double *prop) {
   const ChainDesc &d = *c.d;
@@ -1592,8 +1594,12 @@ __device__ int window_warp(const CV &c, int n, int j0, int m, D &dr, bool rewrit
       }
       __syncwarp();
       PairEst e = {0.f, 0.f, 0.f, 0.f, 0, 0};
-      scan_mirror<2>(c, j0, m, cq, skip, 0, 1, e, lane, NoStop());
-      scan_bounds(d, e);
+      if (LISTS && c.cl && c.N >= kSwapLists) {
+        segment_estimate(c, seg, 0, m, e, lane);
+      } else {
+        scan_mirror<2>(c, j0, m, cq, skip, 0, 1, e, lane, NoStop());
+        scan_bounds(d, e);
+      }
       __syncwarp();
       float t, r;
       est_lane(e, -1.f, t, r);

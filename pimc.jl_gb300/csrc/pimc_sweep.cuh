@@ -307,7 +307,7 @@ __device__ void sweep_one(SmemCtl &sc, double *red, const CV &c, unsigned char *
         for (int n = 0; n < N; ++n) {
           GenDraws dr = gen_draws(make_stream(d, sweep, PH_STAGE, (unsigned)(ph * items + s * N + n)));
           const int m = min(len, 2 + (int)(dr.s.uni(DRAW_CHOICE) * (ell - 1)));
-          const int r = window_warp(cw, n, st, m, dr, false, wsb, nullptr);
+          const int r = window_warp<WARP>(cw, n, st, m, dr, false, wsb, nullptr);
           if (lane == 0) {
             tal[0] += 1.0;
             tal[1] += r == RES_ACCEPT;

@@ -19,7 +19,8 @@ enum : int {
 constexpr int MAX_BEAMS = 16;  // laser beams of an optical-lattice potential
 constexpr int kMaxParticles = 8192;  // particles per chain (pimc_params.N)
 // cell lists where a chain's moves would otherwise scan its rows: staging slots
-// walked window by window (stage_long), swaps (swap_listed)
+// walked window by window (stage_long), swaps (swap_listed) and, with a warp per
+// chain, windows (window_warp)
 constexpr int kLongPairs = 512, kLongTeam = 1024, kLongHard = 2048, kSwapLists = 1280;
 // and windows that stage_slot would take, whose scans of every particle grow with N:
 // in (chain, slot) CTAs of fewer than 512 threads, and in the fused kernel, whose CTA

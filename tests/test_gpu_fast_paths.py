@@ -244,7 +244,7 @@ def test_beam_phases_around_the_table(scale, K, helical, engine_lib):
 @pytest.mark.parametrize("sem", [0, 1])
 @pytest.mark.parametrize("N,L", [(257, 9.0), (513, 9.0), (1100, 16.0), (1300, 20.0)])
 def test_long_chains_decide_as_exact_sums(N, L, sem, engine_lib):
-    """lone chains and split sweeps with swaps in CTAs of 64 threads at lengths
+    """lone chains, split sweeps with swaps in CTAs of 64 threads and warps at lengths
     where the kernels change over (staging in CTAs of 512 threads, the partner
     ratio's particles past the kept ones, swaps bracketed from the cell lists):
     bracketed decisions, with lists and with row scans, give the beads,
@@ -253,13 +253,13 @@ def test_long_chains_decide_as_exact_sums(N, L, sem, engine_lib):
     p = ChainParams(dim=2, N=N, M=9, L=L, T=1.0, lam=0.5, harmonic_omega=0.3, interactions=True, pair_g=1.0,
                     pair_sigma=0.4, r_a=1.0, semantics=sem, seed=61)
     out = []
-    for exact, mode, split in ((1, 0, 0), (0, 0, 0), (0, 2, 0), (0, 0, 1), (0, 2, 1)):
+    for exact, mode, split in ((1, 0, 0), (0, 0, 0), (0, 2, 0), (0, 0, 1), (0, 2, 1), (0, 0, 2), (0, 2, 2)):
         e = Engine(p, Mix(stage_slices=4, stage_max=4, stage_minacc=0.0, stage_maxacc=1.0, swaps_per_sweep=200,
                           swap_slices=5, swap_max=5, swap_minacc=0.0, swap_maxacc=1.0, com_maxstep=2.0))
         e.set_option(OPT_EXACT_DECISIONS, exact)
         e.set_cells(mode)
-        if split:
-            e.set_launch(64, split_phases=1)
+        if split:  # 2: a warp per chain
+            e.set_launch(64, split_phases=split % 2, warp_per_chain=split == 2)
             e.run_batched(3)
         else:
             e.run_plain(3)
